@@ -18,13 +18,29 @@
 // 3 FP64 instructions per pair for one-term kernels, 4 for Brownian + shear
 // (the tile task needs 5 where lo > k). Sum keeps its per-pair rate.
 //
+// From lag D0 on e = 0: every pair lands on its larger member's own slot. There
+// the sums over j separate. beta is a sum of products of powers of x_j and x_k,
+// and fl(x_j + x_k) - x_k is x_j up to the sum's rounding, so
+//   R_s  = N_s sum_j beta(x_j, x_s) N_j      = N_s death_factor(x_s; P),
+//   TH_s = N_s sum_j beta(x_j, x_s) x_j N_j  = N_s death_factor(x_s; T)
+// with the prefix moments P_q, T_q of N and x N over the bins j <= s - D0 (the
+// prep's scan): O(n) work instead of half of all pairs at n = 16384 and q = 512
+// bins per octave, and nearly all of them on coarse grids. The prefix sums add
+// terms of one kind without cancellation. Dropping the rounding of
+// fl(x_j + x_k) moves w by at most u = 2^-53 x_{s+1}/dx_s, so bin s + 1 by
+// u R_s; that bin's own death term is at least N_{s+1}/N_s times R_s, and where
+// u N_s > kMomGuard N_{s+1} (a population that ends or falls steeply within one
+// bin, where a tiny w's rounding would show) the slot keeps its exact pair sum,
+// a task of its own (exact_slot_task).
+//
 // Work split: blocks of 32 output bins aligned to the top of the grid (block
 // t owns bins [n - 32 (t + 1), n - 32 t), as the tiles do, so bin n - 1 is never
-// a block's first bin); a task is one block and one chunk of C lags; the CTA's
-// eight warps take equal contiguous shares of the chunk's lags (each warp sees
-// its runs in order) and their sums are added in warp order. A block with
-// several chunk tasks stores each chunk's 2 x 32 sums; the block's last task
-// (ticket) adds them in chunk order and writes the bins -- deterministic,
+// a block's first bin); a task is one block and one of `parts` equal shares of
+// the lags below D0; the CTA's
+// eight warps take equal contiguous shares of the task's lags (each warp sees
+// its runs in order) and their sums are added in warp order. With several
+// parts each task stores its 2 x 32 sums; the block's last task
+// (ticket) adds them in order and writes the bins -- deterministic,
 // nobody waits.
 //
 // Operand staging (template STAGE): the j-side operands of a task (N_j,
@@ -37,6 +53,7 @@
 #include <cstdint>
 
 #include "agg_tile.cuh"
+#include "agg_moments.cuh"
 
 namespace pbe_gb300 {
 
@@ -45,12 +62,16 @@ constexpr int kLaneWinMax = 1792;                   // staged window, entries pe
 // Bounded waits on the staging barrier: iterations of mbarrier.try_wait.
 constexpr long long kLaneWaitLimit = 1LL << 26;
 
-// Index of task (block t, chunk c): the tasks of chunk c' < c come first.
-__device__ __forceinline__ int lane_task_index(int n, int t, int c, int C)
+// Shares of a block's direct lags: enough tasks to give every CTA several (the
+// last ones then end together), at least 32 lags each (4 per warp). A share
+// longer than the staged window reads its operands from the arrays.
+__host__ __device__ constexpr int lane_parts(int lags, int nblk, int ctas)
 {
-    int base = 0;
-    for (int q = 0; q < c; ++q) base += lane_chunk_blocks(n, q, C);
-    return base + t;
+    int p = (4 * ctas + nblk - 1) / nblk;
+    const int most = (lags + 31) / 32;
+    if (p > most) p = most;
+    if (p > kLaneMaxParts) p = kLaneMaxParts;
+    return p < 1 ? 1 : p;
 }
 
 // ---- bulk TMA copy + mbarrier helpers (shared::cta addresses) -----------------
@@ -107,15 +128,205 @@ struct LaneArgs {
     const double* Ncp;   // N copy
     const double* xcp;   // x copy
     double* part;        // [lane_partial_doubles(n)]
-    int* ticket;         // [lane_blocks(n)] chunk tasks of the block done (reset by the prep)
+    int* ticket;         // [lane_blocks(n)] tasks of the block done (reset by the prep)
     int* err;            // set to 1 when a staging wait gave up
-    int C;               // lag chunk length
+    int parts;           // tasks per block
 };
 
-// One lane task: block t, lag chunk c. All kMainThreads threads of the CTA
-// take part; returns with the CTA synchronised. `phase` is the staging
+// Prefix moments up to bin i of the prep's scan: P_q = sum m_q, T_q = sum m_q x at
+// the binary exponent of x_i.
+template <int K>
+__device__ __forceinline__ void prefix_moments(const AggWs& ws, const double* __restrict__ x, int n,
+                                               int i, double* P, double* T)
+{
+    const int nb = agg_prep_blocks(n), b = i / kPrepThreads;
+    const int dE = b > 0 ? exponent_of(__ldg(x + b * kPrepThreads - 1)) - exponent_of(__ldg(x + i)) : 0;
+#pragma unroll
+    for (int q = 0; q < kMomN; ++q) {
+        P[q] = __ldg(ws.mloc + static_cast<size_t>(q) * n + i) + __ldg(ws.moff + q * nb + b);
+        T[q] = __ldg(ws.mloc + static_cast<size_t>(kMomN + q) * n + i)
+             + scale_down(__ldg(ws.moff + (kMomN + q) * nb + b), dE);
+    }
+}
+
+// Slots of block t (one per lane) whose lags from D0 on are summed pair by pair.
+__device__ __forceinline__ unsigned exact_mask(const AggCellView& v, int t, int Dm)
+{
+    const int s = v.n - kLaneBins * (t + 1) + (threadIdx.x & 31);
+    const bool e = s >= Dm && s <= lane_block_smax(v.n, t) &&
+                   mom_exact_slot(__ldg(v.Nk + s), __ldg(v.Nk + s + 1), __ldg(v.x + s + 1),
+                                  __ldg(v.inv_dx + s));
+    return __ballot_sync(0xffffffffu, e);
+}
+
+// One warp, after its contribution to block t is stored: the block's ticket.
+// True for the last of its `parts` share tasks and one task per exact slot;
+// that one gets the block's sums, added in a fixed order.
+__device__ __forceinline__ bool block_ticket(const AggWs& ws, const LaneArgs& la, int n, int t,
+                                             unsigned exact, double& Rt, double& THt)
+{
+    const int lane = threadIdx.x & 31;
+    const int want = la.parts + __popc(exact);
+    __threadfence();                                   // every lane's stores before the ticket
+    __syncwarp();
+    int last = 0;
+    if (lane == 0) last = (atomicAdd(la.ticket + t, 1) == want - 1);
+    if (!__shfl_sync(0xffffffffu, last, 0)) return false;
+    __threadfence();
+    Rt = 0.0;
+    THt = 0.0;
+    const double* bp = la.part + static_cast<size_t>(t) * la.parts * 64;
+    for (int q = 0; q < la.parts; ++q) {
+        Rt += __ldcg(bp + q * 64 + lane);
+        THt += __ldcg(bp + q * 64 + 32 + lane);
+    }
+    if ((exact >> lane) & 1u) {
+        const int s = n - kLaneBins * (t + 1) + lane;
+        Rt += __ldcg(ws.xsum + 2 * s);
+        THt += __ldcg(ws.xsum + 2 * s + 1);
+    }
+    return true;
+}
+
+// One warp: the bins of block t from its slots' sums (a slot per lane). With
+// `first` the lags from D0 on (prefix moments; not the exact slots) and the
+// death term are added; scatter mode calls it for every share's own sums.
+template <int K, bool SCATTER>
+__device__ void lane_finish(const AggCellView& v, const AggWs& ws, double* rhs, int t, int Dm,
+                            int nclip, unsigned exact, bool first, bool poisoned, double Rt,
+                            double THt)
+{
+    const int n = v.n, lane = threadIdx.x & 31;
+    const int I = n - kLaneBins * (t + 1);
+    const int smax = lane_block_smax(n, t);
+    const int s = I + lane, i = s;
+    const bool slot = s >= 0 && s <= smax;
+    const double xs = slot ? __ldg(v.x + s) : 0.0;
+    const int St = slot ? -ilogb(xs) : 0;
+    double clip0 = 0.0;                                // the lags from D0 on of the clipped slot n - 1
+    if (first && s >= Dm && s <= n - 1 && !((exact >> lane) & 1u)) {
+        double P[kMomN], T[kMomN];
+        prefix_moments<K>(ws, v.x, n, s - Dm, P, T);
+        const double as = __ldg(v.a + s), ias = __ldg(v.ia + s), xv = __ldg(v.x + s);
+        const double Ns = __ldg(v.Nk + s);
+        const double r = Ns * death_factor<K>(xv, as, ias, P, v.b0, v.bbr, v.bsh);
+        const double th = Ns * death_factor<K>(xv, as, ias, T, v.b0, v.bbr, v.bsh);
+        if (slot) {
+            Rt += r;
+            THt += scale_down(th, exponent_of(__ldg(v.x + (s - Dm))) - exponent_of(xv));
+        } else {
+            clip0 = r;
+        }
+    }
+    // own part of bin i (slot i) and the w-part of slot i, owed to bin i + 1
+    double b1 = 0.0, co = 0.0;
+    if (slot) {
+        const double sd = scalbn(__ldg(v.inv_dx + i), -St);
+        b1 = fma(-THt, sd, Rt);
+        co = THt * sd;
+    }
+    const double cin = __shfl_up_sync(0xffffffffu, co, 1);
+    if (i >= 0) {
+        double val = b1;
+        if (lane >= 1) val += cin;
+        val += clip0;
+        if (first) val -= agg_death<K>(v, i);
+        if constexpr (SCATTER) {
+            if (val != 0.0) atomicAdd(rhs + i, val);
+        } else {
+            if (poisoned) val = __longlong_as_double(0x7ff8000000000000LL);
+            if (lane == 0 && I >= 1) {
+                ws.tfirst[t] = val;
+                __threadfence();
+                if (atomicAdd(ws.tticket + t, 1) == 1) {
+                    __threadfence();
+                    rhs[I] = __ldcg(rhs + I) + (__ldcg(ws.tfirst + t) + __ldcg(ws.tcarry + t));
+                }
+            } else {
+                rhs[i] = rhs[i] + val;
+                if (i == n - 1) {
+                    __threadfence();
+                    if (atomicAdd(ws.counter + 3, 1) == nclip) {
+                        __threadfence();
+                        double sc = 0.0;
+                        for (int q = 0; q < nclip; ++q) sc += __ldcg(ws.clip_part + q);
+                        rhs[n - 1] = __ldcg(rhs + (n - 1)) + sc;
+                    }
+                }
+            }
+        }
+    }
+    if constexpr (SCATTER) {
+        if (lane == 31 && slot && co != 0.0) atomicAdd(rhs + i + 1, co);
+    } else if (lane == 31 && t >= 1) {
+        // carry into bin I + 32, the first bin of block t - 1
+        ws.tcarry[t - 1] = co;
+        __threadfence();
+        if (atomicAdd(ws.tticket + (t - 1), 1) == 1) {
+            __threadfence();
+            const int J = I + kLaneBins;
+            rhs[J] = __ldcg(rhs + J) + (__ldcg(ws.tfirst + t - 1) + __ldcg(ws.tcarry + t - 1));
+        }
+    }
+}
+
+// The lags from D0 on of one exact slot, pair by pair: the CTA over j, summed in
+// a fixed order. Such slots cluster at the foot of a population, so each is a
+// task of its own (summed by its block's last task, 90 of them on a run of 3840
+// bins made the whole call 1.5 x slower). `red`: 2 kLaneWarps doubles.
+template <int K, bool SCATTER>
+__device__ void exact_slot_task(const AggCellView& v, const AggWs& ws, const LaneArgs& la,
+                                double* rhs, int s, int nclip, double* red, bool poisoned)
+{
+    const int n = v.n, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int Dm = min(v.D0, n);
+    const int t = (n - 1 - s) / kLaneBins;
+    if (s < Dm || s > lane_block_smax(n, t)) return;   // no such lags (the whole CTA)
+    const double xe = __ldg(v.x + s);
+    const int St = -ilogb(xe);
+    const EwOperandC pc = ew_operand_c(xe, St);
+    const EwOperandA pa = ew_operand_a(xe);
+    const double Ns = __ldg(v.Nk + s), hs = NeedH<K>::k ? __ldg(v.Hk + s) : 0.0;
+    double r = 0.0, th = 0.0;
+    for (int j = tid; j <= s - Dm; j += kMainThreads) {
+        const int d = s - j;
+        const double rate = rate_geo<K>(__ldg(v.Bd + d), __ldg(v.Sd + d), __ldg(v.Nj + j),
+                                        NeedH<K>::j ? __ldg(v.Hj + j) : 0.0, Ns, hs);
+        r += rate;
+        th = fma(rate, sum_minus_scaled_pre(pa, __ldg(v.x + j), pc), th);
+    }
+    r = warp_sum(r);
+    th = warp_sum(th);
+    if (lane == 0) { red[2 * w] = r; red[2 * w + 1] = th; }
+    __syncthreads();
+    if (w == 0) {
+        r = 0.0;
+        th = 0.0;
+        for (int q = 0; q < kLaneWarps; ++q) { r += red[2 * q]; th += red[2 * q + 1]; }
+        if constexpr (SCATTER) {
+            if (lane == 0) {
+                const double co = th * scalbn(__ldg(v.inv_dx + s), -St);
+                atomicAdd(rhs + s, r - co);
+                if (co != 0.0) atomicAdd(rhs + s + 1, co);
+            }
+        } else {
+            if (lane == 0) {
+                ws.xsum[2 * s] = r;
+                ws.xsum[2 * s + 1] = th;
+            }
+            const unsigned em = exact_mask(v, t, Dm);
+            double Rt, THt;
+            if (block_ticket(ws, la, n, t, em, Rt, THt))
+                lane_finish<K, false>(v, ws, rhs, t, Dm, nclip, em, true, poisoned, Rt, THt);
+        }
+    }
+    __syncthreads();
+}
+
+// One lane task: block t, share c of its direct lags. All kMainThreads threads
+// of the CTA take part; returns with the CTA synchronised. `phase` is the staging
 // barrier's parity (flipped per staged task). Gather mode stores / finishes
-// the block's bins; scatter mode flushes this chunk's share with atomics.
+// the block's bins; scatter mode flushes this task's share with atomics.
 template <int K, bool SCATTER, bool STAGE>
 __device__ void lane_task(const AggCellView& v, const AggWs& ws, const LaneArgs& la, double* rhs,
                           int t, int c, int nclip, const LaneSmem& sm, uint64_t* bar,
@@ -123,17 +334,17 @@ __device__ void lane_task(const AggCellView& v, const AggWs& ws, const LaneArgs&
 {
     const int n = v.n;
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    const int C = la.C;
     const int I = n - kLaneBins * (t + 1);
     const int smax = lane_block_smax(n, t);
     const int smin = I > 0 ? I : 0;
-    const int nch = lane_block_chunks(n, t, C);
+    const int Dm = min(v.D0, n);                       // lags summed pair by pair
+    const int C = (Dm + la.parts - 1) / la.parts;
 
     // lags of this task: [dA, dB), dB cut where Ld passes the block's top slot
     // (Ld is nondecreasing; clipped lags hold kLagClipAll)
-    const int dA = c * C;
-    int dB = min(dA + C, smax + 1);
-    // most chunks end below the cut: one load settles it, else bisect
+    const int dA = min(c * C, Dm);
+    int dB = min(min(dA + C, Dm), smax + 1);
+    // most shares end below the cut: one load settles it, else bisect
     if (dB > dA && __ldg(v.Ld + dB - 1) > smax) {
         int lo = dA, hi = dB;
         while (lo < hi) {
@@ -246,86 +457,16 @@ __device__ void lane_task(const AggCellView& v, const AggWs& ws, const LaneArgs&
             Rt += sm.red[(q * 2 + 0) * 32 + lane];
             THt += sm.red[(q * 2 + 1) * 32 + lane];
         }
+        const unsigned em = exact_mask(v, t, Dm);
         bool finish = true;
-        if (!SCATTER && nch > 1) {
-            double* cp = la.part + static_cast<size_t>(lane_task_index(n, t, c, C)) * 64;
-            cp[lane] = Rt;
-            cp[32 + lane] = THt;
-            __threadfence();                           // every lane's sums before the ticket
-            __syncwarp();
-            int last = 0;
-            if (lane == 0) last = (atomicAdd(la.ticket + t, 1) == nch - 1);
-            last = __shfl_sync(0xffffffffu, last, 0);
-            finish = last != 0;
-            if (finish) {
-                __threadfence();
-                Rt = 0.0;
-                THt = 0.0;
-                int idx = t;                           // task index of (t, q), q = 0, 1, ...
-                for (int q = 0; q < nch; ++q) {
-                    const double* pq = la.part + static_cast<size_t>(idx) * 64;
-                    Rt += __ldcg(pq + lane);
-                    THt += __ldcg(pq + 32 + lane);
-                    idx += lane_chunk_blocks(n, q, C);
-                }
-            }
+        if (!SCATTER && (la.parts > 1 || em != 0u)) {
+            double* bp = la.part + (static_cast<size_t>(t) * la.parts + c) * 64;
+            bp[lane] = Rt;
+            bp[32 + lane] = THt;
+            finish = block_ticket(ws, la, n, t, em, Rt, THt);
         }
-        if (finish) {
-            const int i = s;
-            // own part of bin i (slot i) and the w-part of slot i, owed to bin i + 1
-            double b1 = 0.0, co = 0.0;
-            if (slot) {
-                const double sd = scalbn(__ldg(v.inv_dx + i), -St);
-                b1 = fma(-THt, sd, Rt);
-                co = THt * sd;
-            }
-            const double cin = __shfl_up_sync(0xffffffffu, co, 1);
-            if constexpr (SCATTER) {
-                if (i >= 0) {
-                    double val = b1;
-                    if (lane >= 1) val += cin;
-                    if (c == 0) val -= agg_death<K>(v, i);
-                    if (val != 0.0) atomicAdd(rhs + i, val);
-                }
-                if (lane == 31 && slot && co != 0.0) atomicAdd(rhs + i + 1, co);
-            } else {
-                if (i >= 0) {
-                    double val = b1;
-                    if (lane >= 1) val += cin;
-                    val -= agg_death<K>(v, i);
-                    if (poisoned) val = __longlong_as_double(0x7ff8000000000000LL);
-                    if (lane == 0 && I >= 1) {
-                        ws.tfirst[t] = val;
-                        __threadfence();
-                        if (atomicAdd(ws.tticket + t, 1) == 1) {
-                            __threadfence();
-                            rhs[I] = __ldcg(rhs + I) + (__ldcg(ws.tfirst + t) + __ldcg(ws.tcarry + t));
-                        }
-                    } else {
-                        rhs[i] = rhs[i] + val;
-                        if (i == n - 1) {
-                            __threadfence();
-                            if (atomicAdd(ws.counter + 3, 1) == nclip) {
-                                __threadfence();
-                                double sc = 0.0;
-                                for (int q = 0; q < nclip; ++q) sc += __ldcg(ws.clip_part + q);
-                                rhs[n - 1] = __ldcg(rhs + (n - 1)) + sc;
-                            }
-                        }
-                    }
-                }
-                if (lane == 31 && t >= 1) {
-                    // carry into bin I + 32, the first bin of block t - 1
-                    ws.tcarry[t - 1] = co;
-                    __threadfence();
-                    if (atomicAdd(ws.tticket + (t - 1), 1) == 1) {
-                        __threadfence();
-                        const int J = I + kLaneBins;
-                        rhs[J] = __ldcg(rhs + J) + (__ldcg(ws.tfirst + t - 1) + __ldcg(ws.tcarry + t - 1));
-                    }
-                }
-            }
-        }
+        if (finish)
+            lane_finish<K, SCATTER>(v, ws, rhs, t, Dm, nclip, em, !SCATTER || c == 0, poisoned, Rt, THt);
     }
     __syncthreads();
 }

@@ -50,6 +50,118 @@ namespace {
 
 constexpr int W = kTileW;
 
+// Prefix sums of one prep block (see AggWs::mloc), two warps in lane order, and
+// the block totals. The weighted sums run at the exponent of each bin's pivot,
+// so they keep the range of x_j / x_i on grids of any span; a shift between
+// exponents takes integer instructions only. Fixed order: reproducible.
+template <int K>
+__device__ __forceinline__ void prep_prefix(const double* m, double xm, int E, int i, int n,
+                                            const AggWs& ws, double* gsum)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    static_assert(kPrepThreads == 64, "two warps");
+    double P[kMomN], T[kMomN];
+#pragma unroll
+    for (int q = 0; q < kMomN; ++q) { P[q] = m[q]; T[q] = m[q] * xm; }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int dE = __shfl_up_sync(0xffffffffu, E, o) - E;
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) {
+            if (!need_moment<K>(q)) continue;
+            const double p = __shfl_up_sync(0xffffffffu, P[q], o);
+            const double t = __shfl_up_sync(0xffffffffu, T[q], o);
+            if (lane >= o) { P[q] += p; T[q] += scale_down(t, dE); }
+        }
+    }
+    // the first warp's sums enter the second's at its bins' exponents
+    __shared__ int e_s;
+    if (w == 0 && lane == 31) {
+        e_s = E;
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) { gsum[q] = P[q]; gsum[kMomN + q] = T[q]; }
+    }
+    __syncthreads();
+    const int nb = gridDim.x, b = blockIdx.x;
+    const int last = min(n - 1, b * kPrepThreads + kPrepThreads - 1);
+#pragma unroll
+    for (int q = 0; q < kMomN; ++q) {
+        if (!need_moment<K>(q)) continue;
+        if (w == 1 && i < n) {
+            P[q] += gsum[q];
+            T[q] += scale_down(gsum[kMomN + q], e_s - E);
+        }
+        if (i < n) {
+            ws.mloc[static_cast<size_t>(q) * n + i] = P[q];
+            ws.mloc[static_cast<size_t>(kMomN + q) * n + i] = T[q];
+        }
+        if (i == last) {
+            ws.mtot[q * nb + b] = P[q];
+            ws.mtot[(kMomN + q) * nb + b] = T[q];
+        }
+    }
+}
+
+// Scan of the block totals by the prep's last block: each lane sums a run of
+// consecutive blocks, a warp scan adds the runs, each lane writes its blocks'
+// offsets. Warp 0: the moments (their last sums are the death term's moments),
+// warp 1: the weighted ones.
+template <int K>
+__device__ __forceinline__ void prep_offsets(const double* __restrict__ x, int n, int nb,
+                                             const AggWs& ws, int w, int lane)
+{
+    const int per = (nb + 31) / 32;
+    const int b0 = min(nb, lane * per), b1 = min(nb, b0 + per);
+    auto last_exp = [&](int b) { return exponent_of(__ldg(x + min(n - 1, (b + 1) * kPrepThreads - 1))); };
+    // exponent the running sum stands at: that of the last bin before / in the run
+    const int Eb = b0 > 0 ? last_exp(b0 - 1) : 0;
+    int Ee = b1 > 0 ? last_exp(b1 - 1) : 0;
+    const double* tot = ws.mtot + static_cast<size_t>(w) * kMomN * nb;
+    double* off = ws.moff + static_cast<size_t>(w) * kMomN * nb;
+    double S[kMomN];
+#pragma unroll
+    for (int q = 0; q < kMomN; ++q) S[q] = 0.0;
+    int e = Eb;
+    for (int b = b0; b < b1; ++b) {
+        const int en = w ? last_exp(b) : 0;
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q)
+            if (need_moment<K>(q)) S[q] = (w ? scale_down(S[q], e - en) : S[q]) + __ldcg(tot + q * nb + b);
+        e = en;
+    }
+    double R[kMomN];
+#pragma unroll
+    for (int q = 0; q < kMomN; ++q) R[q] = S[q];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int dE = w ? __shfl_up_sync(0xffffffffu, Ee, o) - Ee : 0;
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) {
+            if (!need_moment<K>(q)) continue;
+            const double r = __shfl_up_sync(0xffffffffu, R[q], o);
+            if (lane >= o) R[q] += w ? scale_down(r, dE) : r;
+        }
+    }
+    e = Eb;
+#pragma unroll
+    for (int q = 0; q < kMomN; ++q) {
+        if (!need_moment<K>(q)) continue;
+        if (w == 0 && lane == 31) ws.mom[q] = R[q];
+        const double r = __shfl_up_sync(0xffffffffu, R[q], 1);
+        S[q] = lane > 0 ? r : 0.0;
+    }
+    for (int b = b0; b < b1; ++b) {
+        const int en = w ? last_exp(b) : 0;
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) {
+            if (!need_moment<K>(q)) continue;
+            off[q * nb + b] = S[q];
+            S[q] = (w ? scale_down(S[q], e - en) : S[q]) + __ldcg(tot + q * nb + b);
+        }
+        e = en;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // prep: one thread per bin i. Per-bin values, the lag tables for d = i,
 // moment partials and the geometric-grid deviation.
@@ -66,8 +178,9 @@ constexpr int W = kTileW;
 // call on the same pivots and coefficients wrote it; only the N-dependent
 // values (h, the N copy, moments) and the tickets are rewritten, with the
 // same arithmetic as a FULL call, so the results are bitwise the same.
-// Either way the last block resets counter[2] (the prep's block tickets), so
-// a following call on the same workspace needs no memset.
+// Either way the last block resets counter[2] (the prep's block tickets) and
+// the tile kernel, launched last, counter[5] (the exact slots' list), so a
+// following call on the same workspace needs no memset.
 // ---------------------------------------------------------------------------
 template <int K, bool FULL>
 __global__ void __launch_bounds__(kPrepThreads)
@@ -75,11 +188,14 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
                 double b0, double bbr, double bsh)
 {
     __shared__ double sh[kPrepThreads / 32];
+    __shared__ double gsum[2 * kMomN];
     __shared__ int d0_s;
     __shared__ double ax0_s;
     __shared__ GeoFit fit_s;
     const int i = blockIdx.x * kPrepThreads + threadIdx.x;
     double m[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    double xm = 0.0;     // mantissa and binary exponent of x_i
+    int E = 0;
     double dev = 0.0;
     int d0 = n;      // this thread's lag if its pairs land on their larger member (Ld == d)
     if (FULL && threadIdx.x == 0) {
@@ -102,28 +218,10 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
         ws.h[i] = hi;
         ws.Ncp[i] = Ni;          // 256-byte aligned copies: bulk-copy sources of the lane tasks
         m[0] = iai * Ni; m[1] = Ni; m[2] = ai * Ni; m[3] = (ai * ai) * Ni; m[4] = hi;
+        xm = mantissa_of(xi);
+        E = exponent_of(xi);
         if (i < agg_tiles(n)) { ws.tticket[i] = 0; ws.cticket[i] = 0; }
         if constexpr (FULL) {
-            // launch order of the lane tasks: entry i < full is a full chunk
-            // (chunk by chunk), entry full + rank(t) block t's last chunk
-            const int C = lane_chunk_len(n);
-            const int full = lane_full_tasks(n, C);
-            if (i < full) {
-                int r = i, c = 0;
-                for (;;) {
-                    const int cnt = lane_chunk_blocks(n, c + 1, C);
-                    if (r < cnt) break;
-                    r -= cnt;
-                    ++c;
-                }
-                ws.ltask[2 * i] = r;
-                ws.ltask[2 * i + 1] = c;
-            }
-            if (i < lane_blocks(n)) {
-                const int k = full + lane_last_rank(n, i, C);
-                ws.ltask[2 * k] = i;
-                ws.ltask[2 * k + 1] = lane_block_chunks(n, i, C) - 1;
-            }
             ws.xcp[i] = xi;
             ws.a[i] = ai;
             ws.ia[i] = iai;
@@ -142,19 +240,19 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
             const double v = x0 + xi;       // x[i] <= v: its bracket is at or above i
             const int L = (dbits(v) >= dbits(x[n - 1])) ? kLagClipAll : bracket_from(x, n, v, i);
             ws.Ld[i] = L;
-            if (L == i) d0 = i;
+            if (L == i && i > 0) d0 = i;   // lag 0 carries the pair 1/2: never separated
             if (n >= 2) {
                 dev = geo_dev(fit_s, xi, i);
                 if (!(dev == dev)) dev = 1.0;   // NaN -> not geometric
             }
         }
     }
+    // slots that keep the exact pair sum from D0 on (the list's order does not
+    // matter: each has its own task and its own sums)
+    if (i < n - 1 && mom_exact_slot(N[i], N[i + 1], x[i + 1], ws.inv_dx[i]))
+        ws.xlist[atomicAdd(ws.counter + 5, 1)] = i;
     if (FULL) atomicMin(&d0_s, d0);
-#pragma unroll
-    for (int q = 0; q < 5; ++q) {
-        const double s = block_sum(m[q], sh);
-        if (threadIdx.x == 0) ws.mom_part[blockIdx.x * 8 + q] = s;
-    }
+    prep_prefix<K>(m, xm, E, i, n, ws, gsum);
     if (FULL) {
         dev = warp_max(dev);
         __syncthreads();
@@ -162,6 +260,7 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
         __syncthreads();
     }
     __shared__ int last_s;
+    __syncthreads();                           // the block's totals are written
     if (threadIdx.x == 0) {
         if (FULL) {
             double mx = 0.0;
@@ -179,29 +278,23 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
     // counters of the main kernel. No block waits for another.
     __threadfence();
     const int nb = gridDim.x;
-    // seven reductions over the blocks' partials, spread over the warps: r < 5
-    // one moment each, r = 5 the largest deviation, r = 6 the smallest D0
-    // candidate (lanes stride over the blocks, fixed butterflies)
+    // The scan of the block totals (prefix offsets, and the moments as its last
+    // sums), and, over the warps, the largest deviation and the smallest D0 candidate.
     const int wq = threadIdx.x >> 5, lq = threadIdx.x & 31;
-    for (int r = wq; r < (FULL ? 7 : 5); r += kPrepThreads / 32) {
-        if (r < 5) {
-            double t = 0.0;
-            for (int b = lq; b < nb; b += 32) t += __ldcg(ws.mom_part + b * 8 + r);
-            t = warp_sum(t);
-            if (lq == 0) ws.mom[r] = t;
-        } else if (r == 5) {
-            double m5 = 0.0;
-            for (int b = lq; b < nb; b += 32) m5 = fmax(m5, __ldcg(ws.mom_part + b * 8 + 5));
-            m5 = warp_max(m5);
-            if (lq == 0) sh[0] = m5;
-        } else {
-            int dmin = n;
-            for (int b = lq; b < nb; b += 32)
-                dmin = min(dmin, static_cast<int>(__ldcg(ws.mom_part + b * 8 + 6)));
+    prep_offsets<K>(x, n, nb, ws, wq, lq);
+    if (FULL && wq == 0) {
+        double m5 = 0.0;
+        for (int b = lq; b < nb; b += 32) m5 = fmax(m5, __ldcg(ws.mom_part + b * 8 + 5));
+        m5 = warp_max(m5);
+        if (lq == 0) sh[0] = m5;
+    }
+    if (FULL && wq == 1) {
+        int dmin = n;
+        for (int b = lq; b < nb; b += 32)
+            dmin = min(dmin, static_cast<int>(__ldcg(ws.mom_part + b * 8 + 6)));
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) dmin = min(dmin, __shfl_xor_sync(0xffffffffu, dmin, o));
-            if (lq == 0) d0_s = dmin;
-        }
+        for (int o = 16; o > 0; o >>= 1) dmin = min(dmin, __shfl_xor_sync(0xffffffffu, dmin, o));
+        if (lq == 0) d0_s = dmin;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -212,7 +305,7 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
             const bool geo = n >= 2 && mx <= kGeoTol && x[1] <= 64.0 * x[0];
             ws.mom[5] = geo ? 1.0 : 0.0;
             ws.mom[6] = mx;
-            ws.counter[1] = d0_s;   // lags d >= counter[1] have lo(j, j+d) = j + d
+            ws.counter[1] = d0_s;   // lags d >= counter[1] >= 1 have lo(j, j+d) = j + d
         }
         ws.counter[0] = 0;          // task counter of the main kernel
         ws.counter[2] = 0;          // this kernel's block tickets, ready for the next call
@@ -222,22 +315,25 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
 }
 
 // Clipped pairs (x_j + x_k >= x[n-1], all deposited on bin n-1,
-// src/aggregation_kernels.cuh:191-192), part c of nclip: the lags
-// d = c + nclip (lane + T k) on a geometric grid (pairs j in [n-1-Ld, n-1-d];
-// interleaving spreads the long lags near d = 0 over the parts), the rows
-// j = c + nclip (lane + T k) otherwise.
+// src/aggregation_kernels.cuh:191-192), part c of nclip. On a geometric grid the
+// pairs j in [n-1-Ld, n-1-d] of the lags d = c + nclip (warp + warps k) below
+// dmax (interleaving spreads the long lags near d = 0 over the parts), a warp's
+// lanes over j: a lane per lag left one thread with the q + 1 pairs of lag 0, a
+// chain of 50 us at n = 16384. Otherwise the rows j = c + nclip (lane + T k).
+// Callers that add the lags from D0 on by the prefix sums pass dmax = D0.
 template <int K>
-__device__ double clip_part_sum(const AggCellView& v, int c, int nclip, const TileGroup& G)
+__device__ double clip_part_sum(const AggCellView& v, int c, int nclip, int dmax, const TileGroup& G)
 {
     const int n = v.n;
     double acc = 0.0;
     if (v.geo) {
-        for (int d = c + nclip * G.lane; d < n; d += nclip * G.T) {
+        const int w = G.lane >> 5, l = G.lane & 31, nw = G.T >> 5;
+        for (int d = c + nclip * w; d < dmax; d += nclip * nw) {
             const int L = v.Ld[d];
             const int jhi = n - 1 - d;
             const int jlo = (L >= kLagClipAll) ? 0 : max(0, n - 1 - L);
             const double B = v.Bd[d], S = v.Sd[d];
-            for (int j = jlo; j <= jhi; ++j) {
+            for (int j = jlo + l; j <= jhi; j += 32) {
                 const double hj = NeedH<K>::j ? v.Hj[j] : 0.0;
                 const double hk = NeedH<K>::k ? v.Hk[j + d] : 0.0;
                 acc += rate_geo<K>(B, S, v.Nj[j], hj, v.Nk[j + d], hk);
@@ -303,7 +399,7 @@ __global__ void __launch_bounds__(kMainThreads, 2)
 agg_main_kernel(const double* __restrict__ N, const double* __restrict__ x,
                 double* __restrict__ rhs, AggWs ws, int n, int ntile,
                 int ntasks, int nclip, double b0, double bbr, double bsh, int T, int Cg,
-                int ntasks_lane)
+                int lane_on)
 {
     extern __shared__ double red[];               // [2 W][kMainThreads]
     __shared__ TileShared sm;
@@ -311,6 +407,7 @@ agg_main_kernel(const double* __restrict__ N, const double* __restrict__ x,
     __shared__ int s_last[kMaxGroups];
 
     const int tid = threadIdx.x;
+    if (blockIdx.x == 0 && tid == 0) ws.counter[5] = 0;   // the lane kernel is done with its list
     AggCellView v;
     v.x = x; v.Nk = N; v.Hk = ws.h; v.Nj = N; v.Hj = ws.h; v.Aj = N; v.AHj = ws.h;
     v.Fs = (K == 2) ? ws.h : N;
@@ -324,7 +421,7 @@ agg_main_kernel(const double* __restrict__ N, const double* __restrict__ x,
     for (int q = 0; q < 5; ++q) v.M[q] = ws.mom[q];
 
     // geometric grids run the lane-block kernel instead (launched just before)
-    if (ntasks_lane > 0 && v.geo) return;
+    if (lane_on && v.geo) return;
 
     // groups of T threads pull tasks on their own (no CTA-wide barrier in the loop)
     const int g = tid / T;
@@ -340,7 +437,7 @@ agg_main_kernel(const double* __restrict__ N, const double* __restrict__ x,
 
         if (task < nclip) {
             // a part of the pairs clipped at x[n-1]
-            const double sc = group_sum(clip_part_sum<K>(v, task, nclip, G), sm, G);
+            const double sc = group_sum(clip_part_sum<K>(v, task, nclip, n, G), sm, G);
             if (lane == 0) {
                 if constexpr (SCATTER) {
                     if (sc != 0.0) atomicAdd(rhs + (n - 1), sc);
@@ -438,9 +535,9 @@ agg_main_kernel(const double* __restrict__ N, const double* __restrict__ x,
 
 // ---------------------------------------------------------------------------
 // lane: persistent CTAs pulling lane-block tasks (agg_lane.cuh) on verified
-// geometric grids -- clip tasks first, then (block, lag chunk) tasks largest
-// first in the order of the prep's table ws.ltask (the full chunks, then each
-// block's last chunk by length, so the last wave holds the shortest tasks).
+// geometric grids -- clip tasks first, then the exact slots, then the tasks (block t, share p) of every
+// block's direct lags, share by share with the top blocks first (all shares have
+// equal lags but those of the lowest blocks, which come last).
 // Returns at once on other grids (the tile kernel
 // launched after it takes them). It needs fewer registers than the tile
 // kernel, so more CTAs fit on an SM.
@@ -453,15 +550,15 @@ constexpr int kLaneCtas = PBE_LANE_CTAS;           // CTAs per SM (register budg
 template <int K, bool SCATTER, bool STAGE>
 __global__ void __launch_bounds__(kMainThreads, kLaneCtas)
 agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
-                double* __restrict__ rhs, AggWs ws, int n, int ntasks_lane, int nclip,
-                double b0, double bbr, double bsh, int lane_C)
+                double* __restrict__ rhs, AggWs ws, int n, int nclip, double b0, double bbr,
+                double bsh)
 {
     // per-warp slot sums, then the staged windows (16-byte aligned offsets)
     extern __shared__ __align__(128) double lsmem[];
     __shared__ __align__(8) uint64_t s_bar;
     __shared__ int s_flag;
     __shared__ int s_task;
-    __shared__ double s_wsum[kMainThreads / 32];
+    __shared__ double s_wsum[2 * kLaneWarps];
 
     if (ws.mom[5] == 0.0) return;                  // not geometric: the tile kernel runs
     const int tid = threadIdx.x;
@@ -485,7 +582,11 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
     constexpr int kRed = 2 * kLaneWarps * kLaneBins;     // per-warp R, TH of every slot
     const LaneSmem lsm{lsmem, lsmem + kRed, lsmem + kRed + kLaneWinMax,
                        lsmem + kRed + 2 * kLaneWinMax};
-    const LaneArgs la{ws.Ncp, ws.xcp, ws.lpart, ws.cticket, ws.counter + 4, lane_C};
+    const int nblk = lane_blocks(n);
+    const int parts = lane_parts(min(v.D0, n), nblk, gridDim.x);
+    const int nexact = ws.counter[5];
+    const int ntasks_lane = nclip + nexact + nblk * parts;
+    const LaneArgs la{ws.Ncp, ws.xcp, ws.lpart, ws.cticket, ws.counter + 4, parts};
     const TileGroup G0{0, tid, kMainThreads};
     unsigned phase = 0;
     for (;;) {
@@ -497,7 +598,7 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
         if (task >= ntasks_lane || stop) break;
         if (task < nclip) {
             // a part of the pairs clipped at x[n-1], summed over the CTA in a fixed order
-            double sc = warp_sum(clip_part_sum<K>(v, task, nclip, G0));
+            double sc = warp_sum(clip_part_sum<K>(v, task, nclip, min(n, v.D0), G0));
             if ((tid & 31) == 0) s_wsum[tid >> 5] = sc;
             __syncthreads();
             if (tid == 0) {
@@ -514,9 +615,13 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
             continue;
         }
         task -= nclip;
-        // largest first (the prep's launch order)
-        const int t = __ldg(ws.ltask + 2 * task), c = __ldg(ws.ltask + 2 * task + 1);
-        lane_task<K, SCATTER, STAGE>(v, ws, la, rhs, t, c, nclip, lsm, &s_bar, phase, &s_flag);
+        if (task < nexact) {
+            exact_slot_task<K, SCATTER>(v, ws, la, rhs, ws.xlist[task], nclip, s_wsum, s_flag != 0);
+            continue;
+        }
+        task -= nexact;
+        lane_task<K, SCATTER, STAGE>(v, ws, la, rhs, task % nblk, task / nblk, nclip, lsm, &s_bar,
+                                     phase, &s_flag);
     }
 }
 
@@ -617,10 +722,6 @@ cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_
     // lane-block tasks, taken instead of the tiles when the grid turns out
     // geometric (decided on the device by the prep kernel)
     const int lane_mode = agg_lane_mode();
-    const int lane_C = lane_chunk_len(n);
-    const long long nlane_ll = lane_mode ? lane_tasks(n, lane_C) + nclip : 0;
-    if (nlane_ll > 0x7fffffffLL) return cudaErrorInvalidValue;
-    const int ntasks_lane = static_cast<int>(nlane_ll);
     // chunked gather: many tasks of few lags; single warps keep the fixed-order
     // reduction (2 W T adds per task) small next to a chunk's pairs
     const int T = (Cg < n) ? agg_group_size_chunked() : agg_group_size(ntasks, num_sms);
@@ -633,8 +734,10 @@ cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_
     if (e != cudaSuccess) return e;
     auto lkern = (lane_mode == 2) ? agg_lane_kernel<K, SC, false> : agg_lane_kernel<K, SC, true>;
     const size_t lsmem = sizeof(double) * (2 * kLaneWarps * kLaneBins + 3 * kLaneWinMax);
+    // the number of tasks is known on the device only (it follows D0)
     const long long lcap = static_cast<long long>(kLaneCtas) * num_sms;
-    const int lgrid = static_cast<int>(ntasks_lane < lcap ? ntasks_lane : lcap);
+    const long long lmost = static_cast<long long>(lane_blocks(n)) * kLaneMaxParts + nclip;
+    const int lgrid = static_cast<int>(lmost < lcap ? lmost : lcap);
     if (lane_mode) {
         e = cudaFuncSetAttribute(lkern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(lsmem));
@@ -651,16 +754,20 @@ cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_
         if (e != cudaSuccess) return e;
         agg_prep_kernel<K, true><<<nb, kPrepThreads, 0, s>>>(a.N, a.x, n, ws, a.beta0, a.beta_br,
                                                              a.beta_sh);
-        if (kind == kAggTables) return cudaGetLastError();
+        if (kind == kAggTables) {
+            e = cudaGetLastError();
+            // this call's exact slots are no one's: the next prep starts its own list
+            return e != cudaSuccess ? e : cudaMemsetAsync(ws.counter + 5, 0, sizeof(int), s);
+        }
     }
     const bool prof = g_prof_start && g_prof_stop;
     if (prof) cudaEventRecord(g_prof_start, s);
     if (lane_mode && lgrid > 0)
-        lkern<<<lgrid, kMainThreads, lsmem, s>>>(a.N, a.x, a.rhs, ws, n, ntasks_lane, nclip,
-                                                 a.beta0, a.beta_br, a.beta_sh, lane_C);
+        lkern<<<lgrid, kMainThreads, lsmem, s>>>(a.N, a.x, a.rhs, ws, n, nclip, a.beta0, a.beta_br,
+                                                 a.beta_sh);
     agg_main_kernel<K, SC><<<grid, kMainThreads, smem, s>>>(a.N, a.x, a.rhs, ws, n, ntile, ntasks,
                                                             nclip, a.beta0, a.beta_br, a.beta_sh,
-                                                            T, Cg, ntasks_lane);
+                                                            T, Cg, lane_mode ? 1 : 0);
     if (prof) cudaEventRecord(g_prof_stop, s);
     return cudaGetLastError();
 }

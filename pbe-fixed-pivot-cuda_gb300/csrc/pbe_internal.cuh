@@ -91,6 +91,26 @@ __device__ __forceinline__ double scale_pow2(double v, int s20)
     return __hiloint2double(hi, lo);
 }
 
+// v * 2^s for s <= 0, the exponent taken off the bits (no FP64 instruction);
+// results below the normal range become zero (a zero stays zero for any s),
+// infinities and NaN stay.
+__device__ __forceinline__ double scale_down(double v, int s)
+{
+    const int hi = __double2hiint(v), e = (hi >> 20) & 0x7ff;
+    if (e == 0x7ff) return v;
+    return e > 0 && e + s > 0 ? __hiloint2double(hi + (s << 20), __double2loint(v)) : 0.0;
+}
+
+// Binary exponent and [1, 2) mantissa of a positive normal double.
+__device__ __forceinline__ int exponent_of(double v)
+{
+    return ((__double2hiint(v) >> 20) & 0x7ff) - 1023;
+}
+__device__ __forceinline__ double mantissa_of(double v)
+{
+    return __hiloint2double((__double2hiint(v) & 0x000fffff) | 0x3ff00000, __double2loint(v));
+}
+
 __device__ __forceinline__ double warp_sum(double v)
 {
 #pragma unroll
@@ -247,14 +267,24 @@ struct AggWs {
     int*    cticket;   // [ntile] lag-chunk tasks of the tile done
     int*    counter;   // [8]  [0] task counter, [1] first lag with Ld[d] == d,
                        //      [2] prep blocks done, [3] bin n-1 contributors done,
-                       //      [4] a staging wait of the lane tasks gave up
+                       //      [4] a staging wait of the lane tasks gave up, [5] entries of xlist
     double* Ncp;       // [n + 2] copy of N, 256-byte aligned (bulk-copy source)
     double* xcp;       // [n + 2] copy of x, 256-byte aligned (bulk-copy source)
     double* lpart;     // [lane_partial_doubles(n)] lane-task chunk partials
-    int*    ltask;     // [2 lane_tasks(n)] lane tasks in launch order, (block, chunk) pairs
+    // Prefix sums over the bins (agg_prep_kernel): with m_q = {1/a, 1, a, a^2, x}_q N,
+    // mloc[q n + i] = sum of m_q over the bins of i's prep block up to i, and
+    // mloc[(5 + q) n + i] the same of m_q x 2^-E_i (E = binary exponent of x_i);
+    // moff[q nb + b], moff[(5 + q) nb + b] the sums over all blocks before b (the
+    // latter at the exponent of block b's predecessor's last bin).
+    double* mloc;      // [2 kMomN n]
+    double* mtot;      // [2 kMomN nb_prep] block totals
+    double* moff;      // [2 kMomN nb_prep]
+    int*    xlist;     // [n] slots whose lags from D0 on keep the exact pair sum, counter[5] of them
+    double* xsum;      // [2 n] their R, TH
 };
+constexpr int kMomN = 5;               // moments per prefix (the death term's)
 
-constexpr int agg_prep_blocks(int n) { return (n + kPrepThreads - 1) / kPrepThreads; }
+__host__ __device__ constexpr int agg_prep_blocks(int n) { return (n + kPrepThreads - 1) / kPrepThreads; }
 __host__ __device__ constexpr int agg_tiles(int n) { return (n + kTileW - 1) / kTileW; }
 
 // Gather mode with few tiles per CTA slot (small n): each tile's lags are cut
@@ -365,10 +395,12 @@ __host__ __device__ inline int lane_last_rank(int n, int t, int C)
     return rank;
 }
 
-// Doubles of lane-task chunk partials: tasks x (R, TH) x kLaneBins.
+// Lane tasks of the aggregation pair kernel: each block's direct lags cut into
+// `parts` equal shares, (R, TH) partials of kLaneBins slots per share.
+constexpr int kLaneMaxParts = 8;
 __host__ __device__ constexpr size_t lane_partial_doubles(int n)
 {
-    return static_cast<size_t>(lane_tasks(n, lane_chunk_len(n))) * 2 * kLaneBins;
+    return static_cast<size_t>(lane_blocks(n)) * kLaneMaxParts * 2 * kLaneBins;
 }
 
 // Size of the aggregation scratch for n bins, equal to agg_ws_layout(n) below
@@ -388,7 +420,10 @@ constexpr size_t agg_ws_bytes(int n)
          + align256(sizeof(int) * 8)
          + 2 * align256(sizeof(double) * (static_cast<size_t>(n) + 2))
          + align256(sizeof(double) * lane_partial_doubles(n))
-         + align256(sizeof(int) * 2 * static_cast<size_t>(lane_tasks(n, lane_chunk_len(n))));
+         + align256(sizeof(double) * 2 * kMomN * static_cast<size_t>(n))
+         + 2 * align256(sizeof(double) * 2 * kMomN * static_cast<size_t>(agg_prep_blocks(n)))
+         + align256(sizeof(int) * static_cast<size_t>(n))
+         + align256(sizeof(double) * 2 * static_cast<size_t>(n));
 }
 
 // Carves the aggregation scratch out of `base` (may be null to query the size).
@@ -419,8 +454,12 @@ inline size_t agg_ws_layout(int n, char* base, AggWs* ws)
     w.Ncp       = reinterpret_cast<double*>(take(sizeof(double) * (static_cast<size_t>(n) + 2)));
     w.xcp       = reinterpret_cast<double*>(take(sizeof(double) * (static_cast<size_t>(n) + 2)));
     w.lpart     = reinterpret_cast<double*>(take(sizeof(double) * lane_partial_doubles(n)));
-    w.ltask     = reinterpret_cast<int*>(take(sizeof(int) * 2 *
-                                              static_cast<size_t>(lane_tasks(n, lane_chunk_len(n)))));
+    w.mloc      = reinterpret_cast<double*>(take(sizeof(double) * 2 * kMomN * static_cast<size_t>(n)));
+    const size_t nbm = sizeof(double) * 2 * kMomN * static_cast<size_t>(agg_prep_blocks(n));
+    w.mtot      = reinterpret_cast<double*>(take(nbm));
+    w.moff      = reinterpret_cast<double*>(take(nbm));
+    w.xlist     = reinterpret_cast<int*>(take(sizeof(int) * static_cast<size_t>(n)));
+    w.xsum      = reinterpret_cast<double*>(take(sizeof(double) * 2 * static_cast<size_t>(n)));
     if (ws) *ws = w;
     return off;
 }
