@@ -1,0 +1,261 @@
+// =============================================================================
+// agg_slot.cuh -- aggregation pair sums with one output slot per lane, for any
+// grid: the pair work of the batched kernel (batch_kernels.cu).
+//
+// Slot s collects the pairs (j <= k) whose bracket is lo = s: R_s = sum rate,
+// TH_s = sum rate (fl(x_j + x_k) - x_s) 2^St_s, St_s = -exponent of x_s
+// (reference src/aggregation_kernels.cuh:145-239, regrouped; aggregation.cu has
+// the derivation). The pairs of a slot split in two:
+//
+//  * k = s, j < jcut(s): the sum still lands below x_{s+1}, so the larger member
+//    is the slot's own bin. beta is a sum of products of powers of x_j and x_k,
+//    so these sums come from prefix moments over j (cell_prefix):
+//      R += N_s death_factor(x_s; P),  TH += N_s death_factor(x_s; T),
+//    P, T the moments of N and x N over j < jcut(s). On a geometric grid
+//    jcut(s) = s - D0 + 1 (lags from D0 on); on any other a table per grid. With
+//    q sections an octave D0 is about q log2(1.44 q): 10 lags of n at q = 4, 176
+//    at q = 32. Why the sums may be separated, and when not (mom_exact_slot):
+//    agg_lane.cuh.
+//  * the rest pair by pair (slot_pairs_geo: the lags below D0, runs of lags with
+//    one bracket offset sharing their larger member; slot_pairs_any: a monotone
+//    walk over the rows j).
+//
+// NP = 1: the RHS. NP = 2: its Jacobian-vector product, T(N, v) + T(v, N) with
+// T(a, b) the pair sum with rate beta a_j b_k, both in one pass over the pairs
+// (they share brackets and weights).
+// =============================================================================
+#pragma once
+
+#include "agg_tile.cuh"
+#include "agg_moments.cuh"
+
+namespace pbe_gb300 {
+
+// The grid of a cell (its first n pivots) and the cell's coefficients.
+struct SlotGrid {
+    const double* x;
+    const double* a;        // x^(1/3)
+    const double* ia;       // x^(-1/3)
+    const double* inv_dx;
+    const double* Bd;       // lag factors, c_d = 1/2 on lag 0, no beta (geometric grids)
+    const double* Sd;
+    const int* Ld;          // bracket offset of a lag
+    const int* J0;          // first j with fl(x_j + x_s) >= x_{s+1} (other grids)
+    int n, D0;
+    bool geo;
+    double b0, bbr, bsh;
+};
+
+// One bilinear pass: j side a, k side b. Nj = beta a_j and Hj = beta x_j a_j carry
+// the cell's coefficient (the lag factors do not); Aj = a_j and AHj = x_j a_j for
+// the walk on other grids.
+struct SlotPass {
+    const double* Nj;
+    const double* Hj;
+    const double* Aj;
+    const double* AHj;
+    const double* Nk;
+    const double* Hk;
+};
+
+// Rows j < slot_cut(s) with k = s belong to the prefix sums.
+__device__ __forceinline__ int slot_cut(const SlotGrid& g, int s)
+{
+    if (g.geo) return max(0, s - g.D0 + 1);
+    // the clipped slot n - 1 takes every j < n - 1; the diagonal pair is never in
+    return s >= g.n - 1 ? s : min(__ldg(g.J0 + s), s);
+}
+
+// Lags [d0, d1) of slot s on a geometric grid (uniform d0, d1, smax across the
+// warp; Ld nondecreasing). pc: the slot's pivot, decoded.
+template <int K, int NP>
+__device__ __forceinline__ void slot_pairs_geo(const SlotGrid& g, const SlotPass* p, int s, bool slot,
+                                               int smax, int d0, int d1, const EwOperandC& pc,
+                                               double& R, double& TH)
+{
+    EwOperandA pa = ew_operand_a(0.0);               // x_k of the current run
+    double Q[NP], QT[NP], F[NP], hk[NP];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) { Q[q] = QT[q] = F[q] = hk[q] = 0.0; }
+    int e_cur = -1;
+    for (int d = d0; d < d1; ++d) {
+        const int L = __ldg(g.Ld + d);
+        if (L > smax) break;
+        const int e = L - d;
+        if (e != e_cur) {                              // uniform across the warp
+            e_cur = e;
+            const int k = s - e;
+            const bool kin = slot && k >= 0;
+#pragma unroll
+            for (int q = 0; q < NP; ++q) {
+                if constexpr (K != 1) {
+                    R = fma(F[q], Q[q], R);
+                    TH = fma(F[q], QT[q], TH);
+                    Q[q] = 0.0;
+                    QT[q] = 0.0;
+                }
+                F[q] = kin ? (K == 2 ? p[q].Hk : p[q].Nk)[k] : 0.0;
+                if constexpr (K == 1) hk[q] = kin ? p[q].Hk[k] : 0.0;
+            }
+            pa = ew_operand_a(kin ? __ldg(g.x + k) : 0.0);
+        }
+        const double B = __ldg(g.Bd + d), S = __ldg(g.Sd + d);
+        const int j = s - L;
+        if (slot && j >= 0) {
+            const double th = sum_minus_scaled_pre(pa, __ldg(g.x + j), pc);
+#pragma unroll
+            for (int q = 0; q < NP; ++q) {
+                const double Nj = (K == 2 || K == 4) ? 0.0 : p[q].Nj[j];
+                const double hj = NeedH<K>::j ? p[q].Hj[j] : 0.0;
+                if constexpr (K != 1) {
+                    const double r = q_slot<K>(B, S, Nj, hj);
+                    Q[q] += r;
+                    QT[q] = fma(r, th, QT[q]);
+                } else {
+                    const double r = rate_geo<1>(B, S, Nj, hj, F[q], hk[q]);
+                    R += r;
+                    TH = fma(r, th, TH);
+                }
+            }
+        }
+    }
+    if constexpr (K != 1) {
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            R = fma(F[q], Q[q], R);
+            TH = fma(F[q], QT[q], TH);
+        }
+    }
+}
+
+// beta(x_j, x_k) a_j b_k from per-bin values, every pass.
+template <int K, int NP>
+__device__ __forceinline__ double slot_rate_any(const SlotGrid& g, const SlotPass* p, int j, int k)
+{
+    const double aj = K >= 3 ? __ldg(g.a + j) : 0.0, iaj = K >= 3 ? __ldg(g.ia + j) : 0.0;
+    const double ak = K >= 3 ? __ldg(g.a + k) : 0.0, iak = K >= 3 ? __ldg(g.ia + k) : 0.0;
+    double r = 0.0;
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+        const double v = rate_gen<K>(j == k, g.b0, g.bbr, g.bsh, p[q].Aj[j],
+                                     NeedH<K>::k ? p[q].AHj[j] : 0.0, aj, iaj,
+                                     p[q].Nk[k], NeedH<K>::k ? p[q].Hk[k] : 0.0, ak, iak);
+        r = q == 0 ? v : r + v;
+    }
+    return r;
+}
+
+// Share w of nw of slot s's rows on any grid, but for the pairs of the prefix
+// sums: for each row j the larger members k with x_s <= fl(x_j + x_k) < x_{s+1}
+// lie in one run below the previous row's, so a lane walks down k as j grows.
+template <int K, int NP>
+__device__ __forceinline__ void slot_pairs_any(const SlotGrid& g, const SlotPass* p, int s, bool slot,
+                                               int w, int nw, double& R, double& TH)
+{
+    if (!slot) return;
+    const double* __restrict__ x = g.x;
+    const double xs = __ldg(x + s), xu = __ldg(x + s + 1);
+    const long long lo = dbits(xs), hi = dbits(xu);
+    const int St20 = -exponent_of(xs) * (1 << 20);
+    const int Js = slot_cut(g, s);
+    const int j0 = s > 0 ? min(Js, slot_cut(g, s - 1)) : Js;
+    const int per = (s + 1 - j0 + nw - 1) / nw;
+    const int ja = j0 + w * per, jb = min(s + 1, ja + per);
+    if (ja >= jb) return;
+    // last k <= s with fl(x_ja + x_k) < x_{s+1} (below ja: the rows are done)
+    const double xa = __ldg(x + ja);
+    int k = s, kb = ja - 1;
+    while (kb < k) {
+        const int mid = (kb + k + 1) >> 1;
+        if (dbits(xa + __ldg(x + mid)) < hi) kb = mid; else k = mid - 1;
+    }
+    for (int j = ja; j < jb; ++j) {
+        const double xj = __ldg(x + j);
+        while (k >= j && dbits(xj + __ldg(x + k)) >= hi) --k;
+        if (k < j) break;
+        for (int q = k; q >= j; --q) {
+            const double v = xj + __ldg(x + q);
+            if (dbits(v) < lo) break;
+            if (q == s && j < Js) continue;            // in the prefix sums
+            const double r = slot_rate_any<K, NP>(g, p, j, q);
+            R += r;
+            TH = fma(r, scale_pow2(v - xs, St20), TH);
+        }
+    }
+}
+
+// The prefix part of slot s pair by pair, by one warp (lanes over j, fixed
+// butterfly): for the slots of mom_exact_slot. Valid in every lane.
+template <int K, int NP>
+__device__ __forceinline__ void slot_exact(const SlotGrid& g, const SlotPass* p, int s, double& R,
+                                           double& TH)
+{
+    const int lane = threadIdx.x & 31;
+    const double xs = __ldg(g.x + s);
+    const int St = -exponent_of(xs);
+    const EwOperandA pa = ew_operand_a(xs);
+    const EwOperandC pc = ew_operand_c(xs, St);
+    const int cut = slot_cut(g, s);
+    double r = 0.0, t = 0.0;
+    for (int j = lane; j < cut; j += 32) {
+        double rate, th;
+        if (g.geo) {
+            const int d = s - j;
+            rate = 0.0;
+#pragma unroll
+            for (int q = 0; q < NP; ++q)
+                rate += rate_geo<K>(__ldg(g.Bd + d), __ldg(g.Sd + d), p[q].Nj[j],
+                                    NeedH<K>::j ? p[q].Hj[j] : 0.0, p[q].Nk[s],
+                                    NeedH<K>::k ? p[q].Hk[s] : 0.0);
+            th = sum_minus_scaled_pre(pa, __ldg(g.x + j), pc);
+        } else {
+            rate = slot_rate_any<K, NP>(g, p, j, s);
+            th = scale_pow2((__ldg(g.x + j) + xs) - xs, St * (1 << 20));
+        }
+        r += rate;
+        t = fma(rate, th, t);
+    }
+    R = warp_sum(r);
+    TH = warp_sum(t);
+}
+
+// Clipped pairs (x_j + x_k >= x[n-1], all deposited on bin n-1,
+// src/aggregation_kernels.cuh:191-192) but for those of the prefix sums of slot
+// n - 1, share of thread tid of nt: a warp per lag with its lanes over j on a
+// geometric grid, a thread per row otherwise.
+template <int K, int NP>
+__device__ double slot_clip(const SlotGrid& g, const SlotPass* p, int tid, int nt)
+{
+    const int n = g.n;
+    double acc = 0.0;
+    if (g.geo) {
+        const int l = tid & 31;
+        for (int d = tid >> 5; d < min(n, g.D0); d += nt >> 5) {
+            const int L = __ldg(g.Ld + d);
+            const int jlo = L >= kLagClipAll ? 0 : max(0, n - 1 - L);
+            const double B = __ldg(g.Bd + d), S = __ldg(g.Sd + d);
+            for (int j = jlo + l; j <= n - 1 - d; j += 32)
+#pragma unroll
+                for (int q = 0; q < NP; ++q)
+                    acc += rate_geo<K>(B, S, p[q].Nj[j], NeedH<K>::j ? p[q].Hj[j] : 0.0,
+                                       p[q].Nk[j + d],
+                                       NeedH<K>::k ? p[q].Hk[j + d] : 0.0);
+        }
+    } else {
+        const long long top = dbits(__ldg(g.x + n - 1));
+        for (int j = tid; j < n; j += nt) {
+            const double xj = __ldg(g.x + j);
+            int lo = j, hi = n - 1;                    // x_j + x[n-1] >= x[n-1] always holds
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (dbits(xj + __ldg(g.x + mid)) >= top) hi = mid; else lo = mid + 1;
+            }
+            // k = n - 1 is in the prefix sums, but for the diagonal pair
+            for (int k = lo; k < n - 1 || (k == n - 1 && j == n - 1); ++k)
+                acc += slot_rate_any<K, NP>(g, p, j, k);
+        }
+    }
+    return acc;
+}
+
+} // namespace pbe_gb300

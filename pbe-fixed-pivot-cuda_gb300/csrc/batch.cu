@@ -3,14 +3,13 @@
 // the tile-group autotuner, RK4 as one CUDA graph, the per-cell launch loop,
 // and the pbe_batch_* C ABI (include/pbe_gb300.h).
 //
-// Schedule. Every cell is cut into tiles of kTileW bins; a tile task costs
-// about min(I + W, n) lags. Cells are classed by floor(log2 n). Each class has a group
-// size T (threads per task): a bundle packs 256/T tasks of one class, so a
-// CTA of the persistent kernel runs up to eight small tiles at once. Bundles
-// are sorted by work (largest first) and pulled from an atomic counter. A
-// plan with few tiles (a handful of cells) also cuts each tile's lags into
-// chunks (chunk_setup) and gathers the breakage term in the pair tasks
-// instead of one prep CTA per cell; its VJP takes larger groups.
+// Schedule. Every cell is cut into pair tasks of kSlotBins bins; a task costs
+// about its grid's direct lags. Cells are classed by floor(log2 n). Each class
+// has a group size T (threads per task): a bundle packs 256/T tasks of one
+// class, so a CTA of the pair kernel runs up to eight tasks at once. Bundles
+// are sorted by work (largest first) and launched in that order. A plan of few
+// cells gathers the breakage term in the pair tasks instead of the prep CTAs
+// and gives each cell's prep a cluster of CTAs; its VJP takes larger groups.
 //
 // Per call. The selection function of every bin is evaluated once per call
 // into the plan's cache (sel_cache, SelScope). The adaptive integrators and
@@ -18,7 +17,7 @@
 // solves are left out of the prep and pair launches.
 //
 // Autotuner. With PBE_BATCH_TUNE, each class present in the plan times the
-// persistent kernel on its own tasks for T = 32, 64, 128, 256 (synthetic
+// pair kernel on its own tasks for T = 32, 64, 128, 256 (synthetic
 // state; the work of a tile does not depend on the values) and keeps the
 // fastest. Results are cached per process and device (key: SM count, kernel
 // type, breakage on/off, class) and, when PBE_GB300_TUNE_CACHE names a file,
@@ -60,7 +59,7 @@ struct pbe_batch_plan {
     int group_size[16] = {0};
     int4* d_bundles = nullptr;
     int4* d_tasks = nullptr;
-    std::vector<char> grid_geo;        // grids verified geometric (lag chunks apply)
+    std::vector<int> grid_direct;      // direct lags of a slot (D0), or n on a grid that is not geometric
     std::vector<double> t_q, bw_q;
     double* d_tq = nullptr;
     double* d_bw = nullptr;
@@ -114,7 +113,8 @@ struct pbe_batch_plan {
 namespace pbe_gb300 {
 namespace {
 
-constexpr int W = kTileW;
+constexpr int W = kTileW;        // rows of a VJP tile
+constexpr int SW = kSlotBins;    // bins of a pair task
 constexpr int kClasses = 16;
 
 int n_class(int n)
@@ -124,14 +124,14 @@ int n_class(int n)
     return c;
 }
 
-// Default group size per class (what the autotuner picked on GB300 for the
-// 4096-cell workload: the reduction of 2 (W+1) T partial sums per task costs
-// more than the lanes a small group leaves idle), 128 for very large cells.
-int rule_group_size(int cls)
+// Default group size of the pair tasks: a warp each, until the tasks would leave
+// CTA slots empty (about 4 CTAs of 256 threads per SM); more warps then split a
+// task's direct pairs, at least 16 lags each.
+int rule_group_size(long long tasks, int max_lags, int num_sms)
 {
-    if (cls <= 7) return 64;      // n < 256
-    if (cls <= 13) return 32;     // n < 16384
-    return 128;
+    int T = 32;
+    while (T < kMainThreads && tasks * T < 4LL * kMainThreads * num_sms && max_lags * 32 >= 16 * 2 * T) T <<= 1;
+    return T;
 }
 
 // ---- tune cache ----------------------------------------------------------------
@@ -169,14 +169,19 @@ void tune_cache_store_locked(const TuneKey& k, int t)
 }
 
 // ---- schedule ------------------------------------------------------------------
-struct HostTask { int cell, I, chunk, nct; long long cost; };
+struct HostTask { int cell, I; long long cost; };
 
-long long task_cost(int n, int I, int T)
+// Lags of row tile tasks (VJP): every row meets all n partners.
+long long vjp_task_cost(int n, int T)
 {
-    const long long lags = std::min(I + W, n);
-    const long long it = (lags + T - 1) / T;
+    const long long it = (n + T - 1) / T;
     return it * T + 4LL * T;                          // + reduction / epilogue
 }
+
+// Pairs per slot that a pair task sums directly: the lags below D0 (a grid that
+// is not geometric: about the rows below the first bin), and the epilogue's
+// worth of about 8 pairs.
+long long pair_task_cost(int direct, int I) { return std::min(direct, I + SW) + 8LL; }
 
 // Bundles for the cells of the classes selected by `want` (all when null),
 // each class with its group size gs[class]; sorted by work, largest first.
@@ -186,26 +191,15 @@ void build_schedule(const pbe_batch_plan& p, const int* gs, const bool* want,
                     std::vector<int4>& bundles, std::vector<int4>& tasks, bool vjp = false)
 {
     std::vector<std::vector<HostTask>> per(kClasses);
-    const int Cg = p.d.Cg;
     for (int c = 0; c < p.n_cells; ++c) {
         const int n = p.cell_n[c];
         const int cls = n_class(n);
         if (want && !want[cls]) continue;
         if (vjp) {
-            for (int I = 0; I < n; I += W) per[cls].push_back({c, I, 0, 1, task_cost(n, n, gs[cls])});
+            for (int I = 0; I < n; I += W) per[cls].push_back({c, I, vjp_task_cost(n, gs[cls])});
         } else {
-            // forward tiles aligned to the top: the lowest may start below bin 0;
-            // tile t spans the lags below n - W t, cut into chunks of Cg lags
-            // when the plan has few tiles (chunk_setup)
-            const bool chunks = Cg > 0 && p.grid_geo[p.cell_grid[c]];
-            for (int I = n - W; I > -W; I -= W) {
-                const int span = I + W;
-                const int nct = chunks ? (span + Cg - 1) / Cg : 1;
-                for (int k = 0; k < nct; ++k) {
-                    const int lags = nct > 1 ? std::min(Cg, span - k * Cg) : span;
-                    per[cls].push_back({c, I, k, nct, task_cost(n, lags - W, gs[cls])});
-                }
-            }
+            const int direct = p.grid_direct[p.cell_grid[c]];
+            for (int I = 0; I < n; I += SW) per[cls].push_back({c, I, pair_task_cost(direct, I)});
         }
     }
     struct B { long long cost; int cls; int first; int cnt; };
@@ -232,7 +226,7 @@ void build_schedule(const pbe_batch_plan& p, const int* gs, const bool* want,
         bundles.push_back(make_int4(static_cast<int>(tasks.size()), b.cnt, gs[b.cls], 0));
         for (int k = 0; k < b.cnt; ++k) {
             const HostTask& t = sorted[b.cls][b.first + k];
-            tasks.push_back(make_int4(t.cell, t.I, t.chunk, t.nct));
+            tasks.push_back(make_int4(t.cell, t.I, 0, 0));
         }
     }
 }
@@ -269,7 +263,7 @@ void free_last(pbe_batch_plan* p, int count)
     }
 }
 
-// Times the persistent kernel on the tasks of one class for each group size.
+// Times the pair kernel on the tasks of one class for each group size.
 cudaError_t tune_class(pbe_batch_plan* p, int cls, const pbe_batch_cell_params_t* dparams,
                        double* dN, double* dout, cudaStream_t s, int* best_T)
 {
@@ -277,7 +271,7 @@ cudaError_t tune_class(pbe_batch_plan* p, int cls, const pbe_batch_cell_params_t
     bool want[kClasses] = {false};
     want[cls] = true;
     float best = 0.0f;
-    *best_T = rule_group_size(cls);
+    *best_T = p->group_size[cls];
     cudaEvent_t e0, e1;
     cudaError_t e = cudaEventCreate(&e0);
     if (e != cudaSuccess) return e;
@@ -338,10 +332,10 @@ cudaError_t autotune(pbe_batch_plan* p, bool retune, cudaStream_t s)
     }
     for (int cls = 0; cls < kClasses && e == cudaSuccess; ++cls) {
         if (!present[cls]) continue;
-        const TuneKey key(p->num_sms, p->kernel, (p->nq > 0 ? 1 : 0) | (p->d.Cg > 0 ? 2 : 0), cls);
+        const TuneKey key(p->num_sms, p->kernel, p->nq > 0 ? 1 : 0, cls);
         auto it = g_tune.find(key);
         if (!retune && it != g_tune.end()) { p->group_size[cls] = it->second; continue; }
-        int T = rule_group_size(cls);
+        int T = p->group_size[cls];
         e = tune_class(p, cls, dparams, dN, dout, s, &T);
         if (e == cudaSuccess) {
             p->group_size[cls] = T;
@@ -352,48 +346,27 @@ cudaError_t autotune(pbe_batch_plan* p, bool retune, cudaStream_t s)
     return e;
 }
 
-// Plans with few tiles (a handful of small cells) cut each tile of a cell on a
-// geometric grid into chunks of Cg lags, about kChunkTasks tasks per CTA slot
-// in all; the tile's last chunk task adds the chunk sums in chunk order and runs
-// the epilogue. Cg is fixed for the plan, so a tile has the same chunks in every
-// schedule built from it (tuning, class subsets, the Jacobian-vector pass).
-cudaError_t chunk_setup(pbe_batch_plan* p, long long tiles, cudaStream_t s)
+// Direct lags of every grid (from its tables) and the launch shape of the prep
+// kernels: a thread per two bins of an average cell, up to 256; where the cells
+// are too few for the SMs, clusters of up to 8 CTAs share a cell (a prep of one
+// CTA per cell costs about 30 FP64 operations a bin on one SM: 60 us at n = 3840).
+cudaError_t prep_shape(pbe_batch_plan* p, cudaStream_t s)
 {
     BatchDev& d = p->d;
-    d.Cg = 0;
-    d.cbound = 1;
     std::vector<BatchGridDev> hg(static_cast<size_t>(p->n_grids));
     cudaError_t e = cudaMemcpyAsync(hg.data(), d.grids, hg.size() * sizeof(BatchGridDev),
                                     cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return e;
-    p->grid_geo.assign(static_cast<size_t>(p->n_grids), 0);
-    for (int g = 0; g < p->n_grids; ++g) p->grid_geo[g] = hg[g].geo != 0;
-    if (p->kernel < 0 || tiles >= 4LL * 2 * p->num_sms) return cudaSuccess;
-    long long lags = 0;
-    int max_geo_n = 0;
-    for (int c = 0; c < p->n_cells; ++c) {
-        if (!p->grid_geo[p->cell_grid[c]]) continue;
-        const long long n = p->cell_n[c], nt = (n + W - 1) / W;
-        lags += nt * n - static_cast<long long>(W) * nt * (nt - 1) / 2;
-        max_geo_n = std::max(max_geo_n, p->cell_n[c]);
-    }
-    if (lags == 0) return cudaSuccess;
-    const long long target = static_cast<long long>(kChunkTasks) * 2 *
-                             std::min(p->num_sms, kChunkMaxSms);
-    long long cg = (lags + target - 1) / target;
-    cg = std::max<long long>(((cg + 31) / 32) * 32, kChunkMinLags);
-    if (cg >= max_geo_n) return cudaSuccess;
-    const int Cg = static_cast<int>(cg);
-    const int cbound = (max_geo_n + Cg - 1) / Cg;      // the top tile spans n lags
-    const size_t nt = static_cast<size_t>(tiles);
-    e = plan_alloc(p, &d.cpart, nt * static_cast<size_t>(cbound) * 2 * W);
-    if (e == cudaSuccess) e = plan_alloc(p, &d.cticket, nt);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d.cticket, 0, nt * sizeof(unsigned), s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return e;
-    d.Cg = Cg;
-    d.cbound = cbound;
+    p->grid_direct.assign(static_cast<size_t>(p->n_grids), 0);
+    for (int g = 0; g < p->n_grids; ++g) p->grid_direct[g] = hg[g].geo ? hg[g].D0 : hg[g].n;
+    const long long avg = p->total / p->n_cells;
+    int ranks = 1;
+    while (ranks < 8 && 2LL * ranks * p->n_cells <= 4LL * p->num_sms && p->max_n >= 256 * ranks) ranks <<= 1;
+    int threads = 32;
+    while (threads < 256 && (ranks > 1 || 2LL * threads < avg)) threads <<= 1;
+    d.prep_ranks = ranks;
+    d.prep_threads = threads;
     return cudaSuccess;
 }
 
@@ -459,13 +432,12 @@ cudaError_t create(pbe_batch_plan* p, int n_grids, const int* grid_n, const doub
     std::vector<BatchCellDev> hc(static_cast<size_t>(n_cells));
     p->offsets.resize(static_cast<size_t>(n_cells) + 1);
     long long off = 0;
-    long long tiles = 0;
+    long long ntask = 0;
     for (int c = 0; c < n_cells; ++c) {
-        hc[c] = BatchCellDev{static_cast<int>(off), cell_n[c], cell_grid[c],
-                             static_cast<int>(tiles)};
+        hc[c] = BatchCellDev{static_cast<int>(off), cell_n[c], cell_grid[c], 0};
         p->offsets[c] = off;
         off += cell_n[c];
-        tiles += (cell_n[c] + W - 1) / W;
+        ntask += (cell_n[c] + SW - 1) / SW;
         p->max_n = std::max(p->max_n, cell_n[c]);
     }
     p->offsets[n_cells] = off;
@@ -474,6 +446,7 @@ cudaError_t create(pbe_batch_plan* p, int n_grids, const int* grid_n, const doub
     BatchDev& d = p->d;
     d.n_grids = n_grids; d.n_cells = n_cells; d.kernel = kernel; d.selection = selection;
     d.nq = p->nq; d.num_sms = p->num_sms;
+    d.total = p->total;
     // breakage gather in the pair tasks for plans of at most one wave of prep
     // CTAs (measured: one n = 3840 cell 358 -> 233 us per RHS, 64 cells
     // 1540 -> 1435 us; 1024 cells 20.84 -> 21.12 ms, so those keep the prep)
@@ -493,6 +466,7 @@ cudaError_t create(pbe_batch_plan* p, int n_grids, const int* grid_n, const doub
     if (e == cudaSuccess) e = plan_alloc(p, &d.gSd, G);
     if (e == cudaSuccess) e = plan_alloc(p, &d.gLd, G);
     if (e == cudaSuccess) e = plan_alloc(p, &d.gSl, G);
+    if (e == cudaSuccess) e = plan_alloc(p, &d.gJ0, G);
     if (e == cudaSuccess) e = plan_alloc(p, &d.bfirst, static_cast<size_t>(foff));
     if (e == cudaSuccess) e = plan_alloc(p, &d.bwlo, static_cast<size_t>(woff));
     if (e == cudaSuccess) e = plan_alloc(p, &d.bwhi, static_cast<size_t>(woff));
@@ -505,11 +479,8 @@ cudaError_t create(pbe_batch_plan* p, int n_grids, const int* grid_n, const doub
     if (e == cudaSuccess) e = plan_alloc(p, &d.Bk, C);
     if (e == cudaSuccess) e = plan_alloc(p, &d.k, C);
     if (e == cudaSuccess) e = plan_alloc(p, &d.kacc, C);
-    if (e == cudaSuccess) e = plan_alloc(p, &d.mom, static_cast<size_t>(n_cells) * 8);
-    if (e == cudaSuccess) e = plan_alloc(p, &d.counter, 8);
-    if (e == cudaSuccess) e = plan_alloc(p, &d.tfirst, static_cast<size_t>(tiles));
-    if (e == cudaSuccess) e = plan_alloc(p, &d.tcarry, static_cast<size_t>(tiles));
-    if (e == cudaSuccess) e = plan_alloc(p, &d.tticket, static_cast<size_t>(tiles));
+    if (e == cudaSuccess) e = plan_alloc(p, &d.mom, static_cast<size_t>(n_cells) * kMomStride);
+    if (e == cudaSuccess && kernel >= 0) e = plan_alloc(p, &d.pre, 2 * kMomN * C);
     if (e == cudaSuccess && p->nq > 0) e = plan_alloc(p, &p->sx, C);
     if (e == cudaSuccess && p->nq > 0) e = plan_alloc(p, &p->d_tq, static_cast<size_t>(p->nq));
     if (e == cudaSuccess && p->nq > 0) e = plan_alloc(p, &p->d_bw, static_cast<size_t>(p->nq));
@@ -519,7 +490,6 @@ cudaError_t create(pbe_batch_plan* p, int n_grids, const int* grid_n, const doub
     // finite for the loads that the tile body issues unconditionally
     for (double* a : {d.Y, d.Nj, d.Hj, d.Hk, d.SN, d.Bk, d.k, d.kacc})
         if (e == cudaSuccess) e = cudaMemsetAsync(a, 0, C * sizeof(double), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d.tticket, 0, static_cast<size_t>(tiles) * sizeof(int), s);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d.grids, hg.data(), hg.size() * sizeof(BatchGridDev),
                             cudaMemcpyHostToDevice, s);
@@ -536,16 +506,15 @@ cudaError_t create(pbe_batch_plan* p, int n_grids, const int* grid_n, const doub
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(p->d_bw, bw_q, p->nq * sizeof(double), cudaMemcpyHostToDevice, s);
     }
-    if (e == cudaSuccess) e = batch_kernel_setup(kernel);
     if (e == cudaSuccess) e = batch_grid_tables(d, p->d_tq, p->d_bw, 0, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess) e = chunk_setup(p, tiles, s);
+    if (e == cudaSuccess) e = prep_shape(p, s);
     if (e != cudaSuccess) return e;
-
-    // lag chunks: single-warp groups keep the fixed-order reduction (2 W T adds
-    // per task) small next to a chunk's pairs
+    int max_lags = 1;
+    for (int c = 0; c < n_cells; ++c)
+        max_lags = std::max(max_lags, std::min(cell_n[c], p->grid_direct[cell_grid[c]]));
     for (int cls = 0; cls < kClasses; ++cls)
-        p->group_size[cls] = d.Cg > 0 ? 32 : rule_group_size(cls);
+        p->group_size[cls] = rule_group_size(ntask, max_lags, p->num_sms);
     if (flags & (PBE_BATCH_TUNE | PBE_BATCH_RETUNE)) {
         e = autotune(p, (flags & PBE_BATCH_RETUNE) != 0, s);
         if (e != cudaSuccess) return e;
@@ -722,11 +691,11 @@ cudaError_t vjp_setup(pbe_batch_plan* p, cudaStream_t s)
     for (int c = 0; c < p->n_cells; ++c) tile_off[c + 1] = tile_off[c] + (p->cell_n[c] + W - 1) / W;
     // every row tile meets all n partners, so with few tiles larger groups
     // (fewer tasks per bundle) give each CTA slot a bundle: T >= 256 x (CTA
-    // slots) / tiles, a power of two in [forward T, 256]
+    // slots) / tiles, a power of two up to 256
     int gs[kClasses];
     const long long tiles = tile_off.back();
     for (int c = 0; c < kClasses; ++c) {
-        int T = p->group_size[c] > 0 ? p->group_size[c] : 32;
+        int T = c <= 7 ? 64 : 32;         // n < 256: 64
         while (T < kMainThreads && tiles * T < 256LL * 2 * p->num_sms) T <<= 1;
         gs[c] = T;
     }
@@ -883,30 +852,29 @@ const double kDPErr[7] = {71.0 / 57600.0, 0.0, -71.0 / 16695.0, 71.0 / 1920.0,
                           -17253.0 / 339200.0, 22.0 / 525.0, -1.0 / 40.0};
 
 // ---- Jacobian-vector products and the Rosenbrock integrator -------------------
-// J(N) v = T(N, v) + T(v, N) for the aggregation part (two passes of the pair
-// kernel with the j side from the first vector, batch_kernels.cu) plus the
-// breakage Jacobian at N applied to v (first pass).
-// skip (device, n_cells, or null): cells left out of both passes (their
-// out entries keep their old values).
+// J(N) v = T(N, v) + T(v, N) for the aggregation part (both in one pass over
+// the pairs, batch_kernels.cu) plus the breakage Jacobian at N applied to v.
+// skip (device, n_cells, or null): cells left out (their out entries keep their
+// old values).
 cudaError_t jvp(pbe_batch_plan* p, const double* N, const double* v,
                 const pbe_batch_cell_params_t* prm, double* out, cudaStream_t s,
                 const int* skip = nullptr)
 {
     if (!p->d.Ha) {
-        cudaError_t e = plan_alloc(p, &p->d.Ha, static_cast<size_t>(p->total));
-        if (e != cudaSuccess) { p->d.Ha = nullptr; return e; }
+        const size_t C = static_cast<size_t>(p->total);
+        double *ha = nullptr, *nj = nullptr, *hj = nullptr, *pre = nullptr;
+        cudaError_t e = plan_alloc(p, &nj, C);
+        if (e == cudaSuccess) e = plan_alloc(p, &hj, C);
+        if (e == cudaSuccess && p->kernel >= 0) e = plan_alloc(p, &pre, 2 * kMomN * C);
+        if (e == cudaSuccess) e = plan_alloc(p, &ha, C);
+        if (e != cudaSuccess) return e;
+        p->d.Nj2 = nj; p->d.Hj2 = hj; p->d.pre2 = pre; p->d.Ha = ha;
     }
     BatchDev d = p->d;
     d.skip = skip;
-    BatchDev d1 = d;
-    d1.A = N;
-    cudaError_t e = batch_jvp_prep(d, N, v, N, prm, true, s);
-    if (e == cudaSuccess) e = batch_main(d1, v, prm, out, false, s);
-    BatchDev d2 = d;
-    d2.A = v;
-    d2.brk |= kBrkNone;                    // breakage is linear: first pass only
-    if (e == cudaSuccess) e = batch_jvp_prep(d, v, N, N, prm, false, s);
-    if (e == cudaSuccess) e = batch_main(d2, N, prm, out, true, s);
+    d.A = N;
+    cudaError_t e = batch_jvp_prep(d, v, prm, s);
+    if (e == cudaSuccess) e = batch_main(d, v, prm, out, false, s);
     return e;
 }
 

@@ -16,10 +16,13 @@
 
 namespace pbe_gb300 {
 
+constexpr int kSlotBins = 31;    // bins of a pair task (a warp's lanes: their slots and the one below)
+constexpr int kMomStride = 24;   // doubles of BatchDev::mom per cell
+
 struct BatchGridDev {
     int off;     // first bin in the packed grid arrays
     int n;       // pivots
-    int D0;      // first lag with Ld[d] == d (written by the grid kernel)
+    int D0;      // first lag >= 1 with Ld[d] == d (written by the grid kernel)
     int geo;     // 1 when verified geometric (written by the grid kernel)
     int foff;    // first entry of the grid's run-start table (nq * (n + 2) ints)
     int woff;    // first entry of the grid's fragment weights (nq * n doubles)
@@ -30,7 +33,7 @@ struct BatchCellDev {
     int off;       // first bin in the packed cell arrays
     int n;         // sections of the cell (<= its grid's n)
     int grid;
-    int tile_off;  // first hand-over slot of the cell's tiles (tile t at tile_off + t)
+    int pad;
 };
 
 // Device pointers of a plan: grid tables (static) and per-stage cell arrays.
@@ -41,16 +44,17 @@ struct BatchDev {
     int kernel;        // aggregation kernel type, -1 = no aggregation
     int selection;     // breakage selection, -1 = no breakage
     int nq;            // quadrature points (0 = no breakage)
-    // breakage gather (in the padding after nq, so the struct keeps its size):
-    // bit kBrkTasks: gathered from SN by the pair tasks in their epilogues
+    // breakage gather: bit kBrkTasks: gathered from SN by the pair tasks in their epilogues
     // (their own bins) instead of by the prep kernel (one CTA per cell, into
     // Bk); plans of few cells take it, so that one large cell's prep does not
     // hold up the launch, while many cells balance the prep CTAs anyway.
-    // bit kBrkNone: no breakage term in this pass (the second pass of a
-    // Jacobian-vector product).
     int brk;
+    // launch shape of the prep kernels: CTAs per cell (a cluster) and threads per CTA
+    int prep_ranks, prep_threads;
+    long long total;   // packed length of the per-bin arrays
     // per grid bin (packed by BatchGridDev::off)
     double* gx; double* ga; double* gia; double* ginv_dx; double* gBd; double* gSd; int* gLd;
+    int* gJ0;       // first j with fl(x_j + x_i) >= x_{i+1} (at most i)
     double* gSl;    // shear factor of lag d seen from the larger member: (1 + rho)^3 x_0 / x_d
     // breakage fragment tables: bfirst[foff + q (n+2) + m + 1] = first j with
     // lo(q, j) >= m; bwlo / bwhi[woff + q n + j] = bw_q times the shares of the
@@ -66,27 +70,19 @@ struct BatchDev {
     double* Bk;     // breakage term of the stage (gathered by the prep kernel, brk without kBrkTasks)
     double* k;      // stage derivative (RK4)
     double* kacc;   // k1 + 2 k2 + 2 k3 (+ k4)
-    // Jacobian-vector passes (batch_jvp.cu): the j-side vector of the pass,
-    // unscaled (null for an RHS evaluation), and x times it
+    // prefix moments of the stage state over each cell's bins (cell_prefix):
+    // pre[q total + off + i], 2 kMomN arrays
+    double* pre;
+    // a Jacobian-vector product: the state A (null for an RHS evaluation; Y is
+    // then the direction), x A, the direction's j-side arrays and prefix moments
     const double* A;
-    double* Ha;
-    double* mom;    // [n_cells * 8] moments of the stage state (death term), [5] clip sum
-    int* counter;   // [8] task counter of the persistent kernel
-    // hand-over of a tile's first bin (tiles aligned to the cell's top; tile t
-    // owns bins [n - W (t+1), n - W t)): its own value, the carry of the tile
-    // below, and a ticket that both bump once per launch (odd = second)
-    double* tfirst; double* tcarry; int* tticket;   // [sum of the cells' tiles]
+    double* Ha; double* Nj2; double* Hj2; double* pre2;
+    // [n_cells * kMomStride] 0..4 moments of the stage state (death term), 5..9
+    // of the direction, 10 + r the clipped pairs summed by CTA r of the cell
+    double* mom;
     // schedule
     const int4* bundles;   // {first task, tasks, group size, 0}
-    const int4* tasks;     // {cell, first bin, lag chunk, chunks of the tile}
-    // lag chunks of the tiles (plans with few tiles: see build_schedule):
-    // chunk c of a tile covers the lags [c Cg, (c + 1) Cg); the tile's last
-    // chunk task (a ticket that wraps to 0 with it: no reset needed) adds the
-    // chunks' slot sums in order and runs the epilogue
-    int Cg;                // lags per chunk (0: no chunks)
-    int cbound;            // most chunks of a tile
-    double* cpart;         // [tiles * cbound * 2 kTileW]
-    unsigned* cticket;     // [tiles] lag-chunk tasks of the tile done (wraps at nct)
+    const int4* tasks;     // {cell, first bin, 0, 0}
     int n_bundles;
     int num_sms;
     // [n_cells] or null: a cell with a nonzero entry is left out of the prep
@@ -101,7 +97,6 @@ struct BatchDev {
     const double* Sx;
 };
 constexpr int kBrkTasks = 1;
-constexpr int kBrkNone = 2;
 
 // Scratch of the batched VJP (batch_vjp.cu).
 struct BatchVjpDev {
@@ -177,9 +172,6 @@ struct GmresDev {
 };
 
 // Launchers (batch_kernels.cu). All are asynchronous on `s`.
-// Once per plan, before any launch (and outside stream capture): the
-// persistent kernel's shared-memory attribute for `kernel`.
-cudaError_t batch_kernel_setup(int kernel);
 cudaError_t batch_grid_tables(const BatchDev& d, const double* t_q, const double* bw_q,
                               int max_grid_n, cudaStream_t s);
 // Prep of a stage: state update per `stage`, stage arrays, moments, counter reset.
@@ -230,17 +222,16 @@ cudaError_t batch_ros2_stage(const BatchDev& d, const double* N, const double* K
 cudaError_t batch_ros2_control(const BatchDev& d, double* N, const double* K1, const double* K2,
                                const Rk45Ctl& ctl, cudaStream_t s);
 
-// Prep of one Jacobian-vector pass (batch_kernels.cu, batch_jvp_prep_kernel):
-// j side from A, k side from B, breakage (brk) as the product of its Jacobian
-// at the state G with B, else zero. Followed by batch_main with Y = B and a
-// copy of d whose A = A.
 // Sx[off_c + i] = S(x_i) of cell c's parameters, every bin of the plan
 // (total = the packed length).
 cudaError_t batch_sel(const BatchDev& d, const pbe_batch_cell_params_t* params, double* Sx,
                       long long total, cudaStream_t s);
-cudaError_t batch_jvp_prep(const BatchDev& d, const double* A, const double* B, const double* G,
-                           const pbe_batch_cell_params_t* params, bool brk, cudaStream_t s);
-// Persistent RHS kernel over the plan's bundles: out (+)= RHS(Y) for every cell.
+// Prep of the Jacobian-vector product at d.A along v, followed by batch_main
+// with Y = v and the same d.
+cudaError_t batch_jvp_prep(const BatchDev& d, const double* v, const pbe_batch_cell_params_t* params,
+                           cudaStream_t s);
+// Pair kernel over the plan's bundles: out (+)= RHS(Y) for every cell (d.A set:
+// the Jacobian-vector product at A along Y).
 cudaError_t batch_main(const BatchDev& d, const double* Y, const pbe_batch_cell_params_t* params,
                        double* out, bool accumulate, cudaStream_t s);
 // Same over an explicit bundle list (the autotuner's candidate schedules).

@@ -6,28 +6,32 @@
 // the breakage fragment tables of each grid (brackets, weights, run starts).
 //
 // Per RHS evaluation (two launches):
-//  * batch_prep_kernel, one CTA per cell: the RK4 stage update of the cell's
-//    state, the stage arrays (j-side factors carrying the cell's kernel
-//    coefficients, S(x) N for breakage), the five death moments and the sum
-//    of the cell's clipped pairs.
-//  * batch_main_kernel, persistent: CTAs pull "bundles" from an atomic
-//    counter, largest first. A bundle holds 256/T tile tasks (cell, first bin)
-//    that run side by side on groups of T threads; T is chosen per section
-//    count class by the plan (autotuned or by rule), so a 64-section cell is
-//    not spread over 256 threads. A task runs the shared tile body
-//    (agg_tile.cuh), gathers the breakage term of its bins from S N (a few
-//    fragments per bin and quadrature point), adds the prep kernel's clip sum
-//    and writes its bins once: no atomics, and a fixed summation order for a
-//    fixed schedule. The gather is spread over all tasks instead of one CTA
-//    per cell, so a large cell's prep does not hold up the launch.
+//  * batch_prep_kernel, one cluster of CTAs per cell: the RK4 stage update of the
+//    cell's state, the stage arrays (j-side factors carrying the cell's kernel
+//    coefficients, S(x) N for breakage), the prefix moments over the bins (their
+//    last sums are the death moments) and the sum of the cell's clipped pairs.
+//  * batch_main_kernel: CTAs of 256 threads, each one "bundle" (largest first) of
+//    256/T tasks (cell, first bin) that run side by side on groups of T threads;
+//    T is chosen per section-count class by the plan (autotuned or by rule). A
+//    task owns 31 bins of a cell: a warp's lanes hold their slots and the one
+//    below (agg_slot.cuh), the group's warps split the pairs that the prefix
+//    moments leave, and the group gathers the breakage term of its bins from S N
+//    (a few fragments per bin and quadrature point), adds the clip sum and
+//    writes its bins once: no atomics, and a fixed summation order for a fixed
+//    schedule. The slot below the first bin is summed by two tasks (1 in 32), so
+//    nothing is handed over between tasks.
 // =============================================================================
 #include "batch_internal.cuh"
-#include "agg_tile.cuh"
+#include <cooperative_groups.h>
+
+#include "agg_slot.cuh"
 
 namespace pbe_gb300 {
 namespace {
 
-constexpr int W = kTileW;
+namespace cg = cooperative_groups;
+
+constexpr int SW = kSlotBins;
 
 // ---------------------------------------------------------------------------
 // Grid tables: one CTA per grid. Per bin: a, 1/a, 1/dx; per lag d (= bin
@@ -67,7 +71,18 @@ batch_grid_kernel(BatchDev d)
         const double v = x0 + xi;
         const int L = (dbits(v) >= dbits(x[n - 1])) ? kLagClipAll : bracket_from(x, n, v, i);
         d.gLd[gd->off + i] = L;
-        if (L == i) d0 = min(d0, i);
+        if (L == i && i > 0) d0 = min(d0, i);   // lag 0 carries the pair 1/2: never separated
+        // first j with fl(x_j + x_i) >= x_{i+1}: the prefix sums of slot i on a
+        // grid that is not geometric (monotone in j, so a bisection)
+        int jl = 0, jh = i;
+        if (i < n - 1) {
+            const long long top = dbits(x[i + 1]);
+            while (jl < jh) {
+                const int mid = (jl + jh) >> 1;
+                if (dbits(x[mid] + xi) >= top) jh = mid; else jl = mid + 1;
+            }
+        }
+        d.gJ0[gd->off + i] = jl;
         if (n >= 2) {
             double e = geo_dev(fit, xi, i);
             if (!(e == e)) e = 1.0;
@@ -187,46 +202,6 @@ batch_sel_kernel(BatchDev d, const pbe_batch_cell_params_t* __restrict__ params,
     }
 }
 
-// ---------------------------------------------------------------------------
-// Clipped pairs of a cell (v >= x[n-1], all deposited on bin n-1), summed by
-// the group of the task that owns bin n-1: per lag on a geometric grid (the
-// pairs j in [n-1-Ld, n-1-d]), per row otherwise.
-// ---------------------------------------------------------------------------
-template <int K>
-__device__ double cell_clip(const AggCellView& v, const TileGroup& G)
-{
-    const int n = v.n;
-    double acc = 0.0;
-    if (v.geo) {
-        for (int d = G.lane; d < n; d += G.T) {
-            const int L = v.Ld[d];
-            const int jhi = n - 1 - d;
-            const int jlo = (L >= kLagClipAll) ? 0 : max(0, n - 1 - L);
-            const double B = v.Bd[d], S = v.Sd[d];
-            for (int j = jlo; j <= jhi; ++j) {
-                const double hj = NeedH<K>::j ? v.Hj[j] : 0.0;
-                const double hk = NeedH<K>::k ? v.Hk[j + d] : 0.0;
-                acc += rate_geo<K>(B, S, v.Nj[j], hj, v.Nk[j + d], hk);
-            }
-        }
-    } else {
-        const long long tb = dbits(v.x[n - 1]);
-        for (int j = G.lane; j < n; j += G.T) {
-            const double xj = v.x[j];
-            int lo = j, hi = n - 1;   // xj + x[n-1] >= x[n-1] always holds
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (dbits(xj + v.x[mid]) >= tb) hi = mid; else lo = mid + 1;
-            }
-            const double Nj = v.Aj[j], hj = v.AHj[j], aj = v.a[j], iaj = v.ia[j];
-            for (int k = lo; k < n; ++k)
-                acc += rate_gen<K>(j == k, v.b0, v.bbr, v.bsh, Nj, hj, aj, iaj, v.Nk[k], v.Hk[k],
-                                   v.a[k], v.ia[k]);
-        }
-    }
-    return acc;
-}
-
 // One lane's part of the breakage gather of bin i (0 <= i < n) of a cell:
 // quadrature points q = q0, q0 + nqp, ..., each adding the hi-shares of the
 // fragments bracketed at i-1 and the lo-shares of those at i (bin 0 also the
@@ -258,25 +233,25 @@ __device__ __forceinline__ int brk_lanes(int nq)
     return nqp;
 }
 
-// Breakage term of every bin of a cell (one CTA; the prep kernels without
+// Breakage term of the bins [r0, r1) of a cell (one CTA; the prep kernels without
 // kBrkTasks), minus S_i N_i: a warp covers 32/nqp bins, nqp = the quadrature
 // points rounded up to a power of two (<= 32) lanes per bin.
 __device__ void cell_breakage(const BatchDev& d, const BatchGridDev& gd, const double* SN,
-                              double* Bk, int n)
+                              double* Bk, int n, int r0, int r1)
 {
     const int nqp = brk_lanes(d.nq);
     const int per_warp = 32 / nqp;
     const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    for (int base = w * per_warp; base < n; base += nw * per_warp) {   // uniform per warp
+    for (int base = r0 + w * per_warp; base < r1; base += nw * per_warp) {   // uniform per warp
         const int i = base + l / nqp;
-        double acc = (i < n) ? brk_lane(d, gd, SN, n, i, l % nqp, nqp) : 0.0;
+        double acc = (i < r1) ? brk_lane(d, gd, SN, n, i, l % nqp, nqp) : 0.0;
         for (int o = nqp >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (i < n && (l % nqp) == 0) Bk[i] = acc - SN[i];
+        if (i < r1 && (l % nqp) == 0) Bk[i] = acc - SN[i];
     }
 }
 
-// The same term for the bins I .. I+W-1 of a cell (those in [0, n)), by a
-// task's group into out[0 .. W) (kBrkTasks): the same lanes per bin, loops and
+// The same term for the bins I .. I+SW-1 of a cell (those below n), by a
+// task's group into out[0 .. SW) (kBrkTasks): the same lanes per bin, loops and
 // butterfly, so the sums are bitwise those of cell_breakage.
 __device__ void tile_breakage(const BatchDev& d, const BatchGridDev& gd, const double* SN, int n,
                               int I, double* out, const TileGroup& G)
@@ -284,21 +259,198 @@ __device__ void tile_breakage(const BatchDev& d, const BatchGridDev& gd, const d
     const int nqp = brk_lanes(d.nq);
     const int per_warp = 32 / nqp;
     const int nw = G.T >> 5, w = G.lane >> 5, l = G.lane & 31;
-    for (int base = w * per_warp; base < W; base += nw * per_warp) {   // uniform per warp
+    for (int base = w * per_warp; base < SW; base += nw * per_warp) {   // uniform per warp
         const int t = base + l / nqp;
         const int i = I + t;
-        const bool in = t < W && i >= 0 && i < n;
+        const bool in = t < SW && i < n;
         double acc = in ? brk_lane(d, gd, SN, n, i, l % nqp, nqp) : 0.0;
         for (int o = nqp >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (t < W && (l % nqp) == 0) out[t] = in ? acc - SN[i] : 0.0;
+        if (t < SW && (l % nqp) == 0) out[t] = in ? acc - SN[i] : 0.0;
+    }
+}
+
+// The cell of a cluster of CTAs: its bins are split evenly over the CTAs, and a
+// CTA's bins over its threads in contiguous runs.
+struct CellPart {
+    int rank, ranks;      // this CTA in the cell's cluster
+    int r0, r1;           // its bins
+    int t0, t1;           // this thread's bins
+};
+__device__ __forceinline__ CellPart cell_part(int n)
+{
+    const cg::cluster_group cl = cg::this_cluster();
+    CellPart p;
+    p.rank = static_cast<int>(cl.block_rank());
+    p.ranks = static_cast<int>(cl.num_blocks());
+    const int per = (n + p.ranks - 1) / p.ranks;
+    p.r0 = min(n, p.rank * per);
+    p.r1 = min(n, p.r0 + per);
+    const int c = (p.r1 - p.r0 + static_cast<int>(blockDim.x) - 1) / static_cast<int>(blockDim.x);
+    p.t0 = min(p.r1, p.r0 + c * static_cast<int>(threadIdx.x));
+    p.t1 = min(p.r1, p.t0 + c);
+    return p;
+}
+
+// Prefix moments of y over the cell's bins into pre (AggWs::mloc's sums, here
+// over the whole cell): pre[q stride + i] = sum m_q, pre[(5 + q) stride + i] =
+// sum m_q x at the exponent of x_i, m_q = {1/a, 1, a, a^2, x}_q y; and, by the
+// cluster's CTA 0, the moments over all bins into mom[0..4]. Two passes over a
+// thread's run (totals, then the running sums), a scan of the totals over lanes,
+// warps and CTAs between them. Fixed order for a fixed launch shape.
+constexpr int kPrepMaxWarps = 8;
+struct PrefixShared {
+    double wt[kPrepMaxWarps][2 * kMomN];     // warp totals, then the warps' offsets
+    int we[kPrepMaxWarps];                   // exponent after the warp's last bin
+    double ct[2 * kMomN];                    // CTA totals (read by the cluster's other CTAs)
+    int ce;
+};
+
+template <int K>
+__device__ void cell_prefix(const double* __restrict__ x, const double* __restrict__ a,
+                            const double* __restrict__ ia, const double* y, const CellPart& part,
+                            PrefixShared& sm, double* pre, long long stride, double* mom)
+{
+    const cg::cluster_group cl = cg::this_cluster();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    double P[kMomN], T[kMomN];
+    auto add = [&](int i, int& e) {
+        const double xi = __ldg(x + i), yi = y[i];
+        const int ei = exponent_of(xi);
+        const double ay = (K >= 3) ? __ldg(a + i) * yi : 0.0, xm = mantissa_of(xi);
+        const double m[kMomN] = {(K >= 3) ? __ldg(ia + i) * yi : 0.0, yi, ay,
+                                 (K >= 4) ? __ldg(a + i) * ay : 0.0, xi * yi};
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) {
+            if (!need_moment<K>(q)) continue;
+            P[q] += m[q];
+            T[q] = fma(m[q], xm, ei != e ? scale_down(T[q], e - ei) : T[q]);
+        }
+        e = ei;
+    };
+#pragma unroll
+    for (int q = 0; q < kMomN; ++q) { P[q] = 0.0; T[q] = 0.0; }
+    const int eb = part.t0 > 0 ? exponent_of(__ldg(x + part.t0 - 1)) : 0;   // before the run
+    int e = part.t0 > 0 ? eb : exponent_of(__ldg(x));
+    for (int i = part.t0; i < part.t1; ++i) add(i, e);
+    // inclusive scan of the runs over the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int dE = __shfl_up_sync(0xffffffffu, e, o) - e;
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) {
+            if (!need_moment<K>(q)) continue;
+            const double p = __shfl_up_sync(0xffffffffu, P[q], o);
+            const double t = __shfl_up_sync(0xffffffffu, T[q], o);
+            if (lane >= o) { P[q] += p; T[q] += scale_down(t, dE); }
+        }
+    }
+    if (lane == 31) {
+        sm.we[w] = e;
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) { sm.wt[w][q] = P[q]; sm.wt[w][kMomN + q] = T[q]; }
+    }
+    // the runs before this lane's in the warp (their sum stands at exponent ep)
+    const int eu = __shfl_up_sync(0xffffffffu, e, 1);
+    const int ep = lane > 0 ? eu : eb;
+#pragma unroll
+    for (int q = 0; q < kMomN; ++q) {
+        if (!need_moment<K>(q)) continue;
+        const double p = __shfl_up_sync(0xffffffffu, P[q], 1);
+        const double t = __shfl_up_sync(0xffffffffu, T[q], 1);
+        P[q] = lane > 0 ? p : 0.0;
+        T[q] = lane > 0 ? t : 0.0;
+    }
+    __syncthreads();
+    // lanes 0 .. 2 kMomN - 1 of warp 0, one sum each: the warps' offsets in the CTA
+    const bool weighted = lane >= kMomN;
+    double acc = 0.0;
+    int ea = 0;
+    if (w == 0 && lane < 2 * kMomN) {
+        for (int v = 0; v < nw; ++v) {
+            const double t = sm.wt[v][lane];
+            if (weighted && v > 0) acc = scale_down(acc, ea - sm.we[v]);
+            ea = sm.we[v];
+            acc += t;
+        }
+        sm.ct[lane] = acc;
+        if (lane == 0) sm.ce = ea;
+    }
+    cl.sync();                                        // every CTA's totals are there
+    if (w == 0 && lane < 2 * kMomN) {
+        // the CTAs before this one, then the warps before each warp
+        double base = 0.0;
+        int be = 0;
+        for (int r = 0; r < part.rank; ++r) {
+            const int en = *cl.map_shared_rank(&sm.ce, r);
+            if (weighted && r > 0) base = scale_down(base, be - en);
+            base += *cl.map_shared_rank(&sm.ct[lane], r);
+            be = en;
+        }
+        for (int v = 0; v < nw; ++v) {
+            const double t = sm.wt[v][lane];
+            sm.wt[v][lane] = base;                    // before warp v, at exponent be
+            const int en = sm.we[v];
+            __syncwarp((1u << (2 * kMomN)) - 1u);     // read by every lane
+            if (lane == 0) sm.we[v] = be;
+            if (weighted) base = scale_down(base, be - en);
+            base += t;
+            be = en;
+        }
+        if (part.rank == 0 && lane < kMomN) {
+            double tot = sm.ct[lane];
+            for (int r = 1; r < part.ranks; ++r) tot += *cl.map_shared_rank(&sm.ct[lane], r);
+            mom[lane] = tot;
+        }
+    }
+    __syncthreads();
+    const int wb = sm.we[w];
+#pragma unroll
+    for (int q = 0; q < kMomN; ++q) {
+        if (!need_moment<K>(q)) continue;
+        P[q] += sm.wt[w][q];
+        T[q] += scale_down(sm.wt[w][kMomN + q], wb - ep);
+    }
+    e = part.t0 > 0 ? ep : exponent_of(__ldg(x));
+    for (int i = part.t0; i < part.t1; ++i) {
+        add(i, e);
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) {
+            if (!need_moment<K>(q)) continue;
+            pre[static_cast<long long>(q) * stride + i] = P[q];
+            pre[static_cast<long long>(kMomN + q) * stride + i] = T[q];
+        }
+    }
+}
+
+__device__ __forceinline__ SlotGrid slot_grid(const BatchDev& d, const BatchGridDev& gd, int n,
+                                              const pbe_batch_cell_params_t& P)
+{
+    return SlotGrid{d.gx + gd.off, d.ga + gd.off, d.gia + gd.off, d.ginv_dx + gd.off,
+                    d.gBd + gd.off, d.gSd + gd.off, d.gLd + gd.off, d.gJ0 + gd.off,
+                    n, gd.D0, gd.geo != 0, P.beta0, P.beta_br, P.beta_sh};
+}
+
+// The passes of a launch for the cell at packed offset off: the RHS at Y (one
+// pass), or the Jacobian-vector product at d.A along Y (A with Y, Y with A).
+template <int NP>
+__device__ __forceinline__ void slot_passes(const BatchDev& d, const double* Y, int off, SlotPass* p)
+{
+    const double* y = Y + off;
+    if constexpr (NP == 1) {
+        p[0] = SlotPass{d.Nj + off, d.Hj + off, y, d.Hk + off, y, d.Hk + off};
+    } else {
+        const double* a = d.A + off;
+        p[0] = SlotPass{d.Nj + off, d.Hj + off, a, d.Ha + off, y, d.Hk + off};
+        p[1] = SlotPass{d.Nj2 + off, d.Hj2 + off, y, d.Hk + off, a, d.Ha + off};
     }
 }
 
 // ---------------------------------------------------------------------------
-// Stage prep: one CTA per cell. Pass 1 (per bin): the stage update, the stage
-// arrays (S N for the breakage gather of the pair tasks) and the moment
-// partials. Pass 2 (after a block barrier, so the whole cell's arrays are
-// visible): the moments and the cell's clipped-pair sum (mom[5]).
+// Stage prep: one cluster per cell. Per bin: the stage update and the stage
+// arrays (S N for the breakage gather of the pair tasks); then the prefix
+// moments, and (after a cluster barrier, so the whole cell's arrays are
+// visible) each CTA's part of the cell's clipped pairs (mom[10 + rank]) and of
+// its breakage term.
 // ---------------------------------------------------------------------------
 template <int K>
 __global__ void __launch_bounds__(256)
@@ -306,26 +458,27 @@ batch_prep_kernel(BatchDev d, double* N, const pbe_batch_cell_params_t* __restri
                   int stage, double c, double dt6, StageCombine sc)
 {
     __shared__ double sh[8];
-    if (d.skip && d.skip[blockIdx.x]) return;       // whole block
-    const BatchCellDev cd = d.cells[blockIdx.x];
+    __shared__ PrefixShared psm;
+    const cg::cluster_group cl = cg::this_cluster();
+    const int cell = blockIdx.x / cl.num_blocks();
+    if (d.skip && d.skip[cell]) return;             // whole cluster
+    const BatchCellDev cd = d.cells[cell];
     const BatchGridDev gd = d.grids[cd.grid];
-    const pbe_batch_cell_params_t P = params[blockIdx.x];
+    const pbe_batch_cell_params_t P = params[cell];
     const bool agg = d.kernel >= 0;
     const int F = d.selection;
     const int off = cd.off, n = cd.n;
+    const CellPart part = cell_part(n);
     double* Nc = N + off;
     double* kc = d.k + off;
     double* ac = d.kacc + off;
     double* Yc = d.Y + off;
     const double* x = d.gx + gd.off;
-    const double* a = d.ga + gd.off;
-    const double* ia = d.gia + gd.off;
     // j-side coefficients: Nj = cN * N, Hj = cH * x N
     const double cN = (K <= 2) ? P.beta0 : P.beta_br;
     const double cH = (K == 1 || K == 2) ? P.beta0 : P.beta_sh;
-    double m[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    const double dtc = (stage == kStageCombine) ? sc.dt[blockIdx.x] : 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const double dtc = (stage == kStageCombine) ? sc.dt[cell] : 0.0;
+    for (int i = part.r0 + threadIdx.x; i < part.r1; i += blockDim.x) {
         double y;
         if (stage == kStageCombine) {
             double s_ = 0.0;
@@ -337,16 +490,11 @@ batch_prep_kernel(BatchDev d, double* N, const pbe_batch_cell_params_t* __restri
         }
         if (stage == kStageFinish) continue;
         const double xi = x[i];
-        const double h = xi * y;
         if (agg) {
+            const double h = xi * y;
             if (K != 2 && K != 4) d.Nj[off + i] = cN * y;
             if (NeedH<K>::j) d.Hj[off + i] = cH * h;
             if (NeedH<K>::k) d.Hk[off + i] = h;
-            m[0] = fma(ia[i], y, m[0]);
-            m[1] += y;
-            m[2] = fma(a[i], y, m[2]);
-            m[3] = fma(a[i] * a[i], y, m[3]);
-            m[4] += h;
         }
         if (F >= 0) {
             const double S = d.Sx ? d.Sx[off + i] : sel_value(F, xi, P.S0, P.v_ref, P.alpha, P.v_min);
@@ -354,268 +502,232 @@ batch_prep_kernel(BatchDev d, double* N, const pbe_batch_cell_params_t* __restri
         }
     }
     if (stage == kStageFinish) return;
-    __syncthreads();                       // the cell's stage arrays are complete
+    __syncthreads();                       // this CTA's part of the stage arrays is complete
+    const double* Yk = (stage == kStageRhs || stage == kStageNext) ? Nc : Yc;
+    double* mom = d.mom + static_cast<size_t>(cell) * kMomStride;
     if (agg) {
-#pragma unroll
-        for (int q = 0; q < 5; ++q) {
-            const double s = block_sum(m[q], sh);
-            if (threadIdx.x == 0) d.mom[blockIdx.x * 8 + q] = s;
-        }
-        AggCellView v;
-        v.x = x;
-        v.Nk = (stage == kStageRhs || stage == kStageNext) ? Nc : Yc;
-        v.Hk = d.Hk + off;
-        v.Aj = v.Nk;
-        v.AHj = v.Hk;
-        v.Nj = d.Nj + off;
-        v.Hj = d.Hj + off;
-        v.Fs = v.Nk;
-        v.a = a; v.ia = ia; v.inv_dx = d.ginv_dx + gd.off;
-        v.Bd = d.gBd + gd.off; v.Sd = d.gSd + gd.off; v.Ld = d.gLd + gd.off;
-        v.n = n; v.D0 = gd.D0; v.geo = gd.geo != 0;
-        v.b0 = P.beta0; v.bbr = P.beta_br; v.bsh = P.beta_sh;
-        const TileGroup G{0, static_cast<int>(threadIdx.x), static_cast<int>(blockDim.x)};
-        const double clip = block_sum(cell_clip<K>(v, G), sh);
-        if (threadIdx.x == 0) d.mom[blockIdx.x * 8 + 5] = clip;
+        cell_prefix<K>(x, d.ga + gd.off, d.gia + gd.off, Yk, part, psm, d.pre + off, d.total, mom);
     }
-    if (d.nq > 0 && !(d.brk & kBrkTasks)) cell_breakage(d, gd, d.SN + off, d.Bk + off, n);
-}
-
-// Hand-over of bin `bin` of a cell (the first bin of tile slot `slot`): its
-// owner tile and the tile below each store their part and bump the ticket;
-// the second (odd count: each launch adds two) writes own + carry. The sum of
-// two is the same whichever is second. Called by one thread.
-__device__ __forceinline__ void batch_first_done(const BatchDev& d, double* out, bool accumulate,
-                                                 int bin, int slot)
-{
-    __threadfence();
-    if ((atomicAdd(d.tticket + slot, 1) & 1) == 0) return;
-    __threadfence();
-    const double v = __ldcg(d.tfirst + slot) + __ldcg(d.tcarry + slot);
-    double* o = out + bin;
-    *o = accumulate ? __ldcg(o) + v : v;
+    cl.sync();                             // the cell's stage arrays are complete; all shared reads done
+    if (agg) {
+        const SlotGrid g = slot_grid(d, gd, n, P);
+        SlotPass sp[1];
+        slot_passes<1>(d, Yk - off, off, sp);
+        const double clip = block_sum(slot_clip<K, 1>(g, sp, part.rank * blockDim.x + threadIdx.x,
+                                                      part.ranks * blockDim.x), sh);
+        if (threadIdx.x == 0) mom[10 + part.rank] = clip;
+    }
+    if (d.nq > 0 && !(d.brk & kBrkTasks)) cell_breakage(d, gd, d.SN + off, d.Bk + off, n, part.r0, part.r1);
 }
 
 // ---------------------------------------------------------------------------
-// Prep of one Jacobian-vector pass (one CTA per cell). The aggregation RHS is
-// quadratic: R(N) = T(N, N) with T(a, b) = sum over pairs j <= k of
-// c_d beta(j, k) a_j b_k (deposits as the RHS; death b_i sum_k beta_ik a_k),
-// so J(N) v = T(N, v) + T(v, N), two passes of the persistent pair kernel
-// with the j side from a and the k side from b. This prep builds the j-side
-// arrays from a (coefficient-scaled, and unscaled for the generic path), the
-// k-side x b, the moments of a (death b_i sum_k beta_ik a_k), the clipped
-// pairs' sum of T(a, b), and the breakage input: the breakage RHS is linear
-// in N wherever its guard passes, so with brk its Jacobian-vector product
-// deposits S_j b_j as the RHS deposits S_j N_j, for the bins whose G_j (the
-// state) passes the guard S_j != 0 && G_j > 2.2e-308 (SN = S b there, 0
-// elsewhere; gathered here or by the pair tasks, as for the RHS); the pass
-// without brk runs its pair kernel with kBrkNone.
+// Prep of a Jacobian-vector product at the state A along v (one cluster per
+// cell). The aggregation RHS is quadratic: R(N) = T(N, N) with T(a, b) = sum
+// over pairs j <= k of c_d beta(j, k) a_j b_k (deposits as the RHS; death b_i
+// sum_k beta_ik a_k), so J(N) v = T(N, v) + T(v, N), both in one pass of the
+// pair kernel. This prep builds both vectors' j-side arrays and x products,
+// their prefix moments (mom[0..4] of A, mom[5..9] of v), the clipped pairs, and
+// the breakage input: the breakage RHS is linear in N wherever its guard passes,
+// so its Jacobian-vector product deposits S_j v_j as the RHS deposits S_j N_j,
+// for the bins whose A_j passes the guard S_j != 0 && A_j > 2.2e-308.
 // ---------------------------------------------------------------------------
 template <int K>
 __global__ void __launch_bounds__(256)
-batch_jvp_prep_kernel(BatchDev d, const double* __restrict__ A, const double* __restrict__ Bv,
-                      const double* __restrict__ Gs, const pbe_batch_cell_params_t* __restrict__ params,
-                      int brk)
+batch_jvp_prep_kernel(BatchDev d, const double* __restrict__ v,
+                      const pbe_batch_cell_params_t* __restrict__ params)
 {
     __shared__ double sh[8];
-    if (d.skip && d.skip[blockIdx.x]) return;       // whole block
-    const BatchCellDev cd = d.cells[blockIdx.x];
+    __shared__ PrefixShared psm;
+    const cg::cluster_group cl = cg::this_cluster();
+    const int cell = blockIdx.x / cl.num_blocks();
+    if (d.skip && d.skip[cell]) return;             // whole cluster
+    const BatchCellDev cd = d.cells[cell];
     const BatchGridDev gd = d.grids[cd.grid];
-    const pbe_batch_cell_params_t P = params[blockIdx.x];
+    const pbe_batch_cell_params_t P = params[cell];
     const bool agg = d.kernel >= 0;
     const int F = d.selection;
     const int off = cd.off, n = cd.n;
+    const CellPart part = cell_part(n);
     const double* x = d.gx + gd.off;
-    const double* a = d.ga + gd.off;
-    const double* ia = d.gia + gd.off;
     const double cN = (K <= 2) ? P.beta0 : P.beta_br;
     const double cH = (K == 1 || K == 2) ? P.beta0 : P.beta_sh;
-    double m[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double ya = A[off + i], yb = Bv[off + i];
+    for (int i = part.r0 + threadIdx.x; i < part.r1; i += blockDim.x) {
+        const double ya = d.A[off + i], yb = v[off + i];
         const double xi = x[i];
         if (agg) {
-            const double ha = xi * ya;
-            if (K != 2 && K != 4) d.Nj[off + i] = cN * ya;
-            if (NeedH<K>::j) d.Hj[off + i] = cH * ha;
+            const double ha = xi * ya, hb = xi * yb;
+            if (K != 2 && K != 4) { d.Nj[off + i] = cN * ya; d.Nj2[off + i] = cN * yb; }
+            if (NeedH<K>::j) { d.Hj[off + i] = cH * ha; d.Hj2[off + i] = cH * hb; }
             d.Ha[off + i] = ha;
-            d.Hk[off + i] = xi * yb;
-            m[0] = fma(ia[i], ya, m[0]);
-            m[1] += ya;
-            m[2] = fma(a[i], ya, m[2]);
-            m[3] = fma(a[i] * a[i], ya, m[3]);
-            m[4] += ha;
+            d.Hk[off + i] = hb;
         }
         if (F >= 0) {
-            double sn = 0.0;
-            if (brk) {
-                const double S = d.Sx ? d.Sx[off + i]
-                                      : sel_value(F, xi, P.S0, P.v_ref, P.alpha, P.v_min);
-                sn = (S != 0.0 && Gs[off + i] > kBreakageNMin) ? S * yb : 0.0;
-            }
-            d.SN[off + i] = sn;
+            const double S = d.Sx ? d.Sx[off + i] : sel_value(F, xi, P.S0, P.v_ref, P.alpha, P.v_min);
+            d.SN[off + i] = (S != 0.0 && ya > kBreakageNMin) ? S * yb : 0.0;
         }
     }
-    __syncthreads();                       // the cell's pass arrays are complete
+    __syncthreads();
+    double* mom = d.mom + static_cast<size_t>(cell) * kMomStride;
     if (agg) {
-#pragma unroll
-        for (int q = 0; q < 5; ++q) {
-            const double s_ = block_sum(m[q], sh);
-            if (threadIdx.x == 0) d.mom[blockIdx.x * 8 + q] = s_;
-        }
-        AggCellView v;
-        v.x = x;
-        v.Nk = Bv + off;
-        v.Hk = d.Hk + off;
-        v.Nj = d.Nj + off;
-        v.Hj = d.Hj + off;
-        v.Aj = A + off;
-        v.AHj = d.Ha + off;
-        v.Fs = v.Nk;
-        v.a = a; v.ia = ia; v.inv_dx = d.ginv_dx + gd.off;
-        v.Bd = d.gBd + gd.off; v.Sd = d.gSd + gd.off; v.Ld = d.gLd + gd.off;
-        v.n = n; v.D0 = gd.D0; v.geo = gd.geo != 0;
-        v.b0 = P.beta0; v.bbr = P.beta_br; v.bsh = P.beta_sh;
-        const TileGroup G{0, static_cast<int>(threadIdx.x), static_cast<int>(blockDim.x)};
-        const double clip = block_sum(cell_clip<K>(v, G), sh);
-        if (threadIdx.x == 0) d.mom[blockIdx.x * 8 + 5] = clip;
+        cell_prefix<K>(x, d.ga + gd.off, d.gia + gd.off, d.A + off, part, psm, d.pre + off, d.total, mom);
+        cl.sync();                         // the shared totals are read by every CTA
+        cell_prefix<K>(x, d.ga + gd.off, d.gia + gd.off, v + off, part, psm, d.pre2 + off, d.total, mom + 5);
     }
-    // first pass only (the second runs with kBrkNone)
-    if (d.nq > 0 && !(d.brk & kBrkTasks) && brk) cell_breakage(d, gd, d.SN + off, d.Bk + off, n);
+    cl.sync();                             // the cell's pass arrays are complete
+    if (agg) {
+        const SlotGrid g = slot_grid(d, gd, n, P);
+        SlotPass sp[2];
+        slot_passes<2>(d, v, off, sp);
+        const double clip = block_sum(slot_clip<K, 2>(g, sp, part.rank * blockDim.x + threadIdx.x,
+                                                      part.ranks * blockDim.x), sh);
+        if (threadIdx.x == 0) mom[10 + part.rank] = clip;
+    }
+    if (d.nq > 0 && !(d.brk & kBrkTasks)) cell_breakage(d, gd, d.SN + off, d.Bk + off, n, part.r0, part.r1);
 }
 
-template <int K>
+// Shared memory of a CTA of the pair kernel (per group g < kMaxGroups).
+struct SlotShared {
+    double red[kMaxGroups][2][32];        // per-warp R, TH of every slot
+    double extra[kMaxGroups][SW];         // per-bin breakage (kBrkTasks)
+};
+
+// ---------------------------------------------------------------------------
+// One pair task (cell, first bin I) on a group of T threads: the bins
+// [I, I + 31), lane l of each warp holding slot I - 1 + l. FP64 instructions per
+// slot, Brownian + shear: 4 per direct pair, 22 for the prefix part, 12 for the
+// death term and the bin.
+// ---------------------------------------------------------------------------
+template <int K, int NP>
 __device__ void batch_task(const BatchDev& d, const double* __restrict__ Yg,
                            const pbe_batch_cell_params_t* __restrict__ params, double* out,
-                           bool accumulate, int4 tk, double* red, TileShared& sm,
-                           const TileGroup& G)
+                           bool accumulate, int4 tk, SlotShared& sm, const TileGroup& G)
 {
-    const int c = tk.x, I = tk.y, chunk = tk.z, nct = tk.w;
+    const int c = tk.x, I = tk.y;
     if (d.skip && d.skip[c]) return;                // the whole group
     const BatchCellDev cd = d.cells[c];
     const BatchGridDev gd = d.grids[cd.grid];
-    const int n = cd.n;
+    const int n = cd.n, off = cd.off;
     const bool agg = d.kernel >= 0;
-    AggCellView v;
-    v.x = d.gx + gd.off;
-    v.Nk = Yg + cd.off;
-    v.Hk = d.Hk + cd.off;
-    v.Aj = d.A ? d.A + cd.off : v.Nk;        // a Jacobian-vector pass: the j-side vector
-    v.AHj = d.A ? d.Ha + cd.off : v.Hk;
-    v.Nj = d.Nj + cd.off;
-    v.Hj = d.Hj + cd.off;
-    v.Fs = (K == 2) ? v.Hk : v.Nk;
-    v.a = d.ga + gd.off; v.ia = d.gia + gd.off; v.inv_dx = d.ginv_dx + gd.off;
-    v.Bd = d.gBd + gd.off; v.Sd = d.gSd + gd.off; v.Ld = d.gLd + gd.off;
-    v.n = n;
-    v.D0 = gd.D0;
-    v.geo = gd.geo != 0;
+    const int l = G.lane & 31, w = G.lane >> 5, nw = G.T >> 5;
     const pbe_batch_cell_params_t P = params[c];
-    v.b0 = P.beta0; v.bbr = P.beta_br; v.bsh = P.beta_sh;
-    // values the epilogue needs go through shared memory, so that they hold no
-    // registers during the pair loop (read back after it)
-    if (G.lane < 8) {
-        const int l = G.lane;
-        sm.cinfo[G.g][l] = (l < 5) ? d.mom[c * 8 + l]
-                                   : (l == 5 ? P.beta0 : (l == 6 ? P.beta_br : P.beta_sh));
-    }
-
-    // tiles are aligned to the cell's top: I = n - W (tile + 1), I > -W
-    const int tile = (n - I) / W - 1;
-    const int St = -ilogb(v.x[max(I, 0)]);
+    const SlotGrid g = slot_grid(d, gd, n, P);
+    SlotPass p[NP];
+    slot_passes<NP>(d, Yg, off, p);
+    const int s = I - 1 + l;                        // this lane's slot and bin
+    const bool slot = s >= 0 && s <= n - 2;
+    const double xs = slot ? __ldg(g.x + s) : 1.0;
+    const int St = slot ? -exponent_of(xs) : 0;
+    double R = 0.0, TH = 0.0;
+    unsigned exact = 0u;
     if (agg) {
-        const int d_begin = nct > 1 ? chunk * d.Cg : 0;
-        const int d_end = nct > 1 ? min(n, d_begin + d.Cg) : n;
-        agg_tile_accumulate<K, true>(v, I, d_begin, d_end, St, red, sm, G);   // syncs the group first
-        if (nct > 1) {
-            // this chunk's slot sums; the tile's last chunk task adds all of
-            // them in chunk order and runs the epilogue (nobody waits)
-            constexpr int R2 = TileSlots<true>::rows;
-            const int slot = cd.tile_off + tile;
-            double* cp = d.cpart + static_cast<size_t>(slot) * d.cbound * R2;
-            if (G.lane < R2) cp[chunk * R2 + G.lane] = sm.fin[G.g][G.lane];
-            G.sync();
-            if (G.lane == 0) {
-                __threadfence();
-                // the ticket counts 0 .. nct-1 and wraps to 0 on the last chunk
-                // task, so it is ready for the next launch without a reset
-                sm.last[G.g] = atomicInc(d.cticket + slot, static_cast<unsigned>(nct - 1))
-                               == static_cast<unsigned>(nct - 1);
-            }
-            G.sync();
-            if (!sm.last[G.g]) return;
-            __threadfence();
-            if (G.lane < R2) {
-                double acc = 0.0;
-                for (int q = 0; q < nct; ++q) acc += __ldcg(cp + q * R2 + G.lane);
-                sm.fin[G.g][G.lane] = acc;
-            }
-            G.sync();
+        const int smax = min(I - 1 + 31, n - 2);
+        if (g.geo) {
+            // equal contiguous shares of the lags below D0 (each warp sees its runs in order)
+            const int lags = min(min(n, g.D0), smax + 1);
+            const int per = (lags + nw - 1) / nw;
+            const int d0 = w * per;
+            slot_pairs_geo<K, NP>(g, p, s, slot, smax, d0, min(lags, d0 + per), ew_operand_c(xs, St), R, TH);
+        } else {
+            slot_pairs_any<K, NP>(g, p, s, slot, w, nw, R, TH);
         }
+        // slots that keep the exact pair sums, spread over the group's warps
+        bool ex = false;
+        if (slot && slot_cut(g, s) > 0) {
+            const double xu = __ldg(g.x + s + 1), idx = __ldg(g.inv_dx + s);
 #pragma unroll
-        for (int q = 0; q < 5; ++q) v.M[q] = sm.cinfo[G.g][q];
-        v.b0 = sm.cinfo[G.g][5]; v.bbr = sm.cinfo[G.g][6]; v.bsh = sm.cinfo[G.g][7];
-    }
-    const bool brk = d.nq > 0 && !(d.brk & kBrkNone);
-    const bool brk_tasks = (d.brk & kBrkTasks) != 0;
-    if (brk && brk_tasks) {
-        tile_breakage(d, gd, d.SN + cd.off, n, I, sm.extra[G.g], G);
-        G.sync();
-    }
-    if (G.lane < W) {
-        const int i = I + G.lane;
-        if (i >= 0) {
-            double val = 0.0;
-            if (agg) {
-                double birth = agg_tile_birth<true>(v, I, G.lane, St, sm.fin[G.g]);
-                if (i == n - 1) birth += d.mom[c * 8 + 5];     // clipped pairs (prep)
-                val = birth - agg_death<K>(v, i);
-            }
-            if (brk) val += brk_tasks ? sm.extra[G.g][G.lane] : d.Bk[cd.off + i];   // breakage
-            if (agg && G.lane == 0 && I >= 1) {
-                // the w-part of slot I-1 comes from the tile below
-                d.tfirst[cd.tile_off + tile] = val;
-                batch_first_done(d, out, accumulate, cd.off + I, cd.tile_off + tile);
-            } else {
-                double* o = out + cd.off + i;
-                *o = accumulate ? *o + val : val;
-            }
+            for (int q = 0; q < NP; ++q) ex = ex || mom_exact_slot(p[q].Nk[s], p[q].Nk[s + 1], xu, idx);
         }
-    } else if (agg && G.lane == W && tile >= 1) {
-        // carry into bin I+W, the first bin of the tile above
-        d.tcarry[cd.tile_off + tile - 1] = agg_tile_carry(v, I, St, sm.fin[G.g]);
-        batch_first_done(d, out, accumulate, cd.off + I + W, cd.tile_off + tile - 1);
+        exact = __ballot_sync(0xffffffffu, ex);
+        int turn = 0;
+        for (unsigned m = exact; m != 0u; m &= m - 1u) {
+            const int le = __ffs(m) - 1;
+            if (turn == w) {
+                double r, t;
+                slot_exact<K, NP>(g, p, I - 1 + le, r, t);
+                if (l == le) { R += r; TH += t; }
+            }
+            turn = turn + 1 == nw ? 0 : turn + 1;
+        }
+    }
+    const bool brk = d.nq > 0;
+    const bool brk_tasks = (d.brk & kBrkTasks) != 0;
+    if (brk && brk_tasks) tile_breakage(d, gd, d.SN + off, n, I, sm.extra[G.g], G);
+    if (nw > 1) {
+        sm.red[G.g * nw + w][0][l] = R;
+        sm.red[G.g * nw + w][1][l] = TH;
+    }
+    G.sync();
+    if (w != 0) return;
+    for (int q = 1; q < nw; ++q) {
+        R += sm.red[G.g * nw + q][0][l];
+        TH += sm.red[G.g * nw + q][1][l];
+    }
+    double clip = 0.0, death = 0.0;
+    if (agg && s >= 0 && s < n) {
+        const double as = __ldg(g.a + s), ias = __ldg(g.ia + s), xv = __ldg(g.x + s);
+        const double* mom = d.mom + static_cast<size_t>(c) * kMomStride;
+        const int cut = slot_cut(g, s);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            const double b = p[q].Nk[s];
+            if (cut > 0 && !((exact >> l) & 1u)) {
+                const double* pre = (q == 0 ? d.pre : d.pre2) + off + (cut - 1);
+                double M[kMomN], M1[kMomN];
+#pragma unroll
+                for (int m = 0; m < kMomN; ++m) {
+                    M[m] = need_moment<K>(m) ? pre[m * d.total] : 0.0;
+                    M1[m] = need_moment<K>(m) ? pre[(kMomN + m) * d.total] : 0.0;
+                }
+                const double r = b * death_factor<K>(xv, as, ias, M, g.b0, g.bbr, g.bsh);
+                if (slot) {
+                    const double t = b * death_factor<K>(xv, as, ias, M1, g.b0, g.bbr, g.bsh);
+                    R += r;
+                    TH += scale_down(t, exponent_of(__ldg(g.x + cut - 1)) + St);
+                } else {
+                    clip += r;                      // bin n - 1: clipped
+                }
+            }
+            double M[kMomN];
+#pragma unroll
+            for (int m = 0; m < kMomN; ++m) M[m] = need_moment<K>(m) ? mom[5 * q + m] : 0.0;
+            death += b * death_factor<K>(xv, as, ias, M, g.b0, g.bbr, g.bsh);
+        }
+        if (s == n - 1)
+            for (int r = 0; r < d.prep_ranks; ++r) clip += mom[10 + r];
+    }
+    // the slot's own part of its bin, and its w-part, owed to the bin above
+    double own = 0.0, up = 0.0;
+    if (slot) {
+        const double sd = scalbn(__ldg(g.inv_dx + s), -St);
+        own = fma(-TH, sd, R);
+        up = TH * sd;
+    }
+    const double in = __shfl_up_sync(0xffffffffu, up, 1);
+    if (l >= 1 && s < n) {
+        double val = 0.0;
+        if (agg) val = ((own + in) + clip) - death;
+        if (brk) val += brk_tasks ? sm.extra[G.g][l - 1] : d.Bk[off + s];
+        double* o = out + off + s;
+        *o = accumulate ? *o + val : val;
     }
 }
 
 #ifndef PBE_BATCH_CTAS
-#define PBE_BATCH_CTAS 2
+#define PBE_BATCH_CTAS 3
 #endif
-template <int K>
+template <int K, int NP>
 __global__ void __launch_bounds__(kMainThreads, PBE_BATCH_CTAS)
 batch_main_kernel(BatchDev d, const double* __restrict__ Y,
                   const pbe_batch_cell_params_t* __restrict__ params, double* out, int accumulate,
-                  const int4* __restrict__ bundles, const int4* __restrict__ tasks, int n_bundles)
+                  const int4* __restrict__ bundles, const int4* __restrict__ tasks)
 {
-    extern __shared__ double red[];     // [2 W][kMainThreads]
-    __shared__ TileShared sm;
-    __shared__ int s_b;
-    const int tid = threadIdx.x;
-    for (;;) {
-        if (tid == 0) s_b = atomicAdd(d.counter, 1);
-        __syncthreads();
-        const int b = s_b;
-        __syncthreads();
-        if (b >= n_bundles) break;
-        const int4 bu = bundles[b];     // {first task, tasks, group size, 0}
-        const int T = bu.z;
-        const int g = tid / T;
-        if (g < bu.y) {
-            const TileGroup G{g, tid - g * T, T};
-            batch_task<K>(d, Y, params, out, accumulate != 0, tasks[bu.x + g], red + g * T, sm, G);
-        }
-        __syncthreads();
-    }
+    __shared__ SlotShared sm;
+    const int4 bu = bundles[blockIdx.x];     // {first task, tasks, group size, 0}
+    const int T = bu.z;
+    const int g = threadIdx.x / T;
+    if (g >= bu.y) return;                   // whole groups
+    const TileGroup G{g, static_cast<int>(threadIdx.x) - g * T, T};
+    batch_task<K, NP>(d, Y, params, out, accumulate != 0, tasks[bu.x + g], sm, G);
 }
 
 template <int K>
@@ -623,37 +735,36 @@ cudaError_t main_k(const BatchDev& d, const double* Y, const pbe_batch_cell_para
                    double* out, bool accumulate, const int4* bundles, const int4* tasks,
                    int n_bundles, cudaStream_t s)
 {
-    const size_t smem = sizeof(double) * TileSlots<true>::rows * kMainThreads;
-    cudaError_t e = cudaMemsetAsync(d.counter, 0, sizeof(int), s);
-    if (e != cudaSuccess) return e;
     if (n_bundles <= 0) return cudaSuccess;
-    const int grid = n_bundles < PBE_BATCH_CTAS * d.num_sms ? n_bundles : PBE_BATCH_CTAS * d.num_sms;
-    batch_main_kernel<K><<<grid, kMainThreads, smem, s>>>(d, Y, params, out, accumulate ? 1 : 0,
-                                                          bundles, tasks, n_bundles);
+    if (d.A)
+        batch_main_kernel<K, 2><<<n_bundles, kMainThreads, 0, s>>>(d, Y, params, out, accumulate ? 1 : 0,
+                                                                   bundles, tasks);
+    else
+        batch_main_kernel<K, 1><<<n_bundles, kMainThreads, 0, s>>>(d, Y, params, out, accumulate ? 1 : 0,
+                                                                   bundles, tasks);
     return cudaGetLastError();
 }
 
-template <int K>
-cudaError_t attr_k()
+// Launch shape of the per-cell prep kernels: a cluster of d.prep_ranks CTAs of
+// d.prep_threads threads per cell (prep_shape).
+template <class... P, class... A>
+cudaError_t launch_prep(const BatchDev& d, void (*kern)(P...), cudaStream_t s, A... args)
 {
-    return cudaFuncSetAttribute(batch_main_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(sizeof(double) * TileSlots<true>::rows * kMainThreads));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(d.n_cells) * static_cast<unsigned>(d.prep_ranks));
+    cfg.blockDim = dim3(static_cast<unsigned>(d.prep_threads));
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = static_cast<unsigned>(d.prep_ranks);
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 } // namespace
-
-cudaError_t batch_kernel_setup(int kernel)
-{
-    switch (kernel < 0 ? 0 : kernel) {
-    case 0: return attr_k<0>();
-    case 1: return attr_k<1>();
-    case 2: return attr_k<2>();
-    case 3: return attr_k<3>();
-    case 4: return attr_k<4>();
-    case 5: return attr_k<5>();
-    default: return cudaErrorInvalidValue;
-    }
-}
 
 cudaError_t batch_grid_tables(const BatchDev& d, const double* t_q, const double* bw_q,
                               int max_grid_n, cudaStream_t s)
@@ -671,23 +782,14 @@ cudaError_t prep_any(const BatchDev& d, double* N, const pbe_batch_cell_params_t
 {
     if (d.n_cells <= 0) return cudaErrorInvalidValue;
     switch (d.kernel < 0 ? 0 : d.kernel) {
-    case 0: batch_prep_kernel<0><<<d.n_cells, 256, 0, s>>>(d, N, params, stage, c, dt6, sc); break;
-    case 1: batch_prep_kernel<1><<<d.n_cells, 256, 0, s>>>(d, N, params, stage, c, dt6, sc); break;
-    case 2: batch_prep_kernel<2><<<d.n_cells, 256, 0, s>>>(d, N, params, stage, c, dt6, sc); break;
-    case 3: batch_prep_kernel<3><<<d.n_cells, 256, 0, s>>>(d, N, params, stage, c, dt6, sc); break;
-    case 4: batch_prep_kernel<4><<<d.n_cells, 256, 0, s>>>(d, N, params, stage, c, dt6, sc); break;
-    case 5: batch_prep_kernel<5><<<d.n_cells, 256, 0, s>>>(d, N, params, stage, c, dt6, sc); break;
+    case 0: return launch_prep(d, batch_prep_kernel<0>, s, d, N, params, stage, c, dt6, sc);
+    case 1: return launch_prep(d, batch_prep_kernel<1>, s, d, N, params, stage, c, dt6, sc);
+    case 2: return launch_prep(d, batch_prep_kernel<2>, s, d, N, params, stage, c, dt6, sc);
+    case 3: return launch_prep(d, batch_prep_kernel<3>, s, d, N, params, stage, c, dt6, sc);
+    case 4: return launch_prep(d, batch_prep_kernel<4>, s, d, N, params, stage, c, dt6, sc);
+    case 5: return launch_prep(d, batch_prep_kernel<5>, s, d, N, params, stage, c, dt6, sc);
     default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
-}
-
-template <int K>
-cudaError_t jvp_prep_k(const BatchDev& d, const double* A, const double* B, const double* G,
-                       const pbe_batch_cell_params_t* params, bool brk, cudaStream_t s)
-{
-    batch_jvp_prep_kernel<K><<<d.n_cells, 256, 0, s>>>(d, A, B, G, params, brk ? 1 : 0);
-    return cudaGetLastError();
 }
 
 __global__ void __launch_bounds__(256)
@@ -758,17 +860,17 @@ cudaError_t batch_sel(const BatchDev& d, const pbe_batch_cell_params_t* params, 
     return cudaGetLastError();
 }
 
-cudaError_t batch_jvp_prep(const BatchDev& d, const double* A, const double* B, const double* G,
-                          const pbe_batch_cell_params_t* params, bool brk, cudaStream_t s)
+cudaError_t batch_jvp_prep(const BatchDev& d, const double* v, const pbe_batch_cell_params_t* params,
+                           cudaStream_t s)
 {
-    if (d.n_cells <= 0) return cudaErrorInvalidValue;
+    if (d.n_cells <= 0 || !d.A) return cudaErrorInvalidValue;
     switch (d.kernel < 0 ? 0 : d.kernel) {
-    case 0: return jvp_prep_k<0>(d, A, B, G, params, brk, s);
-    case 1: return jvp_prep_k<1>(d, A, B, G, params, brk, s);
-    case 2: return jvp_prep_k<2>(d, A, B, G, params, brk, s);
-    case 3: return jvp_prep_k<3>(d, A, B, G, params, brk, s);
-    case 4: return jvp_prep_k<4>(d, A, B, G, params, brk, s);
-    case 5: return jvp_prep_k<5>(d, A, B, G, params, brk, s);
+    case 0: return launch_prep(d, batch_jvp_prep_kernel<0>, s, d, v, params);
+    case 1: return launch_prep(d, batch_jvp_prep_kernel<1>, s, d, v, params);
+    case 2: return launch_prep(d, batch_jvp_prep_kernel<2>, s, d, v, params);
+    case 3: return launch_prep(d, batch_jvp_prep_kernel<3>, s, d, v, params);
+    case 4: return launch_prep(d, batch_jvp_prep_kernel<4>, s, d, v, params);
+    case 5: return launch_prep(d, batch_jvp_prep_kernel<5>, s, d, v, params);
     default: return cudaErrorInvalidValue;
     }
 }
