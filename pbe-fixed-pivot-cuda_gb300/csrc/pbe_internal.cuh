@@ -568,6 +568,7 @@ __host__ __device__ inline int vjp_lane_last_rank(int n, int b, int C)
     }
     return rank;
 }
+constexpr int kVjpMom = 32;
 struct VjpWs {
     double* h;         // [n]  x_i N_i
     double* a;         // [n]  x_i^(1/3)
@@ -577,11 +578,20 @@ struct VjpWs {
     double* Sf;        // [n]  shear factor of lag d (1 + rho)^3 (times x of the smaller member)
     double* Sl;        // [n]  the same times x_0 / x_d: times x of the larger member
     int*    Ld;        // [n]  bracket offset of lag d (as AggWs)
-    double* mom_part;  // [nb_prep * 16] moments of N and lambda*N, max deviation
-    double* mom;       // [16] 0..4 moments of N, 5..9 of lambda*N, 10 geo flag
+    double* mom_part;  // [nb_prep * kVjpMom] block partials of mom
+    double* mom;       // [kVjpMom] 0..4 moments of N, 5..9 of lambda N, 10 geo flag, 11 D0,
+                       // 12..16 of |N|, 17..21 of |lambda N|, 22..26 of u |N| |lambda
+                       // step| (u = 2^-53 x_{i+1} / dx_i: what the rounding of a pair's
+                       // volume moves its weight by, at most)
+    // Sums over the bins with m_q = {1/a, 1, a, a^2, x}_q (as AggWs::mloc, block
+    // offsets in moff): [q n + i] over bins up to i of m_q N, [(5 + q) n + i] of
+    // m_q x N at the exponent of x_i; over bins from i on: [(10 + q) n + i] of
+    // m_q lambda N and [(15 + q) n + i] of m_q N D times 2^E_i, E_i the exponent of x_i
+    double* mloc;      // [4 kMomN n]
+    double* mtot;      // [4 kMomN nb_prep]
+    double* moff;      // [4 kMomN nb_prep]
     double* gpart;     // [max(ntile, n / 8) * 4] per-task / per-block parameter partials
     double* vpart;     // [ntile * kVjpMaxChunks * 2 kTileW] row sums per (tile, partner chunk)
-    int*    ltask;     // [2 lane tasks] lane tasks in launch order, (row block, chunk) pairs
     double* lup;       // [lane tasks * 64] lane-task sums of the rows as smaller members
     double* llo;       // [lane tasks * (C + 32)] lane-task sums of the rows as larger members
     int*    counter;   // [8]: 0 tile tasks, 1 lane tasks
@@ -603,14 +613,17 @@ inline size_t vjp_ws_layout(int n, char* base, VjpWs* ws)
     w.Sf       = reinterpret_cast<double*>(take(dn));
     w.Sl       = reinterpret_cast<double*>(take(dn));
     w.Ld       = reinterpret_cast<int*>(take(sizeof(int) * static_cast<size_t>(n)));
-    w.mom_part = reinterpret_cast<double*>(take(sizeof(double) * 16 * static_cast<size_t>(agg_prep_blocks(n))));
-    w.mom      = reinterpret_cast<double*>(take(sizeof(double) * 16));
+    const size_t nbp = static_cast<size_t>(agg_prep_blocks(n));
+    w.mom_part = reinterpret_cast<double*>(take(sizeof(double) * kVjpMom * nbp));
+    w.mom      = reinterpret_cast<double*>(take(sizeof(double) * kVjpMom));
+    w.mloc     = reinterpret_cast<double*>(take(4 * kMomN * dn));
+    w.mtot     = reinterpret_cast<double*>(take(sizeof(double) * 4 * kMomN * nbp));
+    w.moff     = reinterpret_cast<double*>(take(sizeof(double) * 4 * kMomN * nbp));
     w.gpart    = reinterpret_cast<double*>(take(sizeof(double) * 4 * static_cast<size_t>(ntile > nbb ? ntile : nbb)));
     w.vpart    = reinterpret_cast<double*>(take(sizeof(double) * 2 * kTileW * kVjpMaxChunks *
                                                 static_cast<size_t>(ntile)));
     const int C = vjp_lane_chunk(n);
     const size_t ltasks = static_cast<size_t>(vjp_lane_tasks(n, C));
-    w.ltask    = reinterpret_cast<int*>(take(sizeof(int) * 2 * ltasks));
     w.lup      = reinterpret_cast<double*>(take(sizeof(double) * 2 * kLaneBins * ltasks));
     w.llo      = reinterpret_cast<double*>(take(sizeof(double) * (C + 32) * ltasks));
     w.counter  = reinterpret_cast<int*>(take(sizeof(int) * 8));

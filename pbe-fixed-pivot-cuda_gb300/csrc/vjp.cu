@@ -50,8 +50,9 @@ constexpr int VW = kVW;                 // rows per task
 
 // -------------------------------------------------------------------------
 // prep: per-bin values, lag factors (no beta, no diagonal 1/2), moments of N
-// and lambda*N, geometric deviation. Moment slots per block (stride 16):
-// 0..4 sum N{1/a, 1, a, a^2, x}, 5..9 the same of lambda*N, 10 max dev.
+// and lambda*N, geometric deviation, and the sums over the bins that the lags
+// from D0 on reduce to (VjpWs::mloc). Block partials as VjpWs::mom, the maximum
+// deviation in slot 10 and the smallest D0 candidate in slot 11.
 // Modes: kVjpFull everything; kVjpTables the grid-only part (cube roots, lag
 // tables, bracket offsets, deviation) for callers that keep the workspace for
 // one set of pivots (the RK4 tape); kVjpStage the N- and lambda-dependent
@@ -59,15 +60,53 @@ constexpr int VW = kVW;                 // rows per task
 // -------------------------------------------------------------------------
 enum { kVjpFull = 0, kVjpTables = 1, kVjpStage = 2 };
 
+// Running sums of v over the prep block's bins, from the first up (SUF = false)
+// or from the last down (true); SCALED: each bin's value is relative to 2^E
+// (prefix: the sum at bin i stands at 2^E_i, a term of a lower bin is scaled
+// down; suffix: at 2^-E_i, a term of a higher bin is scaled down).
+template <bool SUF, bool SCALED>
+__device__ __forceinline__ void block_scan(double* v, int E, double* sv, int* se)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    static_assert(kPrepThreads == 64, "two warps");
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int Es = SUF ? __shfl_down_sync(0xffffffffu, E, o) : __shfl_up_sync(0xffffffffu, E, o);
+        const int sh = SUF ? E - Es : Es - E;
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) {
+            const double u = SUF ? __shfl_down_sync(0xffffffffu, v[q], o)
+                                 : __shfl_up_sync(0xffffffffu, v[q], o);
+            if (SUF ? lane + o < 32 : lane >= o) v[q] += SCALED ? scale_down(u, sh) : u;
+        }
+    }
+    __syncthreads();
+    if (SUF ? (w == 1 && lane == 0) : (w == 0 && lane == 31)) {
+        *se = E;
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) sv[q] = v[q];
+    }
+    __syncthreads();
+    if (SUF ? w == 0 : w == 1) {
+        const int sh = SUF ? E - *se : *se - E;
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) v[q] += SCALED ? scale_down(sv[q], sh) : sv[q];
+    }
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(kPrepThreads)
 vjp_prep_kernel(const double* __restrict__ N, const double* __restrict__ x,
                 const double* __restrict__ lam, int n, VjpWs ws)
 {
-    __shared__ double sh[kPrepThreads / 32];
+    __shared__ double sh[kPrepThreads / 32][kVjpMom];
+    __shared__ double sv[kMomN];
+    __shared__ int se;
     __shared__ double ax0_s;
     __shared__ GeoFit fit_s;
     const int i = blockIdx.x * kPrepThreads + threadIdx.x;
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int nb = gridDim.x, b = blockIdx.x;
     if constexpr (MODE != kVjpStage) {
         if (threadIdx.x == 0) {
             ax0_s = cbrt(x[0]);
@@ -75,12 +114,12 @@ vjp_prep_kernel(const double* __restrict__ N, const double* __restrict__ x,
         }
         __syncthreads();
     }
-    double m[10];
-#pragma unroll
-    for (int q = 0; q < 10; ++q) m[q] = 0.0;
     double dev = 0.0;
+    int d0 = n;
+    const double xi = x[min(i, n - 1)];          // bins beyond the last add zeros
+    double w[kMomN] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    double Ni = 0.0, li = 0.0, Di = 0.0, dl = 0.0;
     if (i < n) {
-        const double xi = x[i];
         double ai, iai;
         if constexpr (MODE == kVjpStage) {
             ai = ws.a[i];
@@ -97,100 +136,173 @@ vjp_prep_kernel(const double* __restrict__ N, const double* __restrict__ x,
             ws.Sf[i] = (s * s) * s;
             ws.Sl[i] = (s * s) * s * (x0 / xi);
             const double v = x0 + xi;
-            ws.Ld[i] = (dbits(v) >= dbits(x[n - 1])) ? kLagClipAll : bracket_from(x, n, v, i);
-            // launch order of the lane tasks: entry i < full is a full chunk
-            // (chunk by chunk), entry full + rank(b) row block b's last chunk
-            const int C = vjp_lane_chunk(n);
-            const int full = vjp_lane_full_tasks(n, C);
-            if (i < full) {
-                int r = i, c = 0;
-                for (;;) {
-                    const int cnt = vjp_lane_chunk_blocks(n, c + 1, C);
-                    if (r < cnt) break;
-                    r -= cnt;
-                    ++c;
-                }
-                ws.ltask[2 * i] = r;
-                ws.ltask[2 * i + 1] = c;
-            }
-            if (i < vjp_lane_chunk_blocks(n, 0, C)) {
-                const int dmax = n - 1 - kLaneBins * i;
-                const int k = full + vjp_lane_last_rank(n, i, C);
-                ws.ltask[2 * k] = i;
-                ws.ltask[2 * k + 1] = (dmax + C - 1) / C - 1;
-            }
+            const int L = (dbits(v) >= dbits(x[n - 1])) ? kLagClipAll : bracket_from(x, n, v, i);
+            ws.Ld[i] = L;
+            if (L == i && i > 0) d0 = i;
             if (n >= 2) {
                 dev = geo_dev(fit_s, xi, i);
                 if (!(dev == dev)) dev = 1.0;
             }
         }
         if constexpr (MODE != kVjpTables) {
-            const double Ni = N[i], li = lam[i];
-            ws.h[i] = xi * Ni;
-            ws.D[i] = (i < n - 1) ? (lam[i + 1] - li) / (x[i + 1] - xi) : 0.0;
-            const double w[5] = {iai, 1.0, ai, ai * ai, xi};
-#pragma unroll
-            for (int q = 0; q < 5; ++q) {
-                m[q] = w[q] * Ni;
-                m[5 + q] = w[q] * (li * Ni);
+            Ni = N[i];
+            li = lam[i];
+            if (i < n - 1) {
+                dl = lam[i + 1] - li;
+                Di = dl / (x[i + 1] - xi);
             }
+            ws.h[i] = xi * Ni;
+            ws.D[i] = Di;
+            w[0] = iai; w[1] = 1.0; w[2] = ai; w[3] = ai * ai; w[4] = xi;
         }
     }
     if constexpr (MODE != kVjpTables) {
+        const int E = exponent_of(xi);
+        const double xm = mantissa_of(xi);
+        // the block's share of the moments
+        const double u = (i < n - 1) ? 1.1102230246251565e-16 * (x[i + 1] / (x[i + 1] - xi)) : 0.0;
+        const double c[5] = {Ni, li * Ni, fabs(Ni), fabs(li * Ni), u * fabs(dl * Ni)};
 #pragma unroll
-        for (int q = 0; q < 10; ++q) {
-            const double s = block_sum(m[q], sh);
-            if (threadIdx.x == 0) ws.mom_part[blockIdx.x * 16 + q] = s;
-        }
+        for (int g = 0; g < 5; ++g)
+#pragma unroll
+            for (int q = 0; q < kMomN; ++q) {
+                const double t = warp_sum(w[q] * c[g]);
+                if (lane == 0) sh[wp][(g < 2 ? 5 * g : 2 + 5 * g) + q] = t;
+            }
+        // the sums over the bins
+        double v[kMomN];
+        auto store = [&](int k, int edge) {
+#pragma unroll
+            for (int q = 0; q < kMomN; ++q) {
+                if (i < n) ws.mloc[static_cast<size_t>(k * kMomN + q) * n + i] = v[q];
+                if (i == edge) ws.mtot[(k * kMomN + q) * nb + b] = v[q];
+            }
+        };
+        const int first = b * kPrepThreads, last = min(n - 1, first + kPrepThreads - 1);
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) v[q] = w[q] * Ni;
+        block_scan<false, false>(v, E, sv, &se);
+        store(0, last);
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) v[q] = (w[q] * Ni) * xm;
+        block_scan<false, true>(v, E, sv, &se);
+        store(1, last);
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) v[q] = w[q] * c[1];
+        block_scan<true, false>(v, E, sv, &se);
+        store(2, first);
+        const double ND = Ni * scalbn(Di, E);
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) v[q] = w[q] * ND;
+        block_scan<true, true>(v, E, sv, &se);
+        store(3, first);
     }
     if constexpr (MODE != kVjpStage) {
         dev = warp_max(dev);
-        __syncthreads();
-        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = dev;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double mx = 0.0;
-            for (int w = 0; w < kPrepThreads / 32; ++w) mx = fmax(mx, sh[w]);
-            ws.mom_part[blockIdx.x * 16 + 10] = mx;
-        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) d0 = min(d0, __shfl_xor_sync(0xffffffffu, d0, o));
+        if (lane == 0) { sh[wp][10] = dev; sh[wp][11] = static_cast<double>(d0); }
+    }
+    __syncthreads();
+    if (threadIdx.x < kVjpMom) {
+        const int q = threadIdx.x;
+        const double s0 = sh[0][q], s1 = sh[1][q];
+        const bool grid_only = q == 10 || q == 11;
+        if (q < 27 && (MODE == kVjpFull || (MODE == kVjpTables) == grid_only))
+            ws.mom_part[b * kVjpMom + q] = q == 10 ? fmax(s0, s1) : q == 11 ? fmin(s0, s1) : s0 + s1;
     }
 }
 
-// One block: the reductions over the prep blocks' partials, one per warp and
-// round (lanes stride over the blocks, fixed butterflies): the ten moments
-// (kVjpFull, kVjpStage) and the geometric flag (kVjpFull, kVjpTables); resets
-// the task counters (kVjpFull, kVjpStage).
+// One block: the reductions over the prep blocks' partials, spread over the
+// warps: warps 0..3 scan the block totals of the four groups of sums into
+// offsets (each lane a run of consecutive blocks, a warp scan over the runs);
+// warps 4..7 the moments (kVjpFull, kVjpStage), the geometric flag and D0
+// (kVjpFull, kVjpTables), lanes striding over the blocks, fixed butterflies.
+// Resets the task counters (kVjpFull, kVjpStage).
 template <int MODE>
 __global__ void __launch_bounds__(256)
 vjp_fin_kernel(const double* __restrict__ x, int n, VjpWs ws)
 {
-    __shared__ double mx_s;
     const int nb = (n + kPrepThreads - 1) / kPrepThreads;
     const int wq = threadIdx.x >> 5, lq = threadIdx.x & 31;
-    for (int r = wq; r < 11; r += 8) {
-        double t = 0.0;
-        if (r < 10) {
-            if (MODE == kVjpTables) continue;
-            for (int b = lq; b < nb; b += 32) t += ws.mom_part[b * 16 + r];
-            t = warp_sum(t);
-            if (lq == 0) ws.mom[r] = t;
-        } else {
-            if (MODE == kVjpStage) continue;
-            for (int b = lq; b < nb; b += 32) t = fmax(t, ws.mom_part[b * 16 + 10]);
-            t = warp_max(t);
-            if (lq == 0) mx_s = t;
+    if (wq < 4) {
+        if (MODE == kVjpTables) return;
+        const bool suf = wq >= 2, scaled = (wq & 1) != 0;
+        const int per = (nb + 31) / 32;
+        const int k0 = min(nb, lq * per), k1 = min(nb, k0 + per);
+        // k-th block in the scan's direction, and the exponent its total stands at
+        auto blk = [&](int k) { return suf ? nb - 1 - k : k; };
+        auto tag = [&](int k) {
+            const int b = blk(k);
+            return exponent_of(__ldg(x + (suf ? b * kPrepThreads : min(n - 1, (b + 1) * kPrepThreads - 1))));
+        };
+        auto shift = [&](double v, int from, int to) {
+            return scaled ? scale_down(v, suf ? to - from : from - to) : v;
+        };
+        const double* tot = ws.mtot + static_cast<size_t>(wq) * kMomN * nb;
+        double* off = ws.moff + static_cast<size_t>(wq) * kMomN * nb;
+        const int e0 = k0 > 0 ? tag(k0 - 1) : tag(0), e1 = k1 > 0 ? tag(k1 - 1) : e0;
+        double S[kMomN], R[kMomN];
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) S[q] = 0.0;
+        int e = e0;
+        for (int k = k0; k < k1; ++k) {
+            const int en = tag(k);
+#pragma unroll
+            for (int q = 0; q < kMomN; ++q) S[q] = shift(S[q], e, en) + tot[q * nb + blk(k)];
+            e = en;
         }
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) R[q] = S[q];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int es = __shfl_up_sync(0xffffffffu, e1, o);
+#pragma unroll
+            for (int q = 0; q < kMomN; ++q) {
+                const double r = __shfl_up_sync(0xffffffffu, R[q], o);
+                if (lq >= o) R[q] += shift(r, es, e1);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) {
+            const double r = __shfl_up_sync(0xffffffffu, R[q], 1);
+            S[q] = lq > 0 ? r : 0.0;
+        }
+        e = e0;
+        for (int k = k0; k < k1; ++k) {
+            const int en = tag(k);
+#pragma unroll
+            for (int q = 0; q < kMomN; ++q) {
+                off[q * nb + blk(k)] = S[q];
+                S[q] = shift(S[q], e, en) + tot[q * nb + blk(k)];
+            }
+            e = en;
+        }
+        return;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        if (MODE != kVjpStage) {
+    for (int r = wq - 4; r < 27; r += 4) {
+        double t = 0.0;
+        if (r == 10 || r == 11) {
+            if (MODE == kVjpStage) continue;
+            if (r == 11) t = static_cast<double>(n);
+            for (int b = lq; b < nb; b += 32) {
+                const double v = ws.mom_part[b * kVjpMom + r];
+                t = r == 10 ? fmax(t, v) : fmin(t, v);
+            }
+            t = r == 10 ? warp_max(t) : -warp_max(-t);
+            // the largest deviation decides the geometric flag
             const bool ratio_ok = n >= 2 && x[1] <= 64.0 * x[0];
-            ws.mom[10] = (n >= 2 && mx_s <= kGeoTol && ratio_ok) ? 1.0 : 0.0;
+            if (r == 10) t = (n >= 2 && t <= kGeoTol && ratio_ok) ? 1.0 : 0.0;
+        } else {
+            if (MODE == kVjpTables) continue;
+            for (int b = lq; b < nb; b += 32) t += ws.mom_part[b * kVjpMom + r];
+            t = warp_sum(t);
         }
-        if (MODE != kVjpTables) {
-            ws.counter[0] = 0;
-            ws.counter[1] = 0;
-        }
+        if (lq == 0) ws.mom[r] = t;
+    }
+    if (threadIdx.x == 128 && MODE != kVjpTables) {
+        ws.counter[0] = 0;
+        ws.counter[1] = 0;
     }
 }
 
@@ -303,9 +415,11 @@ __global__ void __launch_bounds__(128) vjp_gfin_kernel(int ntile, VjpWs ws, doub
 // every lane's W at the end of the share. Brownian + shear: 7 FP64
 // instructions per pair (P; P Bf, P Sf; two sums of the smaller member; two
 // FMAs into W) against 8 for the two visits of the tile path.
-// Tasks (row block, lag chunk) run largest first from the prep's launch-order
-// table. Determinism: the windows of the CTA's warps are added in warp order;
-// the rows kernel adds the tasks' sums in a fixed order.
+// Only the lags below D0: from there on every pair lands on its larger member's
+// own slot, lo = k, and the sums separate (vjp_lane_rows_kernel).
+// Tasks (row block, lag chunk) run chunk by chunk; all but the lowest-lag rows'
+// have equal length. Determinism: the windows of the CTA's warps are added in
+// warp order; the rows kernel adds the tasks' sums in a fixed order.
 // -------------------------------------------------------------------------
 #ifndef PBE_VJP_LANE_CTAS
 #define PBE_VJP_LANE_CTAS 3
@@ -320,7 +434,7 @@ constexpr int kVLaneMaxChunks = 64;        // vjp_lane_chunks(n, C) bound
 template <int K>
 __global__ void __launch_bounds__(kMainThreads, kVLaneCtas)
 vjp_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
-                const double* __restrict__ lam, VjpWs ws, int n, int ntasks, int C,
+                const double* __restrict__ lam, VjpWs ws, int n, int C,
                 double b0, double bbr, double bsh)
 {
     extern __shared__ double esm[];               // [kLaneWarps][per_max + 32] W windows
@@ -335,21 +449,27 @@ vjp_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
     const double lamlast = lam[n - 1];
     const int ew = (C + kLaneWarps - 1) / kLaneWarps + 32;
     double* eb = esm + w * ew;
+    const int Dm = static_cast<int>(ws.mom[11]);
 
     for (;;) {
         if (tid == 0) s_task = atomicAdd(ws.counter + 1, 1);
         __syncthreads();
         const int task = s_task;
         __syncthreads();
-        if (task >= ntasks) break;
-        // largest first (the prep's launch order); the sums are stored under the
-        // chunk-major index sum_{c' < c} blocks(c') + b that the rows kernel reads
-        const int b = __ldg(ws.ltask + 2 * task), c = __ldg(ws.ltask + 2 * task + 1);
-        int tix = b;
-        for (int q = 0; q < c; ++q) tix += vjp_lane_chunk_blocks(n, q, C);
+        // task `task` of the chunk-major order: chunk c of row block b (lags
+        // 1 + c C and up, below D0); tix is also where the rows kernel finds its sums
+        int b = task, c = 0;
+        while (1 + c * C < Dm) {
+            const int cnt = vjp_lane_chunk_blocks(n, c, C);
+            if (cnt == 0 || b < cnt) break;
+            b -= cnt;
+            ++c;
+        }
+        if (1 + c * C >= Dm || vjp_lane_chunk_blocks(n, c, C) == 0) break;
+        const int tix = task;
         const int J = kLaneBins * b;
         const int dA = 1 + c * C;
-        const int dB = min(dA + C, n - J);        // lags [dA, dB), dB - 1 <= n - 1 - J
+        const int dB = min(min(dA + C, n - J), Dm);   // lags [dA, dB), dB - 1 <= n - 1 - J
         const int len = dB - dA;
         const int per = (len + kLaneWarps - 1) / kLaneWarps;
         const int dw0 = dA + w * per;
@@ -435,7 +555,7 @@ vjp_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
         // the task's window: entry i is row J + dA - 1 + i, i < len + 32; warp q's
         // window starts at i = q per and holds its share's length + 32 entries
         double* seg = ws.llo + static_cast<size_t>(tix) * (C + 32);
-        for (int i = tid; i < len + 32; i += kMainThreads) {
+        for (int i = tid; i < C + 32; i += kMainThreads) {   // zeros beyond len + 32
             double sum = 0.0;
             for (int q = 0; q < kLaneWarps; ++q) {
                 const int q0 = q * per, q1 = min(len, q0 + per);
@@ -449,16 +569,51 @@ vjp_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
     }
 }
 
+// Sums over the bins (VjpWs::mloc) at bin i: group k's five values; for the
+// scaled groups at i's exponent.
+template <bool SUF, bool SCALED>
+__device__ __forceinline__ void bin_sums(const VjpWs& ws, const double* __restrict__ x, int n, int k,
+                                         int i, double* v)
+{
+    const int nb = agg_prep_blocks(n), b = i / kPrepThreads;
+    int sh = 0;
+    if (SCALED) {
+        const int ib = SUF ? (b + 1) * kPrepThreads : b * kPrepThreads - 1;   // the neighbour block's edge
+        const int eb = ib >= 0 && ib < n ? exponent_of(__ldg(x + ib)) : 0, ei = exponent_of(__ldg(x + i));
+        sh = SUF ? ei - eb : eb - ei;
+        if (ib < 0 || ib >= n) sh = 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kMomN; ++q) {
+        const double o = ws.moff[(k * kMomN + q) * nb + b];
+        v[q] = ws.mloc[static_cast<size_t>(k * kMomN + q) * n + i] + (SCALED ? scale_down(o, sh) : o);
+    }
+}
+
 // Rows of the lane path: one CTA per row block b (rows 32 b + lane). Warp g
 // adds the larger-member sums of the row blocks b' = g, g + 32, ... <= b (the
 // chunk holding lag d = m - 32 b' and, for the first 32 lags of a chunk, the
 // tail of the chunk before); warp 0 adds the 32 in order, the block's own
-// smaller-member sums chunk by chunk, the diagonal pair, the death moments,
-// and stores dL/dN_m and the block's parameter partials.
+// smaller-member sums chunk by chunk, the diagonal pair, the lags from D0 on,
+// the death moments, and stores dL/dN_m and the block's parameter partials.
+//
+// Lags from D0 on: lo = k and fl(x_j + x_k) - x_k is x_j up to the sum's
+// rounding, so P = lambda_k + x_j D_k and, with beta a sum of products of powers
+// of x_j and x_k, row m's sums are
+//   as the larger member   lambda_m beta[P(m - D0)] + D_m beta[T(m - D0)]
+//   as the smaller member  beta[SL(m + D0)] + x_m beta[SD(m + D0)]
+// (beta[M]: the death polynomial at x_m; P, T the moments of N and x N over the
+// bins up to an index, SL, SD those of lambda N and D N from an index up).
+// Leaving out the rounding changes P by at most u_k |lambda_{k+1} - lambda_k|,
+// u_k = 2^-53 x_{k+1}/dx_k. Bounded over all partners with the moments of
+// |N|, |lambda N| and u |N| |lambda step|, it may move a row by at most
+// kVjpGuard of the row's sum of |terms|; rows where it could (a lambda that is
+// nonzero on few bins) take their lags from D0 on pair by pair.
 #ifndef PBE_VROWS_WARPS
-#define PBE_VROWS_WARPS 32
+#define PBE_VROWS_WARPS 16
 #endif
 constexpr int kVRowsWarps = PBE_VROWS_WARPS;
+constexpr double kVjpGuard = 5e-13;
 
 template <int K>
 __global__ void __launch_bounds__(kVRowsWarps * 32)
@@ -468,11 +623,16 @@ vjp_lane_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
 {
     __shared__ double lw[kVRowsWarps][kLaneBins];
     __shared__ int base[kVLaneMaxChunks + 1];
+    __shared__ double xs3[3][kLaneBins];           // exact rows: larger-member sum, smaller-member sums
+    __shared__ double red[kVRowsWarps];
+    __shared__ unsigned exact_s;
     if (ws.mom[10] == 0.0) return;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b = gridDim.x - 1 - blockIdx.x;      // top row blocks (the most lower blocks) first
     const int m = kLaneBins * b + lane;
-    const int nchunks = vjp_lane_chunks(n, C);
+    const int Dm = static_cast<int>(ws.mom[11]);   // lags below Dm were summed pair by pair
+    int nchunks = 0;                               // chunks that hold such lags
+    while (nchunks < kVLaneMaxChunks && 1 + nchunks * C < Dm && vjp_lane_chunk_blocks(n, nchunks, C) > 0) ++nchunks;
     if (threadIdx.x == 0) {
         int sacc = 0;
         for (int c = 0; c < nchunks; ++c) {
@@ -480,14 +640,35 @@ vjp_lane_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
             sacc += vjp_lane_chunk_blocks(n, c, C);
         }
     }
+    // rows that take the lags from D0 on pair by pair
+    if (w == 0) {
+        bool ex = false;
+        if (m < n && (m >= Dm || m + Dm < n)) {
+            const double xm = x[m], am = ws.a[m], iam = ws.ia[m];
+            const double c0 = fabs(b0), c1 = fabs(bbr), c2 = fabs(bsh);
+            const double A = death_factor<K>(xm, am, iam, ws.mom + 12, c0, c1, c2);
+            const double AL = death_factor<K>(xm, am, iam, ws.mom + 17, c0, c1, c2);
+            double err = death_factor<K>(xm, am, iam, ws.mom + 22, c0, c1, c2);
+            if (m < n - 1) {
+                const double xu = x[m + 1];
+                err = fma(1.1102230246251565e-16 * (xu / (xu - xm)) * fabs(lam[m + 1]), A, err);
+            }
+            ex = err > kVjpGuard * fma(fabs(lam[m]), A, AL);
+        }
+        const unsigned em = __ballot_sync(0xffffffffu, ex);
+        if (lane == 0) exact_s = em;
+    }
     __syncthreads();
+    const unsigned exact = exact_s;
     const size_t S = static_cast<size_t>(C) + 32;
     double acc = 0.0;
-    if (m < n) {
-        // the loads of several row blocks in flight: addresses do not depend on acc
+    if (m < n && nchunks > 0) {
+        // the loads of several row blocks in flight: addresses do not depend on acc.
+        // Lower blocks whose window reaches row m: lags d < Dm + 32
         const float invC = 1.0f / static_cast<float>(C);
+        const int bp0 = max(0, (kLaneBins * b - Dm) / kLaneBins - 1);
 #pragma unroll 4
-        for (int bp = w; bp <= b; bp += kVRowsWarps) {
+        for (int bp = bp0 + w; bp <= b; bp += kVRowsWarps) {
             const int d = m - kLaneBins * bp;
             // c1 = d / C: the float quotient, corrected by one either way
             int c1 = __float2int_rz(static_cast<float>(d) * invC);
@@ -496,15 +677,51 @@ vjp_lane_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
             const int idx = d - c1 * C;
             double v = 0.0;
             if (d >= 1) {
-                if (c1 >= 1 && idx < 32) v = __ldcg(ws.llo + (base[c1 - 1] + bp) * S + C + idx);
+                if (c1 >= 1 && idx < 32 && c1 - 1 < nchunks)
+                    v = __ldcg(ws.llo + (base[c1 - 1] + bp) * S + C + idx);
                 // chunk c1 exists for block bp when its first lag 1 + c1 C <= n - 1 - 32 bp
-                if (1 + c1 * C <= n - 1 - kLaneBins * bp) v += __ldcg(ws.llo + (base[c1] + bp) * S + idx);
+                if (c1 < nchunks && 1 + c1 * C <= n - 1 - kLaneBins * bp)
+                    v += __ldcg(ws.llo + (base[c1] + bp) * S + idx);
             }
             acc += v;
         }
     }
     lw[w][lane] = acc;
     __syncthreads();
+
+    // exact rows, one after the other: the CTA over the partners, fixed order
+    for (unsigned em = exact; em != 0u; em &= em - 1u) {
+        const int le = __ffs(em) - 1, r = kLaneBins * b + le;
+        const double xr = x[r], Dr = ws.D[r], lr = lam[r];
+        const EwOperandA ar = ew_operand_a(xr);
+        const EwOperandB br = ew_operand_b(xr);
+        const EwOperandC cr = ew_operand_c(xr, 0);
+        double W = 0.0, U0 = 0.0, U1 = 0.0;
+        for (int j = threadIdx.x; j <= r - Dm; j += kVRowsWarps * 32) {     // r the larger member
+            const int d = r - j;
+            const double P = r < n - 1 ? fma(sum_minus_scaled_pre(ar, x[j], cr), Dr, lr) : lr;
+            if constexpr (K == 0) W = fma(P, b0 * N[j], W);
+            if constexpr (K == 1) W = fma(P, b0 * fma(N[j], xr, ws.h[j]), W);
+            if constexpr (K == 2) W = fma(P * xr, b0 * ws.h[j], W);
+            if constexpr (K == 3 || K == 5) W = fma(P * ws.Bf[d], bbr * N[j], W);
+            if constexpr (K == 4 || K == 5) W = fma(P * ws.Sf[d], bsh * ws.h[j], W);
+        }
+        for (int k = r + Dm + threadIdx.x; k < n; k += kVRowsWarps * 32) {  // r the smaller member
+            const int d = k - r;
+            const double xk = x[k], Nk = N[k];
+            double P = lam[k];
+            if (k < n - 1)
+                P = fma(sum_minus_scaled_dec(ew_operand_a(xk), br, ew_operand_c(xk, 0)), ws.D[k], P);
+            if constexpr (K == 0) U0 = fma(P, Nk, U0);
+            if constexpr (K == 1) U0 = fma(P, fma(xr, Nk, ws.h[k]), U0);
+            if constexpr (K == 2) U0 = fma(P, xr * ws.h[k], U0);
+            if constexpr (K == 3 || K == 5) U0 = fma(P * ws.Bf[d], Nk, U0);
+            if constexpr (K == 4 || K == 5) U1 = fma(P * ws.Sf[d], xr * Nk, U1);
+        }
+        const double t[3] = {block_sum(W, red), block_sum(U0, red), block_sum(U1, red)};
+        if (threadIdx.x < 3) xs3[threadIdx.x][le] = t[threadIdx.x];
+        __syncthreads();
+    }
     if (w != 0) return;
 
     double gB = 0.0, gS = 0.0;
@@ -512,7 +729,7 @@ vjp_lane_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
         double Wm = 0.0;
 #pragma unroll
         for (int q = 0; q < kVRowsWarps; ++q) Wm += lw[q][lane];
-        const int dmax = n - 1 - kLaneBins * b;
+        const int dmax = min(n - 1 - kLaneBins * b, Dm - 1);
         const int nchb = dmax >= 1 ? (dmax + C - 1) / C : 0;
         double U0 = 0.0, U1 = 0.0;
         for (int c = 0; c < nchb; ++c) {
@@ -543,6 +760,37 @@ vjp_lane_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
         if constexpr (K == 2) { Tv0 = xm * U0; Td0 = xm * d0; }
         if constexpr (K == 4 || K == 5) { Tv1 = xm * U1; Td1 = xm * d1; }
         const double am = ws.a[m], iam = ws.ia[m];
+        // the lags from D0 on
+        if ((exact >> lane) & 1u) {
+            Wm += xs3[0][lane];
+            Tv0 += xs3[1][lane];
+            Tv1 += xs3[2][lane];
+        } else {
+            const int Em = exponent_of(xm);
+            if (m >= Dm) {
+                double p[kMomN], t[kMomN];
+                bin_sums<false, false>(ws, x, n, 0, m - Dm, p);
+                Wm = fma(lm, death_factor<K>(xm, am, iam, p, b0, bbr, bsh), Wm);
+                if (m < n - 1) {
+                    bin_sums<false, true>(ws, x, n, 1, m - Dm, t);
+                    const double ft = death_factor<K>(xm, am, iam, t, b0, bbr, bsh);
+                    Wm += scale_down(scalbn(ws.D[m], Em) * ft, exponent_of(x[m - Dm]) - Em);
+                }
+            }
+            if (m + Dm < n) {
+                double sl[kMomN], sd[kMomN];
+                bin_sums<true, false>(ws, x, n, 2, m + Dm, sl);
+                bin_sums<true, true>(ws, x, n, 3, m + Dm, sd);
+                const int sh = Em - exponent_of(x[m + Dm]);
+                const double xmm = mantissa_of(xm);
+                if constexpr (K != 4)
+                    Tv0 += moment_factor<K, 0>(xm, am, iam, sl) +
+                           scale_down(xmm * moment_factor<K, 0>(xm, am, iam, sd), sh);
+                if constexpr (K == 4 || K == 5)
+                    Tv1 += moment_factor<K, 1>(xm, am, iam, sl) +
+                           scale_down(xmm * moment_factor<K, 1>(xm, am, iam, sd), sh);
+            }
+        }
         const double* M = ws.mom;
         const double* Lm = ws.mom + 5;
         double g = Wm;
@@ -699,8 +947,7 @@ cudaError_t agg_vjp_k(const AggVjpArgs& a, const VjpWs& ws, int num_sms, cudaStr
     if (lane_on) {
         const size_t lsmem = sizeof(double) * kLaneWarps * ((C + kLaneWarps - 1) / kLaneWarps + 32);
         const int lgrid = static_cast<int>(ltasks < kVLaneCtas * num_sms ? ltasks : kVLaneCtas * num_sms);
-        vjp_lane_kernel<K><<<lgrid, kMainThreads, lsmem, s>>>(a.N, a.x, a.lam, ws, n,
-                                                              static_cast<int>(ltasks), C,
+        vjp_lane_kernel<K><<<lgrid, kMainThreads, lsmem, s>>>(a.N, a.x, a.lam, ws, n, C,
                                                               a.beta0, a.beta_br, a.beta_sh);
     }
     vjp_main_kernel<K><<<grid, kMainThreads, smem, s>>>(a.N, a.x, a.lam, ws, n, ntile, nch, lane_on);
