@@ -23,10 +23,11 @@ __device__ __forceinline__ constexpr bool need_moment(int q)
 constexpr double kMomGuard = 2.5e-13;
 
 // The slot's lags from D0 on must be summed pair by pair (see the file header):
-// u |N_s| > kMomGuard |N_{s+1}|, u = 2^-53 x_{s+1} / dx_s.
+// u |N_s| > kMomGuard |N_{s+1}|, u = 2^-53 x_{s+1} / dx_s (2^53 on the other
+// side, so that no product underflows for subnormal N).
 __device__ __forceinline__ bool mom_exact_slot(double Ns, double Nup, double xup, double inv_dx)
 {
-    return fabs(Nup) * kMomGuard < (1.1102230246251565e-16 * (xup * inv_dx)) * fabs(Ns);
+    return fabs(Nup) * (kMomGuard * 9007199254740992.0) < (xup * inv_dx) * fabs(Ns);
 }
 
 } // namespace pbe_gb300

@@ -1,6 +1,7 @@
 // =============================================================================
 // agg_slot.cuh -- aggregation pair sums with one output slot per lane, for any
-// grid: the pair work of the batched kernel (batch_kernels.cu).
+// grid: the pair work of the batched kernel (batch_kernels.cu) and, on grids that
+// are not geometric, of the single-instance kernel (agg_lane.cuh).
 //
 // Slot s collects the pairs (j <= k) whose bracket is lo = s: R_s = sum rate,
 // TH_s = sum rate (fl(x_j + x_k) - x_s) 2^St_s, St_s = -exponent of x_s
@@ -26,12 +27,14 @@
 // =============================================================================
 #pragma once
 
-#include "agg_tile.cuh"
+#include "agg_rates.cuh"
 #include "agg_moments.cuh"
 
 namespace pbe_gb300 {
 
-// The grid of a cell (its first n pivots) and the cell's coefficients.
+// The grid of a cell (its first n pivots) and the cell's coefficients. The lag
+// factors carry the coefficients in single-instance use (Nj = a_j, Hj = x_j a_j
+// then), and not in batched use.
 struct SlotGrid {
     const double* x;
     const double* a;        // x^(1/3)
@@ -184,20 +187,20 @@ __device__ __forceinline__ void slot_pairs_any(const SlotGrid& g, const SlotPass
     }
 }
 
-// The prefix part of slot s pair by pair, by one warp (lanes over j, fixed
-// butterfly): for the slots of mom_exact_slot. Valid in every lane.
+// Thread tid of nt's share of the prefix part of slot s, pair by pair: for the
+// slots of mom_exact_slot.
 template <int K, int NP>
-__device__ __forceinline__ void slot_exact(const SlotGrid& g, const SlotPass* p, int s, double& R,
-                                           double& TH)
+__device__ __forceinline__ void slot_exact_part(const SlotGrid& g, const SlotPass* p, int s, int tid,
+                                                int nt, double& r, double& t)
 {
-    const int lane = threadIdx.x & 31;
     const double xs = __ldg(g.x + s);
     const int St = -exponent_of(xs);
     const EwOperandA pa = ew_operand_a(xs);
     const EwOperandC pc = ew_operand_c(xs, St);
     const int cut = slot_cut(g, s);
-    double r = 0.0, t = 0.0;
-    for (int j = lane; j < cut; j += 32) {
+    r = 0.0;
+    t = 0.0;
+    for (int j = tid; j < cut; j += nt) {
         double rate, th;
         if (g.geo) {
             const int d = s - j;
@@ -215,6 +218,15 @@ __device__ __forceinline__ void slot_exact(const SlotGrid& g, const SlotPass* p,
         r += rate;
         t = fma(rate, th, t);
     }
+}
+
+// The same by one warp, summed by a fixed butterfly. Valid in every lane.
+template <int K, int NP>
+__device__ __forceinline__ void slot_exact(const SlotGrid& g, const SlotPass* p, int s, double& R,
+                                           double& TH)
+{
+    double r, t;
+    slot_exact_part<K, NP>(g, p, s, threadIdx.x & 31, 32, r, t);
     R = warp_sum(r);
     TH = warp_sum(t);
 }

@@ -15,7 +15,7 @@
 // least-squares problem is updated with Givens rotations by thread 0.
 // =============================================================================
 #include "batch_internal.cuh"
-#include "agg_tile.cuh"
+#include "agg_rates.cuh"
 
 namespace pbe_gb300 {
 namespace {

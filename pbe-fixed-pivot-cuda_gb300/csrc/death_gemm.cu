@@ -24,7 +24,7 @@
 // this form is measured beside the moment form rather than used by the RHS.
 // =============================================================================
 #include "batch_internal.cuh"
-#include "agg_tile.cuh"
+#include "agg_rates.cuh"
 
 namespace pbe_gb300 {
 namespace {

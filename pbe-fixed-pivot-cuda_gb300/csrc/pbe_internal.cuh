@@ -19,12 +19,11 @@
 namespace pbe_gb300 {
 
 // ---- launch geometry --------------------------------------------------------
-constexpr int kTileW        = 12;    // output bins owned by one task (125 regs, no spill)
+constexpr int kTileW        = 12;    // rows of a VJP row-tile task
 constexpr int kMainThreads  = 256;   // threads per aggregation task CTA
-constexpr int kPrepThreads  = 64;    // per-bin prep kernels: small blocks spread the
+constexpr int kPrepThreads  = 64;    // bins of a prep block: small blocks spread the
                                      // cube roots and divisions over every SM
 constexpr int kMaxClipTasks = 32;    // tasks summing the pairs clipped at x[n-1]
-constexpr int kRedRows      = 2 * (kTileW + 1);   // R[0..W], TH[0..W]
 
 // A grid is treated as geometric when |log(x_i/x_0) - i*log(r)| <= kGeoTol for
 // every i (r fitted from the end points). Then the pivot ratio x_{j+d}/x_j
@@ -51,13 +50,12 @@ struct GeoFit {
     double s_lo;     // step, low part
 };
 
-__device__ __forceinline__ GeoFit geo_fit(double x0, double xl, int n)
+// From the end points' exponents and the log2 of their mantissas.
+__device__ __forceinline__ GeoFit geo_fit_from(int E0, double f0, int El, double fl, int n)
 {
     GeoFit g;
-    g.E0 = ilogb(x0);
-    g.f0 = log2(scalbn(x0, -g.E0));
-    const int El = ilogb(xl);
-    const double fl = log2(scalbn(xl, -El));
+    g.E0 = E0;
+    g.f0 = f0;
     const double m = static_cast<double>(n > 1 ? n - 1 : 1);
     const double L_hi = static_cast<double>(El) - static_cast<double>(g.E0);   // exact
     const double L_lo = fl - g.f0;
@@ -67,17 +65,26 @@ __device__ __forceinline__ GeoFit geo_fit(double x0, double xl, int n)
     return g;
 }
 
-// |ln(x_i / x_0) - i ln r| for the fitted r (natural-log units).
-__device__ __forceinline__ double geo_dev(const GeoFit& g, double xi, int i)
+__device__ __forceinline__ GeoFit geo_fit(double x0, double xl, int n)
 {
-    const int Ei = ilogb(xi);
-    const double fi = log2(scalbn(xi, -Ei));
+    const int E0 = ilogb(x0), El = ilogb(xl);
+    return geo_fit_from(E0, log2(scalbn(x0, -E0)), El, log2(scalbn(xl, -El)), n);
+}
+
+// |ln(x_i / x_0) - i ln r| for the fitted r (natural-log units).
+__device__ __forceinline__ double geo_dev_from(const GeoFit& g, int Ei, double fi, int i)
+{
     const double di = static_cast<double>(i);
     const double p_hi = di * g.s_hi;
     const double p_lo = fma(di, g.s_hi, -p_hi) + di * g.s_lo;
     const double dev2 = ((static_cast<double>(Ei) - static_cast<double>(g.E0)) - p_hi)
                       + ((fi - g.f0) - p_lo);
     return fabs(dev2) * 0.6931471805599453;
+}
+__device__ __forceinline__ double geo_dev(const GeoFit& g, double xi, int i)
+{
+    const int Ei = ilogb(xi);
+    return geo_dev_from(g, Ei, log2(scalbn(xi, -Ei)), i);
 }
 
 // v * 2^s for a normal (or zero) double, by adding s to the exponent field:
@@ -260,14 +267,15 @@ struct AggWs {
     double* mom_part;  // [nb_prep * 8] per-block moment partials
     double* mom;       // [8]  M_{-1/3}, M_0, M_{1/3}, M_{2/3}, M_1, geo flag, max dev
     double* clip_part; // [kMaxClipTasks] sums of clipped pair rates, one per clip task
-    double* tfirst;    // [ntile] gather mode: tile's own value of its first bin
-    double* tcarry;    // [ntile] gather mode: the lower neighbour's carry into that bin
-    int*    tticket;   // [ntile] contributors to the tile's first bin done (0, 1, 2)
-    double* cpart;     // [ntile * agg_chunk_bound(n) * 2 kTileW] lag-chunk partials of R, TH
-    int*    cticket;   // [ntile] lag-chunk tasks of the tile done
+    int*    J0;        // [n]  first j with fl(x_j + x_i) >= x_{i+1} (at most i)
+    double* tfirst;    // [nblk] gather mode: block's own value of its first bin
+    double* tcarry;    // [nblk] gather mode: the lower neighbour's carry into that bin
+    int*    tticket;   // [nblk] contributors to the block's first bin done (0, 1, 2)
+    int*    cticket;   // [nblk] tasks of the block done
     int*    counter;   // [8]  [0] task counter, [1] first lag with Ld[d] == d,
                        //      [2] prep blocks done, [3] bin n-1 contributors done,
-                       //      [4] a staging wait of the lane tasks gave up, [5] entries of xlist
+                       //      [4] a staging wait of the lane tasks gave up, [5] entries of xlist,
+                       //      [6] CTAs of the pair kernel done
     double* Ncp;       // [n + 2] copy of N, 256-byte aligned (bulk-copy source)
     double* xcp;       // [n + 2] copy of x, 256-byte aligned (bulk-copy source)
     double* lpart;     // [lane_partial_doubles(n)] lane-task chunk partials
@@ -285,22 +293,6 @@ struct AggWs {
 constexpr int kMomN = 5;               // moments per prefix (the death term's)
 
 __host__ __device__ constexpr int agg_prep_blocks(int n) { return (n + kPrepThreads - 1) / kPrepThreads; }
-__host__ __device__ constexpr int agg_tiles(int n) { return (n + kTileW - 1) / kTileW; }
-
-// Gather mode with few tiles per CTA slot (small n): each tile's lags are cut
-// into chunks of at least kChunkMinLags lags, about kChunkTasks tasks per CTA
-// slot in all, on GPUs of up to kChunkMaxSms SMs; agg_chunk_bound(n) chunks per
-// tile at most (the scratch is sized for it whatever the GPU).
-constexpr int kChunkTasks = 8;
-constexpr int kChunkMaxSms = 256;
-constexpr int kChunkMinLags = 256;
-__host__ __device__ constexpr int agg_chunk_bound(int n)
-{
-    const int a = (n + kChunkMinLags - 1) / kChunkMinLags;
-    const int b = n > 0 ? (2 * kTileW * kChunkTasks * 2 * kChunkMaxSms + n - 1) / n + 1 : 1;
-    const int m = a < b ? a : b;
-    return m < 1 ? 1 : m;
-}
 
 constexpr size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
@@ -408,15 +400,12 @@ __host__ __device__ constexpr size_t lane_partial_doubles(int n)
 constexpr size_t agg_ws_bytes(int n)
 {
     const size_t dn = align256(sizeof(double) * static_cast<size_t>(n));
-    return 6 * dn + align256(sizeof(int) * static_cast<size_t>(n))
+    return 6 * dn + 2 * align256(sizeof(int) * static_cast<size_t>(n))
          + align256(sizeof(double) * 8 * static_cast<size_t>(agg_prep_blocks(n)))
          + align256(sizeof(double) * 8)
          + align256(sizeof(double) * kMaxClipTasks)
-         + 2 * align256(sizeof(double) * static_cast<size_t>(agg_tiles(n)))
-         + align256(sizeof(int) * static_cast<size_t>(agg_tiles(n)))
-         + align256(sizeof(double) * 2 * kTileW * static_cast<size_t>(agg_tiles(n)) *
-                    static_cast<size_t>(agg_chunk_bound(n)))
-         + align256(sizeof(int) * static_cast<size_t>(agg_tiles(n)))
+         + 2 * align256(sizeof(double) * static_cast<size_t>(lane_blocks(n)))
+         + 2 * align256(sizeof(int) * static_cast<size_t>(lane_blocks(n)))
          + align256(sizeof(int) * 8)
          + 2 * align256(sizeof(double) * (static_cast<size_t>(n) + 2))
          + align256(sizeof(double) * lane_partial_doubles(n))
@@ -443,12 +432,11 @@ inline size_t agg_ws_layout(int n, char* base, AggWs* ws)
     w.mom_part  = reinterpret_cast<double*>(take(sizeof(double) * 8 * static_cast<size_t>(agg_prep_blocks(n))));
     w.mom       = reinterpret_cast<double*>(take(sizeof(double) * 8));
     w.clip_part = reinterpret_cast<double*>(take(sizeof(double) * kMaxClipTasks));
-    const size_t nt = static_cast<size_t>(agg_tiles(n));
+    w.J0        = reinterpret_cast<int*>(take(sizeof(int) * static_cast<size_t>(n)));
+    const size_t nt = static_cast<size_t>(lane_blocks(n));
     w.tfirst    = reinterpret_cast<double*>(take(sizeof(double) * nt));
     w.tcarry    = reinterpret_cast<double*>(take(sizeof(double) * nt));
     w.tticket   = reinterpret_cast<int*>(take(sizeof(int) * nt));
-    w.cpart     = reinterpret_cast<double*>(take(sizeof(double) * 2 * kTileW * nt *
-                                                 static_cast<size_t>(agg_chunk_bound(n))));
     w.cticket   = reinterpret_cast<int*>(take(sizeof(int) * nt));
     w.counter   = reinterpret_cast<int*>(take(sizeof(int) * 8));
     w.Ncp       = reinterpret_cast<double*>(take(sizeof(double) * (static_cast<size_t>(n) + 2)));

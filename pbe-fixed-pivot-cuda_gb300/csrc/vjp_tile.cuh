@@ -6,12 +6,12 @@
 // per row m, up to two partner sums of P (the lambda interpolated at the
 // pair's birth volume) times N_k (or x_k N_k) times the lag factor (see
 // vjp.cu for the derivation). It runs on a group of T threads (runtime
-// value, named barrier, like agg_tile.cuh); the T partials of every row are
+// value, named barrier); the T partials of every row are
 // reduced in a fixed order.
 // =============================================================================
 #pragma once
 
-#include "agg_tile.cuh"
+#include "agg_rates.cuh"
 
 namespace pbe_gb300 {
 
