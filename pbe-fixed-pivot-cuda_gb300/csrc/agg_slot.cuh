@@ -66,7 +66,7 @@ __device__ __forceinline__ int slot_cut(const SlotGrid& g, int s)
 {
     if (g.geo) return max(0, s - g.D0 + 1);
     // the clipped slot n - 1 takes every j < n - 1; the diagonal pair is never in
-    return s >= g.n - 1 ? s : min(__ldg(g.J0 + s), s);
+    return s >= g.n - 1 ? s : min(g.J0[s], s);
 }
 
 // Lags [d0, d1) of slot s on a geometric grid (uniform d0, d1, smax across the
@@ -82,7 +82,7 @@ __device__ __forceinline__ void slot_pairs_geo(const SlotGrid& g, const SlotPass
     for (int q = 0; q < NP; ++q) { Q[q] = QT[q] = F[q] = hk[q] = 0.0; }
     int e_cur = -1;
     for (int d = d0; d < d1; ++d) {
-        const int L = __ldg(g.Ld + d);
+        const int L = g.Ld[d];
         if (L > smax) break;
         const int e = L - d;
         if (e != e_cur) {                              // uniform across the warp
@@ -102,7 +102,7 @@ __device__ __forceinline__ void slot_pairs_geo(const SlotGrid& g, const SlotPass
             }
             pa = ew_operand_a(kin ? __ldg(g.x + k) : 0.0);
         }
-        const double B = __ldg(g.Bd + d), S = __ldg(g.Sd + d);
+        const double B = g.Bd[d], S = g.Sd[d];
         const int j = s - L;
         if (slot && j >= 0) {
             const double th = sum_minus_scaled_pre(pa, __ldg(g.x + j), pc);
@@ -135,8 +135,8 @@ __device__ __forceinline__ void slot_pairs_geo(const SlotGrid& g, const SlotPass
 template <int K, int NP>
 __device__ __forceinline__ double slot_rate_any(const SlotGrid& g, const SlotPass* p, int j, int k)
 {
-    const double aj = K >= 3 ? __ldg(g.a + j) : 0.0, iaj = K >= 3 ? __ldg(g.ia + j) : 0.0;
-    const double ak = K >= 3 ? __ldg(g.a + k) : 0.0, iak = K >= 3 ? __ldg(g.ia + k) : 0.0;
+    const double aj = K >= 3 ? g.a[j] : 0.0, iaj = K >= 3 ? g.ia[j] : 0.0;
+    const double ak = K >= 3 ? g.a[k] : 0.0, iak = K >= 3 ? g.ia[k] : 0.0;
     double r = 0.0;
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
@@ -207,7 +207,7 @@ __device__ __forceinline__ void slot_exact_part(const SlotGrid& g, const SlotPas
             rate = 0.0;
 #pragma unroll
             for (int q = 0; q < NP; ++q)
-                rate += rate_geo<K>(__ldg(g.Bd + d), __ldg(g.Sd + d), p[q].Nj[j],
+                rate += rate_geo<K>(g.Bd[d], g.Sd[d], p[q].Nj[j],
                                     NeedH<K>::j ? p[q].Hj[j] : 0.0, p[q].Nk[s],
                                     NeedH<K>::k ? p[q].Hk[s] : 0.0);
             th = sum_minus_scaled_pre(pa, __ldg(g.x + j), pc);
@@ -231,6 +231,50 @@ __device__ __forceinline__ void slot_exact(const SlotGrid& g, const SlotPass* p,
     TH = warp_sum(t);
 }
 
+// Warp w of nw's part of the 32 slots s = I - 1 + lane (I the first bin): the
+// direct pairs, and its turns of the slots that keep their exact pair sums
+// (spread over the warps). Returns the mask of those slots; the prefix part of
+// the others is left to the caller.
+template <int K, int NP>
+__device__ __forceinline__ unsigned slot_warp(const SlotGrid& g, const SlotPass* p, int I, int w, int nw,
+                                              double& R, double& TH)
+{
+    const int l = threadIdx.x & 31, s = I - 1 + l, n = g.n;
+    const bool slot = s >= 0 && s <= n - 2;
+    R = 0.0;
+    TH = 0.0;
+    if (g.geo) {
+        // equal contiguous shares of the lags below D0 (each warp sees its runs in order)
+        const int smax = min(I - 1 + 31, n - 2);
+        const double xs = slot ? __ldg(g.x + s) : 1.0;
+        const int lags = min(min(n, g.D0), smax + 1);
+        const int per = (lags + nw - 1) / nw;
+        const int d0 = w * per;
+        slot_pairs_geo<K, NP>(g, p, s, slot, smax, d0, min(lags, d0 + per),
+                              ew_operand_c(xs, -exponent_of(xs)), R, TH);
+    } else {
+        slot_pairs_any<K, NP>(g, p, s, slot, w, nw, R, TH);
+    }
+    bool ex = false;
+    if (slot && slot_cut(g, s) > 0) {
+        const double xu = __ldg(g.x + s + 1), idx = g.inv_dx[s];
+#pragma unroll
+        for (int q = 0; q < NP; ++q) ex = ex || mom_exact_slot(p[q].Nk[s], p[q].Nk[s + 1], xu, idx);
+    }
+    const unsigned exact = __ballot_sync(0xffffffffu, ex);
+    int turn = 0;
+    for (unsigned m = exact; m != 0u; m &= m - 1u) {
+        const int le = __ffs(m) - 1;
+        if (turn == w) {
+            double r, t;
+            slot_exact<K, NP>(g, p, I - 1 + le, r, t);
+            if (l == le) { R += r; TH += t; }
+        }
+        turn = turn + 1 == nw ? 0 : turn + 1;
+    }
+    return exact;
+}
+
 // Clipped pairs (x_j + x_k >= x[n-1], all deposited on bin n-1,
 // src/aggregation_kernels.cuh:191-192) but for those of the prefix sums of slot
 // n - 1, share of thread tid of nt: a warp per lag with its lanes over j on a
@@ -243,9 +287,9 @@ __device__ double slot_clip(const SlotGrid& g, const SlotPass* p, int tid, int n
     if (g.geo) {
         const int l = tid & 31;
         for (int d = tid >> 5; d < min(n, g.D0); d += nt >> 5) {
-            const int L = __ldg(g.Ld + d);
+            const int L = g.Ld[d];
             const int jlo = L >= kLagClipAll ? 0 : max(0, n - 1 - L);
-            const double B = __ldg(g.Bd + d), S = __ldg(g.Sd + d);
+            const double B = g.Bd[d], S = g.Sd[d];
             for (int j = jlo + l; j <= n - 1 - d; j += 32)
 #pragma unroll
                 for (int q = 0; q < NP; ++q)

@@ -30,13 +30,16 @@
 //    last of them and of the task owning bin n-1 adds their parts, in order, to
 //    rhs[n-1].
 //
-// Kernels per call: prep (per-bin values, lag tables, prefix moments, geometric
+// Kernels per call: up to kSmallMaxN sections, one cluster kernel in gather mode
+// (agg_small_kernel); else prep (per-bin values, lag tables, prefix moments, geometric
 // check; its last block finishes moments, flag and counters) -> pair kernel
 // (persistent CTAs pulling tasks from an atomic counter, agg_lane.cuh). GATHER
 // mode: each output bin is written once, from sums reduced in a fixed order ->
 // bitwise reproducible. SCATTER mode: every task flushes its bins with FP64
 // atomicAdd.
 // =============================================================================
+#include <cooperative_groups.h>
+
 #include "pbe_internal.cuh"
 #include "agg_lane.cuh"
 
@@ -460,6 +463,301 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
     if (tid == 0 && atomicAdd(ws.counter + 6, 1) == static_cast<int>(gridDim.x) - 1) ws.counter[5] = 0;
 }
 
+// ---------------------------------------------------------------------------
+// Small instances (gather mode, n <= kSmallMaxN): the whole call as one cluster,
+// CTA r owning the bins [31 r, 31 r + 31) (a warp's lanes: their slots and the
+// one below, so nothing is handed over). At these sizes a call is a chain of
+// latencies -- two launches, a memset, tickets with memory fences, the FP64
+// chains of the prep -- not work: 24 us of it at n = 64 in the kernels above.
+//  1. grid tables and moments of the CTA's bins as agg_prep_kernel (warp 0 the
+//     moments and their scan, warp 1 logarithms, brackets and J0, warp 2 the
+//     geometric fit and 1/dx, warp 3 the lag factors), totals in shared memory;
+//  2. cluster barrier; every CTA adds the others' totals (distributed shared
+//     memory): prefix offsets, moments, geometric flag, D0;
+//  3. the slots' pairs over the CTA's eight warps, the bins by warp 0.
+// KIND as the launcher's: kAggTables stops after 2 and keeps the tables,
+// kAggStage takes them from the workspace.
+// ---------------------------------------------------------------------------
+enum { kAggFull = 0, kAggTables = 1, kAggStage = 2 };
+constexpr int kSmallBins = 31;
+constexpr int kSmallMaxCtas = 16;
+constexpr int kSmallMaxN = kSmallBins * kSmallMaxCtas;
+
+template <int K, int KIND>
+__global__ void __launch_bounds__(kMainThreads)
+agg_small_kernel(const double* __restrict__ N, const double* __restrict__ x, double* __restrict__ rhs,
+                 AggWs ws, int n, double b0, double bbr, double bsh)
+{
+    namespace cg = cooperative_groups;
+    const cg::cluster_group cl = cg::this_cluster();
+    __shared__ double tot[2 * kMomN];                  // this CTA's totals (read by the cluster)
+    __shared__ int te_s, d0_s;                         // exponent of its last bin, its D0 candidate
+    __shared__ double dev_s;
+    __shared__ double off[kSmallMaxCtas][2 * kMomN];   // sums over the CTAs before r
+    __shared__ int oe[kSmallMaxCtas];                  // exponent they stand at
+    __shared__ double M_s[kMomN];
+    __shared__ double a_s[32];
+    __shared__ double ax0_s;
+    __shared__ GeoFit fit_s;
+    __shared__ int D0_all;
+    __shared__ int geo_all;
+    __shared__ double red[kLaneWarps][2][32];
+    __shared__ double csum[kLaneWarps];
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int r = static_cast<int>(cl.block_rank()), ranks = static_cast<int>(cl.num_blocks());
+    const int I = kSmallBins * r;
+    const int i = I + lane;
+    const bool on = lane < kSmallBins && i < n;
+    const int last = min(I + kSmallBins - 1, n - 1);   // the CTA's last bin
+    const double xi = x[on ? i : last];
+
+    // 1. grid tables and moments
+    int Ei = 0, d0 = n;
+    double fi = 0.0;
+    if (w == 0) {
+        double ai, iai;
+        if constexpr (KIND == kAggStage) {
+            ai = ws.a[on ? i : last];
+            iai = ws.ia[on ? i : last];
+        } else {
+            ai = cbrt(xi);
+            iai = 1.0 / ai;
+            if (on) { ws.a[i] = ai; ws.ia[i] = iai; }
+            a_s[lane] = ai;
+        }
+        if constexpr (KIND != kAggTables) {
+            const double Ni = on ? N[i] : 0.0;
+            const double hi = xi * Ni, xm = mantissa_of(xi);
+            const int E = exponent_of(xi);
+            if (on) ws.h[i] = hi;
+            double P[kMomN] = {iai * Ni, Ni, ai * Ni, (ai * ai) * Ni, hi}, T[kMomN];
+#pragma unroll
+            for (int q = 0; q < kMomN; ++q) T[q] = P[q] * xm;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int dE = __shfl_up_sync(0xffffffffu, E, o) - E;
+#pragma unroll
+                for (int q = 0; q < kMomN; ++q) {
+                    if (!need_moment<K>(q)) continue;
+                    const double p = __shfl_up_sync(0xffffffffu, P[q], o);
+                    const double t = __shfl_up_sync(0xffffffffu, T[q], o);
+                    if (lane >= o) { P[q] += p; T[q] += scale_down(t, dE); }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < kMomN; ++q) {
+                if (!need_moment<K>(q)) continue;
+                if (on) {
+                    ws.mloc[q * n + i] = P[q];
+                    ws.mloc[(kMomN + q) * n + i] = T[q];
+                }
+                if (lane == 31) { tot[q] = P[q]; tot[kMomN + q] = T[q]; }
+            }
+            if (lane == 31) te_s = E;
+        }
+    }
+    if constexpr (KIND != kAggStage) {
+        if (w == 1) {
+            Ei = ilogb(xi);
+            fi = log2(scalbn(xi, -Ei));
+            const float lx0 = log2_approx(__ldg(x));
+            const float span = log2_approx(__ldg(x + n - 1)) - lx0;
+            const float inv_span = (n > 1 && span > 0.0f) ? static_cast<float>(n - 1) / span : 0.0f;
+            if (on) {
+                const double v = x[0] + xi;
+                const int L = (dbits(v) >= dbits(x[n - 1])) ? kLagClipAll : bracket_from(x, n, v, i);
+                ws.Ld[i] = L;
+                if (L == i && i > 0) d0 = i;           // lag 0 carries the pair 1/2: never separated
+                ws.J0[i] = i < n - 1 ? first_above(x, i, xi, x[i + 1], lx0, inv_span) : i;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) d0 = min(d0, __shfl_xor_sync(0xffffffffu, d0, o));
+        } else if (w == 2) {
+            const double xe = x[lane == 1 ? n - 1 : 0];
+            const int Ee = ilogb(xe);
+            const double fe = log2(scalbn(xe, -Ee));
+            const double f1 = __shfl_sync(0xffffffffu, fe, 1);
+            const int E1 = __shfl_sync(0xffffffffu, Ee, 1);
+            if (lane == 0) fit_s = geo_fit_from(Ee, fe, E1, f1, n);
+            if (on) ws.inv_dx[i] = (i < n - 1) ? 1.0 / (x[i + 1] - xi) : 0.0;
+        } else if (w == 3) {
+            const double c0 = cbrt(x[0]);
+            if (lane == 0) ax0_s = c0;
+        }
+        __syncthreads();
+        if (w == 1) {
+            double dev = (on && n >= 2) ? geo_dev_from(fit_s, Ei, fi, i) : 0.0;
+            if (!(dev == dev)) dev = 1.0;              // NaN -> not geometric
+            dev = warp_max(dev);
+            if (lane == 0) { dev_s = dev; d0_s = d0; }
+        } else if (w == 3 && on) {
+            const double c = (i == 0) ? 0.5 : 1.0;
+            double B = 0.0, S = 0.0;
+            if constexpr (K <= 2) B = c * b0;
+            if constexpr (K >= 3) {
+                const double rho = a_s[lane] / ax0_s;
+                if constexpr (K == 3 || K == 5) B = c * bbr * (rho + 1.0 / rho + 2.0);
+                if constexpr (K == 4 || K == 5) { const double t = 1.0 + rho; S = c * bsh * (t * t) * t; }
+            }
+            ws.Bd[i] = B;
+            ws.Sd[i] = S;
+        }
+    }
+    cl.sync();
+
+    // 2. the other CTAs' totals
+    if (w == 0 && lane < 2 * kMomN && KIND != kAggTables) {
+        const bool weighted = lane >= kMomN;
+        double acc = 0.0;
+        int e = 0;
+        for (int q = 0; q < ranks; ++q) {
+            const int en = *cl.map_shared_rank(&te_s, q);
+            off[q][lane] = acc;
+            if (lane == 0) oe[q] = e;
+            if (weighted && q > 0) acc = scale_down(acc, e - en);
+            acc += *cl.map_shared_rank(&tot[lane], q);
+            e = en;
+        }
+        if (!weighted) M_s[lane] = acc;
+    }
+    if (w == 1) {
+        if constexpr (KIND == kAggStage) {
+            if (lane == 0) { geo_all = ws.mom[5] != 0.0 ? 1 : 0; D0_all = ws.counter[1]; }
+        } else {
+            double dev = 0.0;
+            int dm = n;
+            if (lane < ranks) {
+                dev = *cl.map_shared_rank(&dev_s, lane);
+                dm = *cl.map_shared_rank(&d0_s, lane);
+            }
+            dev = warp_max(dev);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) dm = min(dm, __shfl_xor_sync(0xffffffffu, dm, o));
+            if (lane == 0) {
+                // neighbour ratio <= 64: precondition of sum_minus_scaled
+                geo_all = (n >= 2 && dev <= kGeoTol && x[1] <= 64.0 * x[0]) ? 1 : 0;
+                D0_all = dm;
+                if (KIND == kAggTables && r == 0) {
+                    ws.mom[5] = geo_all ? 1.0 : 0.0;
+                    ws.counter[1] = dm;
+                }
+            }
+        }
+    }
+    cl.sync();            // offsets in place; nobody reads another CTA's memory from here on
+    if constexpr (KIND == kAggTables) return;
+
+    // 3. pairs and bins
+    const SlotGrid g{x, ws.a, ws.ia, ws.inv_dx, ws.Bd, ws.Sd, ws.Ld, ws.J0, n, D0_all, geo_all != 0,
+                     b0, bbr, bsh};
+    const SlotPass p{N, ws.h, N, ws.h, N, ws.h};
+    double R, TH;
+    const unsigned exact = slot_warp<K, 1>(g, &p, I, w, kLaneWarps, R, TH);
+    red[w][0][lane] = R;
+    red[w][1][lane] = TH;
+    if (last == n - 1) {
+        const double c = warp_sum(slot_clip<K, 1>(g, &p, tid, kMainThreads));
+        if (lane == 0) csum[w] = c;
+    }
+    __syncthreads();
+    if (w != 0) return;
+    R = 0.0;
+    TH = 0.0;
+#pragma unroll
+    for (int q = 0; q < kLaneWarps; ++q) { R += red[q][0][lane]; TH += red[q][1][lane]; }
+    const int s = I - 1 + lane;                        // this lane's slot and bin
+    const bool slot = s >= 0 && s <= n - 2;
+    double death = 0.0, clip = 0.0, own = 0.0, up = 0.0;
+    if (s >= 0 && s < n) {
+        const double xs = x[s], as = g.a[s], ias = g.ia[s], Ns = N[s];
+        const int St = -exponent_of(xs);
+        death = Ns * death_factor<K>(xs, as, ias, M_s, b0, bbr, bsh);
+        const int cut = slot_cut(g, s);
+        if (cut > 0 && !((exact >> lane) & 1u)) {
+            const int j = cut - 1, b = j / kSmallBins, Ej = exponent_of(x[j]);
+            double P[kMomN], T[kMomN];
+#pragma unroll
+            for (int q = 0; q < kMomN; ++q) {
+                P[q] = T[q] = 0.0;
+                if (!need_moment<K>(q)) continue;
+                P[q] = ws.mloc[q * n + j] + off[b][q];
+                T[q] = ws.mloc[(kMomN + q) * n + j] + scale_down(off[b][kMomN + q], oe[b] - Ej);
+            }
+            const double rr = Ns * death_factor<K>(xs, as, ias, P, b0, bbr, bsh);
+            if (slot) {
+                R += rr;
+                TH += scale_down(Ns * death_factor<K>(xs, as, ias, T, b0, bbr, bsh), Ej + St);
+            } else {
+                clip = rr;                             // bin n - 1: clipped
+            }
+        }
+        if (slot) {
+            const double sd = scalbn(g.inv_dx[s], -St);
+            own = fma(-TH, sd, R);
+            up = TH * sd;
+        } else {
+#pragma unroll
+            for (int q = 0; q < kLaneWarps; ++q) clip += csum[q];
+        }
+    }
+    const double in = __shfl_up_sync(0xffffffffu, up, 1);
+    if (lane >= 1 && s < n) rhs[s] = rhs[s] + (((own + in) + clip) - death);
+}
+
+// One cluster of the device can hold 16 CTAs of this kernel (a size beyond the
+// portable 8, asked for once per kernel).
+template <int K, int KIND>
+bool small_cluster_ok(int ranks)
+{
+    if (ranks <= 8) return true;
+    static const bool ok = []() {
+        auto kern = agg_small_kernel<K, KIND>;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(kSmallMaxCtas);
+        cfg.blockDim = dim3(kMainThreads);
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = kSmallMaxCtas;
+        at.val.clusterDim.y = 1;
+        at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int num = 0;
+        if (cudaOccupancyMaxActiveClusters(&num, kern, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        return num > 0;
+    }();
+    return ok;
+}
+
+template <int K, int KIND>
+cudaError_t launch_small(const AggArgs& a, const AggWs& ws, cudaStream_t s, int ranks)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(ranks));
+    cfg.blockDim = dim3(kMainThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = static_cast<unsigned>(ranks);
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const bool prof = KIND != kAggTables && g_prof_start && g_prof_stop;
+    if (prof) cudaEventRecord(g_prof_start, s);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, agg_small_kernel<K, KIND>, a.N, a.x, a.rhs, ws, a.n,
+                                             a.beta0, a.beta_br, a.beta_sh);
+    if (prof) cudaEventRecord(g_prof_stop, s);
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
 // Tasks that sum the clipped pairs (about n + 1.2 q^2 pairs on a grid with q bins
 // per octave, up to half of all pairs on others).
 int agg_clip_tasks(int n)
@@ -470,13 +768,21 @@ int agg_clip_tasks(int n)
 
 // kind: kAggFull = tables + pair kernel (the drop-in calls), kAggTables =
 // the FULL prep only, kAggStage = the light prep + pair kernel on a
-// workspace whose tables an earlier kAggTables / kAggFull call wrote.
-enum { kAggFull = 0, kAggTables = 1, kAggStage = 2 };
-
+// workspace whose tables an earlier kAggTables call wrote.
 template <int K, bool SC>
 cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_t s, int kind)
 {
     const int n = a.n;
+    if (!SC && n <= kSmallMaxN) {
+        // measured against the two kernels below, whole calls: n = 64 X -> X us
+        const int ranks = (n + kSmallBins - 1) / kSmallBins;
+        if (small_cluster_ok<K, kAggFull>(ranks) && small_cluster_ok<K, kAggTables>(ranks) &&
+            small_cluster_ok<K, kAggStage>(ranks)) {
+            if (kind == kAggFull) return launch_small<K, kAggFull>(a, ws, s, ranks);
+            if (kind == kAggTables) return launch_small<K, kAggTables>(a, ws, s, ranks);
+            return launch_small<K, kAggStage>(a, ws, s, ranks);
+        }
+    }
     const int nb = agg_prep_blocks(n);
     const int nclip = agg_clip_tasks(n);
     auto kern = agg_lane_kernel<K, SC>;

@@ -615,40 +615,9 @@ __device__ void batch_task(const BatchDev& d, const double* __restrict__ Yg,
     slot_passes<NP>(d, Yg, off, p);
     const int s = I - 1 + l;                        // this lane's slot and bin
     const bool slot = s >= 0 && s <= n - 2;
-    const double xs = slot ? __ldg(g.x + s) : 1.0;
-    const int St = slot ? -exponent_of(xs) : 0;
+    const int St = slot ? -exponent_of(__ldg(g.x + s)) : 0;
     double R = 0.0, TH = 0.0;
-    unsigned exact = 0u;
-    if (agg) {
-        const int smax = min(I - 1 + 31, n - 2);
-        if (g.geo) {
-            // equal contiguous shares of the lags below D0 (each warp sees its runs in order)
-            const int lags = min(min(n, g.D0), smax + 1);
-            const int per = (lags + nw - 1) / nw;
-            const int d0 = w * per;
-            slot_pairs_geo<K, NP>(g, p, s, slot, smax, d0, min(lags, d0 + per), ew_operand_c(xs, St), R, TH);
-        } else {
-            slot_pairs_any<K, NP>(g, p, s, slot, w, nw, R, TH);
-        }
-        // slots that keep the exact pair sums, spread over the group's warps
-        bool ex = false;
-        if (slot && slot_cut(g, s) > 0) {
-            const double xu = __ldg(g.x + s + 1), idx = __ldg(g.inv_dx + s);
-#pragma unroll
-            for (int q = 0; q < NP; ++q) ex = ex || mom_exact_slot(p[q].Nk[s], p[q].Nk[s + 1], xu, idx);
-        }
-        exact = __ballot_sync(0xffffffffu, ex);
-        int turn = 0;
-        for (unsigned m = exact; m != 0u; m &= m - 1u) {
-            const int le = __ffs(m) - 1;
-            if (turn == w) {
-                double r, t;
-                slot_exact<K, NP>(g, p, I - 1 + le, r, t);
-                if (l == le) { R += r; TH += t; }
-            }
-            turn = turn + 1 == nw ? 0 : turn + 1;
-        }
-    }
+    const unsigned exact = agg ? slot_warp<K, NP>(g, p, I, w, nw, R, TH) : 0u;
     const bool brk = d.nq > 0;
     const bool brk_tasks = (d.brk & kBrkTasks) != 0;
     if (brk && brk_tasks) tile_breakage(d, gd, d.SN + off, n, I, sm.extra[G.g], G);
