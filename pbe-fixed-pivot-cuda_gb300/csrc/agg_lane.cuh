@@ -32,6 +32,18 @@
 // bin, where a tiny w's rounding would show) the slot keeps its exact pair sum,
 // a task of its own (exact_slot_task).
 //
+// Lags below D0 on fine grids (win_grid; gather mode; N without negative entries):
+// the runs from lag Dm on are long enough to separate too. In run e, lags [d1, d2),
+// slot s has k = s - e and the window j in [k - d2 + 1, k - d1], so
+//   R += sum_q c_q(x_k) N_k M_q,  TH += sum_q c_q N_k M_{q+3} + (x_k - x_s) R_run,
+// M_m = sum over the window of x_j^(m/3) N_j, from two table values (and whole
+// blocks of 64 between them): windows of any length and place without a
+// subtraction, so sums of one sign keep their relative precision. At 512 sections
+// an octave 1324 lags stay pairs and 137 runs cover the other 3560. The rounding of
+// fl(x_j + x_k), left out as above, moves bins s and s + 1 by at most u R_win; the
+// finishing warp compares that with what these bins are known to receive and lose
+// (kMomGuard), and slots beyond it sum those lags pair by pair.
+//
 // On other grids the same holds for the rows j < J0(s), the first j with
 // fl(x_j + x_s) >= x_{s+1}.
 //
@@ -41,7 +53,7 @@
 // (of each slot's rows on other grids); the CTA's eight warps take equal
 // contiguous shares of the task's lags (each warp sees its runs in order) and
 // their sums are added in warp order. With several parts each task stores its
-// 2 x 32 sums; the block's last task (ticket) adds them in order and writes the
+// 4 x 32 sums; the block's last task (ticket) adds them in order and writes the
 // bins -- deterministic, nobody waits.
 //
 // Operand staging (geometric grids): the j-side operands of a task (N_j,
@@ -62,12 +74,17 @@ constexpr int kLaneWinMax = 1792;                   // staged window, entries pe
 // Bounded waits on the staging barrier: iterations of mbarrier.try_wait.
 constexpr long long kLaneWaitLimit = 1LL << 26;
 
-// Shares of a block's direct lags: enough tasks to give every CTA several (the
-// last ones then end together), at least 32 lags each (4 per warp). A share
-// longer than the staged window reads its operands from the arrays.
+// Shares of a block's pairs (`lags`: pairs of a slot). Long shares: enough tasks
+// to give every CTA four, so that the last ones end together. A task costs a few
+// microseconds beside its pairs (fetch, staging, sums, ticket), so where that would
+// leave a share less than 192 pairs a slot, as many shares as fit the CTAs in one
+// round (n = 3840, 456 CTAs: 8 shares in two rounds 57 us, 3 shares in one 42). At
+// least 32 pairs a share (4 per warp). A share longer than the staged window reads
+// its operands from the arrays.
 __host__ __device__ constexpr int lane_parts(int lags, int nblk, int ctas)
 {
     int p = (4 * ctas + nblk - 1) / nblk;
+    if (p > kLaneMaxParts || lags < 192 * p) p = ctas / nblk;
     const int most = (lags + 31) / 32;
     if (p > most) p = most;
     if (p > kLaneMaxParts) p = kLaneMaxParts;
@@ -116,7 +133,7 @@ __device__ __forceinline__ void fence_proxy_async_smem()
 
 // Shared memory of a lane task (carved from the kernel's dynamic buffer).
 struct LaneSmem {
-    double* red;     // [kLaneWarps][2][32] per-warp R, TH
+    double* red;     // [kLaneWarps][4][32] per-warp R, TH of the pairs and of the windows
     double* wN;      // [kLaneWinMax] staged N_j   (K needs N on the j side)
     double* wH;      // [kLaneWinMax] staged x_j N_j
     double* wX;      // [kLaneWinMax] staged x_j
@@ -131,6 +148,8 @@ struct LaneArgs {
     int* ticket;         // [lane_blocks(n)] tasks of the block done (reset by the prep)
     int* err;            // set to 1 when a staging wait gave up
     int parts;           // tasks per block
+    int Dm;              // lags summed pair by pair (geometric grids)
+    int eh, el;          // runs eh .. el (descending) summed by windows; eh < el: none
 };
 
 // The call as its tasks see it: the grid with the lag tables, the one pass
@@ -168,11 +187,16 @@ __device__ __forceinline__ unsigned exact_mask(const LaneView& v, int t)
     return __ballot_sync(0xffffffffu, e);
 }
 
+// The sums of a slot: pairs (and prefix part), windows.
+struct SlotSums {
+    double R, TH, Rw, Tw;
+};
+
 // One warp, after its contribution to block t is stored: the block's ticket.
 // True for the last of its `parts` share tasks and one task per exact slot;
 // that one gets the block's sums, added in a fixed order.
 __device__ __forceinline__ bool block_ticket(const AggWs& ws, const LaneArgs& la, int n, int t,
-                                             unsigned exact, double& Rt, double& THt)
+                                             unsigned exact, SlotSums& u)
 {
     const int lane = threadIdx.x & 31;
     const int want = la.parts + __popc(exact);
@@ -182,67 +206,188 @@ __device__ __forceinline__ bool block_ticket(const AggWs& ws, const LaneArgs& la
     if (lane == 0) last = (atomicAdd(la.ticket + t, 1) == want - 1);
     if (!__shfl_sync(0xffffffffu, last, 0)) return false;
     __threadfence();
-    Rt = 0.0;
-    THt = 0.0;
-    const double* bp = la.part + static_cast<size_t>(t) * la.parts * 64;
-    for (int q = 0; q < la.parts; ++q) {
-        Rt += __ldcg(bp + q * 64 + lane);
-        THt += __ldcg(bp + q * 64 + 32 + lane);
+    u = SlotSums{0.0, 0.0, 0.0, 0.0};
+    const double* bp = la.part + static_cast<size_t>(t) * la.parts * 128 + lane;
+    for (int q = 0; q < la.parts; ++q, bp += 128) {
+        u.R += __ldcg(bp);
+        u.TH += __ldcg(bp + 32);
+        u.Rw += __ldcg(bp + 64);
+        u.Tw += __ldcg(bp + 96);
     }
     if ((exact >> lane) & 1u) {
         const int s = n - kLaneBins * (t + 1) + lane;
-        Rt += __ldcg(ws.xsum + 2 * s);
-        THt += __ldcg(ws.xsum + 2 * s + 1);
+        u.R += __ldcg(ws.xsum + 2 * s);
+        u.TH += __ldcg(ws.xsum + 2 * s + 1);
     }
     return true;
 }
 
-// One warp: the bins of block t from its slots' sums (a slot per lane). With
-// `first` the prefix part (not of the exact slots) and the death term are added;
-// scatter mode calls it for every share's own sums.
-template <int K, bool SCATTER>
-__device__ void lane_finish(const LaneView& v, const AggWs& ws, double* rhs, int t,
-                            int nclip, unsigned exact, bool first, bool poisoned, double Rt,
-                            double THt)
+// The runs eh .. el of slot s by windows: Rw += rates, Tw += rates (v - x_s), not
+// scaled. Every lane of the warp takes part.
+template <int K>
+__device__ __forceinline__ void lane_windows(const LaneView& v, const AggWs& ws, int s, bool slot, int eh,
+                                             int el, double& Rw, double& Tw)
 {
-    const int n = v.g.n, lane = threadIdx.x & 31;
+    const int n = v.g.n;
+    const size_t ns = static_cast<size_t>(n);
+    const double xs = slot ? __ldg(v.g.x + s) : 0.0;
+    for (int e = eh; e >= el; --e) {
+        const int d1 = __ldg(ws.rend + e + 1), d2 = __ldg(ws.rend + e);
+        const int k = s - e, b = k - d1;
+        if (!slot || b < 0) continue;
+        const int a = max(0, k - d2 + 1);
+        const int A = a >> 6, B = b >> 6;
+        const double* pb = ws.wtab + b;                // the part from the middle (or a block's start) to b
+        const double* pa = ws.wtab + a;                // the part from a to the middle (or a block's end)
+        bool two = true;
+        if (A != B) {
+            pb += 4 * kWinMom * ns;
+            pa += 5 * kWinMom * ns;
+        } else if ((a & 63) == 0) {
+            pb += 4 * kWinMom * ns;
+            two = false;
+        } else {                                       // b - a >= 4: they differ in bit 2 or above
+            const size_t l = static_cast<size_t>(31 - __clz(a ^ b) - 2) * kWinMom * ns;
+            pb += l;
+            pa += l;
+        }
+        double M[kWinMom];
+#pragma unroll
+        for (int m = 0; m < kWinMom; ++m) {
+            M[m] = 0.0;
+            if (need_window<K>(m)) M[m] = __ldg(pb + m * ns) + (two ? __ldg(pa + m * ns) : 0.0);
+        }
+        for (int q = A + 1; q < B; ++q)                // whole blocks of 64 between
+#pragma unroll
+            for (int m = 0; m < kWinMom; ++m)
+                if (need_window<K>(m)) M[m] += __ldg(ws.wtab + (4 * kWinMom + m) * ns + q * 64 + 63);
+        double r = 0.0;
+#pragma unroll
+        for (int q = 0; q < kMomN; ++q) {
+            if (!need_moment<K>(q)) continue;
+            const double c = __ldg(ws.wc + q * ns + k);
+            r = fma(c, M[q], r);
+            Tw = fma(c, M[q + 3], Tw);
+        }
+        Rw += r;
+        Tw = fma(__ldg(v.g.x + k) - xs, r, Tw);
+    }
+}
+
+// The lags [Dm, D0) of slot s pair by pair, by one warp (lanes over the lags,
+// fixed butterfly). Valid in every lane.
+template <int K>
+__device__ __forceinline__ void exact_runs(const LaneView& v, int s, int Dm, double& R, double& TH)
+{
+    const int lane = threadIdx.x & 31;
+    const double xs = __ldg(v.g.x + s);
+    const EwOperandC pc = ew_operand_c(xs, -exponent_of(xs));
+    double r = 0.0, t = 0.0;
+    for (int d = Dm + lane; d < min(v.g.D0, v.g.n); d += 32) {
+        const int L = __ldg(v.g.Ld + d);
+        const int j = s - L, k = j + d;
+        if (j < 0) break;                              // Ld is nondecreasing
+        const double rate = rate_geo<K>(__ldg(v.g.Bd + d), __ldg(v.g.Sd + d), __ldg(v.p.Nj + j),
+                                        NeedH<K>::j ? __ldg(v.p.Hj + j) : 0.0, __ldg(v.p.Nk + k),
+                                        NeedH<K>::k ? __ldg(v.p.Hk + k) : 0.0);
+        r += rate;
+        t = fma(rate, sum_minus_scaled_pre(ew_operand_a(__ldg(v.g.x + k)), __ldg(v.g.x + j), pc), t);
+    }
+    R = warp_sum(r);
+    TH = warp_sum(t);
+}
+
+// The bins of block t from its slots' sums (a slot per lane of warp 0), by the
+// CTA; `finish` and u are warp 0's. With `first` the prefix part (not of the exact
+// slots) and the death term are added; scatter mode calls it for every share's own
+// sums. s_ex: shared memory, [2][32] and a mask behind it.
+template <int K, bool SCATTER>
+__device__ void lane_finish(const LaneView& v, const AggWs& ws, const LaneArgs& la, double* rhs, int t,
+                            int nclip, unsigned exact, bool finish, bool first, bool poisoned,
+                            SlotSums u, double (*s_ex)[32], unsigned* s_mask)
+{
+    const int n = v.g.n, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int I = n - kLaneBins * (t + 1);
     const int smax = lane_block_smax(n, t);
     const int s = I + lane, i = s;
     const bool slot = s >= 0 && s <= smax;
-    const double xs = slot ? __ldg(v.g.x + s) : 0.0;
-    const int St = slot ? -exponent_of(xs) : 0;
     double clip0 = 0.0;                                // the prefix part of the clipped slot n - 1
-    double death = 0.0;
-    if (first && s >= 0 && s <= n - 1) {
-        const double as = __ldg(v.g.a + s), ias = __ldg(v.g.ia + s), xv = __ldg(v.g.x + s);
-        const double Ns = __ldg(v.p.Nk + s);
-        death = Ns * death_factor<K>(xv, as, ias, v.M, v.g.b0, v.g.bbr, v.g.bsh);
-        const int cut = slot_cut(v.g, s);
-        if (cut > 0 && !((exact >> lane) & 1u)) {
-            double P[kMomN], T[kMomN];
-            prefix_moments<K>(ws, v.g.x, n, cut - 1, P, T);
-            const double r = Ns * death_factor<K>(xv, as, ias, P, v.g.b0, v.g.bbr, v.g.bsh);
-            const double th = Ns * death_factor<K>(xv, as, ias, T, v.g.b0, v.g.bbr, v.g.bsh);
-            if (slot) {
-                Rt += r;
-                THt += scale_down(th, exponent_of(__ldg(v.g.x + cut - 1)) + St);
-            } else {
-                clip0 = r;
+    double death = 0.0, sd = 0.0, own = 0.0, up = 0.0;
+    int St = 0;
+    if (w == 0 && finish) {
+        const double xs = slot ? __ldg(v.g.x + s) : 0.0;
+        St = slot ? -exponent_of(xs) : 0;
+        if (first && s >= 0 && s <= n - 1) {
+            const double as = __ldg(v.g.a + s), ias = __ldg(v.g.ia + s), xv = __ldg(v.g.x + s);
+            const double Ns = __ldg(v.p.Nk + s);
+            death = Ns * death_factor<K>(xv, as, ias, v.M, v.g.b0, v.g.bbr, v.g.bsh);
+            const int cut = slot_cut(v.g, s);
+            if (cut > 0 && !((exact >> lane) & 1u)) {
+                double P[kMomN], T[kMomN];
+                prefix_moments<K>(ws, v.g.x, n, cut - 1, P, T);
+                const double r = Ns * death_factor<K>(xv, as, ias, P, v.g.b0, v.g.bbr, v.g.bsh);
+                const double th = Ns * death_factor<K>(xv, as, ias, T, v.g.b0, v.g.bbr, v.g.bsh);
+                if (slot) {
+                    u.R += r;
+                    u.TH += scale_down(th, exponent_of(__ldg(v.g.x + cut - 1)) + St);
+                } else {
+                    clip0 = r;
+                }
+            }
+        }
+        u.Tw = scalbn(u.Tw, St);
+        // own part of bin i (slot i) and the w-part of slot i, owed to bin i + 1
+        if (slot) {
+            const double idx = __ldg(v.g.inv_dx + i);
+            sd = scalbn(idx, -St);
+            own = fma(-(u.TH + u.Tw), sd, u.R + u.Rw);
+            up = (u.TH + u.Tw) * sd;
+        }
+    }
+    if (!SCATTER && la.eh >= la.el) {
+        // windows: slots where the rounding they leave out may show in bin s or s + 1
+        if (w == 0) {
+            bool ex = false;
+            const double below = __shfl_up_sync(0xffffffffu, up, 1);
+            const double dn = __shfl_down_sync(0xffffffffu, death, 1);
+            const double on = __shfl_down_sync(0xffffffffu, own, 1);
+            if (finish && slot && u.Rw != 0.0) {
+                const double xu = __ldg(v.g.x + s + 1);
+                const double err = (1.1102230246251565e-16 * (xu * __ldg(v.g.inv_dx + s))) * u.Rw;
+                double dup = dn;
+                if (lane == 31)
+                    dup = __ldg(v.p.Nk + s + 1) * death_factor<K>(xu, __ldg(v.g.a + s + 1), __ldg(v.g.ia + s + 1),
+                                                                  v.M, v.g.b0, v.g.bbr, v.g.bsh);
+                const double here = fmax(own, 0.0) + (lane > 0 ? below : 0.0) + death;
+                const double next = up + (lane < 31 ? fmax(on, 0.0) : 0.0) + dup;
+                ex = !(err <= kMomGuard * here && err <= kMomGuard * next);
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, ex);
+            if (lane == 0) *s_mask = m;
+        }
+        __syncthreads();
+        const unsigned mask = *s_mask;
+        if (mask != 0u) {
+            int turn = 0;
+            for (unsigned m = mask; m != 0u; m &= m - 1u, turn = (turn + 1) & (kLaneWarps - 1)) {
+                if (turn != w) continue;
+                const int le = __ffs(m) - 1;
+                double r, th;
+                exact_runs<K>(v, I + le, la.Dm, r, th);
+                if (lane == 0) { s_ex[0][le] = r; s_ex[1][le] = th; }
+            }
+            __syncthreads();
+            if (w == 0 && ((mask >> lane) & 1u)) {
+                own = fma(-(u.TH + s_ex[1][lane]), sd, u.R + s_ex[0][lane]);
+                up = (u.TH + s_ex[1][lane]) * sd;
             }
         }
     }
-    // own part of bin i (slot i) and the w-part of slot i, owed to bin i + 1
-    double b1 = 0.0, co = 0.0;
-    if (slot) {
-        const double sd = scalbn(__ldg(v.g.inv_dx + i), -St);
-        b1 = fma(-THt, sd, Rt);
-        co = THt * sd;
-    }
-    const double cin = __shfl_up_sync(0xffffffffu, co, 1);
+    if (w != 0 || !finish) return;
+    const double in = __shfl_up_sync(0xffffffffu, up, 1);
     if (i >= 0) {
-        double val = b1;
-        if (lane >= 1) val += cin;
+        double val = own;
+        if (lane >= 1) val += in;
         val += clip0;
         val -= death;
         if constexpr (SCATTER) {
@@ -271,10 +416,10 @@ __device__ void lane_finish(const LaneView& v, const AggWs& ws, double* rhs, int
         }
     }
     if constexpr (SCATTER) {
-        if (lane == 31 && slot && co != 0.0) atomicAdd(rhs + i + 1, co);
+        if (lane == 31 && slot && up != 0.0) atomicAdd(rhs + i + 1, up);
     } else if (lane == 31 && t >= 1) {
         // carry into bin I + 32, the first bin of block t - 1
-        ws.tcarry[t - 1] = co;
+        ws.tcarry[t - 1] = up;
         __threadfence();
         if (atomicAdd(ws.tticket + (t - 1), 1) == 1) {
             __threadfence();
@@ -290,7 +435,8 @@ __device__ void lane_finish(const LaneView& v, const AggWs& ws, double* rhs, int
 // bins made the whole call 1.5 x slower). `red`: 2 kLaneWarps doubles.
 template <int K, bool SCATTER>
 __device__ void exact_slot_task(const LaneView& v, const AggWs& ws, const LaneArgs& la,
-                                double* rhs, int s, int nclip, double* red, bool poisoned)
+                                double* rhs, int s, int nclip, double* red, bool poisoned,
+                                double (*s_ex)[32], unsigned* s_mask)
 {
     const int n = v.g.n, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int t = (n - 1 - s) / kLaneBins;
@@ -304,6 +450,9 @@ __device__ void exact_slot_task(const LaneView& v, const AggWs& ws, const LaneAr
     th = warp_sum(th);
     if (lane == 0) { red[2 * w] = r; red[2 * w + 1] = th; }
     __syncthreads();
+    SlotSums u{0.0, 0.0, 0.0, 0.0};
+    unsigned em = 0u;
+    bool finish = false;
     if (w == 0) {
         r = 0.0;
         th = 0.0;
@@ -319,12 +468,12 @@ __device__ void exact_slot_task(const LaneView& v, const AggWs& ws, const LaneAr
                 ws.xsum[2 * s] = r;
                 ws.xsum[2 * s + 1] = th;
             }
-            const unsigned em = exact_mask(v, t);
-            double Rt, THt;
-            if (block_ticket(ws, la, n, t, em, Rt, THt))
-                lane_finish<K, false>(v, ws, rhs, t, nclip, em, true, poisoned, Rt, THt);
+            em = exact_mask(v, t);
+            finish = block_ticket(ws, la, n, t, em, u);
         }
     }
+    if constexpr (!SCATTER)
+        lane_finish<K, false>(v, ws, la, rhs, t, nclip, em, finish, true, poisoned, u, s_ex, s_mask);
     __syncthreads();
 }
 
@@ -387,7 +536,7 @@ __device__ __forceinline__ void lane_pairs(const LaneView& v, int s, bool slot, 
 template <int K, bool SCATTER>
 __device__ void lane_task(const LaneView& v, const AggWs& ws, const LaneArgs& la, double* rhs,
                           int t, int c, int nclip, const LaneSmem& sm, uint64_t* bar,
-                          unsigned& phase, int* s_flag)
+                          unsigned& phase, int* s_flag, double (*s_ex)[32], unsigned* s_mask)
 {
     const int n = v.g.n;
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
@@ -396,9 +545,9 @@ __device__ void lane_task(const LaneView& v, const AggWs& ws, const LaneArgs& la
     const int smin = I > 0 ? I : 0;
     const int s = I + lane;
     const bool slot = (s >= smin && s <= smax);
-    double R = 0.0, TH = 0.0;
+    double R = 0.0, TH = 0.0, Rw = 0.0, Tw = 0.0;
     if (v.g.geo) {
-        const int Dm = min(v.g.D0, n);                 // lags summed pair by pair
+        const int Dm = la.Dm;                          // lags summed pair by pair
         const int C = (Dm + la.parts - 1) / la.parts;
         // lags of this task: [dA, dB), dB cut where Ld passes the block's top slot
         // (Ld is nondecreasing; clipped lags hold kLagClipAll)
@@ -448,32 +597,51 @@ __device__ void lane_task(const LaneView& v, const AggWs& ws, const LaneArgs& la
         const int per = (dB - dA + kLaneWarps - 1) / kLaneWarps;
         const int dw0 = dA + w * per;
         if (!*s_flag) lane_pairs<K>(v, s, slot, dw0, min(dB, dw0 + per), pN, pH, pX, R, TH);
+        if (!SCATTER && la.eh >= la.el) {
+            // and of the runs summed by windows
+            const int ne = la.eh - la.el + 1, sh = la.parts * kLaneWarps, q = c * kLaneWarps + w;
+            lane_windows<K>(v, ws, s, slot, la.eh - ne * q / sh, la.eh - ne * (q + 1) / sh + 1, Rw, Tw);
+        }
     } else {
         slot_pairs_any<K, 1>(v.g, &v.p, s, slot, c * kLaneWarps + w, la.parts * kLaneWarps, R, TH);
     }
-    sm.red[(w * 2 + 0) * 32 + lane] = R;
-    sm.red[(w * 2 + 1) * 32 + lane] = TH;
+    constexpr int NS = SCATTER ? 2 : 4;
+    double* red = sm.red + w * NS * 32 + lane;
+    red[0] = R;
+    red[32] = TH;
+    if constexpr (!SCATTER) {
+        red[64] = Rw;
+        red[96] = Tw;
+    }
     __syncthreads();
     const bool poisoned = *s_flag != 0;
 
+    SlotSums u{0.0, 0.0, 0.0, 0.0};
+    unsigned em = 0u;
+    bool finish = false;
     if (w == 0) {
-        double Rt = 0.0, THt = 0.0;
 #pragma unroll
         for (int q = 0; q < kLaneWarps; ++q) {
-            Rt += sm.red[(q * 2 + 0) * 32 + lane];
-            THt += sm.red[(q * 2 + 1) * 32 + lane];
+            const double* rq = sm.red + q * NS * 32 + lane;
+            u.R += rq[0];
+            u.TH += rq[32];
+            if constexpr (!SCATTER) {
+                u.Rw += rq[64];
+                u.Tw += rq[96];
+            }
         }
-        const unsigned em = exact_mask(v, t);
-        bool finish = true;
+        em = exact_mask(v, t);
+        finish = true;
         if (!SCATTER && (la.parts > 1 || em != 0u)) {
-            double* bp = la.part + (static_cast<size_t>(t) * la.parts + c) * 64;
-            bp[lane] = Rt;
-            bp[32 + lane] = THt;
-            finish = block_ticket(ws, la, n, t, em, Rt, THt);
+            double* bp = la.part + (static_cast<size_t>(t) * la.parts + c) * 128 + lane;
+            bp[0] = u.R;
+            bp[32] = u.TH;
+            bp[64] = u.Rw;
+            bp[96] = u.Tw;
+            finish = block_ticket(ws, la, n, t, em, u);
         }
-        if (finish)
-            lane_finish<K, SCATTER>(v, ws, rhs, t, nclip, em, !SCATTER || c == 0, poisoned, Rt, THt);
     }
+    lane_finish<K, SCATTER>(v, ws, la, rhs, t, nclip, em, finish, !SCATTER || c == 0, poisoned, u, s_ex, s_mask);
     __syncthreads();
 }
 

@@ -30,4 +30,22 @@ __device__ __forceinline__ bool mom_exact_slot(double Ns, double Nup, double xup
     return fabs(Nup) * (kMomGuard * 9007199254740992.0) < (xup * inv_dx) * fabs(Ns);
 }
 
+// Window sums (agg_lane.cuh) pay on grids of about 64 sections an octave and more:
+// neighbour ratio at most kWinRatio = 2^(1/64). The tables hold x^2 N unscaled, so
+// the pivots stay within 2^-300 .. 2^300. Lags up to x_d = kWinStart x_0 are summed
+// pair by pair: from there on a run has at least 6 lags (1 + x_d / x_0, within
+// one), a window more than 4 bins, and costs 21 FP64 instructions against 4 a pair.
+constexpr double kWinRatio = 1.0109;
+constexpr double kWinStart = 6.0;
+__device__ __forceinline__ bool win_grid(const double* __restrict__ x, int n)
+{
+    return n >= 2 && x[1] <= kWinRatio * x[0] && exponent_of(x[0]) > -300 && exponent_of(x[n - 1]) < 300;
+}
+// Moments m_{-1..6} (index m + 1) that kernel type K's windows need.
+template <int K>
+__device__ __forceinline__ constexpr bool need_window(int m)
+{
+    return (m < kMomN && need_moment<K>(m)) || (m >= 3 && need_moment<K>(m - 3));
+}
+
 } // namespace pbe_gb300

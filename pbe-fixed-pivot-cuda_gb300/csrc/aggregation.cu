@@ -98,6 +98,64 @@ __device__ __forceinline__ void prep_prefix(const double* m, double xm, int E, i
     }
 }
 
+// Window tables of one prep block (AggWs::wtab) and the coefficients of its bins as
+// larger members (AggWs::wc). p and s run through the prefix and suffix sums within
+// aligned groups of 1, 2, 4 .. bins: joining two groups, the right half's prefixes
+// gain the left half's total and the left half's suffixes the right half's, one
+// add a lane, step and moment (p of the left half's last lane and s of the right
+// half's first are those totals).
+template <int K>
+__device__ __forceinline__ void prep_windows(const double* m, double xi, double Ni, double hi,
+                                             int i, int n, const AggWs& ws, double (*wtot)[kWinMom],
+                                             double b0, double bbr, double bsh)
+{
+    const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & 1;   // two whole warps
+    const size_t ns = static_cast<size_t>(n);
+    double p[kWinMom], s[kWinMom];
+#pragma unroll
+    for (int q = 0; q < kWinMom; ++q) {
+        if (!need_window<K>(q)) continue;
+        double v = q < kMomN ? m[q < kMomN ? q : 0] : xi * m[q >= 3 ? q - 3 : 0];
+        p[q] = s[q] = v;
+#pragma unroll
+        for (int h = 1; h < 32; h <<= 1) {
+            const bool right = (lane & h) != 0;
+            const int src = (lane & ~(2 * h - 1)) + (right ? h - 1 : h);
+            const double t = __shfl_sync(0xffffffffu, right ? s[q] : p[q], src);
+            if (h >= 4 && i < n) {
+                const int l = h == 4 ? 0 : h == 8 ? 1 : 2;
+                ws.wtab[(l * kWinMom + q) * ns + i] = right ? p[q] : s[q];
+            }
+            if (right) p[q] += t; else s[q] += t;
+        }
+        if (i < n) ws.wtab[(3 * kWinMom + q) * ns + i] = w ? p[q] : s[q];
+        if (lane == 31) wtot[w][q] = p[q];
+    }
+    asm volatile("bar.sync 3, %0;" :: "n"(kPrepThreads) : "memory");
+    if (i >= n) return;
+#pragma unroll
+    for (int q = 0; q < kWinMom; ++q) {
+        if (!need_window<K>(q)) continue;
+        ws.wtab[(4 * kWinMom + q) * ns + i] = w ? p[q] + wtot[0][q] : p[q];
+        ws.wtab[(5 * kWinMom + q) * ns + i] = w ? s[q] : s[q] + wtot[1][q];
+    }
+    // beta(x_j, x_k) = sum_q c_q(x_k) m_q(x_j), m_q = {1/a, 1, a, a^2, x}
+    double c[kMomN] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    if constexpr (K == 0) c[1] = b0 * Ni;
+    if constexpr (K == 1) { c[1] = b0 * hi; c[4] = b0 * Ni; }
+    if constexpr (K == 2) c[4] = b0 * hi;
+    if constexpr (K == 3 || K == 5) { c[0] = bbr * m[2]; c[1] = 2.0 * bbr * Ni; c[2] = bbr * m[0]; }
+    if constexpr (K == 4 || K == 5) {
+        c[1] = fma(bsh, hi, c[1]);
+        c[2] = fma(3.0 * bsh, m[3], c[2]);
+        c[3] = (3.0 * bsh) * m[2];
+        c[4] = bsh * Ni;
+    }
+#pragma unroll
+    for (int q = 0; q < kMomN; ++q)
+        if (need_moment<K>(q)) ws.wc[q * ns + i] = c[q];
+}
+
 // Scan of the block totals by the prep's last block: each lane sums a run of
 // consecutive blocks, a warp scan adds the runs, each lane writes its blocks'
 // offsets. Warp 0: the moments (their last sums are the death term's moments),
@@ -160,8 +218,8 @@ __device__ __forceinline__ void prep_offsets(const double* __restrict__ x, int n
 
 // ---------------------------------------------------------------------------
 // prep: blocks of 64 bins. Threads 0..63 (a thread per bin): cube roots, the
-// moments' terms and their prefix sums. Threads 64..127 (FULL, the same bins):
-// the grid's part --
+// moments' terms and their prefix sums. The last 64 threads (the same bins): the
+// window tables of fine grids. Threads 64..127 (FULL): the grid's part --
 //   Bd[d], Sd[d] for d = i: beta(x_j, x_{j+d}) = Bd + x_j Sd on a geometric grid,
 //   times c_d (1/2 for d = 0), with rho = x_d^(1/3) / x_0^(1/3):
 //     Constant/Sum/Product: Bd = c_d beta0 (the x dependence stays per pair)
@@ -170,7 +228,7 @@ __device__ __forceinline__ void prep_offsets(const double* __restrict__ x, int n
 //   Ld[d]: bracket of x_0 + x_d (kLagClipAll when it reaches x[n-1]); 1/dx; J0;
 //   the geometric-grid deviation.
 // The kernel is a chain of dependent FP64 instructions (cube root, divisions,
-// log2: some 40 clocks each): the two halves of a block run theirs side by side.
+// log2: some 40 clocks each): the parts of a block run theirs side by side.
 //
 // FULL = false (stage calls of a caller that keeps the workspace, e.g. the RK4
 // tape): every grid-only entry -- a, ia, inv_dx, the x copy, Bd, Sd, Ld, J0, the
@@ -182,7 +240,8 @@ __device__ __forceinline__ void prep_offsets(const double* __restrict__ x, int n
 // the pair kernel's last CTA counter[5] (the exact slots' list), so a
 // following call on the same workspace needs no memset.
 // ---------------------------------------------------------------------------
-constexpr int kPrepFullThreads = 2 * kPrepThreads;
+constexpr int kPrepFullThreads = 3 * kPrepThreads;
+constexpr int kPrepStageThreads = 2 * kPrepThreads;
 
 // First j <= i with fl(x_j + x_i) >= x_{i+1} (i when there is none below), from a
 // guess on the geometric grid through the end points, then galloping.
@@ -209,13 +268,15 @@ __device__ __forceinline__ int first_above(const double* __restrict__ x, int i, 
 }
 
 template <int K, bool FULL>
-__global__ void __launch_bounds__(FULL ? kPrepFullThreads : kPrepThreads)
+__global__ void __launch_bounds__(FULL ? kPrepFullThreads : kPrepStageThreads)
 agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int n, AggWs ws,
                 double b0, double bbr, double bsh)
 {
     __shared__ double dev_s[kPrepThreads / 32];
     __shared__ double gsum[2 * kMomN];
-    __shared__ double a_s[kPrepThreads];
+    __shared__ double wtot[kPrepThreads / 32][kWinMom];
+    __shared__ int neg_s[kPrepThreads / 32];
+    __shared__ double a_s[kPrepThreads], ia_s[kPrepThreads];
     __shared__ double ax0_s;
     __shared__ GeoFit fit_s;
     __shared__ int d0_s[kPrepThreads / 32];
@@ -227,11 +288,10 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
         double m[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
         double xm = 0.0;     // mantissa and binary exponent of x_i
         int E = 0;
-        double ai = 0.0;
+        double ai = 0.0, iai = 0.0, Ni = 0.0;
         if (i < n) {
-            const double Ni = N[i];
+            Ni = N[i];
             const double hi = xi * Ni;
-            double iai;
             if constexpr (FULL) {
                 ai = cbrt(xi);
                 iai = 1.0 / ai;
@@ -261,10 +321,27 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
         }
         if constexpr (FULL) {
             a_s[tid] = ai;
+            ia_s[tid] = iai;
             __syncwarp();
             asm volatile("bar.arrive 2, %0;" :: "n"(kPrepFullThreads) : "memory");
         }
+        const unsigned neg = __ballot_sync(0xffffffffu, !(Ni >= 0.0));   // negative, or NaN
+        if (lane == 0) neg_s[wp] = neg != 0u;
         prep_prefix<K>(m, xm, E, i, n, ws, gsum);
+    } else if (wp >= (FULL ? 4 : 2)) {
+        // window tables; FULL: the cube roots of the first two warps
+        if constexpr (FULL) asm volatile("bar.sync 2, %0;" :: "n"(kPrepFullThreads) : "memory");
+        if (win_grid(x, n)) {
+            double Ni = 0.0, ai = 0.0, iai = 0.0;
+            if (i < n) {
+                Ni = N[i];
+                ai = FULL ? a_s[tid & (kPrepThreads - 1)] : ws.a[i];
+                iai = FULL ? ia_s[tid & (kPrepThreads - 1)] : ws.ia[i];
+            }
+            const double hi = xi * Ni;
+            const double m[5] = {iai * Ni, Ni, ai * Ni, (ai * ai) * Ni, hi};
+            prep_windows<K>(m, xi, Ni, hi, i, n, ws, wtot, b0, bbr, bsh);
+        }
     } else if constexpr (FULL) {
         // the fit's end points on lanes 0 and 1 of the third warp, the cube root of
         // x_0 on the fourth, beside the bins' own logarithms
@@ -290,6 +367,18 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
             const int L = (dbits(v) >= dbits(x[n - 1])) ? kLagClipAll : bracket_from(x, n, v, i);
             ws.Ld[i] = L;
             if (L == i && i > 0) d0 = i;    // lag 0 carries the pair 1/2: never separated
+            // runs of lags with one bracket offset e = L - i: where this one ends,
+            // the last run, and the first run that windows sum (win_grid)
+            const int e = L - i;
+            if (L < kLagClipAll) {
+                const double vn = i + 1 < n ? x[0] + x[i + 1] : 0.0;
+                const bool over = i + 1 >= n || dbits(vn) >= dbits(x[n - 1]);
+                if (over || dbits(vn) < dbits(x[L + 1])) ws.rend[e] = i + 1;
+                if (over) ws.counter[9] = e;
+            }
+            const double start = kWinStart * x[0];
+            if (xi >= start && (i == 0 || x[i - 1] < start)) ws.counter[8] = L < kLagClipAll ? e - 1 : 0;
+            if (i == n - 1 && xi < start) ws.counter[8] = 0;
             ws.J0[i] = i < n - 1 ? first_above(x, i, xi, x[i + 1], lx0, inv_span) : i;
         }
         __syncwarp();
@@ -322,6 +411,7 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
             ws.mom_part[blockIdx.x * 8 + 5] = fmax(dev_s[0], dev_s[1]);
             ws.mom_part[blockIdx.x * 8 + 6] = static_cast<double>(min(d0_s[0], d0_s[1]));
         }
+        ws.mom_part[blockIdx.x * 8 + 7] = (neg_s[0] | neg_s[1]) ? 1.0 : 0.0;
         __threadfence();                       // partials visible before the ticket
         last_s = (atomicAdd(ws.counter + 2, 1) == static_cast<int>(gridDim.x) - 1);
     }
@@ -335,7 +425,13 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
     const int nb = gridDim.x;
     if (wp < 2) {
         prep_offsets<K>(x, n, nb, ws, wp, lane);
-    } else if (wp == 2) {
+        if (wp == 1) {
+            double neg = 0.0;
+            for (int b = lane; b < nb; b += 32) neg = fmax(neg, __ldcg(ws.mom_part + b * 8 + 7));
+            neg = warp_max(neg);
+            if (lane == 0) ws.mom[7] = neg;    // some N_i is negative or NaN
+        }
+    } else if (FULL && wp == 2) {
         double m5 = 0.0;
         for (int b = lane; b < nb; b += 32) m5 = fmax(m5, __ldcg(ws.mom_part + b * 8 + 5));
         m5 = warp_max(m5);
@@ -346,7 +442,7 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
             ws.mom[5] = geo ? 1.0 : 0.0;
             ws.mom[6] = m5;
         }
-    } else {
+    } else if (FULL && wp == 3) {
         int dmin = n;
         for (int b = lane; b < nb; b += 32)
             dmin = min(dmin, static_cast<int>(__ldcg(ws.mom_part + b * 8 + 6)));
@@ -401,6 +497,8 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
     __shared__ int s_flag;
     __shared__ int s_task;
     __shared__ double s_wsum[2 * kLaneWarps];
+    __shared__ double s_ex[2][32];
+    __shared__ unsigned s_mask;
 
     const int tid = threadIdx.x;
     LaneView v;
@@ -415,15 +513,22 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
         s_flag = 0;
     }
     __syncthreads();
-    constexpr int kRed = 2 * kLaneWarps * kLaneBins;     // per-warp R, TH of every slot
+    constexpr int kRed = 4 * kLaneWarps * kLaneBins;     // per-warp sums of every slot
     const LaneSmem lsm{lsmem, lsmem + kRed, lsmem + kRed + kLaneWinMax,
                        lsmem + kRed + 2 * kLaneWinMax};
     const int nblk = lane_blocks(n);
     // direct pairs of a slot: its lags below D0; on other grids at most its rows
-    const int parts = lane_parts(v.g.geo ? min(v.g.D0, n) : n, nblk, gridDim.x);
+    int Dm = min(v.g.D0, n), eh = 0, el = 1;
+    if (!SCATTER && v.g.geo && ws.mom[7] == 0.0 && win_grid(x, n)) {
+        eh = ws.counter[8];
+        el = max(1, ws.counter[9]);
+        if (eh >= el) Dm = ws.rend[eh + 1];
+    }
+    // (a window counts as 5 pairs)
+    const int parts = lane_parts(v.g.geo ? Dm + 5 * max(0, eh - el + 1) : n, nblk, gridDim.x);
     const int nexact = ws.counter[5];
     const int ntasks = nclip + nexact + nblk * parts;
-    const LaneArgs la{ws.Ncp, ws.xcp, ws.lpart, ws.cticket, ws.counter + 4, parts};
+    const LaneArgs la{ws.Ncp, ws.xcp, ws.lpart, ws.cticket, ws.counter + 4, parts, Dm, eh, el};
     unsigned phase = 0;
     for (;;) {
         if (tid == 0) s_task = atomicAdd(ws.counter, 1);
@@ -453,11 +558,13 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
         }
         task -= nclip;
         if (task < nexact) {
-            exact_slot_task<K, SCATTER>(v, ws, la, rhs, ws.xlist[task], nclip, s_wsum, s_flag != 0);
+            exact_slot_task<K, SCATTER>(v, ws, la, rhs, ws.xlist[task], nclip, s_wsum, s_flag != 0,
+                                        s_ex, &s_mask);
             continue;
         }
         task -= nexact;
-        lane_task<K, SCATTER>(v, ws, la, rhs, task % nblk, task / nblk, nclip, lsm, &s_bar, phase, &s_flag);
+        lane_task<K, SCATTER>(v, ws, la, rhs, task % nblk, task / nblk, nclip, lsm, &s_bar, phase, &s_flag,
+                              s_ex, &s_mask);
     }
     // the last CTA leaves the exact slots' list empty for the next prep
     if (tid == 0 && atomicAdd(ws.counter + 6, 1) == static_cast<int>(gridDim.x) - 1) ws.counter[5] = 0;
@@ -786,7 +893,7 @@ cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_
     const int nb = agg_prep_blocks(n);
     const int nclip = agg_clip_tasks(n);
     auto kern = agg_lane_kernel<K, SC>;
-    const size_t smem = sizeof(double) * (2 * kLaneWarps * kLaneBins + 3 * kLaneWinMax);
+    const size_t smem = sizeof(double) * (4 * kLaneWarps * kLaneBins + 3 * kLaneWinMax);
     // the number of tasks is known on the device only (it follows D0)
     const long long cap = static_cast<long long>(kLaneCtas) * num_sms;
     const long long most = static_cast<long long>(lane_blocks(n)) * kLaneMaxParts + nclip;
@@ -798,7 +905,7 @@ cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_
     if (e != cudaSuccess) return e;
     if (kind == kAggStage) {
         // counter[2] and [5] were left at 0 by the previous call on this workspace
-        agg_prep_kernel<K, false><<<nb, kPrepThreads, 0, s>>>(a.N, a.x, n, ws, a.beta0, a.beta_br,
+        agg_prep_kernel<K, false><<<nb, kPrepStageThreads, 0, s>>>(a.N, a.x, n, ws, a.beta0, a.beta_br,
                                                               a.beta_sh);
     } else {
         e = cudaMemsetAsync(ws.counter, 0, 8 * sizeof(int), s);   // prep's block tickets

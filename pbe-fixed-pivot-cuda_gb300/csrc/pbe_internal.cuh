@@ -272,10 +272,12 @@ struct AggWs {
     double* tcarry;    // [nblk] gather mode: the lower neighbour's carry into that bin
     int*    tticket;   // [nblk] contributors to the block's first bin done (0, 1, 2)
     int*    cticket;   // [nblk] tasks of the block done
-    int*    counter;   // [8]  [0] task counter, [1] first lag with Ld[d] == d,
+    int*    counter;   // [16] [0] task counter, [1] first lag with Ld[d] == d,
                        //      [2] prep blocks done, [3] bin n-1 contributors done,
                        //      [4] a staging wait of the lane tasks gave up, [5] entries of xlist,
-                       //      [6] CTAs of the pair kernel done
+                       //      [6] CTAs of the pair kernel done, [8] the first (largest)
+                       //      offset whose run is summed by windows, [9] the last run's
+                       //      offset (both grid-only)
     double* Ncp;       // [n + 2] copy of N, 256-byte aligned (bulk-copy source)
     double* xcp;       // [n + 2] copy of x, 256-byte aligned (bulk-copy source)
     double* lpart;     // [lane_partial_doubles(n)] lane-task chunk partials
@@ -287,10 +289,19 @@ struct AggWs {
     double* mloc;      // [2 kMomN n]
     double* mtot;      // [2 kMomN nb_prep] block totals
     double* moff;      // [2 kMomN nb_prep]
+    // Window tables (prep_windows; fine geometric grids): with M_m = x^(m/3) N, m =
+    // -1..6, wtab[(v 8 + m + 1) n + i] for v = 0..3 the sum from i to the middle of
+    // its aligned block of 2^(v+3) bins (suffix in the left half, prefix in the
+    // right half), v = 4 / 5 the prefix / suffix sum within i's block of 64 bins
+    double* wtab;      // [6 * 8 n]
+    double* wc;        // [kMomN n] N_i times beta's coefficient of m_q(x_j) at x_k = x_i
+    int*    rend;      // [n + 1] end (exclusive) of the run of lags with bracket offset e
     int*    xlist;     // [n] slots whose lags from D0 on keep the exact pair sum, counter[5] of them
     double* xsum;      // [2 n] their R, TH
 };
 constexpr int kMomN = 5;               // moments per prefix (the death term's)
+constexpr int kWinMom = 8;             // moments of a window: kMomN of N and, x_j / x_j^(-1/3) on, of x N
+constexpr int kWinTabs = 6 * kWinMom;  // window table values per bin
 
 __host__ __device__ constexpr int agg_prep_blocks(int n) { return (n + kPrepThreads - 1) / kPrepThreads; }
 
@@ -388,11 +399,11 @@ __host__ __device__ inline int lane_last_rank(int n, int t, int C)
 }
 
 // Lane tasks of the aggregation pair kernel: each block's direct lags cut into
-// `parts` equal shares, (R, TH) partials of kLaneBins slots per share.
+// `parts` equal shares, four partial sums of kLaneBins slots per share.
 constexpr int kLaneMaxParts = 8;
 __host__ __device__ constexpr size_t lane_partial_doubles(int n)
 {
-    return static_cast<size_t>(lane_blocks(n)) * kLaneMaxParts * 2 * kLaneBins;
+    return static_cast<size_t>(lane_blocks(n)) * kLaneMaxParts * 4 * kLaneBins;
 }
 
 // Size of the aggregation scratch for n bins, equal to agg_ws_layout(n) below
@@ -406,13 +417,16 @@ constexpr size_t agg_ws_bytes(int n)
          + align256(sizeof(double) * kMaxClipTasks)
          + 2 * align256(sizeof(double) * static_cast<size_t>(lane_blocks(n)))
          + 2 * align256(sizeof(int) * static_cast<size_t>(lane_blocks(n)))
-         + align256(sizeof(int) * 8)
+         + align256(sizeof(int) * 16)
          + 2 * align256(sizeof(double) * (static_cast<size_t>(n) + 2))
          + align256(sizeof(double) * lane_partial_doubles(n))
          + align256(sizeof(double) * 2 * kMomN * static_cast<size_t>(n))
          + 2 * align256(sizeof(double) * 2 * kMomN * static_cast<size_t>(agg_prep_blocks(n)))
          + align256(sizeof(int) * static_cast<size_t>(n))
-         + align256(sizeof(double) * 2 * static_cast<size_t>(n));
+         + align256(sizeof(double) * 2 * static_cast<size_t>(n))
+         + align256(sizeof(double) * kWinTabs * static_cast<size_t>(n))
+         + align256(sizeof(double) * kMomN * static_cast<size_t>(n))
+         + align256(sizeof(int) * (static_cast<size_t>(n) + 1));
 }
 
 // Carves the aggregation scratch out of `base` (may be null to query the size).
@@ -438,7 +452,7 @@ inline size_t agg_ws_layout(int n, char* base, AggWs* ws)
     w.tcarry    = reinterpret_cast<double*>(take(sizeof(double) * nt));
     w.tticket   = reinterpret_cast<int*>(take(sizeof(int) * nt));
     w.cticket   = reinterpret_cast<int*>(take(sizeof(int) * nt));
-    w.counter   = reinterpret_cast<int*>(take(sizeof(int) * 8));
+    w.counter   = reinterpret_cast<int*>(take(sizeof(int) * 16));
     w.Ncp       = reinterpret_cast<double*>(take(sizeof(double) * (static_cast<size_t>(n) + 2)));
     w.xcp       = reinterpret_cast<double*>(take(sizeof(double) * (static_cast<size_t>(n) + 2)));
     w.lpart     = reinterpret_cast<double*>(take(sizeof(double) * lane_partial_doubles(n)));
@@ -448,6 +462,9 @@ inline size_t agg_ws_layout(int n, char* base, AggWs* ws)
     w.moff      = reinterpret_cast<double*>(take(nbm));
     w.xlist     = reinterpret_cast<int*>(take(sizeof(int) * static_cast<size_t>(n)));
     w.xsum      = reinterpret_cast<double*>(take(sizeof(double) * 2 * static_cast<size_t>(n)));
+    w.wtab      = reinterpret_cast<double*>(take(sizeof(double) * kWinTabs * static_cast<size_t>(n)));
+    w.wc        = reinterpret_cast<double*>(take(sizeof(double) * kMomN * static_cast<size_t>(n)));
+    w.rend      = reinterpret_cast<int*>(take(sizeof(int) * (static_cast<size_t>(n) + 1)));
     if (ws) *ws = w;
     return off;
 }

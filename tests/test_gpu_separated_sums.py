@@ -86,3 +86,23 @@ def test_separated_jvp_matches_oracle(kernel, b0, bbr, bsh, grid):
                             out, prm) == 0
             for got, (x, N, v, ref, scale, what) in zip(plan.split(out.cpu().numpy()), group):
                 assert_close(got, ref, scale, "jvp " + what)
+
+
+@pytest.mark.parametrize("n,q", [(497, 64.0), (641, 64.0), (700, 512.0), (1500, 128.0), (3000, 256.0)])
+@pytest.mark.parametrize("kernel,b0,bbr,bsh", AGG_KERNELS, ids=[str(k[0]) for k in AGG_KERNELS])
+def test_window_sums_match_oracle(kernel, b0, bbr, bsh, n, q):
+    """Fine grids, where runs of lags with one bracket offset are summed by window
+    tables: windows within a block of 64 bins, across one edge and across whole
+    blocks, cut at bin 0; a grid that ends before the lags that land on their larger
+    member (n = 700, q = 512); populations the windows' rounding rule rejects, and
+    one with a negative entry (no windows at all)."""
+    rng = np.random.default_rng(90 + kernel)
+    x = pg.grids.geometric_pow2(n, 1e-21, q)
+    p = agg_params(n, kernel, b0, bbr, bsh, x)
+    for what, N in [*populations(x, rng), ("sparse", np.where(np.arange(n) % 97 == 5, 1e9, 0.0)),
+                    ("negative", -np.abs(rng.standard_normal(n)) + 0.5)]:
+        ref, scale, _ = oracle_agg(N, x, p)
+        for mode in (pg.MODE_GATHER, pg.MODE_SCATTER):
+            code, got = gpu_agg(N, x, p, mode)
+            assert code == 0
+            assert_close(got, ref, scale, "k=%d n=%d q=%g %s mode %d" % (kernel, n, q, what, mode))
