@@ -39,7 +39,7 @@
 // M_m = sum over the window of x_j^(m/3) N_j, from two table values (and whole
 // blocks of 64 between them): windows of any length and place without a
 // subtraction, so sums of one sign keep their relative precision. At 512 sections
-// an octave 1324 lags stay pairs and 137 runs cover the other 3560. The rounding of
+// an octave 1189 lags stay pairs and 135 runs cover the other 3690. The rounding of
 // fl(x_j + x_k), left out as above, moves bins s and s + 1 by at most u R_win; the
 // finishing warp compares that with what these bins are known to receive and lose
 // (kMomGuard), and slots beyond it sum those lags pair by pair.
@@ -47,40 +47,35 @@
 // On other grids the same holds for the rows j < J0(s), the first j with
 // fl(x_j + x_s) >= x_{s+1}.
 //
-// Work split: blocks of 32 output bins aligned to the top of the grid (block
-// t owns bins [n - 32 (t + 1), n - 32 t), so bin n - 1 is never a block's first
-// bin); a task is one block and one of `parts` equal shares of the lags below D0
+// Work split: blocks of 31 output bins aligned to the top of the grid (slot_blocks);
+// a task is one block and one of `parts` equal shares of the lags below D0
 // (of each slot's rows on other grids); the CTA's eight warps take equal
 // contiguous shares of the task's lags (each warp sees its runs in order) and
 // their sums are added in warp order. With several parts each task stores its
-// 4 x 32 sums; the block's last task (ticket) adds them in order and writes the
-// bins -- deterministic, nobody waits.
+// 5 x 32 sums; the block's last task (ticket) adds them in order and writes the
+// bins -- deterministic, nobody waits. Beside its pairs a task is a chain of
+// latencies of a microsecond each (n = 3840: 24 of 41 us once, 19 of 37 now), so
+// the prefix part and the death term come from a warp of share 0 while the others
+// sum pairs, and the slot below a block's first bin is summed twice instead of
+// handed over.
 //
-// Operand staging (geometric grids): the j-side operands of a task (N_j,
-// x_j N_j, x_j for j in one contiguous window of at most kLaneWinMax entries)
-// are copied into shared memory with bulk TMA copies (cp.async.bulk, mbarrier
-// completion).
+// The j-side operands are read through L1: a share's window (32 + its lags entries
+// of N, x N and x) staged in shared memory by bulk copies measured the same with
+// these shorter shares (n = 3840: 37.5 and 37.5 us, n = 16384: 291.5 and 291.5).
 // =============================================================================
 #pragma once
-
-#include <cstdint>
 
 #include "agg_slot.cuh"
 
 namespace pbe_gb300 {
 
 constexpr int kLaneWarps = kMainThreads / 32;       // warps sharing a task's lags
-constexpr int kLaneWinMax = 1792;                   // staged window, entries per array (even)
-// Bounded waits on the staging barrier: iterations of mbarrier.try_wait.
-constexpr long long kLaneWaitLimit = 1LL << 26;
-
 // Shares of a block's pairs (`lags`: pairs of a slot). Long shares: enough tasks
 // to give every CTA four, so that the last ones end together. A task costs a few
 // microseconds beside its pairs (fetch, staging, sums, ticket), so where that would
 // leave a share less than 192 pairs a slot, as many shares as fit the CTAs in one
 // round (n = 3840, 456 CTAs: 8 shares in two rounds 57 us, 3 shares in one 42). At
-// least 32 pairs a share (4 per warp). A share longer than the staged window reads
-// its operands from the arrays.
+// least 32 pairs a share (4 per warp).
 __host__ __device__ constexpr int lane_parts(int lags, int nblk, int ctas)
 {
     int p = (4 * ctas + nblk - 1) / nblk;
@@ -91,62 +86,19 @@ __host__ __device__ constexpr int lane_parts(int lags, int nblk, int ctas)
     return p < 1 ? 1 : p;
 }
 
-// ---- bulk TMA copy + mbarrier helpers (shared::cta addresses) -----------------
-__device__ __forceinline__ unsigned smem_addr(const void* p)
-{
-    return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_addr(bar)), "r"(count) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                 :: "r"(smem_addr(bar)), "r"(bytes) : "memory");
-}
-// global -> shared bulk copy; dst, src 16-byte aligned, bytes a multiple of 16.
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 :: "r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar)) : "memory");
-}
-// Waits for the barrier's phase `parity` to complete; false after kLaneWaitLimit tries.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity)
-{
-    const unsigned a = smem_addr(bar);
-    for (long long it = 0; it < kLaneWaitLimit; ++it) {
-        unsigned done;
-        asm volatile("{\n\t.reg .pred p;\n\t"
-                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                     "selp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done) : "r"(a), "r"(parity) : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-__device__ __forceinline__ void fence_proxy_async_smem()
-{
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-// Shared memory of a lane task (carved from the kernel's dynamic buffer).
+// Shared memory of a CTA.
 struct LaneSmem {
-    double* red;     // [kLaneWarps][4][32] per-warp R, TH of the pairs and of the windows
-    double* wN;      // [kLaneWinMax] staged N_j   (K needs N on the j side)
-    double* wH;      // [kLaneWinMax] staged x_j N_j
-    double* wX;      // [kLaneWinMax] staged x_j
+    double red[kLaneWarps][4][32];   // per-warp R, TH of the pairs and of the windows
+    double D[32];                    // the bins' death terms
+    double sum[2 * kLaneWarps];      // CTA-wide sums
+    unsigned mask;
+    int task;
 };
 
-// Staged copies of N and x (scratch, 256-byte aligned, at least n + 2 entries)
-// and the chunk partials / tickets of the lane path.
+// The shares of the blocks and what they sum.
 struct LaneArgs {
-    const double* Ncp;   // N copy
-    const double* xcp;   // x copy
     double* part;        // [lane_partial_doubles(n)]
-    int* ticket;         // [lane_blocks(n)] tasks of the block done (reset by the prep)
-    int* err;            // set to 1 when a staging wait gave up
+    int* ticket;         // [slot_blocks(n)] tasks of the block done (reset by the prep)
     int parts;           // tasks per block
     int Dm;              // lags summed pair by pair (geometric grids)
     int eh, el;          // runs eh .. el (descending) summed by windows; eh < el: none
@@ -180,16 +132,17 @@ __device__ __forceinline__ void prefix_moments(const AggWs& ws, const double* __
 // Slots of block t (one per lane) whose prefix part is summed pair by pair.
 __device__ __forceinline__ unsigned exact_mask(const LaneView& v, int t)
 {
-    const int s = v.g.n - kLaneBins * (t + 1) + (threadIdx.x & 31);
-    const bool e = s >= 0 && s <= lane_block_smax(v.g.n, t) && slot_cut(v.g, s) > 0 &&
+    const int n = v.g.n, s = n - kSlotBins * (t + 1) - 1 + (threadIdx.x & 31);
+    const bool e = s >= 0 && s <= n - 2 && slot_cut(v.g, s) > 0 &&
                    mom_exact_slot(__ldg(v.p.Nk + s), __ldg(v.p.Nk + s + 1), __ldg(v.g.x + s + 1),
-                                  __ldg(v.g.inv_dx + s));
+                                  v.g.inv_dx[s]);
     return __ballot_sync(0xffffffffu, e);
 }
 
-// The sums of a slot: pairs (and prefix part), windows.
+// The sums of a lane: its slot's pairs and prefix part, its windows, its bin's
+// death term (less what is clipped from the prefix part of slot n - 1).
 struct SlotSums {
-    double R, TH, Rw, Tw;
+    double R, TH, Rw, Tw, D;
 };
 
 // One warp, after its contribution to block t is stored: the block's ticket.
@@ -206,20 +159,48 @@ __device__ __forceinline__ bool block_ticket(const AggWs& ws, const LaneArgs& la
     if (lane == 0) last = (atomicAdd(la.ticket + t, 1) == want - 1);
     if (!__shfl_sync(0xffffffffu, last, 0)) return false;
     __threadfence();
-    u = SlotSums{0.0, 0.0, 0.0, 0.0};
-    const double* bp = la.part + static_cast<size_t>(t) * la.parts * 128 + lane;
-    for (int q = 0; q < la.parts; ++q, bp += 128) {
+    u = SlotSums{0.0, 0.0, 0.0, 0.0, 0.0};
+    const double* bp = la.part + static_cast<size_t>(t) * la.parts * kLanePart + lane;
+    for (int q = 0; q < la.parts; ++q, bp += kLanePart) {
         u.R += __ldcg(bp);
         u.TH += __ldcg(bp + 32);
         u.Rw += __ldcg(bp + 64);
         u.Tw += __ldcg(bp + 96);
+        if (q == 0) u.D = __ldcg(bp + 128);
     }
     if ((exact >> lane) & 1u) {
-        const int s = n - kLaneBins * (t + 1) + lane;
+        const int s = n - kSlotBins * (t + 1) - 1 + lane;
         u.R += __ldcg(ws.xsum + 2 * s);
         u.TH += __ldcg(ws.xsum + 2 * s + 1);
     }
     return true;
+}
+
+// One warp: the prefix part of block t's slots (but the exact ones) and the death
+// term of its bins.
+template <int K>
+__device__ __forceinline__ void lane_base(const LaneView& v, const AggWs& ws, int t, unsigned exact,
+                                          double& R, double& TH, double& D)
+{
+    const int n = v.g.n, lane = threadIdx.x & 31;
+    const int s = n - kSlotBins * (t + 1) - 1 + lane;
+    R = TH = D = 0.0;
+    if (s < 0 || s >= n) return;
+    const double as = v.g.a[s], ias = v.g.ia[s], xv = __ldg(v.g.x + s), Ns = __ldg(v.p.Nk + s);
+    const int cut = slot_cut(v.g, s);
+    if (cut > 0 && !((exact >> lane) & 1u)) {
+        double P[kMomN], T[kMomN];
+        prefix_moments<K>(ws, v.g.x, n, cut - 1, P, T);
+        const double r = Ns * death_factor<K>(xv, as, ias, P, v.g.b0, v.g.bbr, v.g.bsh);
+        const double th = Ns * death_factor<K>(xv, as, ias, T, v.g.b0, v.g.bbr, v.g.bsh);
+        if (s <= n - 2) {
+            R = r;
+            TH = scale_down(th, exponent_of(__ldg(v.g.x + cut - 1)) - exponent_of(xv));
+        } else {
+            D = -r;                                    // clipped: all of it stays in bin n - 1
+        }
+    }
+    D += Ns * death_factor<K>(xv, as, ias, v.M, v.g.b0, v.g.bbr, v.g.bsh);
 }
 
 // The runs eh .. el of slot s by windows: Rw += rates, Tw += rates (v - x_s), not
@@ -274,157 +255,101 @@ __device__ __forceinline__ void lane_windows(const LaneView& v, const AggWs& ws,
     }
 }
 
-// The lags [Dm, D0) of slot s pair by pair, by one warp (lanes over the lags,
-// fixed butterfly). Valid in every lane.
+// The lags [Dm, D0) of slot s pair by pair, by the CTA (threads over the lags),
+// summed in a fixed order; red: 2 kLaneWarps doubles of shared memory. Valid in
+// every thread; CTA synchronised.
 template <int K>
-__device__ __forceinline__ void exact_runs(const LaneView& v, int s, int Dm, double& R, double& TH)
+__device__ __forceinline__ void exact_runs(const LaneView& v, int s, int Dm, double* red, double& R,
+                                           double& TH)
 {
-    const int lane = threadIdx.x & 31;
     const double xs = __ldg(v.g.x + s);
     const EwOperandC pc = ew_operand_c(xs, -exponent_of(xs));
     double r = 0.0, t = 0.0;
-    for (int d = Dm + lane; d < min(v.g.D0, v.g.n); d += 32) {
-        const int L = __ldg(v.g.Ld + d);
+    for (int d = Dm + static_cast<int>(threadIdx.x); d < min(v.g.D0, v.g.n); d += kMainThreads) {
+        const int L = v.g.Ld[d];
         const int j = s - L, k = j + d;
         if (j < 0) break;                              // Ld is nondecreasing
-        const double rate = rate_geo<K>(__ldg(v.g.Bd + d), __ldg(v.g.Sd + d), __ldg(v.p.Nj + j),
-                                        NeedH<K>::j ? __ldg(v.p.Hj + j) : 0.0, __ldg(v.p.Nk + k),
-                                        NeedH<K>::k ? __ldg(v.p.Hk + k) : 0.0);
+        const double rate = rate_geo<K>(v.g.Bd[d], v.g.Sd[d], __ldg(v.p.Nj + j),
+                                        NeedH<K>::j ? v.p.Hj[j] : 0.0, __ldg(v.p.Nk + k),
+                                        NeedH<K>::k ? v.p.Hk[k] : 0.0);
         r += rate;
         t = fma(rate, sum_minus_scaled_pre(ew_operand_a(__ldg(v.g.x + k)), __ldg(v.g.x + j), pc), t);
     }
-    R = warp_sum(r);
-    TH = warp_sum(t);
+    r = warp_sum(r);
+    t = warp_sum(t);
+    if ((threadIdx.x & 31) == 0) { red[2 * (threadIdx.x >> 5)] = r; red[2 * (threadIdx.x >> 5) + 1] = t; }
+    __syncthreads();
+    R = TH = 0.0;
+    for (int q = 0; q < kLaneWarps; ++q) { R += red[2 * q]; TH += red[2 * q + 1]; }
+    __syncthreads();
 }
 
-// The bins of block t from its slots' sums (a slot per lane of warp 0), by the
-// CTA; `finish` and u are warp 0's. With `first` the prefix part (not of the exact
-// slots) and the death term are added; scatter mode calls it for every share's own
-// sums. s_ex: shared memory, [2][32] and a mask behind it.
+// The bins of block t from its lanes' sums in warp 0, by the CTA; `finish` and u
+// are warp 0's. Scatter mode calls it for every share's own sums.
 template <int K, bool SCATTER>
 __device__ void lane_finish(const LaneView& v, const AggWs& ws, const LaneArgs& la, double* rhs, int t,
-                            int nclip, unsigned exact, bool finish, bool first, bool poisoned,
-                            SlotSums u, double (*s_ex)[32], unsigned* s_mask)
+                            int nclip, bool finish, SlotSums u, LaneSmem& sm)
 {
     const int n = v.g.n, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int I = n - kLaneBins * (t + 1);
-    const int smax = lane_block_smax(n, t);
-    const int s = I + lane, i = s;
-    const bool slot = s >= 0 && s <= smax;
-    double clip0 = 0.0;                                // the prefix part of the clipped slot n - 1
-    double death = 0.0, sd = 0.0, own = 0.0, up = 0.0;
-    int St = 0;
-    if (w == 0 && finish) {
-        const double xs = slot ? __ldg(v.g.x + s) : 0.0;
-        St = slot ? -exponent_of(xs) : 0;
-        if (first && s >= 0 && s <= n - 1) {
-            const double as = __ldg(v.g.a + s), ias = __ldg(v.g.ia + s), xv = __ldg(v.g.x + s);
-            const double Ns = __ldg(v.p.Nk + s);
-            death = Ns * death_factor<K>(xv, as, ias, v.M, v.g.b0, v.g.bbr, v.g.bsh);
-            const int cut = slot_cut(v.g, s);
-            if (cut > 0 && !((exact >> lane) & 1u)) {
-                double P[kMomN], T[kMomN];
-                prefix_moments<K>(ws, v.g.x, n, cut - 1, P, T);
-                const double r = Ns * death_factor<K>(xv, as, ias, P, v.g.b0, v.g.bbr, v.g.bsh);
-                const double th = Ns * death_factor<K>(xv, as, ias, T, v.g.b0, v.g.bbr, v.g.bsh);
-                if (slot) {
-                    u.R += r;
-                    u.TH += scale_down(th, exponent_of(__ldg(v.g.x + cut - 1)) + St);
-                } else {
-                    clip0 = r;
-                }
-            }
-        }
+    const int s = n - kSlotBins * (t + 1) - 1 + lane;  // this lane's slot and bin
+    const bool slot = s >= 0 && s <= n - 2;
+    double sd = 0.0, own = 0.0, up = 0.0;              // the slot's own part of bin s, its w-part of bin s + 1
+    if (w == 0 && finish && slot) {
+        const int St = -exponent_of(__ldg(v.g.x + s));
         u.Tw = scalbn(u.Tw, St);
-        // own part of bin i (slot i) and the w-part of slot i, owed to bin i + 1
-        if (slot) {
-            const double idx = __ldg(v.g.inv_dx + i);
-            sd = scalbn(idx, -St);
-            own = fma(-(u.TH + u.Tw), sd, u.R + u.Rw);
-            up = (u.TH + u.Tw) * sd;
-        }
+        sd = scalbn(v.g.inv_dx[s], -St);
+        own = fma(-(u.TH + u.Tw), sd, u.R + u.Rw);
+        up = (u.TH + u.Tw) * sd;
     }
     if (!SCATTER && la.eh >= la.el) {
         // windows: slots where the rounding they leave out may show in bin s or s + 1
         if (w == 0) {
             bool ex = false;
             const double below = __shfl_up_sync(0xffffffffu, up, 1);
-            const double dn = __shfl_down_sync(0xffffffffu, death, 1);
+            const double dn = __shfl_down_sync(0xffffffffu, u.D, 1);
             const double on = __shfl_down_sync(0xffffffffu, own, 1);
             if (finish && slot && u.Rw != 0.0) {
                 const double xu = __ldg(v.g.x + s + 1);
-                const double err = (1.1102230246251565e-16 * (xu * __ldg(v.g.inv_dx + s))) * u.Rw;
-                double dup = dn;
+                const double err = (1.1102230246251565e-16 * (xu * v.g.inv_dx[s])) * u.Rw;
+                double dup = fmax(dn, 0.0);
                 if (lane == 31)
-                    dup = __ldg(v.p.Nk + s + 1) * death_factor<K>(xu, __ldg(v.g.a + s + 1), __ldg(v.g.ia + s + 1),
+                    dup = __ldg(v.p.Nk + s + 1) * death_factor<K>(xu, v.g.a[s + 1], v.g.ia[s + 1],
                                                                   v.M, v.g.b0, v.g.bbr, v.g.bsh);
-                const double here = fmax(own, 0.0) + (lane > 0 ? below : 0.0) + death;
+                const double here = fmax(own, 0.0) + (lane > 0 ? below : 0.0) + u.D;
                 const double next = up + (lane < 31 ? fmax(on, 0.0) : 0.0) + dup;
-                ex = !(err <= kMomGuard * here && err <= kMomGuard * next);
+                // (slot I - 1 matters to bin I alone here)
+                ex = !((lane == 0 || err <= kMomGuard * here) && err <= kMomGuard * next);
             }
             const unsigned m = __ballot_sync(0xffffffffu, ex);
-            if (lane == 0) *s_mask = m;
+            if (lane == 0) sm.mask = m;
         }
         __syncthreads();
-        const unsigned mask = *s_mask;
-        if (mask != 0u) {
-            int turn = 0;
-            for (unsigned m = mask; m != 0u; m &= m - 1u, turn = (turn + 1) & (kLaneWarps - 1)) {
-                if (turn != w) continue;
-                const int le = __ffs(m) - 1;
-                double r, th;
-                exact_runs<K>(v, I + le, la.Dm, r, th);
-                if (lane == 0) { s_ex[0][le] = r; s_ex[1][le] = th; }
-            }
-            __syncthreads();
-            if (w == 0 && ((mask >> lane) & 1u)) {
-                own = fma(-(u.TH + s_ex[1][lane]), sd, u.R + s_ex[0][lane]);
-                up = (u.TH + s_ex[1][lane]) * sd;
+        for (unsigned m = sm.mask; m != 0u; m &= m - 1u) {
+            const int le = __ffs(m) - 1;
+            double r, th;
+            exact_runs<K>(v, n - kSlotBins * (t + 1) - 1 + le, la.Dm, sm.sum, r, th);
+            if (w == 0 && lane == le) {
+                own = fma(-(u.TH + th), sd, u.R + r);
+                up = (u.TH + th) * sd;
             }
         }
     }
     if (w != 0 || !finish) return;
     const double in = __shfl_up_sync(0xffffffffu, up, 1);
-    if (i >= 0) {
-        double val = own;
-        if (lane >= 1) val += in;
-        val += clip0;
-        val -= death;
-        if constexpr (SCATTER) {
-            if (val != 0.0) atomicAdd(rhs + i, val);
-        } else {
-            if (poisoned) val = __longlong_as_double(0x7ff8000000000000LL);
-            if (lane == 0 && I >= 1) {
-                ws.tfirst[t] = val;
-                __threadfence();
-                if (atomicAdd(ws.tticket + t, 1) == 1) {
-                    __threadfence();
-                    rhs[I] = __ldcg(rhs + I) + (__ldcg(ws.tfirst + t) + __ldcg(ws.tcarry + t));
-                }
-            } else {
-                rhs[i] = rhs[i] + val;
-                if (i == n - 1) {
-                    __threadfence();
-                    if (atomicAdd(ws.counter + 3, 1) == nclip) {
-                        __threadfence();
-                        double sc = 0.0;
-                        for (int q = 0; q < nclip; ++q) sc += __ldcg(ws.clip_part + q);
-                        rhs[n - 1] = __ldcg(rhs + (n - 1)) + sc;
-                    }
-                }
-            }
-        }
-    }
     if constexpr (SCATTER) {
-        if (lane == 31 && slot && up != 0.0) atomicAdd(rhs + i + 1, up);
-    } else if (lane == 31 && t >= 1) {
-        // carry into bin I + 32, the first bin of block t - 1
-        ws.tcarry[t - 1] = up;
-        __threadfence();
-        if (atomicAdd(ws.tticket + (t - 1), 1) == 1) {
+        // (slot I - 1: its w-part enters bin I as `in`; slot I + 30's leaves by lane 0 above)
+        const double val = (own + in) - u.D;
+        if (lane >= 1 && s >= 0 && val != 0.0) atomicAdd(rhs + s, val);
+    } else if (lane >= 1 && s >= 0) {
+        rhs[s] = rhs[s] + ((own + in) - u.D);
+        if (s == n - 1) {
             __threadfence();
-            const int J = I + kLaneBins;
-            rhs[J] = __ldcg(rhs + J) + (__ldcg(ws.tfirst + t - 1) + __ldcg(ws.tcarry + t - 1));
+            if (atomicAdd(ws.counter + 3, 1) == nclip) {
+                __threadfence();
+                double sc = 0.0;
+                for (int q = 0; q < nclip; ++q) sc += __ldcg(ws.clip_part + q);
+                rhs[n - 1] = __ldcg(rhs + (n - 1)) + sc;
+            }
         }
     }
 }
@@ -432,216 +357,113 @@ __device__ void lane_finish(const LaneView& v, const AggWs& ws, const LaneArgs& 
 // The prefix part of one exact slot, pair by pair: the CTA over j, summed in
 // a fixed order. Such slots cluster at the foot of a population, so each is a
 // task of its own (summed by its block's last task, 90 of them on a run of 3840
-// bins made the whole call 1.5 x slower). `red`: 2 kLaneWarps doubles.
+// bins made the whole call 1.5 x slower). red: 2 kLaneWarps doubles.
 template <int K, bool SCATTER>
 __device__ void exact_slot_task(const LaneView& v, const AggWs& ws, const LaneArgs& la,
-                                double* rhs, int s, int nclip, double* red, bool poisoned,
-                                double (*s_ex)[32], unsigned* s_mask)
+                                double* rhs, int s, int nclip, LaneSmem& sm)
 {
     const int n = v.g.n, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    const int t = (n - 1 - s) / kLaneBins;
     const int cut = slot_cut(v.g, s);
-    if (cut <= 0 || s > lane_block_smax(n, t)) return;   // no such pairs (the whole CTA)
-    const double xe = __ldg(v.g.x + s);
-    const int St = -exponent_of(xe);
+    if (cut <= 0 || s > n - 2) return;                 // no such pairs (the whole CTA)
     double r, th;
     slot_exact_part<K, 1>(v.g, &v.p, s, tid, kMainThreads, r, th);
     r = warp_sum(r);
     th = warp_sum(th);
-    if (lane == 0) { red[2 * w] = r; red[2 * w + 1] = th; }
+    if (lane == 0) { sm.sum[2 * w] = r; sm.sum[2 * w + 1] = th; }
     __syncthreads();
-    SlotSums u{0.0, 0.0, 0.0, 0.0};
-    unsigned em = 0u;
-    bool finish = false;
-    if (w == 0) {
-        r = 0.0;
-        th = 0.0;
-        for (int q = 0; q < kLaneWarps; ++q) { r += red[2 * q]; th += red[2 * q + 1]; }
-        if constexpr (SCATTER) {
-            if (lane == 0) {
-                const double co = th * scalbn(__ldg(v.g.inv_dx + s), -St);
-                atomicAdd(rhs + s, r - co);
-                if (co != 0.0) atomicAdd(rhs + s + 1, co);
-            }
-        } else {
-            if (lane == 0) {
-                ws.xsum[2 * s] = r;
-                ws.xsum[2 * s + 1] = th;
-            }
-            em = exact_mask(v, t);
-            finish = block_ticket(ws, la, n, t, em, u);
-        }
-    }
-    if constexpr (!SCATTER)
-        lane_finish<K, false>(v, ws, la, rhs, t, nclip, em, finish, true, poisoned, u, s_ex, s_mask);
+    r = 0.0;
+    th = 0.0;
+    for (int q = 0; q < kLaneWarps; ++q) { r += sm.sum[2 * q]; th += sm.sum[2 * q + 1]; }
     __syncthreads();
-}
-
-// The lags [dw0, dw1) of a warp's slots on a geometric grid, with the operands of
-// the task staged (pN, pH, pX indexed by j).
-template <int K>
-__device__ __forceinline__ void lane_pairs(const LaneView& v, int s, bool slot, int dw0, int dw1,
-                                           const double* pN, const double* pH, const double* pX,
-                                           double& R, double& TH)
-{
-    const double xs = slot ? __ldg(v.g.x + s) : 0.0;
-    const EwOperandC pc = ew_operand_c(xs, slot ? -exponent_of(xs) : 0);   // the slot pivot, decoded once
-    EwOperandA pa = ew_operand_a(0.0);                // x_k of the current run
-    double Q = 0.0, QT = 0.0, F = 0.0, hk = 0.0;
-    int e_cur = -1;
-    for (int d = dw0; d < dw1; ++d) {
-        const int L = __ldg(v.g.Ld + d);
-        const int e = L - d;
-        if (e != e_cur) {                              // uniform across the warp
-            if constexpr (K != 1) {
-                R = fma(F, Q, R);
-                TH = fma(F, QT, TH);
-                Q = 0.0;
-                QT = 0.0;
-            }
-            e_cur = e;
-            const int k = s - e;
-            const bool kin = slot && k >= 0;
-            F = kin ? __ldg((K == 2 ? v.p.Hk : v.p.Nk) + k) : 0.0;
-            pa = ew_operand_a(kin ? __ldg(v.g.x + k) : 0.0);
-            if constexpr (K == 1) hk = kin ? __ldg(v.p.Hk + k) : 0.0;
+    if constexpr (SCATTER) {
+        if (tid == 0) {
+            const double co = th * scalbn(v.g.inv_dx[s], exponent_of(__ldg(v.g.x + s)));
+            atomicAdd(rhs + s, r - co);
+            if (co != 0.0) atomicAdd(rhs + s + 1, co);
         }
-        const double B = __ldg(v.g.Bd + d), S = __ldg(v.g.Sd + d);
-        const int j = s - L;
-        if (slot && j >= 0) {
-            const double Nj = pN[j];
-            const double hj = NeedH<K>::j ? pH[j] : 0.0;
-            const double th = sum_minus_scaled_pre(pa, pX[j], pc);
-            if constexpr (K != 1) {
-                const double q = q_slot<K>(B, S, Nj, hj);
-                Q += q;
-                QT = fma(q, th, QT);
-            } else {
-                const double rate = rate_geo<1>(B, S, Nj, hj, F, hk);
-                R += rate;
-                TH = fma(rate, th, TH);
-            }
+    } else {
+        if (tid == 0) {
+            ws.xsum[2 * s] = r;
+            ws.xsum[2 * s + 1] = th;
         }
-    }
-    if constexpr (K != 1) {
-        R = fma(F, Q, R);
-        TH = fma(F, QT, TH);
+        // the slot's own block, and the one above when the slot is the one below its bins
+        const int up = n - 1 - s, t1 = up / kSlotBins;
+        for (int t = t1; t >= 0 && (t == t1 || (t == t1 - 1 && up % kSlotBins == 0)); --t) {
+            SlotSums u{0.0, 0.0, 0.0, 0.0, 0.0};
+            bool finish = false;
+            if (w == 0) finish = block_ticket(ws, la, n, t, exact_mask(v, t), u);
+            lane_finish<K, false>(v, ws, la, rhs, t, nclip, finish, u, sm);
+            __syncthreads();
+        }
     }
 }
 
 // One lane task: block t, share c of its direct pairs. All kMainThreads threads
-// of the CTA take part; returns with the CTA synchronised. `phase` is the staging
-// barrier's parity (flipped per staged task). Gather mode stores / finishes
-// the block's bins; scatter mode flushes this task's share with atomics.
+// of the CTA take part; returns with the CTA synchronised. Gather mode stores /
+// finishes the block's bins; scatter mode flushes this task's share with atomics.
 template <int K, bool SCATTER>
 __device__ void lane_task(const LaneView& v, const AggWs& ws, const LaneArgs& la, double* rhs,
-                          int t, int c, int nclip, const LaneSmem& sm, uint64_t* bar,
-                          unsigned& phase, int* s_flag, double (*s_ex)[32], unsigned* s_mask)
+                          int t, int c, int nclip, LaneSmem& sm)
 {
     const int n = v.g.n;
-    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    const int I = n - kLaneBins * (t + 1);
-    const int smax = lane_block_smax(n, t);
-    const int smin = I > 0 ? I : 0;
-    const int s = I + lane;
-    const bool slot = (s >= smin && s <= smax);
-    double R = 0.0, TH = 0.0, Rw = 0.0, Tw = 0.0;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int I = n - kSlotBins * (t + 1);
+    const int smax = min(I + kSlotBins - 1, n - 2);
+    const int s = I - 1 + lane;
+    const bool slot = s >= 0 && s <= smax;
+    double R = 0.0, TH = 0.0, Rw = 0.0, Tw = 0.0, D = 0.0;
+    const unsigned em = w <= 1 ? exact_mask(v, t) : 0u;
+    if (w == 1 && c == 0) lane_base<K>(v, ws, t, em, R, TH, D);
+    double r = 0.0, th = 0.0;
     if (v.g.geo) {
-        const int Dm = la.Dm;                          // lags summed pair by pair
-        const int C = (Dm + la.parts - 1) / la.parts;
-        // lags of this task: [dA, dB), dB cut where Ld passes the block's top slot
-        // (Ld is nondecreasing; clipped lags hold kLagClipAll)
-        const int dA = min(c * C, Dm);
-        int dB = min(min(dA + C, Dm), smax + 1);
-        // most shares end below the cut: one load settles it, else bisect
-        if (dB > dA && __ldg(v.g.Ld + dB - 1) > smax) {
-            int lo = dA, hi = dB;
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (__ldg(v.g.Ld + mid) > smax) hi = mid; else lo = mid + 1;
-            }
-            dB = lo;
-        }
-
-        // j-side operand pointers: the staged window or the arrays themselves
-        const double* pN = v.p.Nj;
-        const double* pH = v.p.Hj;
-        const double* pX = v.g.x;
-        if (dB > dA) {
-            int jw0 = smin - __ldg(v.g.Ld + dB - 1);
-            jw0 = jw0 > 0 ? (jw0 & ~1) : 0;
-            int jw1 = smax - __ldg(v.g.Ld + dA) + 1;       // exclusive, <= n - 1
-            jw1 = (jw1 + 1) & ~1;                           // <= n: copies are padded
-            const int cnt = jw1 - jw0;
-            if (cnt > 0 && cnt <= kLaneWinMax) {
-                const unsigned bytes = static_cast<unsigned>(cnt) * 8u;
-                if (tid == 0) {
-                    fence_proxy_async_smem();              // earlier generic reads of the window
-                    mbar_expect_tx(bar, (NeedH<K>::j ? 3u : 2u) * bytes);
-                    bulk_g2s(sm.wN, la.Ncp + jw0, bytes, bar);
-                    if constexpr (NeedH<K>::j) bulk_g2s(sm.wH, v.p.Hj + jw0, bytes, bar);
-                    bulk_g2s(sm.wX, la.xcp + jw0, bytes, bar);
-                }
-                if (!mbar_wait(bar, phase)) {
-                    // the copy never completed: flag it, poison the block's bins, leave
-                    if (tid == 0) *la.err = 1;
-                    *s_flag = 1;
-                }
-                phase ^= 1u;
-                pN = sm.wN - jw0;
-                pH = sm.wH - jw0;
-                pX = sm.wX - jw0;
-            }
-        }
-        // this warp's contiguous share of the lags
-        const int per = (dB - dA + kLaneWarps - 1) / kLaneWarps;
-        const int dw0 = dA + w * per;
-        if (!*s_flag) lane_pairs<K>(v, s, slot, dw0, min(dB, dw0 + per), pN, pH, pX, R, TH);
         if (!SCATTER && la.eh >= la.el) {
-            // and of the runs summed by windows
+            // this warp's share of the runs summed by windows
             const int ne = la.eh - la.el + 1, sh = la.parts * kLaneWarps, q = c * kLaneWarps + w;
             lane_windows<K>(v, ws, s, slot, la.eh - ne * q / sh, la.eh - ne * (q + 1) / sh + 1, Rw, Tw);
         }
+        // and its contiguous share of the task's lags [dA, dB), dB cut where Ld passes
+        // the block's top slot (Ld is nondecreasing; clipped lags hold kLagClipAll)
+        const int C = (la.Dm + la.parts - 1) / la.parts;
+        const int dA = min(c * C, la.Dm);
+        const int dB = min(min(dA + C, la.Dm), smax + 1);
+        const int per = (dB - dA + kLaneWarps - 1) / kLaneWarps;
+        const int dw0 = dA + w * per;
+        const double xs = slot ? __ldg(v.g.x + s) : 1.0;
+        slot_pairs_geo<K, 1>(v.g, &v.p, s, slot, smax, dw0, min(dB, dw0 + per),
+                             ew_operand_c(xs, -exponent_of(xs)), r, th);
     } else {
-        slot_pairs_any<K, 1>(v.g, &v.p, s, slot, c * kLaneWarps + w, la.parts * kLaneWarps, R, TH);
+        slot_pairs_any<K, 1>(v.g, &v.p, s, slot, c * kLaneWarps + w, la.parts * kLaneWarps, r, th);
     }
-    constexpr int NS = SCATTER ? 2 : 4;
-    double* red = sm.red + w * NS * 32 + lane;
-    red[0] = R;
-    red[32] = TH;
-    if constexpr (!SCATTER) {
-        red[64] = Rw;
-        red[96] = Tw;
-    }
+    sm.red[w][0][lane] = R + r;
+    sm.red[w][1][lane] = TH + th;
+    sm.red[w][2][lane] = Rw;
+    sm.red[w][3][lane] = Tw;
+    if (w == 1) sm.D[lane] = D;
     __syncthreads();
-    const bool poisoned = *s_flag != 0;
 
-    SlotSums u{0.0, 0.0, 0.0, 0.0};
-    unsigned em = 0u;
+    SlotSums u{0.0, 0.0, 0.0, 0.0, 0.0};
     bool finish = false;
     if (w == 0) {
 #pragma unroll
         for (int q = 0; q < kLaneWarps; ++q) {
-            const double* rq = sm.red + q * NS * 32 + lane;
-            u.R += rq[0];
-            u.TH += rq[32];
-            if constexpr (!SCATTER) {
-                u.Rw += rq[64];
-                u.Tw += rq[96];
-            }
+            u.R += sm.red[q][0][lane];
+            u.TH += sm.red[q][1][lane];
+            u.Rw += sm.red[q][2][lane];
+            u.Tw += sm.red[q][3][lane];
         }
-        em = exact_mask(v, t);
+        u.D = sm.D[lane];
         finish = true;
         if (!SCATTER && (la.parts > 1 || em != 0u)) {
-            double* bp = la.part + (static_cast<size_t>(t) * la.parts + c) * 128 + lane;
+            double* bp = la.part + (static_cast<size_t>(t) * la.parts + c) * kLanePart + lane;
             bp[0] = u.R;
             bp[32] = u.TH;
             bp[64] = u.Rw;
             bp[96] = u.Tw;
+            if (c == 0) bp[128] = u.D;
             finish = block_ticket(ws, la, n, t, em, u);
         }
     }
-    lane_finish<K, SCATTER>(v, ws, la, rhs, t, nclip, em, finish, !SCATTER || c == 0, poisoned, u, s_ex, s_mask);
+    lane_finish<K, SCATTER>(v, ws, la, rhs, t, nclip, finish, u, sm);
     __syncthreads();
 }
 

@@ -30,6 +30,9 @@ __device__ __forceinline__ bool mom_exact_slot(double Ns, double Nup, double xup
     return fabs(Nup) * (kMomGuard * 9007199254740992.0) < (xup * inv_dx) * fabs(Ns);
 }
 
+// The same for a row of the VJP (vjp.cu), relative to its sum of |terms|.
+constexpr double kVjpGuard = 5e-13;
+
 // Window sums (agg_lane.cuh) pay on grids of about 64 sections an octave and more:
 // neighbour ratio at most kWinRatio = 2^(1/64). The tables hold x^2 N unscaled, so
 // the pivots stay within 2^-300 .. 2^300. Lags up to x_d = kWinStart x_0 are summed

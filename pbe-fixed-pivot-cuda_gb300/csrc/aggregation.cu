@@ -231,10 +231,10 @@ __device__ __forceinline__ void prep_offsets(const double* __restrict__ x, int n
 // log2: some 40 clocks each): the parts of a block run theirs side by side.
 //
 // FULL = false (stage calls of a caller that keeps the workspace, e.g. the RK4
-// tape): every grid-only entry -- a, ia, inv_dx, the x copy, Bd, Sd, Ld, J0, the
+// tape): every grid-only entry -- a, ia, inv_dx, Bd, Sd, Ld, J0, the window runs, the
 // geometric flag mom[5..6] and D0 in counter[1] -- is left as an earlier FULL
 // call on the same pivots and coefficients wrote it; only the N-dependent
-// values (h, the N copy, moments) and the tickets are rewritten, with the
+// values (h, moments, window tables) and the tickets are rewritten, with the
 // same arithmetic as a FULL call, so the results are bitwise the same.
 // Either way the last block resets counter[2] (the prep's block tickets) and
 // the pair kernel's last CTA counter[5] (the exact slots' list), so a
@@ -297,17 +297,15 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
                 iai = 1.0 / ai;
                 ws.a[i] = ai;
                 ws.ia[i] = iai;
-                ws.xcp[i] = xi;
             } else {
                 ai = ws.a[i];
                 iai = ws.ia[i];
             }
             ws.h[i] = hi;
-            ws.Ncp[i] = Ni;          // 256-byte aligned copies: bulk-copy sources of the lane tasks
             m[0] = iai * Ni; m[1] = Ni; m[2] = ai * Ni; m[3] = (ai * ai) * Ni; m[4] = hi;
             xm = mantissa_of(xi);
             E = exponent_of(xi);
-            if (i < lane_blocks(n)) { ws.tticket[i] = 0; ws.cticket[i] = 0; }
+            if (i < slot_blocks(n)) ws.cticket[i] = 0;
             // slots that keep the exact pair sum of their prefix part (the list's
             // order does not matter: each has its own task and its own sums)
             if (i < n - 1) {
@@ -441,6 +439,8 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
             const bool geo = n >= 2 && m5 <= kGeoTol && x[1] <= 64.0 * x[0];
             ws.mom[5] = geo ? 1.0 : 0.0;
             ws.mom[6] = m5;
+            const int eh = __ldcg(ws.counter + 8);
+            ws.counter[10] = eh >= max(1, __ldcg(ws.counter + 9)) ? __ldcg(ws.rend + eh + 1) : 0;
         }
     } else if (FULL && wp == 3) {
         int dmin = n;
@@ -454,7 +454,6 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
         ws.counter[0] = 0;          // task counter of the pair kernel
         ws.counter[2] = 0;          // this kernel's block tickets, ready for the next call
         ws.counter[3] = 0;          // contributors to bin n-1 done (clip tasks + top block)
-        ws.counter[4] = 0;          // lane-task staging error flag
         ws.counter[6] = 0;          // CTAs of the pair kernel done
     }
 }
@@ -481,9 +480,9 @@ __device__ __forceinline__ void clip_contributor_done(double* rhs, int n, const 
 // have equal lags but those of the lowest blocks, which come last).
 // ---------------------------------------------------------------------------
 #ifndef PBE_LANE_CTAS
-#define PBE_LANE_CTAS 3
+#define PBE_LANE_CTAS 4
 #endif
-constexpr int kLaneCtas = PBE_LANE_CTAS;           // CTAs per SM (register budget)
+constexpr int kLaneCtas = PBE_LANE_CTAS;   // CTAs per SM (64 registers; 3: an irregular grid 115 us, not 97, others the same)
 
 template <int K, bool SCATTER>
 __global__ void __launch_bounds__(kMainThreads, kLaneCtas)
@@ -491,14 +490,7 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
                 double* __restrict__ rhs, AggWs ws, int n, int nclip, double b0, double bbr,
                 double bsh)
 {
-    // per-warp slot sums, then the staged windows (16-byte aligned offsets)
-    extern __shared__ __align__(128) double lsmem[];
-    __shared__ __align__(8) uint64_t s_bar;
-    __shared__ int s_flag;
-    __shared__ int s_task;
-    __shared__ double s_wsum[2 * kLaneWarps];
-    __shared__ double s_ex[2][32];
-    __shared__ unsigned s_mask;
+    __shared__ LaneSmem sm;
 
     const int tid = threadIdx.x;
     LaneView v;
@@ -508,44 +500,31 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
 #pragma unroll
     for (int q = 0; q < kMomN; ++q) v.M[q] = ws.mom[q];
 
-    if (tid == 0) {
-        mbar_init(&s_bar, 1);
-        s_flag = 0;
-    }
-    __syncthreads();
-    constexpr int kRed = 4 * kLaneWarps * kLaneBins;     // per-warp sums of every slot
-    const LaneSmem lsm{lsmem, lsmem + kRed, lsmem + kRed + kLaneWinMax,
-                       lsmem + kRed + 2 * kLaneWinMax};
-    const int nblk = lane_blocks(n);
+    const int nblk = slot_blocks(n);
     // direct pairs of a slot: its lags below D0; on other grids at most its rows
     int Dm = min(v.g.D0, n), eh = 0, el = 1;
     if (!SCATTER && v.g.geo && ws.mom[7] == 0.0 && win_grid(x, n)) {
         eh = ws.counter[8];
         el = max(1, ws.counter[9]);
-        if (eh >= el) Dm = ws.rend[eh + 1];
+        if (eh >= el) Dm = ws.counter[10];
     }
     // (a window counts as 5 pairs)
     const int parts = lane_parts(v.g.geo ? Dm + 5 * max(0, eh - el + 1) : n, nblk, gridDim.x);
     const int nexact = ws.counter[5];
     const int ntasks = nclip + nexact + nblk * parts;
-    const LaneArgs la{ws.Ncp, ws.xcp, ws.lpart, ws.cticket, ws.counter + 4, parts, Dm, eh, el};
-    unsigned phase = 0;
-    for (;;) {
-        if (tid == 0) s_task = atomicAdd(ws.counter, 1);
-        __syncthreads();
-        int task = s_task;
-        const int stop = s_flag;
-        __syncthreads();
-        if (task >= ntasks || stop) break;
+    const LaneArgs la{ws.lpart, ws.cticket, parts, Dm, eh, el};
+    for (int next = blockIdx.x;;) {                      // the first task by the CTA's own index
+        int task = next;
+        if (task >= ntasks) break;
         if (task < nclip) {
             // a part of the clipped pairs (but for the prefix part of slot n - 1),
             // summed over the CTA in a fixed order
             double sc = warp_sum(slot_clip<K, 1>(v.g, &v.p, task * kMainThreads + tid, nclip * kMainThreads));
-            if ((tid & 31) == 0) s_wsum[tid >> 5] = sc;
+            if ((tid & 31) == 0) sm.sum[tid >> 5] = sc;
             __syncthreads();
             if (tid == 0) {
                 sc = 0.0;
-                for (int w = 0; w < kLaneWarps; ++w) sc += s_wsum[w];
+                for (int w = 0; w < kLaneWarps; ++w) sc += sm.sum[w];
                 if constexpr (SCATTER) {
                     if (sc != 0.0) atomicAdd(rhs + (n - 1), sc);
                 } else {
@@ -554,17 +533,16 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
                 }
             }
             __syncthreads();
-            continue;
+        } else if ((task -= nclip) < nexact) {
+            exact_slot_task<K, SCATTER>(v, ws, la, rhs, ws.xlist[task], nclip, sm);
+        } else {
+            task -= nexact;
+            lane_task<K, SCATTER>(v, ws, la, rhs, task % nblk, task / nblk, nclip, sm);
         }
-        task -= nclip;
-        if (task < nexact) {
-            exact_slot_task<K, SCATTER>(v, ws, la, rhs, ws.xlist[task], nclip, s_wsum, s_flag != 0,
-                                        s_ex, &s_mask);
-            continue;
-        }
-        task -= nexact;
-        lane_task<K, SCATTER>(v, ws, la, rhs, task % nblk, task / nblk, nclip, lsm, &s_bar, phase, &s_flag,
-                              s_ex, &s_mask);
+        if (tid == 0) sm.task = static_cast<int>(gridDim.x) + atomicAdd(ws.counter, 1);
+        __syncthreads();
+        next = sm.task;
+        __syncthreads();
     }
     // the last CTA leaves the exact slots' list empty for the next prep
     if (tid == 0 && atomicAdd(ws.counter + 6, 1) == static_cast<int>(gridDim.x) - 1) ws.counter[5] = 0;
@@ -893,16 +871,11 @@ cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_
     const int nb = agg_prep_blocks(n);
     const int nclip = agg_clip_tasks(n);
     auto kern = agg_lane_kernel<K, SC>;
-    const size_t smem = sizeof(double) * (4 * kLaneWarps * kLaneBins + 3 * kLaneWinMax);
     // the number of tasks is known on the device only (it follows D0)
     const long long cap = static_cast<long long>(kLaneCtas) * num_sms;
-    const long long most = static_cast<long long>(lane_blocks(n)) * kLaneMaxParts + nclip;
+    const long long most = static_cast<long long>(slot_blocks(n)) * kLaneMaxParts + nclip;
     const int grid = static_cast<int>(most < cap ? most : cap);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
     if (kind == kAggStage) {
         // counter[2] and [5] were left at 0 by the previous call on this workspace
         agg_prep_kernel<K, false><<<nb, kPrepStageThreads, 0, s>>>(a.N, a.x, n, ws, a.beta0, a.beta_br,
@@ -920,7 +893,7 @@ cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_
     }
     const bool prof = g_prof_start && g_prof_stop;
     if (prof) cudaEventRecord(g_prof_start, s);
-    kern<<<grid, kMainThreads, smem, s>>>(a.N, a.x, a.rhs, ws, n, nclip, a.beta0, a.beta_br, a.beta_sh);
+    kern<<<grid, kMainThreads, 0, s>>>(a.N, a.x, a.rhs, ws, n, nclip, a.beta0, a.beta_br, a.beta_sh);
     if (prof) cudaEventRecord(g_prof_stop, s);
     return cudaGetLastError();
 }

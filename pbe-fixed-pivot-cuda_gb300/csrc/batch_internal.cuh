@@ -16,7 +16,6 @@
 
 namespace pbe_gb300 {
 
-constexpr int kSlotBins = 31;    // bins of a pair task (a warp's lanes: their slots and the one below)
 constexpr int kMomStride = 24;   // doubles of BatchDev::mom per cell
 
 struct BatchGridDev {

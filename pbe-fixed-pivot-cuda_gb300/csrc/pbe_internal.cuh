@@ -268,19 +268,14 @@ struct AggWs {
     double* mom;       // [8]  M_{-1/3}, M_0, M_{1/3}, M_{2/3}, M_1, geo flag, max dev
     double* clip_part; // [kMaxClipTasks] sums of clipped pair rates, one per clip task
     int*    J0;        // [n]  first j with fl(x_j + x_i) >= x_{i+1} (at most i)
-    double* tfirst;    // [nblk] gather mode: block's own value of its first bin
-    double* tcarry;    // [nblk] gather mode: the lower neighbour's carry into that bin
-    int*    tticket;   // [nblk] contributors to the block's first bin done (0, 1, 2)
     int*    cticket;   // [nblk] tasks of the block done
     int*    counter;   // [16] [0] task counter, [1] first lag with Ld[d] == d,
                        //      [2] prep blocks done, [3] bin n-1 contributors done,
-                       //      [4] a staging wait of the lane tasks gave up, [5] entries of xlist,
+                       //      [5] entries of xlist,
                        //      [6] CTAs of the pair kernel done, [8] the first (largest)
                        //      offset whose run is summed by windows, [9] the last run's
-                       //      offset (both grid-only)
-    double* Ncp;       // [n + 2] copy of N, 256-byte aligned (bulk-copy source)
-    double* xcp;       // [n + 2] copy of x, 256-byte aligned (bulk-copy source)
-    double* lpart;     // [lane_partial_doubles(n)] lane-task chunk partials
+                       //      offset, [10] the first lag of run [8] (grid-only)
+    double* lpart;     // [lane_partial_doubles(n)] partial sums of the blocks' shares
     // Prefix sums over the bins (agg_prep_kernel): with m_q = {1/a, 1, a, a^2, x}_q N,
     // mloc[q n + i] = sum of m_q over the bins of i's prep block up to i, and
     // mloc[(5 + q) n + i] the same of m_q x 2^-E_i (E = binary exponent of x_i);
@@ -398,12 +393,18 @@ __host__ __device__ inline int lane_last_rank(int n, int t, int C)
     return rank;
 }
 
-// Lane tasks of the aggregation pair kernel: each block's direct lags cut into
-// `parts` equal shares, four partial sums of kLaneBins slots per share.
+// Pair tasks: blocks of kSlotBins output bins, a warp's lanes holding their slots
+// and the one below the first (summed by both neighbours, so that nothing is handed
+// over). The single-instance kernel aligns its blocks to the top of the grid (block
+// t owns [n - 31 (t + 1), n - 31 t)) and cuts each block's pairs into `parts` equal
+// shares, five partial sums of 32 slots per share.
+constexpr int kSlotBins = 31;
+__host__ __device__ constexpr int slot_blocks(int n) { return (n + kSlotBins - 1) / kSlotBins; }
 constexpr int kLaneMaxParts = 8;
+constexpr int kLanePart = 5 * 32;      // doubles of a share's partial sums
 __host__ __device__ constexpr size_t lane_partial_doubles(int n)
 {
-    return static_cast<size_t>(lane_blocks(n)) * kLaneMaxParts * 4 * kLaneBins;
+    return static_cast<size_t>(slot_blocks(n)) * kLaneMaxParts * kLanePart;
 }
 
 // Size of the aggregation scratch for n bins, equal to agg_ws_layout(n) below
@@ -415,10 +416,8 @@ constexpr size_t agg_ws_bytes(int n)
          + align256(sizeof(double) * 8 * static_cast<size_t>(agg_prep_blocks(n)))
          + align256(sizeof(double) * 8)
          + align256(sizeof(double) * kMaxClipTasks)
-         + 2 * align256(sizeof(double) * static_cast<size_t>(lane_blocks(n)))
-         + 2 * align256(sizeof(int) * static_cast<size_t>(lane_blocks(n)))
+         + align256(sizeof(int) * static_cast<size_t>(slot_blocks(n)))
          + align256(sizeof(int) * 16)
-         + 2 * align256(sizeof(double) * (static_cast<size_t>(n) + 2))
          + align256(sizeof(double) * lane_partial_doubles(n))
          + align256(sizeof(double) * 2 * kMomN * static_cast<size_t>(n))
          + 2 * align256(sizeof(double) * 2 * kMomN * static_cast<size_t>(agg_prep_blocks(n)))
@@ -447,14 +446,8 @@ inline size_t agg_ws_layout(int n, char* base, AggWs* ws)
     w.mom       = reinterpret_cast<double*>(take(sizeof(double) * 8));
     w.clip_part = reinterpret_cast<double*>(take(sizeof(double) * kMaxClipTasks));
     w.J0        = reinterpret_cast<int*>(take(sizeof(int) * static_cast<size_t>(n)));
-    const size_t nt = static_cast<size_t>(lane_blocks(n));
-    w.tfirst    = reinterpret_cast<double*>(take(sizeof(double) * nt));
-    w.tcarry    = reinterpret_cast<double*>(take(sizeof(double) * nt));
-    w.tticket   = reinterpret_cast<int*>(take(sizeof(int) * nt));
-    w.cticket   = reinterpret_cast<int*>(take(sizeof(int) * nt));
+    w.cticket   = reinterpret_cast<int*>(take(sizeof(int) * static_cast<size_t>(slot_blocks(n))));
     w.counter   = reinterpret_cast<int*>(take(sizeof(int) * 16));
-    w.Ncp       = reinterpret_cast<double*>(take(sizeof(double) * (static_cast<size_t>(n) + 2)));
-    w.xcp       = reinterpret_cast<double*>(take(sizeof(double) * (static_cast<size_t>(n) + 2)));
     w.lpart     = reinterpret_cast<double*>(take(sizeof(double) * lane_partial_doubles(n)));
     w.mloc      = reinterpret_cast<double*>(take(sizeof(double) * 2 * kMomN * static_cast<size_t>(n)));
     const size_t nbm = sizeof(double) * 2 * kMomN * static_cast<size_t>(agg_prep_blocks(n));

@@ -613,7 +613,6 @@ __device__ __forceinline__ void bin_sums(const VjpWs& ws, const double* __restri
 #define PBE_VROWS_WARPS 16
 #endif
 constexpr int kVRowsWarps = PBE_VROWS_WARPS;
-constexpr double kVjpGuard = 5e-13;
 
 template <int K>
 __global__ void __launch_bounds__(kVRowsWarps * 32)

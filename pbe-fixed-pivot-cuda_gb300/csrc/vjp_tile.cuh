@@ -11,6 +11,7 @@
 // =============================================================================
 #pragma once
 
+#include "agg_moments.cuh"
 #include "agg_rates.cuh"
 
 namespace pbe_gb300 {
