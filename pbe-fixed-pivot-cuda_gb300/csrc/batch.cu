@@ -60,6 +60,7 @@ struct pbe_batch_plan {
     int4* d_bundles = nullptr;
     int4* d_tasks = nullptr;
     std::vector<int> grid_direct;      // direct lags of a slot (D0), or n on a grid that is not geometric
+    std::vector<char> grid_geo;        // grids verified geometric
     std::vector<double> t_q, bw_q;
     double* d_tq = nullptr;
     double* d_bw = nullptr;
@@ -169,7 +170,7 @@ void tune_cache_store_locked(const TuneKey& k, int t)
 }
 
 // ---- schedule ------------------------------------------------------------------
-struct HostTask { int cell, I; long long cost; };
+struct HostTask { int cell, I, slot; long long cost; };
 
 // Lags of row tile tasks (VJP): every row meets all n partners.
 long long vjp_task_cost(int n, int T)
@@ -185,21 +186,29 @@ long long pair_task_cost(int direct, int I) { return std::min(direct, I + SW) + 
 
 // Bundles for the cells of the classes selected by `want` (all when null),
 // each class with its group size gs[class]; sorted by work, largest first.
-// vjp: row tiles of the VJP, whose work does not depend on the first row (every
-// row meets all n partners).
+// kTasksPair: the pair kernel's tasks of every cell; kTasksRows: the VJP's blocks
+// of 32 rows of the cells on geometric grids; kTasksTiles: its row tiles of the
+// other cells (their work does not depend on the first row). slot_off: first task
+// slot of each cell (VJP).
+enum TaskKind { kTasksPair, kTasksRows, kTasksTiles };
 void build_schedule(const pbe_batch_plan& p, const int* gs, const bool* want,
-                    std::vector<int4>& bundles, std::vector<int4>& tasks, bool vjp = false)
+                    std::vector<int4>& bundles, std::vector<int4>& tasks, TaskKind kind = kTasksPair,
+                    const int* slot_off = nullptr)
 {
     std::vector<std::vector<HostTask>> per(kClasses);
     for (int c = 0; c < p.n_cells; ++c) {
         const int n = p.cell_n[c];
         const int cls = n_class(n);
         if (want && !want[cls]) continue;
-        if (vjp) {
-            for (int I = 0; I < n; I += W) per[cls].push_back({c, I, vjp_task_cost(n, gs[cls])});
-        } else {
-            const int direct = p.grid_direct[p.cell_grid[c]];
-            for (int I = 0; I < n; I += SW) per[cls].push_back({c, I, pair_task_cost(direct, I)});
+        const int direct = p.grid_direct[p.cell_grid[c]];
+        const bool geo = p.grid_geo[p.cell_grid[c]] != 0;
+        if (kind == kTasksPair) {
+            for (int I = 0; I < n; I += SW) per[cls].push_back({c, I, 0, pair_task_cost(direct, I)});
+        } else if (kind == kTasksRows && geo) {
+            for (int I = 0; I < n; I += 32)
+                per[cls].push_back({c, I, slot_off[c] + I / 32, std::min(direct, std::max(n - I, I + 32)) + 8LL});
+        } else if (kind == kTasksTiles && !geo) {
+            for (int I = 0; I < n; I += W) per[cls].push_back({c, I, slot_off[c] + I / W, vjp_task_cost(n, gs[cls])});
         }
     }
     struct B { long long cost; int cls; int first; int cnt; };
@@ -226,7 +235,7 @@ void build_schedule(const pbe_batch_plan& p, const int* gs, const bool* want,
         bundles.push_back(make_int4(static_cast<int>(tasks.size()), b.cnt, gs[b.cls], 0));
         for (int k = 0; k < b.cnt; ++k) {
             const HostTask& t = sorted[b.cls][b.first + k];
-            tasks.push_back(make_int4(t.cell, t.I, 0, 0));
+            tasks.push_back(make_int4(t.cell, t.I, t.slot, 0));
         }
     }
 }
@@ -359,7 +368,11 @@ cudaError_t prep_shape(pbe_batch_plan* p, cudaStream_t s)
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return e;
     p->grid_direct.assign(static_cast<size_t>(p->n_grids), 0);
-    for (int g = 0; g < p->n_grids; ++g) p->grid_direct[g] = hg[g].geo ? hg[g].D0 : hg[g].n;
+    p->grid_geo.assign(static_cast<size_t>(p->n_grids), 0);
+    for (int g = 0; g < p->n_grids; ++g) {
+        p->grid_geo[g] = hg[g].geo != 0;
+        p->grid_direct[g] = hg[g].geo ? hg[g].D0 : hg[g].n;
+    }
     const long long avg = p->total / p->n_cells;
     int ranks = 1;
     while (ranks < 8 && 2LL * ranks * p->n_cells <= 4LL * p->num_sms && p->max_n >= 256 * ranks) ranks <<= 1;
@@ -687,40 +700,53 @@ cudaError_t vjp_setup(pbe_batch_plan* p, cudaStream_t s)
     if (p->vjp_ready) return cudaSuccess;
     BatchVjpDev& vd = p->vd;
     const size_t C = static_cast<size_t>(p->total);
-    std::vector<int> tile_off(static_cast<size_t>(p->n_cells) + 1, 0);
-    for (int c = 0; c < p->n_cells; ++c) tile_off[c + 1] = tile_off[c] + (p->cell_n[c] + W - 1) / W;
+    std::vector<int> slot_off(static_cast<size_t>(p->n_cells) + 1, 0);
+    long long tiles = 0, rows = 0;
+    int max_lags = 1;
+    for (int c = 0; c < p->n_cells; ++c) {
+        const int n = p->cell_n[c], g = p->cell_grid[c];
+        const bool by_rows = p->grid_geo[g] != 0;
+        const int cnt = by_rows ? (n + 31) / 32 : (n + W - 1) / W;
+        slot_off[c + 1] = slot_off[c] + cnt;
+        (by_rows ? rows : tiles) += cnt;
+        if (by_rows) max_lags = std::max(max_lags, std::min(n, p->grid_direct[g]));
+    }
     // every row tile meets all n partners, so with few tiles larger groups
     // (fewer tasks per bundle) give each CTA slot a bundle: T >= 256 x (CTA
     // slots) / tiles, a power of two up to 256
-    int gs[kClasses];
-    const long long tiles = tile_off.back();
+    int gs[kClasses], gr[kClasses];
     for (int c = 0; c < kClasses; ++c) {
         int T = c <= 7 ? 64 : 32;         // n < 256: 64
         while (T < kMainThreads && tiles * T < 256LL * 2 * p->num_sms) T <<= 1;
         gs[c] = T;
+        gr[c] = rule_group_size(rows, max_lags, p->num_sms);
     }
-    std::vector<int4> b;
-    std::vector<int4> t;
-    build_schedule(*p, gs, nullptr, b, t, true);
+    std::vector<int4> b, t, rb, rt;
+    build_schedule(*p, gs, nullptr, b, t, kTasksTiles, slot_off.data());
+    build_schedule(*p, gr, nullptr, rb, rt, kTasksRows, slot_off.data());
     int* dto = nullptr;
-    int4* db = nullptr;
-    int4* dt = nullptr;
+    int4 *db = nullptr, *dt = nullptr, *drb = nullptr, *drt = nullptr;
     cudaError_t e = plan_alloc(p, &vd.h, C);
     if (e == cudaSuccess) e = plan_alloc(p, &vd.D, C);
-    if (e == cudaSuccess) e = plan_alloc(p, &vd.mom, static_cast<size_t>(p->n_cells) * 16);
-    if (e == cudaSuccess) e = plan_alloc(p, &vd.tpart, 2 * static_cast<size_t>(tile_off.back()));
-    if (e == cudaSuccess) e = plan_alloc(p, &dto, tile_off.size());
+    if (e == cudaSuccess) e = plan_alloc(p, &vd.mom, static_cast<size_t>(p->n_cells) * kVjpMomStride);
+    if (e == cudaSuccess && rows > 0) e = plan_alloc(p, &vd.pre, 4 * kMomN * C);
+    if (e == cudaSuccess) e = plan_alloc(p, &vd.tpart, 2 * static_cast<size_t>(slot_off.back()));
+    if (e == cudaSuccess) e = plan_alloc(p, &dto, slot_off.size());
     if (e == cudaSuccess) e = plan_alloc(p, &vd.counter, 8);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dto, tile_off.data(), tile_off.size() * sizeof(int),
+        e = cudaMemcpyAsync(dto, slot_off.data(), slot_off.size() * sizeof(int),
                             cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = upload_schedule(p, b, t, &db, &dt, s);
+    if (e == cudaSuccess) e = upload_schedule(p, rb, rt, &drb, &drt, s);
     if (e == cudaSuccess) e = batch_vjp_setup(p->kernel);
     if (e != cudaSuccess) return e;
     vd.tile_off = dto;
     vd.bundles = db;
     vd.tasks = dt;
     vd.n_bundles = static_cast<int>(b.size());
+    vd.rbundles = drb;
+    vd.rtasks = drt;
+    vd.n_rbundles = static_cast<int>(rb.size());
     p->vjp_ready = true;
     return cudaSuccess;
 }

@@ -98,15 +98,27 @@ struct BatchDev {
 constexpr int kBrkTasks = 1;
 
 // Scratch of the batched VJP (batch_vjp.cu).
+constexpr int kVjpMomStride = 16 + 18 * 8;   // doubles of BatchVjpDev::mom per cell
 struct BatchVjpDev {
     double* h;             // x N per cell bin
     double* D;             // lambda slopes per cell bin
-    double* mom;           // [n_cells * 16]: moments of N (0..4) and of lambda N (5..9)
-    double* tpart;         // [2 * tiles]: parameter partials per row tile
-    const int* tile_off;   // [n_cells + 1]: first row-tile slot of each cell
-    const int4* bundles;   // row-tile bundles {first task, tasks, group size, 0}
-    const int4* tasks;     // {cell, first row, 0, 1}
+    // [n_cells * kVjpMomStride] moments of N (0..4) and of lambda N (5..9); by each
+    // CTA r of the cell's prep cluster, at 16 + 18 r: its parts of the moments of
+    // |N|, |lambda N| and u |N| |lambda step| (5 each, VjpWs::mom) and of the
+    // breakage parameter gradients (3)
+    double* mom;
+    double* pre;           // [2 * 2 kMomN * total] sums over the bins: VjpWs::mloc's four groups
+    double* tpart;         // [2 * slots]: parameter partials per task
+    const int* tile_off;   // [n_cells + 1]: first task slot of each cell
+    // row tiles of the cells on grids that are not geometric: bundles {first task,
+    // tasks, group size, 0}, tasks {cell, first row, slot, 0}
+    const int4* bundles;
+    const int4* tasks;
     int n_bundles;
+    // blocks of 32 rows of the cells on geometric grids
+    const int4* rbundles;
+    const int4* rtasks;
+    int n_rbundles;
     int* counter;
 };
 

@@ -22,14 +22,11 @@
 //    nothing is handed over between tasks.
 // =============================================================================
 #include "batch_internal.cuh"
-#include <cooperative_groups.h>
-
 #include "agg_slot.cuh"
+#include "batch_scan.cuh"
 
 namespace pbe_gb300 {
 namespace {
-
-namespace cg = cooperative_groups;
 
 constexpr int SW = kSlotBins;
 
@@ -202,11 +199,10 @@ batch_sel_kernel(BatchDev d, const pbe_batch_cell_params_t* __restrict__ params,
     }
 }
 
-// One lane's part of the breakage gather of bin i (0 <= i < n) of a cell:
+// One lane's part of the breakage gather of bin i (0 < i < n) of a cell:
 // quadrature points q = q0, q0 + nqp, ..., each adding the hi-shares of the
-// fragments bracketed at i-1 and the lo-shares of those at i (bin 0 also the
-// fragments clipped below x[0]). The nqp lanes of a bin then add their parts
-// in a fixed butterfly.
+// fragments bracketed at i-1 and the lo-shares of those at i. The nqp lanes of a
+// bin then add their parts in a fixed butterfly.
 __device__ __forceinline__ double brk_lane(const BatchDev& d, const BatchGridDev& gd,
                                            const double* SN, int n, int i, int q0, int nqp)
 {
@@ -219,11 +215,26 @@ __device__ __forceinline__ double brk_lane(const BatchDev& d, const BatchGridDev
         const int fa = min(max(fq[i], 0), n);         // first j with lo >= i-1
         const int fb = min(max(fq[i + 1], fa), n);    // first j with lo >= i
         const int fc = min(max(fq[i + 2], fb), n);    // first j with lo >= i+1
-        if (i == 0) { for (int j = 0; j < fb; ++j) acc = fma(SN[j], wl[j], acc); }
-        else        { for (int j = fa; j < fb; ++j) acc = fma(SN[j], wh[j], acc); }
+        for (int j = fa; j < fb; ++j) acc = fma(SN[j], wh[j], acc);
         for (int j = fb; j < fc; ++j) acc = fma(SN[j], wl[j], acc);
     }
     return acc;
+}
+
+// Bin 0 by one warp, its lanes over the parents: the lo-shares of the fragments
+// clipped below x[0] and of those bracketed at 0 (with small table entries that is
+// some hundred parents a point, 18 us for one lane at 128 sections an octave).
+// Valid in every lane.
+__device__ __forceinline__ double brk_bin0(const BatchDev& d, const BatchGridDev& gd, const double* SN, int n)
+{
+    const int ng = gd.n;
+    double acc = 0.0;
+    for (int q = 0; q < d.nq; ++q) {
+        const int fc = min(max(d.bfirst[gd.foff + q * (ng + 2) + 2], 0), n);   // first j with lo >= 1
+        const double* wl = d.bwlo + gd.woff + q * ng;
+        for (int j = threadIdx.x & 31; j < fc; j += 32) acc = fma(SN[j], wl[j], acc);
+    }
+    return warp_sum(acc);
 }
 
 __device__ __forceinline__ int brk_lanes(int nq)
@@ -244,9 +255,13 @@ __device__ void cell_breakage(const BatchDev& d, const BatchGridDev& gd, const d
     const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, l = threadIdx.x & 31;
     for (int base = r0 + w * per_warp; base < r1; base += nw * per_warp) {   // uniform per warp
         const int i = base + l / nqp;
-        double acc = (i < r1) ? brk_lane(d, gd, SN, n, i, l % nqp, nqp) : 0.0;
+        double acc = (i < r1 && i > 0) ? brk_lane(d, gd, SN, n, i, l % nqp, nqp) : 0.0;
         for (int o = nqp >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (i < r1 && (l % nqp) == 0) Bk[i] = acc - SN[i];
+        if (i < r1 && i > 0 && (l % nqp) == 0) Bk[i] = acc - SN[i];
+    }
+    if (r0 == 0 && w == nw - 1) {
+        const double acc = brk_bin0(d, gd, SN, n);
+        if (l == 0) Bk[0] = acc - SN[0];
     }
 }
 
@@ -262,163 +277,14 @@ __device__ void tile_breakage(const BatchDev& d, const BatchGridDev& gd, const d
     for (int base = w * per_warp; base < SW; base += nw * per_warp) {   // uniform per warp
         const int t = base + l / nqp;
         const int i = I + t;
-        const bool in = t < SW && i < n;
+        const bool in = t < SW && i > 0 && i < n;
         double acc = in ? brk_lane(d, gd, SN, n, i, l % nqp, nqp) : 0.0;
         for (int o = nqp >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (t < SW && (l % nqp) == 0) out[t] = in ? acc - SN[i] : 0.0;
+        if (t < SW && i > 0 && (l % nqp) == 0) out[t] = in ? acc - SN[i] : 0.0;
     }
-}
-
-// The cell of a cluster of CTAs: its bins are split evenly over the CTAs, and a
-// CTA's bins over its threads in contiguous runs.
-struct CellPart {
-    int rank, ranks;      // this CTA in the cell's cluster
-    int r0, r1;           // its bins
-    int t0, t1;           // this thread's bins
-};
-__device__ __forceinline__ CellPart cell_part(int n)
-{
-    const cg::cluster_group cl = cg::this_cluster();
-    CellPart p;
-    p.rank = static_cast<int>(cl.block_rank());
-    p.ranks = static_cast<int>(cl.num_blocks());
-    const int per = (n + p.ranks - 1) / p.ranks;
-    p.r0 = min(n, p.rank * per);
-    p.r1 = min(n, p.r0 + per);
-    const int c = (p.r1 - p.r0 + static_cast<int>(blockDim.x) - 1) / static_cast<int>(blockDim.x);
-    p.t0 = min(p.r1, p.r0 + c * static_cast<int>(threadIdx.x));
-    p.t1 = min(p.r1, p.t0 + c);
-    return p;
-}
-
-// Prefix moments of y over the cell's bins into pre (AggWs::mloc's sums, here
-// over the whole cell): pre[q stride + i] = sum m_q, pre[(5 + q) stride + i] =
-// sum m_q x at the exponent of x_i, m_q = {1/a, 1, a, a^2, x}_q y; and, by the
-// cluster's CTA 0, the moments over all bins into mom[0..4]. Two passes over a
-// thread's run (totals, then the running sums), a scan of the totals over lanes,
-// warps and CTAs between them. Fixed order for a fixed launch shape.
-constexpr int kPrepMaxWarps = 8;
-struct PrefixShared {
-    double wt[kPrepMaxWarps][2 * kMomN];     // warp totals, then the warps' offsets
-    int we[kPrepMaxWarps];                   // exponent after the warp's last bin
-    double ct[2 * kMomN];                    // CTA totals (read by the cluster's other CTAs)
-    int ce;
-};
-
-template <int K>
-__device__ void cell_prefix(const double* __restrict__ x, const double* __restrict__ a,
-                            const double* __restrict__ ia, const double* y, const CellPart& part,
-                            PrefixShared& sm, double* pre, long long stride, double* mom)
-{
-    const cg::cluster_group cl = cg::this_cluster();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    double P[kMomN], T[kMomN];
-    auto add = [&](int i, int& e) {
-        const double xi = __ldg(x + i), yi = y[i];
-        const int ei = exponent_of(xi);
-        const double ay = (K >= 3) ? __ldg(a + i) * yi : 0.0, xm = mantissa_of(xi);
-        const double m[kMomN] = {(K >= 3) ? __ldg(ia + i) * yi : 0.0, yi, ay,
-                                 (K >= 4) ? __ldg(a + i) * ay : 0.0, xi * yi};
-#pragma unroll
-        for (int q = 0; q < kMomN; ++q) {
-            if (!need_moment<K>(q)) continue;
-            P[q] += m[q];
-            T[q] = fma(m[q], xm, ei != e ? scale_down(T[q], e - ei) : T[q]);
-        }
-        e = ei;
-    };
-#pragma unroll
-    for (int q = 0; q < kMomN; ++q) { P[q] = 0.0; T[q] = 0.0; }
-    const int eb = part.t0 > 0 ? exponent_of(__ldg(x + part.t0 - 1)) : 0;   // before the run
-    int e = part.t0 > 0 ? eb : exponent_of(__ldg(x));
-    for (int i = part.t0; i < part.t1; ++i) add(i, e);
-    // inclusive scan of the runs over the warp
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int dE = __shfl_up_sync(0xffffffffu, e, o) - e;
-#pragma unroll
-        for (int q = 0; q < kMomN; ++q) {
-            if (!need_moment<K>(q)) continue;
-            const double p = __shfl_up_sync(0xffffffffu, P[q], o);
-            const double t = __shfl_up_sync(0xffffffffu, T[q], o);
-            if (lane >= o) { P[q] += p; T[q] += scale_down(t, dE); }
-        }
-    }
-    if (lane == 31) {
-        sm.we[w] = e;
-#pragma unroll
-        for (int q = 0; q < kMomN; ++q) { sm.wt[w][q] = P[q]; sm.wt[w][kMomN + q] = T[q]; }
-    }
-    // the runs before this lane's in the warp (their sum stands at exponent ep)
-    const int eu = __shfl_up_sync(0xffffffffu, e, 1);
-    const int ep = lane > 0 ? eu : eb;
-#pragma unroll
-    for (int q = 0; q < kMomN; ++q) {
-        if (!need_moment<K>(q)) continue;
-        const double p = __shfl_up_sync(0xffffffffu, P[q], 1);
-        const double t = __shfl_up_sync(0xffffffffu, T[q], 1);
-        P[q] = lane > 0 ? p : 0.0;
-        T[q] = lane > 0 ? t : 0.0;
-    }
-    __syncthreads();
-    // lanes 0 .. 2 kMomN - 1 of warp 0, one sum each: the warps' offsets in the CTA
-    const bool weighted = lane >= kMomN;
-    double acc = 0.0;
-    int ea = 0;
-    if (w == 0 && lane < 2 * kMomN) {
-        for (int v = 0; v < nw; ++v) {
-            const double t = sm.wt[v][lane];
-            if (weighted && v > 0) acc = scale_down(acc, ea - sm.we[v]);
-            ea = sm.we[v];
-            acc += t;
-        }
-        sm.ct[lane] = acc;
-        if (lane == 0) sm.ce = ea;
-    }
-    cl.sync();                                        // every CTA's totals are there
-    if (w == 0 && lane < 2 * kMomN) {
-        // the CTAs before this one, then the warps before each warp
-        double base = 0.0;
-        int be = 0;
-        for (int r = 0; r < part.rank; ++r) {
-            const int en = *cl.map_shared_rank(&sm.ce, r);
-            if (weighted && r > 0) base = scale_down(base, be - en);
-            base += *cl.map_shared_rank(&sm.ct[lane], r);
-            be = en;
-        }
-        for (int v = 0; v < nw; ++v) {
-            const double t = sm.wt[v][lane];
-            sm.wt[v][lane] = base;                    // before warp v, at exponent be
-            const int en = sm.we[v];
-            __syncwarp((1u << (2 * kMomN)) - 1u);     // read by every lane
-            if (lane == 0) sm.we[v] = be;
-            if (weighted) base = scale_down(base, be - en);
-            base += t;
-            be = en;
-        }
-        if (part.rank == 0 && lane < kMomN) {
-            double tot = sm.ct[lane];
-            for (int r = 1; r < part.ranks; ++r) tot += *cl.map_shared_rank(&sm.ct[lane], r);
-            mom[lane] = tot;
-        }
-    }
-    __syncthreads();
-    const int wb = sm.we[w];
-#pragma unroll
-    for (int q = 0; q < kMomN; ++q) {
-        if (!need_moment<K>(q)) continue;
-        P[q] += sm.wt[w][q];
-        T[q] += scale_down(sm.wt[w][kMomN + q], wb - ep);
-    }
-    e = part.t0 > 0 ? ep : exponent_of(__ldg(x));
-    for (int i = part.t0; i < part.t1; ++i) {
-        add(i, e);
-#pragma unroll
-        for (int q = 0; q < kMomN; ++q) {
-            if (!need_moment<K>(q)) continue;
-            pre[static_cast<long long>(q) * stride + i] = P[q];
-            pre[static_cast<long long>(kMomN + q) * stride + i] = T[q];
-        }
+    if (I == 0 && w == nw - 1) {
+        const double acc = brk_bin0(d, gd, SN, n);
+        if (l == 0) out[0] = acc - SN[0];
     }
 }
 
@@ -506,7 +372,7 @@ batch_prep_kernel(BatchDev d, double* N, const pbe_batch_cell_params_t* __restri
     const double* Yk = (stage == kStageRhs || stage == kStageNext) ? Nc : Yc;
     double* mom = d.mom + static_cast<size_t>(cell) * kMomStride;
     if (agg) {
-        cell_prefix<K>(x, d.ga + gd.off, d.gia + gd.off, Yk, part, psm, d.pre + off, d.total, mom);
+        cell_prefix<K>(x, d.ga + gd.off, d.gia + gd.off, Yk, part, n, psm, d.pre + off, d.total, mom);
     }
     cl.sync();                             // the cell's stage arrays are complete; all shared reads done
     if (agg) {
@@ -569,9 +435,9 @@ batch_jvp_prep_kernel(BatchDev d, const double* __restrict__ v,
     __syncthreads();
     double* mom = d.mom + static_cast<size_t>(cell) * kMomStride;
     if (agg) {
-        cell_prefix<K>(x, d.ga + gd.off, d.gia + gd.off, d.A + off, part, psm, d.pre + off, d.total, mom);
+        cell_prefix<K>(x, d.ga + gd.off, d.gia + gd.off, d.A + off, part, n, psm, d.pre + off, d.total, mom);
         cl.sync();                         // the shared totals are read by every CTA
-        cell_prefix<K>(x, d.ga + gd.off, d.gia + gd.off, v + off, part, psm, d.pre2 + off, d.total, mom + 5);
+        cell_prefix<K>(x, d.ga + gd.off, d.gia + gd.off, v + off, part, n, psm, d.pre2 + off, d.total, mom + 5);
     }
     cl.sync();                             // the cell's pass arrays are complete
     if (agg) {
@@ -714,25 +580,6 @@ cudaError_t main_k(const BatchDev& d, const double* Y, const pbe_batch_cell_para
     return cudaGetLastError();
 }
 
-// Launch shape of the per-cell prep kernels: a cluster of d.prep_ranks CTAs of
-// d.prep_threads threads per cell (prep_shape).
-template <class... P, class... A>
-cudaError_t launch_prep(const BatchDev& d, void (*kern)(P...), cudaStream_t s, A... args)
-{
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(d.n_cells) * static_cast<unsigned>(d.prep_ranks));
-    cfg.blockDim = dim3(static_cast<unsigned>(d.prep_threads));
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = static_cast<unsigned>(d.prep_ranks);
-    at.val.clusterDim.y = 1;
-    at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 } // namespace
 
 cudaError_t batch_grid_tables(const BatchDev& d, const double* t_q, const double* bw_q,
@@ -751,12 +598,12 @@ cudaError_t prep_any(const BatchDev& d, double* N, const pbe_batch_cell_params_t
 {
     if (d.n_cells <= 0) return cudaErrorInvalidValue;
     switch (d.kernel < 0 ? 0 : d.kernel) {
-    case 0: return launch_prep(d, batch_prep_kernel<0>, s, d, N, params, stage, c, dt6, sc);
-    case 1: return launch_prep(d, batch_prep_kernel<1>, s, d, N, params, stage, c, dt6, sc);
-    case 2: return launch_prep(d, batch_prep_kernel<2>, s, d, N, params, stage, c, dt6, sc);
-    case 3: return launch_prep(d, batch_prep_kernel<3>, s, d, N, params, stage, c, dt6, sc);
-    case 4: return launch_prep(d, batch_prep_kernel<4>, s, d, N, params, stage, c, dt6, sc);
-    case 5: return launch_prep(d, batch_prep_kernel<5>, s, d, N, params, stage, c, dt6, sc);
+    case 0: return launch_prep(d, batch_prep_kernel<0>, d.prep_threads, s, d, N, params, stage, c, dt6, sc);
+    case 1: return launch_prep(d, batch_prep_kernel<1>, d.prep_threads, s, d, N, params, stage, c, dt6, sc);
+    case 2: return launch_prep(d, batch_prep_kernel<2>, d.prep_threads, s, d, N, params, stage, c, dt6, sc);
+    case 3: return launch_prep(d, batch_prep_kernel<3>, d.prep_threads, s, d, N, params, stage, c, dt6, sc);
+    case 4: return launch_prep(d, batch_prep_kernel<4>, d.prep_threads, s, d, N, params, stage, c, dt6, sc);
+    case 5: return launch_prep(d, batch_prep_kernel<5>, d.prep_threads, s, d, N, params, stage, c, dt6, sc);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -834,12 +681,12 @@ cudaError_t batch_jvp_prep(const BatchDev& d, const double* v, const pbe_batch_c
 {
     if (d.n_cells <= 0 || !d.A) return cudaErrorInvalidValue;
     switch (d.kernel < 0 ? 0 : d.kernel) {
-    case 0: return launch_prep(d, batch_jvp_prep_kernel<0>, s, d, v, params);
-    case 1: return launch_prep(d, batch_jvp_prep_kernel<1>, s, d, v, params);
-    case 2: return launch_prep(d, batch_jvp_prep_kernel<2>, s, d, v, params);
-    case 3: return launch_prep(d, batch_jvp_prep_kernel<3>, s, d, v, params);
-    case 4: return launch_prep(d, batch_jvp_prep_kernel<4>, s, d, v, params);
-    case 5: return launch_prep(d, batch_jvp_prep_kernel<5>, s, d, v, params);
+    case 0: return launch_prep(d, batch_jvp_prep_kernel<0>, d.prep_threads, s, d, v, params);
+    case 1: return launch_prep(d, batch_jvp_prep_kernel<1>, d.prep_threads, s, d, v, params);
+    case 2: return launch_prep(d, batch_jvp_prep_kernel<2>, d.prep_threads, s, d, v, params);
+    case 3: return launch_prep(d, batch_jvp_prep_kernel<3>, d.prep_threads, s, d, v, params);
+    case 4: return launch_prep(d, batch_jvp_prep_kernel<4>, d.prep_threads, s, d, v, params);
+    case 5: return launch_prep(d, batch_jvp_prep_kernel<5>, d.prep_threads, s, d, v, params);
     default: return cudaErrorInvalidValue;
     }
 }
