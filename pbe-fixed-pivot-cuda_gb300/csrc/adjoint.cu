@@ -74,6 +74,8 @@ __global__ void __launch_bounds__(256)
 rk_stage_kernel(double* N, const double* k, double* acc, double* Y, int n, int q, double c,
                 double dt6)
 {
+    const int dep = dep_wait();
+    k += dep; n += dep;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double ki = k[i];
@@ -93,6 +95,8 @@ rk_stage_kernel(double* N, const double* k, double* acc, double* Y, int n, int q
 __global__ void __launch_bounds__(256)
 adj_coeff_kernel(double* a, const double* lp, double* mu, double w, double c, int n, int first)
 {
+    const int dep = dep_wait();
+    lp += dep; n += dep;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     a[i] = first ? w * lp[i] : fma(c, mu[i], w * lp[i]);
@@ -101,6 +105,8 @@ adj_coeff_kernel(double* a, const double* lp, double* mu, double w, double c, in
 
 __global__ void __launch_bounds__(256) adj_sum_kernel(double* lsum, const double* mu, int n)
 {
+    const int dep = dep_wait();
+    mu += dep; n += dep;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) lsum[i] += mu[i];
 }
@@ -162,7 +168,8 @@ cudaError_t step(pbe_rk4_tape* t, int m, double* N, double* Ys, cudaStream_t s)
         e = rhs(t, m, in, s);
         if (e != cudaSuccess) break;
         double* Yout = (q < 3) ? (Ys ? Ys + (q + 1) * un : t->Y) : t->Y;
-        rk_stage_kernel<<<blocks(t->n), 256, 0, s>>>(N, t->k, t->acc, Yout, t->n, q, cs[q], dt6);
+        launch_dep(rk_stage_kernel, dim3(blocks(t->n)), 256, 0, s, 1, N, t->k, t->acc, Yout, t->n, q, cs[q],
+                   dt6);
         e = cudaGetLastError();
     }
     return e;
@@ -238,12 +245,12 @@ cudaError_t enqueue_backward(pbe_rk4_tape* t, const double* lamT, double* gN0, d
             e = cudaMemcpyAsync(lsum, lam, sizeof(double) * un, cudaMemcpyDeviceToDevice, s);
             for (int q = 3; q >= 0 && e == cudaSuccess; --q) {
                 const double w = (q == 0 || q == 3) ? c6 : 2.0 * c6;
-                adj_coeff_kernel<<<blocks(t->n), 256, 0, s>>>(t->a, lam, t->mu, w,
-                                                              q < 3 ? cs[q] : 0.0, t->n, q == 3);
+                launch_dep(adj_coeff_kernel, dim3(blocks(t->n)), 256, 0, s, 1, t->a, lam, t->mu, w,
+                           q < 3 ? cs[q] : 0.0, t->n, q == 3);
                 e = cudaGetLastError();
                 if (e == cudaSuccess) e = vjp(t, m, Ys + q * un, g_agg, g_brk, s);
                 if (e == cudaSuccess) {
-                    adj_sum_kernel<<<blocks(t->n), 256, 0, s>>>(lsum, t->mu, t->n);
+                    launch_dep(adj_sum_kernel, dim3(blocks(t->n)), 256, 0, s, 1, lsum, t->mu, t->n);
                     e = cudaGetLastError();
                 }
             }

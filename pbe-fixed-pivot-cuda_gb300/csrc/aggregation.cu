@@ -272,6 +272,8 @@ __global__ void __launch_bounds__(FULL ? kPrepFullThreads : kPrepStageThreads)
 agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int n, AggWs ws,
                 double b0, double bbr, double bsh)
 {
+    const int dep = dep_wait();
+    N += dep; x += dep; n += dep;
     __shared__ double dev_s[kPrepThreads / 32];
     __shared__ double gsum[2 * kMomN];
     __shared__ double wtot[kPrepThreads / 32][kWinMom];
@@ -490,6 +492,8 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
                 double* __restrict__ rhs, AggWs ws, int n, int nclip, double b0, double bbr,
                 double bsh)
 {
+    const int dep = dep_wait();
+    N += dep; x += dep; rhs += dep; n += dep;
     __shared__ LaneSmem sm;
 
     const int tid = threadIdx.x;
@@ -573,6 +577,8 @@ __global__ void __launch_bounds__(kMainThreads)
 agg_small_kernel(const double* __restrict__ N, const double* __restrict__ x, double* __restrict__ rhs,
                  AggWs ws, int n, double b0, double bbr, double bsh)
 {
+    const int dep = dep_wait();
+    N += dep; x += dep; rhs += dep; n += dep;
     namespace cg = cooperative_groups;
     const cg::cluster_group cl = cg::this_cluster();
     __shared__ double tot[2 * kMomN];                  // this CTA's totals (read by the cluster)
@@ -824,21 +830,12 @@ bool small_cluster_ok(int ranks)
 template <int K, int KIND>
 cudaError_t launch_small(const AggArgs& a, const AggWs& ws, cudaStream_t s, int ranks)
 {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(ranks));
-    cfg.blockDim = dim3(kMainThreads);
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = static_cast<unsigned>(ranks);
-    at.val.clusterDim.y = 1;
-    at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
     const bool prof = KIND != kAggTables && g_prof_start && g_prof_stop;
     if (prof) cudaEventRecord(g_prof_start, s);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, agg_small_kernel<K, KIND>, a.N, a.x, a.rhs, ws, a.n,
-                                             a.beta0, a.beta_br, a.beta_sh);
+    const cudaError_t e = launch_dep(agg_small_kernel<K, KIND>, dim3(static_cast<unsigned>(ranks)),
+                                     kMainThreads, 0,
+                                     s, static_cast<unsigned>(ranks), a.N, a.x, a.rhs, ws, a.n, a.beta0,
+                                     a.beta_br, a.beta_sh);
     if (prof) cudaEventRecord(g_prof_stop, s);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -878,13 +875,13 @@ cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_
     cudaError_t e = cudaSuccess;
     if (kind == kAggStage) {
         // counter[2] and [5] were left at 0 by the previous call on this workspace
-        agg_prep_kernel<K, false><<<nb, kPrepStageThreads, 0, s>>>(a.N, a.x, n, ws, a.beta0, a.beta_br,
-                                                              a.beta_sh);
+        launch_dep(agg_prep_kernel<K, false>, dim3(nb), kPrepStageThreads, 0, s, 1, a.N, a.x, n, ws,
+                   a.beta0, a.beta_br, a.beta_sh);
     } else {
         e = cudaMemsetAsync(ws.counter, 0, 8 * sizeof(int), s);   // prep's block tickets
         if (e != cudaSuccess) return e;
-        agg_prep_kernel<K, true><<<nb, kPrepFullThreads, 0, s>>>(a.N, a.x, n, ws, a.beta0, a.beta_br,
-                                                                 a.beta_sh);
+        launch_dep(agg_prep_kernel<K, true>, dim3(nb), kPrepFullThreads, 0, s, 1, a.N, a.x, n, ws, a.beta0,
+                   a.beta_br, a.beta_sh);
         if (kind == kAggTables) {
             e = cudaGetLastError();
             // this call's exact slots are no one's: the next prep starts its own list
@@ -893,7 +890,8 @@ cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_
     }
     const bool prof = g_prof_start && g_prof_stop;
     if (prof) cudaEventRecord(g_prof_start, s);
-    kern<<<grid, kMainThreads, 0, s>>>(a.N, a.x, a.rhs, ws, n, nclip, a.beta0, a.beta_br, a.beta_sh);
+    launch_dep(kern, dim3(grid), kMainThreads, 0, s, 1, a.N, a.x, a.rhs, ws, n, nclip, a.beta0, a.beta_br,
+               a.beta_sh);
     if (prof) cudaEventRecord(g_prof_stop, s);
     return cudaGetLastError();
 }

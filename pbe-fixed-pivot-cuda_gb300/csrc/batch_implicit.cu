@@ -53,6 +53,8 @@ gmres_start_kernel(BatchDev d, GmresDev g, const double* __restrict__ N,
                    const double* __restrict__ r, const pbe_batch_cell_params_t* __restrict__ params,
                    int first)
 {
+    const int dep = dep_wait();
+    N += dep; r += dep; params += dep;
     __shared__ double sh[8];
     __shared__ double m_s[5];
     const int c = blockIdx.x;
@@ -131,6 +133,7 @@ gmres_start_kernel(BatchDev d, GmresDev g, const double* __restrict__ N,
 __global__ void __launch_bounds__(256)
 gmres_arnoldi_kernel(BatchDev d, GmresDev g, int j)
 {
+    dep_wait();
     __shared__ double sh[8];
     __shared__ double h_s[kGmresMaxDim + 1];
     __shared__ int more_s;
@@ -214,6 +217,8 @@ __global__ void __launch_bounds__(256)
 gmres_finish_kernel(BatchDev d, GmresDev g, double* __restrict__ xo, double* __restrict__ resid,
                     int acc, int final)
 {
+    const int dep = dep_wait();
+    xo += dep; resid += dep;
     __shared__ double y_s[kGmresMaxDim];
     const int c = blockIdx.x;
     const BatchCellDev cd = d.cells[c];
@@ -253,6 +258,8 @@ __global__ void __launch_bounds__(256)
 gmres_restart_kernel(BatchDev d, GmresDev g, const double* __restrict__ r,
                      const double* __restrict__ x)
 {
+    const int dep = dep_wait();
+    r += dep; x += dep;
     const int c = blockIdx.x;
     if (g.conv[c] || (g.skip && g.skip[c])) return;      // whole block
     const BatchCellDev cd = d.cells[c];
@@ -268,6 +275,8 @@ __global__ void __launch_bounds__(256)
 lincomb_kernel(double* __restrict__ out, double a, const double* __restrict__ X, double b,
                const double* __restrict__ Y, long long total)
 {
+    const int dep = dep_wait();
+    out += dep; X += dep; Y += dep;
     for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += 256LL * gridDim.x) {
         const double ax = a * X[i];
         out[i] = Y ? fma(b, Y[i], ax) : ax;
@@ -279,6 +288,8 @@ __global__ void __launch_bounds__(256)
 ros_update_kernel(double* __restrict__ N, double c1, const double* __restrict__ K1, double c2,
                   const double* __restrict__ K2, long long total)
 {
+    const int dep = dep_wait();
+    N += dep; K1 += dep; K2 += dep;
     for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += 256LL * gridDim.x)
         N[i] = N[i] + fma(c1, K1[i], c2 * K2[i]);
 }
@@ -297,6 +308,8 @@ __global__ void __launch_bounds__(256)
 ros2_stage_kernel(BatchDev d, const double* __restrict__ N, const double* __restrict__ K1,
                   double* __restrict__ Y, double* __restrict__ gtc, Rk45Ctl ctl, double gamma)
 {
+    const int dep = dep_wait();
+    N += dep; K1 += dep; Y += dep; gtc += dep;
     const int c = blockIdx.x;
     const BatchCellDev cd = d.cells[c];
     const double dt = ctl.dt[c];           // 0 for a finished cell: Y = N
@@ -309,6 +322,8 @@ __global__ void __launch_bounds__(256)
 ros2_control_kernel(BatchDev d, double* __restrict__ N, const double* __restrict__ K1,
                     const double* __restrict__ K2, Rk45Ctl ctl)
 {
+    const int dep = dep_wait();
+    N += dep; K1 += dep; K2 += dep;
     __shared__ double sh[8];
     __shared__ int accept_s;
     const int c = blockIdx.x;
@@ -357,7 +372,7 @@ template <int K>
 cudaError_t start_k(const BatchDev& d, const GmresDev& g, const double* N, const double* r,
                     const pbe_batch_cell_params_t* params, bool first, cudaStream_t s)
 {
-    gmres_start_kernel<K><<<d.n_cells, 256, 0, s>>>(d, g, N, r, params, first ? 1 : 0);
+    launch_dep(gmres_start_kernel<K>, dim3(d.n_cells), 256, 0, s, 1, d, g, N, r, params, first ? 1 : 0);
     return cudaGetLastError();
 }
 
@@ -386,49 +401,51 @@ cudaError_t batch_gmres_start(const BatchDev& d, const GmresDev& g, const double
 
 cudaError_t batch_gmres_arnoldi(const BatchDev& d, const GmresDev& g, int j, cudaStream_t s)
 {
-    gmres_arnoldi_kernel<<<d.n_cells, 256, 0, s>>>(d, g, j);
+    launch_dep(gmres_arnoldi_kernel, dim3(d.n_cells), 256, 0, s, 1, d, g, j);
     return cudaGetLastError();
 }
 
 cudaError_t batch_gmres_finish(const BatchDev& d, const GmresDev& g, double* x, double* resid,
                                bool acc, bool final, cudaStream_t s)
 {
-    gmres_finish_kernel<<<d.n_cells, 256, 0, s>>>(d, g, x, resid, acc ? 1 : 0, final ? 1 : 0);
+    launch_dep(gmres_finish_kernel, dim3(d.n_cells), 256, 0, s, 1, d, g, x, resid, acc ? 1 : 0,
+               final ? 1 : 0);
     return cudaGetLastError();
 }
 
 cudaError_t batch_gmres_restart(const BatchDev& d, const GmresDev& g, const double* r,
                                 const double* x, cudaStream_t s)
 {
-    gmres_restart_kernel<<<d.n_cells, 256, 0, s>>>(d, g, r, x);
+    launch_dep(gmres_restart_kernel, dim3(d.n_cells), 256, 0, s, 1, d, g, r, x);
     return cudaGetLastError();
 }
 
 cudaError_t batch_lincomb(double* out, double a, const double* X, double b, const double* Y,
                           long long total, int num_sms, cudaStream_t s)
 {
-    lincomb_kernel<<<elementwise_grid(total, num_sms), 256, 0, s>>>(out, a, X, b, Y, total);
+    launch_dep(lincomb_kernel, dim3(elementwise_grid(total, num_sms)), 256, 0, s, 1, out, a, X, b, Y, total);
     return cudaGetLastError();
 }
 
 cudaError_t batch_ros2_stage(const BatchDev& d, const double* N, const double* K1, double* Y,
                              double* gtc, const Rk45Ctl& ctl, double gamma, cudaStream_t s)
 {
-    ros2_stage_kernel<<<d.n_cells, 256, 0, s>>>(d, N, K1, Y, gtc, ctl, gamma);
+    launch_dep(ros2_stage_kernel, dim3(d.n_cells), 256, 0, s, 1, d, N, K1, Y, gtc, ctl, gamma);
     return cudaGetLastError();
 }
 
 cudaError_t batch_ros2_control(const BatchDev& d, double* N, const double* K1, const double* K2,
                                const Rk45Ctl& ctl, cudaStream_t s)
 {
-    ros2_control_kernel<<<d.n_cells, 256, 0, s>>>(d, N, K1, K2, ctl);
+    launch_dep(ros2_control_kernel, dim3(d.n_cells), 256, 0, s, 1, d, N, K1, K2, ctl);
     return cudaGetLastError();
 }
 
 cudaError_t batch_ros_update(double* N, double c1, const double* K1, double c2, const double* K2,
                              long long total, int num_sms, cudaStream_t s)
 {
-    ros_update_kernel<<<elementwise_grid(total, num_sms), 256, 0, s>>>(N, c1, K1, c2, K2, total);
+    launch_dep(ros_update_kernel, dim3(elementwise_grid(total, num_sms)), 256, 0, s, 1, N, c1, K1, c2, K2,
+               total);
     return cudaGetLastError();
 }
 

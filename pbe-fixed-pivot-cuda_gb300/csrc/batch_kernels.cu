@@ -40,6 +40,7 @@ constexpr int SW = kSlotBins;
 __global__ void __launch_bounds__(256)
 batch_grid_kernel(BatchDev d)
 {
+    dep_wait();
     __shared__ double sh[8];
     __shared__ int d0_s;
     BatchGridDev* gd = d.grids + blockIdx.x;
@@ -107,6 +108,8 @@ batch_grid_kernel(BatchDev d)
 __global__ void __launch_bounds__(256)
 batch_frag_kernel(BatchDev d, const double* __restrict__ t_q, const double* __restrict__ bw_q)
 {
+    const int dep = dep_wait();
+    t_q += dep; bw_q += dep;
     const BatchGridDev gd = d.grids[blockIdx.x];
     const int n = gd.n, nq = d.nq;
     const double* x = d.gx + gd.off;
@@ -174,6 +177,8 @@ __global__ void __launch_bounds__(256)
 cell_stage_kernel(double* N, const double* k, double* kacc, double* Y, int n, int stage,
                   double c, double dt6)
 {
+    const int dep = dep_wait();
+    k += dep; n += dep;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) stage_update(stage, N, k, kacc, Y, i, c, dt6);
 }
@@ -186,6 +191,8 @@ __global__ void __launch_bounds__(256)
 batch_sel_kernel(BatchDev d, const pbe_batch_cell_params_t* __restrict__ params,
                  double* __restrict__ Sx, long long total)
 {
+    const int dep = dep_wait();
+    params += dep; Sx += dep;
     for (long long e = blockIdx.x * 256LL + threadIdx.x; e < total; e += 256LL * gridDim.x) {
         int lo = 0, hi = d.n_cells;          // cells[lo].off <= e < cells[hi].off
         while (hi - lo > 1) {
@@ -323,6 +330,8 @@ __global__ void __launch_bounds__(256)
 batch_prep_kernel(BatchDev d, double* N, const pbe_batch_cell_params_t* __restrict__ params,
                   int stage, double c, double dt6, StageCombine sc)
 {
+    const int dep = dep_wait();
+    params += dep;
     __shared__ double sh[8];
     __shared__ PrefixShared psm;
     const cg::cluster_group cl = cg::this_cluster();
@@ -402,6 +411,8 @@ __global__ void __launch_bounds__(256)
 batch_jvp_prep_kernel(BatchDev d, const double* __restrict__ v,
                       const pbe_batch_cell_params_t* __restrict__ params)
 {
+    const int dep = dep_wait();
+    v += dep; params += dep;
     __shared__ double sh[8];
     __shared__ PrefixShared psm;
     const cg::cluster_group cl = cg::this_cluster();
@@ -556,6 +567,8 @@ batch_main_kernel(BatchDev d, const double* __restrict__ Y,
                   const pbe_batch_cell_params_t* __restrict__ params, double* out, int accumulate,
                   const int4* __restrict__ bundles, const int4* __restrict__ tasks)
 {
+    const int dep = dep_wait();
+    Y += dep; params += dep; bundles += dep; tasks += dep;
     __shared__ SlotShared sm;
     const int4 bu = bundles[blockIdx.x];     // {first task, tasks, group size, 0}
     const int T = bu.z;
@@ -572,11 +585,11 @@ cudaError_t main_k(const BatchDev& d, const double* Y, const pbe_batch_cell_para
 {
     if (n_bundles <= 0) return cudaSuccess;
     if (d.A)
-        batch_main_kernel<K, 2><<<n_bundles, kMainThreads, 0, s>>>(d, Y, params, out, accumulate ? 1 : 0,
-                                                                   bundles, tasks);
+        launch_dep(batch_main_kernel<K, 2>, dim3(n_bundles), kMainThreads, 0, s, 1, d, Y, params, out,
+                   accumulate ? 1 : 0, bundles, tasks);
     else
-        batch_main_kernel<K, 1><<<n_bundles, kMainThreads, 0, s>>>(d, Y, params, out, accumulate ? 1 : 0,
-                                                                   bundles, tasks);
+        launch_dep(batch_main_kernel<K, 1>, dim3(n_bundles), kMainThreads, 0, s, 1, d, Y, params, out,
+                   accumulate ? 1 : 0, bundles, tasks);
     return cudaGetLastError();
 }
 
@@ -587,8 +600,8 @@ cudaError_t batch_grid_tables(const BatchDev& d, const double* t_q, const double
 {
     (void)max_grid_n;
     if (d.n_grids <= 0) return cudaErrorInvalidValue;
-    batch_grid_kernel<<<d.n_grids, 256, 0, s>>>(d);
-    if (d.nq > 0) batch_frag_kernel<<<d.n_grids, 256, 0, s>>>(d, t_q, bw_q);
+    launch_dep(batch_grid_kernel, dim3(d.n_grids), 256, 0, s, 1, d);
+    if (d.nq > 0) launch_dep(batch_frag_kernel, dim3(d.n_grids), 256, 0, s, 1, d, t_q, bw_q);
     return cudaGetLastError();
 }
 
@@ -612,6 +625,8 @@ __global__ void __launch_bounds__(256)
 rk45_control_kernel(BatchDev d, double* N, const double* __restrict__ Y, StageCombine e,
                     double* k0, Rk45Ctl ctl)
 {
+    const int dep = dep_wait();
+    Y += dep;
     __shared__ double sh[8];
     __shared__ int accept_s;
     const int c = blockIdx.x;
@@ -672,7 +687,8 @@ cudaError_t batch_sel(const BatchDev& d, const pbe_batch_cell_params_t* params, 
 {
     if (d.n_cells <= 0 || d.selection < 0 || total <= 0) return cudaErrorInvalidValue;
     const long long b = (total + 255) / 256, cap = 16LL * (d.num_sms > 0 ? d.num_sms : 1);
-    batch_sel_kernel<<<static_cast<int>(b < cap ? b : cap), 256, 0, s>>>(d, params, Sx, total);
+    launch_dep(batch_sel_kernel, dim3(static_cast<int>(b < cap ? b : cap)), 256, 0, s, 1, d, params, Sx,
+               total);
     return cudaGetLastError();
 }
 
@@ -701,7 +717,7 @@ cudaError_t batch_rk45_control(const BatchDev& d, double* N, const double* Y,
                                const StageCombine& err, double* k0, const Rk45Ctl& ctl,
                                cudaStream_t s)
 {
-    rk45_control_kernel<<<d.n_cells, 256, 0, s>>>(d, N, Y, err, k0, ctl);
+    launch_dep(rk45_control_kernel, dim3(d.n_cells), 256, 0, s, 1, d, N, Y, err, k0, ctl);
     return cudaGetLastError();
 }
 
@@ -731,7 +747,7 @@ cudaError_t cell_stage(double* N, const double* k, double* kacc, double* Y, int 
                        double c, double dt6, cudaStream_t s)
 {
     if (n <= 0) return cudaErrorInvalidValue;
-    cell_stage_kernel<<<(n + 255) / 256, 256, 0, s>>>(N, k, kacc, Y, n, stage, c, dt6);
+    launch_dep(cell_stage_kernel, dim3((n + 255) / 256), 256, 0, s, 1, N, k, kacc, Y, n, stage, c, dt6);
     return cudaGetLastError();
 }
 

@@ -193,18 +193,9 @@ __device__ __forceinline__ void cell_prefix(const double* __restrict__ x, const 
 template <class... P, class... A>
 cudaError_t launch_prep(const BatchDev& d, void (*kern)(P...), int threads, cudaStream_t s, A... args)
 {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(d.n_cells) * static_cast<unsigned>(d.prep_ranks));
-    cfg.blockDim = dim3(static_cast<unsigned>(threads));
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = static_cast<unsigned>(d.prep_ranks);
-    at.val.clusterDim.y = 1;
-    at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
+    const unsigned ranks = static_cast<unsigned>(d.prep_ranks);
+    return launch_dep(kern, dim3(static_cast<unsigned>(d.n_cells) * ranks), static_cast<unsigned>(threads), 0, s,
+                      ranks, args...);
 }
 
 } // namespace pbe_gb300

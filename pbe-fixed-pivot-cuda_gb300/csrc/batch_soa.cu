@@ -22,6 +22,8 @@ __global__ void __launch_bounds__(kTile * 8)
 soa_kernel(BatchDev d, const double* __restrict__ src, double* __restrict__ dst, long long ld,
            int max_n)
 {
+    const int dep = dep_wait();
+    src += dep; dst += dep;
     __shared__ double tile[kTile][kTile + 1];
     const int c0 = blockIdx.x * kTile, i0 = blockIdx.y * kTile;
     const int tx = threadIdx.x & (kTile - 1), ty = threadIdx.x / kTile;   // 32 x 8 threads
@@ -69,8 +71,8 @@ cudaError_t batch_soa(const BatchDev& d, const double* src, double* dst, long lo
     if (d.n_cells <= 0 || max_n <= 0) return cudaSuccess;
     const dim3 grid((d.n_cells + kTile - 1) / kTile, (max_n + kTile - 1) / kTile);
     if (grid.y > 65535u) return cudaErrorInvalidValue;
-    if (to_packed) soa_kernel<true><<<grid, kTile * 8, 0, s>>>(d, src, dst, ld, max_n);
-    else soa_kernel<false><<<grid, kTile * 8, 0, s>>>(d, src, dst, ld, max_n);
+    if (to_packed) launch_dep(soa_kernel<true>, dim3(grid), kTile * 8, 0, s, 1, d, src, dst, ld, max_n);
+    else launch_dep(soa_kernel<false>, dim3(grid), kTile * 8, 0, s, 1, d, src, dst, ld, max_n);
     return cudaGetLastError();
 }
 

@@ -85,6 +85,8 @@ batch_vjp_prep_kernel(BatchDev d, BatchVjpDev vd, const double* __restrict__ N,
                       const double* __restrict__ lam, double* __restrict__ gN,
                       const pbe_batch_cell_params_t* __restrict__ params)
 {
+    const int dep = dep_wait();
+    N += dep; lam += dep; gN += dep; params += dep;
     __shared__ double sh[8];
     __shared__ double msh[kPrepMaxWarps][3 * kMomN];
     __shared__ PrefixShared psm;
@@ -275,6 +277,8 @@ batch_vjp_row_kernel(BatchDev d, BatchVjpDev vd, const double* __restrict__ N,
                      const double* __restrict__ lam, double* __restrict__ gN,
                      const pbe_batch_cell_params_t* __restrict__ params)
 {
+    const int dep = dep_wait();
+    N += dep; lam += dep; gN += dep; params += dep;
     __shared__ RowShared sm;
     const int4 bu = vd.rbundles[blockIdx.x];  // {first task, tasks, group size, 0}
     const int T = bu.z;
@@ -468,6 +472,8 @@ batch_vjp_main_kernel(BatchDev d, BatchVjpDev vd, const double* __restrict__ N,
                       const double* __restrict__ lam, double* __restrict__ gN,
                       const pbe_batch_cell_params_t* __restrict__ params)
 {
+    const int dep = dep_wait();
+    N += dep; lam += dep; gN += dep; params += dep;
     extern __shared__ double red[];     // [kVRows][kMainThreads]
     __shared__ VjpShared sm;
     __shared__ int s_b;
@@ -495,6 +501,8 @@ template <int K>
 __global__ void __launch_bounds__(256)
 batch_vjp_gfin_kernel(BatchDev d, BatchVjpDev vd, double* __restrict__ gparams)
 {
+    const int dep = dep_wait();
+    gparams += dep;
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, l = threadIdx.x & 31;
     if (c >= d.n_cells) return;
     if (d.kernel >= 0) {
@@ -531,16 +539,18 @@ cudaError_t vjp_k(const BatchDev& d, const BatchVjpDev& vd, const double* N, con
     if (e != cudaSuccess) return e;
     if (d.kernel >= 0) {
         if (vd.n_rbundles > 0)
-            batch_vjp_row_kernel<K><<<vd.n_rbundles, kMainThreads, 0, s>>>(d, vd, N, lam, gN, params);
+            launch_dep(batch_vjp_row_kernel<K>, dim3(vd.n_rbundles), kMainThreads, 0, s, 1, d, vd, N, lam,
+                       gN, params);
         if (vd.n_bundles > 0) {
             e = cudaMemsetAsync(vd.counter, 0, sizeof(int), s);
             if (e != cudaSuccess) return e;
             const int grid = vd.n_bundles < 2 * d.num_sms ? vd.n_bundles : 2 * d.num_sms;
             const size_t smem = sizeof(double) * kVRows * kMainThreads;
-            batch_vjp_main_kernel<K><<<grid, kMainThreads, smem, s>>>(d, vd, N, lam, gN, params);
+            launch_dep(batch_vjp_main_kernel<K>, dim3(grid), kMainThreads, smem, s, 1, d, vd, N, lam, gN,
+                       params);
         }
     }
-    batch_vjp_gfin_kernel<K><<<(d.n_cells + 7) / 8, 256, 0, s>>>(d, vd, gparams);
+    launch_dep(batch_vjp_gfin_kernel<K>, dim3((d.n_cells + 7) / 8), 256, 0, s, 1, d, vd, gparams);
     return cudaGetLastError();
 }
 
@@ -556,6 +566,8 @@ __global__ void __launch_bounds__(256)
 adj_coeff_kernel(double* a, const double* lp, double* mu, double w, double c, long long n,
                  int first)
 {
+    const int dep = dep_wait();
+    lp += dep;
     const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     a[i] = first ? w * lp[i] : fma(c, mu[i], w * lp[i]);
@@ -564,6 +576,8 @@ adj_coeff_kernel(double* a, const double* lp, double* mu, double w, double c, lo
 
 __global__ void __launch_bounds__(256) adj_sum_kernel(double* lsum, const double* mu, long long n)
 {
+    const int dep = dep_wait();
+    mu += dep;
     const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n) lsum[i] += mu[i];
 }
@@ -601,14 +615,14 @@ cudaError_t batch_vjp(const BatchDev& d, const BatchVjpDev& vd, const double* N,
 cudaError_t batch_adj_coeff(double* a, const double* lp, double* mu, double w, double c,
                             long long n, bool first, cudaStream_t s)
 {
-    adj_coeff_kernel<<<static_cast<int>((n + 255) / 256), 256, 0, s>>>(a, lp, mu, w, c, n,
-                                                                       first ? 1 : 0);
+    launch_dep(adj_coeff_kernel, dim3(static_cast<int>((n + 255) / 256)), 256, 0, s, 1, a, lp, mu, w, c, n,
+               first ? 1 : 0);
     return cudaGetLastError();
 }
 
 cudaError_t batch_adj_sum(double* lsum, const double* mu, long long n, cudaStream_t s)
 {
-    adj_sum_kernel<<<static_cast<int>((n + 255) / 256), 256, 0, s>>>(lsum, mu, n);
+    launch_dep(adj_sum_kernel, dim3(static_cast<int>((n + 255) / 256)), 256, 0, s, 1, lsum, mu, n);
     return cudaGetLastError();
 }
 

@@ -50,6 +50,8 @@ brk_prep_kernel(const double* __restrict__ N, const double* __restrict__ x,
                 const double* __restrict__ t_q, const double* __restrict__ bw_q, int n, int nq,
                 BrkWs ws, double S0, double v_ref, double alpha, double v_min)
 {
+    const int dep = dep_wait();
+    N += dep; x += dep; t_q += dep; bw_q += dep; n += dep;
     __shared__ double sh[8];
     const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const bool live = idx < static_cast<long long>(n) * nq;   // every lane takes part in the shuffle
@@ -120,6 +122,8 @@ brk_prep_kernel(const double* __restrict__ N, const double* __restrict__ x,
 __global__ void __launch_bounds__(256)
 brk_gather_kernel(double* __restrict__ rhs, int n, int nq, BrkWs ws)
 {
+    const int dep = dep_wait();
+    rhs += dep; n += dep;
     __shared__ double sh[8];
     int nqp = 1;
     while (nqp < nq && nqp < 32) nqp <<= 1;
@@ -352,6 +356,13 @@ __device__ __forceinline__ void brk_bin0(const double* __restrict__ N, const dou
     __shared__ double s_pre[32 * kBinWarpsMax];
     constexpr bool kS0 = (F == 0 || F == 3);
     const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, w = tid >> 5, W = T >> 5;
+    bool waited = !(F == 1 || F == 2);
+    auto wait = [&]() {                        // for SN (brk_bin_kernel)
+        if (waited) return;
+        const int dep = dep_wait();
+        SN += dep; rhs += dep;
+        waited = true;
+    };
     const bool mid0 = n >= 2;                  // bracket 0 is [x0, x1); else all of it is bin 0's
     const double x1 = mid0 ? __ldg(x + 1) : 0.0;
     const double inv0 = mid0 ? 1.0 / (x1 - __ldg(x)) : 0.0;
@@ -368,6 +379,7 @@ __device__ __forceinline__ void brk_bin0(const double* __restrict__ N, const dou
         const int f1 = mid0 ? first_parent_spec(x, n, 1, tq, first_parent_guess(lx1, ltq, lx0, inv_span, n)).f
                             : n;
         fm = max(fm, f0);
+        wait();
         double lo = 0.0;
         for (int j = f0; j < f1; ++j) {
             const double u = bin_unit<F>(N, x, SN, j, v_min);
@@ -375,6 +387,7 @@ __device__ __forceinline__ void brk_bin0(const double* __restrict__ N, const dou
         }
         term = fma(bw, lo, term);
     }
+    wait();
     for (int o = 16; o > 0; o >>= 1) fm = max(fm, __shfl_xor_sync(0xffffffffu, fm, o));
     if (lane == 0) s_fmax[w] = fm;
     __syncthreads();
@@ -423,6 +436,15 @@ brk_bin_kernel(const double* __restrict__ N, const double* __restrict__ x,
                double* __restrict__ rhs, int n, int nq, const double* __restrict__ SN,
                double S0, double v_ref, double alpha, double v_min)
 {
+    // After brk_sn_kernel (Linear, PowerLaw) the search for the parents' ranges runs
+    // beside it -- it passed its own wait, so the pivots and the table are there -- and
+    // the wait comes before the first S_j N_j; else at once.
+    bool waited = false;
+    if constexpr (F == 0 || F == 3) {
+        const int dep = dep_wait();
+        waited = true;
+        N += dep; x += dep; t_q += dep; bw_q += dep; rhs += dep; n += dep;
+    }
     if ((F == 0 || F == 3) && S0 == 0.0) return;     // S = 0 everywhere: no breakage at all
     __shared__ double s_acc[kBinWarpsMax][32];
     // index of a volume on the geometric grid through x[0] and x[n-1] (guesses only)
@@ -505,6 +527,11 @@ brk_bin_kernel(const double* __restrict__ N, const double* __restrict__ x,
         // every lane runs every shuffle (full mask), then selects
         const int up = __shfl_down_sync(0xffffffffu, f, 1);
         const int fn = (lane < 31) ? up : ft;                   // f(c + 1)
+        if (!waited) {
+            const int dep = dep_wait();
+            SN += dep; rhs += dep;
+            waited = true;
+        }
         bracket_shares<F>(N, x, SN, v_min, f, fn, v, tq, bw, xc, mid, top, A, H);
     }
     // bin c: the lower shares A - H/dx_c; bin c + 1: the upper shares H/dx_c
@@ -527,12 +554,17 @@ brk_bin_kernel(const double* __restrict__ N, const double* __restrict__ x,
 }
 
 // S_j N_j with the reference's guard, one thread per bin (Linear and
-// PowerLaw selections: one division or pow per bin instead of per fragment).
+// PowerLaw selections: one division or pow per bin instead of per fragment. Formed by
+// the fragments' warps instead, without this kernel: Linear 6.5 us for 6.6 at n = 480
+// and 8 points, 24 for 10 at n = 8191 and 16; PowerLaw 16 for 12 and 138 for 15).
 template <int F>
 __global__ void __launch_bounds__(256)
 brk_sn_kernel(const double* __restrict__ N, const double* __restrict__ x, int n, double* SN,
               double S0, double v_ref, double alpha, double v_min)
 {
+    const int dep = dep_wait();
+    N += dep; x += dep; n += dep;
+    dep_launch();                              // the search of brk_bin_kernel runs beside this
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const double S = selection<F>(x[j], S0, v_ref, alpha, v_min);
@@ -556,6 +588,8 @@ brk_scatter_kernel(const double* __restrict__ N, const double* __restrict__ x,
                    const double* __restrict__ t_q, const double* __restrict__ bw_q, double* rhs,
                    int n, int nq, double S0, double v_ref, double alpha, double v_min)
 {
+    const int dep = dep_wait();
+    N += dep; x += dep; t_q += dep; bw_q += dep; n += dep;
     const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= static_cast<long long>(n) * nq) return;
     const int q = static_cast<int>(idx / n);
@@ -580,39 +614,36 @@ cudaError_t launch_f(const BrkArgs& a, bool scatter, void* ws_base, cudaStream_t
     const long long m = static_cast<long long>(a.n) * a.n_quad;
     const int grid = static_cast<int>((m + 255) / 256);
     if (scatter) {
-        brk_scatter_kernel<F><<<grid, 256, 0, s>>>(a.N, a.x, a.t_q, a.bw_q, a.rhs, a.n, a.n_quad,
-                                                   a.S0, a.v_ref, a.alpha, a.v_min);
+        launch_dep(brk_scatter_kernel<F>, dim3(grid), 256, 0, s, 1, a.N, a.x, a.t_q, a.bw_q, a.rhs, a.n,
+                   a.n_quad, a.S0, a.v_ref, a.alpha, a.v_min);
     } else {
         BrkWs ws;
         brk_ws_layout(a.n, a.n_quad, static_cast<char*>(ws_base), &ws);
         if (kind == kBrkFull && brk_gather_path() == 0) {
             if (F == 1 || F == 2)
-                brk_sn_kernel<F><<<(a.n + 255) / 256, 256, 0, s>>>(a.N, a.x, a.n, ws.SN, a.S0,
-                                                                  a.v_ref, a.alpha, a.v_min);
+                launch_dep(brk_sn_kernel<F>, dim3((a.n + 255) / 256), 256, 0, s, 1, a.N, a.x, a.n, ws.SN,
+                           a.S0, a.v_ref, a.alpha, a.v_min);
             const int W = a.n_quad < kBinWarpsMax ? a.n_quad : kBinWarpsMax;
-            brk_bin_kernel<F><<<1 + (a.n - 1 + kBrkBins - 1) / kBrkBins, 32 * W, 0, s>>>(
-                a.N, a.x, a.t_q, a.bw_q, a.rhs, a.n, a.n_quad, ws.SN, a.S0, a.v_ref, a.alpha,
-                a.v_min);
+            launch_dep(brk_bin_kernel<F>, dim3(1 + (a.n - 1 + kBrkBins - 1) / kBrkBins), 32 * W, 0, s, 1,
+                       a.N, a.x, a.t_q, a.bw_q, a.rhs, a.n, a.n_quad, ws.SN, a.S0, a.v_ref, a.alpha, a.v_min);
             return cudaGetLastError();
         }
         if (kind == kBrkTables) {
-            brk_prep_kernel<F, kBrkTables><<<grid, 256, 0, s>>>(a.N, a.x, a.t_q, a.bw_q, a.n,
-                                                                a.n_quad, ws, a.S0, a.v_ref,
-                                                                a.alpha, a.v_min);
+            launch_dep(brk_prep_kernel<F, kBrkTables>, dim3(grid), 256, 0, s, 1, a.N, a.x, a.t_q, a.bw_q,
+                       a.n, a.n_quad, ws, a.S0, a.v_ref, a.alpha, a.v_min);
             return cudaGetLastError();
         }
         if (kind == kBrkStage)
-            brk_prep_kernel<F, kBrkStage><<<grid, 256, 0, s>>>(a.N, a.x, a.t_q, a.bw_q, a.n,
-                                                               a.n_quad, ws, a.S0, a.v_ref,
-                                                               a.alpha, a.v_min);
+            launch_dep(brk_prep_kernel<F, kBrkStage>, dim3(grid), 256, 0, s, 1, a.N, a.x, a.t_q, a.bw_q,
+                       a.n, a.n_quad, ws, a.S0, a.v_ref, a.alpha, a.v_min);
         else
-            brk_prep_kernel<F, kBrkFull><<<grid, 256, 0, s>>>(a.N, a.x, a.t_q, a.bw_q, a.n,
-                                                              a.n_quad, ws, a.S0, a.v_ref,
-                                                              a.alpha, a.v_min);
+            launch_dep(brk_prep_kernel<F, kBrkFull>, dim3(grid), 256, 0, s, 1, a.N, a.x, a.t_q, a.bw_q, a.n,
+                       a.n_quad, ws, a.S0, a.v_ref, a.alpha, a.v_min);
         int nqp = 1;
         while (nqp < a.n_quad && nqp < 32) nqp <<= 1;
         const int per_block = 8 * (32 / nqp);               // bins per 256-thread block
-        brk_gather_kernel<<<(a.n + per_block - 1) / per_block, 256, 0, s>>>(a.rhs, a.n, a.n_quad, ws);
+        launch_dep(brk_gather_kernel, dim3((a.n + per_block - 1) / per_block), 256, 0, s, 1, a.rhs, a.n,
+                   a.n_quad, ws);
     }
     return cudaGetLastError();
 }
@@ -631,6 +662,11 @@ cudaError_t brk_dispatch(const BrkArgs& a, bool scatter, void* ws_base, cudaStre
     }
 }
 } // namespace
+
+bool brk_needs_scratch(const BrkArgs& a, bool scatter)
+{
+    return !scatter && (a.selection == 1 || a.selection == 2 || brk_gather_path() != 0);
+}
 
 cudaError_t brk_launch(const BrkArgs& a, bool scatter, void* ws_base, cudaStream_t s)
 {

@@ -99,6 +99,8 @@ __global__ void __launch_bounds__(kPrepThreads)
 vjp_prep_kernel(const double* __restrict__ N, const double* __restrict__ x,
                 const double* __restrict__ lam, int n, VjpWs ws)
 {
+    const int dep = dep_wait();
+    N += dep; x += dep; lam += dep; n += dep;
     __shared__ double sh[kPrepThreads / 32][kVjpMom];
     __shared__ double sv[kMomN];
     __shared__ int se;
@@ -223,6 +225,8 @@ template <int MODE>
 __global__ void __launch_bounds__(256)
 vjp_fin_kernel(const double* __restrict__ x, int n, VjpWs ws)
 {
+    const int dep = dep_wait();
+    x += dep; n += dep;
     const int nb = (n + kPrepThreads - 1) / kPrepThreads;
     const int wq = threadIdx.x >> 5, lq = threadIdx.x & 31;
     if (wq < 4) {
@@ -315,6 +319,8 @@ __global__ void __launch_bounds__(kMainThreads, 2)
 vjp_main_kernel(const double* __restrict__ N, const double* __restrict__ x,
                 const double* __restrict__ lam, VjpWs ws, int n, int ntile, int nch, int lane_on)
 {
+    const int dep = dep_wait();
+    N += dep; x += dep; lam += dep; n += dep;
     extern __shared__ double red[];               // [kVRows][kMainThreads]
     __shared__ VjpShared sm;
     __shared__ int s_task;
@@ -351,6 +357,8 @@ vjp_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
                 const double* __restrict__ lam, double* __restrict__ gN, VjpWs ws, int n,
                 int ntile, int nch, double b0, double bbr, double bsh, int lane_on)
 {
+    const int dep = dep_wait();
+    N += dep; x += dep; lam += dep; gN += dep; n += dep;
     __shared__ double fin[8][kVRows];
     if (lane_on && ws.mom[10] != 0.0) return;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -394,6 +402,7 @@ vjp_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
 __global__ void __launch_bounds__(128) vjp_gfin_kernel(int ntile, VjpWs ws, double* gp, int nslots,
                                                        int nlane)
 {
+    dep_wait();
     const int q = threadIdx.x >> 5, l = threadIdx.x & 31;
     if (q >= nslots) return;
     if (nlane > 0 && ws.mom[10] != 0.0) ntile = nlane;
@@ -437,6 +446,8 @@ vjp_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
                 const double* __restrict__ lam, VjpWs ws, int n, int C,
                 double b0, double bbr, double bsh)
 {
+    const int dep = dep_wait();
+    N += dep; x += dep; lam += dep; n += dep;
     extern __shared__ double esm[];               // [kLaneWarps][per_max + 32] W windows
     __shared__ double red[kLaneWarps][2][kLaneBins];
     __shared__ int s_task;
@@ -620,6 +631,8 @@ vjp_lane_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
                      const double* __restrict__ lam, double* __restrict__ gN, VjpWs ws, int n,
                      int C, double b0, double bbr, double bsh)
 {
+    const int dep = dep_wait();
+    N += dep; x += dep; lam += dep; gN += dep; n += dep;
     __shared__ double lw[kVRowsWarps][kLaneBins];
     __shared__ int base[kVLaneMaxChunks + 1];
     __shared__ double xs3[3][kLaneBins];           // exact rows: larger-member sum, smaller-member sums
@@ -830,6 +843,8 @@ brk_vjp_kernel(const double* __restrict__ N, const double* __restrict__ x,
                int nq, int nqp, double S0, double v_ref, double alpha, double v_min,
                const double* __restrict__ Ssel, const int* __restrict__ lo_tab)
 {
+    const int dep = dep_wait();
+    N += dep; x += dep; t_q += dep; bw_q += dep; lam += dep; gN += dep; Ssel += dep; lo_tab += dep; n += dep;
     __shared__ double sh[8];
     const int l = threadIdx.x % nqp;
     const int j = (blockIdx.x * blockDim.x + threadIdx.x) / nqp;
@@ -931,31 +946,32 @@ cudaError_t agg_vjp_k(const AggVjpArgs& a, const VjpWs& ws, int num_sms, cudaStr
     const long long ltasks = vjp_lane_tasks(n, C);
     const int lane_on = (vjp_lane_mode() && ltasks > 0 && vjp_lane_chunks(n, C) <= kVLaneMaxChunks) ? 1 : 0;
     if (kind == kVjpTables) {
-        vjp_prep_kernel<kVjpTables><<<nb, kPrepThreads, 0, s>>>(a.N, a.x, a.lam, n, ws);
-        vjp_fin_kernel<kVjpTables><<<1, 256, 0, s>>>(a.x, n, ws);
+        launch_dep(vjp_prep_kernel<kVjpTables>, dim3(nb), kPrepThreads, 0, s, 1, a.N, a.x, a.lam, n, ws);
+        launch_dep(vjp_fin_kernel<kVjpTables>, dim3(1), 256, 0, s, 1, a.x, n, ws);
         return cudaGetLastError();
     }
     if (kind == kVjpStage) {
-        vjp_prep_kernel<kVjpStage><<<nb, kPrepThreads, 0, s>>>(a.N, a.x, a.lam, n, ws);
-        vjp_fin_kernel<kVjpStage><<<1, 256, 0, s>>>(a.x, n, ws);
+        launch_dep(vjp_prep_kernel<kVjpStage>, dim3(nb), kPrepThreads, 0, s, 1, a.N, a.x, a.lam, n, ws);
+        launch_dep(vjp_fin_kernel<kVjpStage>, dim3(1), 256, 0, s, 1, a.x, n, ws);
     } else {
-        vjp_prep_kernel<kVjpFull><<<nb, kPrepThreads, 0, s>>>(a.N, a.x, a.lam, n, ws);
-        vjp_fin_kernel<kVjpFull><<<1, 256, 0, s>>>(a.x, n, ws);
+        launch_dep(vjp_prep_kernel<kVjpFull>, dim3(nb), kPrepThreads, 0, s, 1, a.N, a.x, a.lam, n, ws);
+        launch_dep(vjp_fin_kernel<kVjpFull>, dim3(1), 256, 0, s, 1, a.x, n, ws);
     }
     const int nrb = (n + kLaneBins - 1) / kLaneBins;
     if (lane_on) {
         const size_t lsmem = sizeof(double) * kLaneWarps * ((C + kLaneWarps - 1) / kLaneWarps + 32);
         const int lgrid = static_cast<int>(ltasks < kVLaneCtas * num_sms ? ltasks : kVLaneCtas * num_sms);
-        vjp_lane_kernel<K><<<lgrid, kMainThreads, lsmem, s>>>(a.N, a.x, a.lam, ws, n, C,
-                                                              a.beta0, a.beta_br, a.beta_sh);
+        launch_dep(vjp_lane_kernel<K>, dim3(lgrid), kMainThreads, lsmem, s, 1, a.N, a.x, a.lam, ws, n, C,
+                   a.beta0, a.beta_br, a.beta_sh);
     }
-    vjp_main_kernel<K><<<grid, kMainThreads, smem, s>>>(a.N, a.x, a.lam, ws, n, ntile, nch, lane_on);
-    vjp_rows_kernel<K><<<(ntile + 7) / 8, 256, 0, s>>>(a.N, a.x, a.lam, a.gN, ws, n, ntile, nch,
-                                                       a.beta0, a.beta_br, a.beta_sh, lane_on);
+    launch_dep(vjp_main_kernel<K>, dim3(grid), kMainThreads, smem, s, 1, a.N, a.x, a.lam, ws, n, ntile, nch,
+               lane_on);
+    launch_dep(vjp_rows_kernel<K>, dim3((ntile + 7) / 8), 256, 0, s, 1, a.N, a.x, a.lam, a.gN, ws, n, ntile,
+               nch, a.beta0, a.beta_br, a.beta_sh, lane_on);
     if (lane_on)
-        vjp_lane_rows_kernel<K><<<nrb, kVRowsWarps * 32, 0, s>>>(a.N, a.x, a.lam, a.gN, ws, n, C, a.beta0,
-                                                    a.beta_br, a.beta_sh);
-    vjp_gfin_kernel<<<1, 128, 0, s>>>(ntile, ws, a.gp, 3, lane_on ? nrb : 0);
+        launch_dep(vjp_lane_rows_kernel<K>, dim3(nrb), kVRowsWarps * 32, 0, s, 1, a.N, a.x, a.lam, a.gN, ws,
+                   n, C, a.beta0, a.beta_br, a.beta_sh);
+    launch_dep(vjp_gfin_kernel, dim3(1), 128, 0, s, 1, ntile, ws, a.gp, 3, lane_on ? nrb : 0);
     return cudaGetLastError();
 }
 
@@ -966,10 +982,9 @@ cudaError_t brk_vjp_f(const BrkVjpArgs& a, const VjpWs& ws, cudaStream_t s, cons
     int nqp = 1;
     while (nqp < a.n_quad && nqp < 32) nqp <<= 1;
     const int nb = static_cast<int>((static_cast<long long>(a.n) * nqp + 255) / 256);
-    brk_vjp_kernel<F><<<nb, 256, 0, s>>>(a.N, a.x, a.t_q, a.bw_q, a.lam, a.gN, ws.gpart, a.n,
-                                         a.n_quad, nqp, a.S0, a.v_ref, a.alpha, a.v_min, Ssel,
-                                         lo_tab);
-    vjp_gfin_kernel<<<1, 128, 0, s>>>(nb, ws, a.gp, 4, 0);
+    launch_dep(brk_vjp_kernel<F>, dim3(nb), 256, 0, s, 1, a.N, a.x, a.t_q, a.bw_q, a.lam, a.gN, ws.gpart,
+               a.n, a.n_quad, nqp, a.S0, a.v_ref, a.alpha, a.v_min, Ssel, lo_tab);
+    launch_dep(vjp_gfin_kernel, dim3(1), 128, 0, s, 1, nb, ws, a.gp, 4, 0);
     return cudaGetLastError();
 }
 
