@@ -165,7 +165,9 @@ cudaError_t brk_call(const double* N, const double* x, const double* t_q, const 
     if (e != cudaSuccess) return e;
     const bool scatter = resolve_mode(mode) == PBE_MODE_SCATTER;
     BrkArgs a{N, x, t_q, bw_q, rhs, p->n, p->n_quad, p->selection, p->S0, p->v_ref, p->alpha, p->v_min};
-    const size_t need = scatter ? 0 : brk_ws_layout(p->n, p->n_quad, nullptr, nullptr);
+    // a caller's scratch has to hold the layout; without one only what the call uses is taken
+    const size_t need = scatter || (!ws && !brk_needs_scratch(a, scatter))
+                            ? 0 : brk_ws_layout(p->n, p->n_quad, nullptr, nullptr);
     return with_scratch(need, ws, ws_bytes, s, st, [&](void* w) {
         return brk_launch(a, scatter, w, s);
     });

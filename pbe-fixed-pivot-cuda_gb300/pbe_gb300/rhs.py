@@ -19,29 +19,41 @@ from ._lib import AggregationParams, BreakageParams, MODE_DEFAULT
 Array = Union["torch.Tensor", int, None]  # noqa: F821
 
 
+_torch = None          # the module, once a call has needed it (an import statement a call costs 0.3 us)
+
+
+def _load_torch():
+    global _torch
+    import torch
+
+    _torch = torch
+    return torch
+
+
 def _ptr(a: Array, name: str) -> Optional[int]:
+    # a call has up to seven of these and a small one is bound by the host (64 sections,
+    # aggregation + breakage: 32 us of host time a pass): the common case first
+    torch = _torch or _load_torch()
+    if isinstance(a, torch.Tensor):
+        if a.dtype is not torch.float64:
+            raise TypeError("%s must be float64 (got %s)" % (name, a.dtype))
+        if not a.is_cuda:
+            raise TypeError("%s must be a CUDA tensor" % name)
+        if not a.is_contiguous():
+            raise TypeError("%s must be contiguous" % name)
+        return a.data_ptr()
     if a is None:
         return None
     if isinstance(a, int):
         return a or None
-    import torch
-
-    if not isinstance(a, torch.Tensor):
-        raise TypeError("%s must be a torch tensor or a device address" % name)
-    if a.dtype != torch.float64:
-        raise TypeError("%s must be float64 (got %s)" % (name, a.dtype))
-    if not a.is_cuda:
-        raise TypeError("%s must be a CUDA tensor" % name)
-    if not a.is_contiguous():
-        raise TypeError("%s must be contiguous" % name)
-    return a.data_ptr()
+    raise TypeError("%s must be a torch tensor or a device address" % name)
 
 
 def _stream(stream) -> Optional[int]:
     if stream is None:
-        import torch
-
-        return torch.cuda.current_stream().cuda_stream or None
+        # the current stream's handle without a Stream object (2.9 us a call on the host)
+        torch = _torch or _load_torch()
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()) or None
     if isinstance(stream, int):
         return stream or None
     return stream.cuda_stream or None
