@@ -250,11 +250,29 @@ vjp_fin_kernel(const double* __restrict__ x, int n, VjpWs ws)
 #pragma unroll
         for (int q = 0; q < kMomN; ++q) S[q] = 0.0;
         int e = e0;
-        for (int k = k0; k < k1; ++k) {
-            const int en = tag(k);
+        // kRun blocks' totals and exponents at a time, loaded together (as the forward's
+        // prep_offsets: a load at a time is a chain of 0.7 us each)
+        constexpr int kRun = 4;
+        double t[kRun][kMomN];
+        int en[kRun];
+        auto load = [&](int k) {
 #pragma unroll
-            for (int q = 0; q < kMomN; ++q) S[q] = shift(S[q], e, en) + tot[q * nb + blk(k)];
-            e = en;
+            for (int u = 0; u < kRun; ++u) {
+                const int c = min(k + u, nb - 1);
+                en[u] = tag(c);
+#pragma unroll
+                for (int q = 0; q < kMomN; ++q) t[u][q] = tot[q * nb + blk(c)];
+            }
+        };
+        for (int k = k0; k < k1; k += kRun) {
+            load(k);
+#pragma unroll
+            for (int u = 0; u < kRun; ++u) {
+                if (k + u >= k1) break;
+#pragma unroll
+                for (int q = 0; q < kMomN; ++q) S[q] = shift(S[q], e, en[u]) + t[u][q];
+                e = en[u];
+            }
         }
 #pragma unroll
         for (int q = 0; q < kMomN; ++q) R[q] = S[q];
@@ -273,14 +291,18 @@ vjp_fin_kernel(const double* __restrict__ x, int n, VjpWs ws)
             S[q] = lq > 0 ? r : 0.0;
         }
         e = e0;
-        for (int k = k0; k < k1; ++k) {
-            const int en = tag(k);
+        for (int k = k0; k < k1; k += kRun) {
+            load(k);
 #pragma unroll
-            for (int q = 0; q < kMomN; ++q) {
-                off[q * nb + blk(k)] = S[q];
-                S[q] = shift(S[q], e, en) + tot[q * nb + blk(k)];
+            for (int u = 0; u < kRun; ++u) {
+                if (k + u >= k1) break;
+#pragma unroll
+                for (int q = 0; q < kMomN; ++q) {
+                    off[q * nb + blk(k + u)] = S[q];
+                    S[q] = shift(S[q], e, en[u]) + t[u][q];
+                }
+                e = en[u];
             }
-            e = en;
         }
         return;
     }
@@ -299,6 +321,7 @@ vjp_fin_kernel(const double* __restrict__ x, int n, VjpWs ws)
             if (r == 10) t = (n >= 2 && t <= kGeoTol && ratio_ok) ? 1.0 : 0.0;
         } else {
             if (MODE == kVjpTables) continue;
+#pragma unroll 8
             for (int b = lq; b < nb; b += 32) t += ws.mom_part[b * kVjpMom + r];
             t = warp_sum(t);
         }
