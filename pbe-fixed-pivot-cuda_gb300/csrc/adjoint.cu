@@ -32,7 +32,7 @@
 #include <new>
 #include <vector>
 
-#include "pbe_internal.cuh"
+#include "tape_stage.cuh"
 #include "pbe_gb300.h"
 
 struct pbe_rk4_tape {
@@ -67,39 +67,39 @@ struct pbe_rk4_tape {
 namespace pbe_gb300 {
 namespace {
 
-// Stage q of one RK4 step (same rounding as the reference's host loop):
-// q = 0: acc = k; Y = N + c k.   q = 1, 2: acc += 2 k; Y = N + c k.
-// q = 3: acc += k; N += dt6 acc.
-__global__ void __launch_bounds__(256)
-rk_stage_kernel(double* N, const double* k, double* acc, double* Y, int n, int q, double c,
-                double dt6)
+// A stage update of its own, for instances without breakage (with it, the breakage's
+// gather does it).
+__global__ void __launch_bounds__(256) rk_stage_kernel(const double* k, int n, RkStage st)
 {
     const int dep = dep_wait();
     k += dep; n += dep;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double ki = k[i];
-    if (q == 0) {
-        acc[i] = ki;
-        Y[i] = __dadd_rn(N[i], __dmul_rn(c, ki));
-    } else if (q < 3) {
-        acc[i] = __dadd_rn(acc[i], __dmul_rn(2.0, ki));
-        Y[i] = __dadd_rn(N[i], __dmul_rn(c, ki));
-    } else {
-        const double s = __dadd_rn(acc[i], ki);
-        N[i] = __dadd_rn(N[i], __dmul_rn(dt6, s));
-    }
+    if (i < n) rk_update(st, i, k[i]);
 }
 
-// a = w lam' (+ c mu), then mu = 0 (ready for the next VJP).
+// a = w lam' and mu = 0, before the last stage's VJP.
 __global__ void __launch_bounds__(256)
-adj_coeff_kernel(double* a, const double* lp, double* mu, double w, double c, int n, int first)
+adj_coeff_kernel(double* a, const double* lp, double* mu, double w, int n)
 {
     const int dep = dep_wait();
     lp += dep; n += dep;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    a[i] = first ? w * lp[i] : fma(c, mu[i], w * lp[i]);
+    a[i] = w * lp[i];
+    mu[i] = 0.0;
+}
+
+// lsum += mu of one stage, and a = w lam' + c mu, mu = 0 for the next.
+__global__ void __launch_bounds__(256)
+adj_next_kernel(double* lsum, double* a, const double* lp, double* mu, double w, double c, int n)
+{
+    const int dep = dep_wait();
+    lp += dep; n += dep;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double m = mu[i];
+    lsum[i] += m;
+    a[i] = fma(c, m, w * lp[i]);
     mu[i] = 0.0;
 }
 
@@ -136,23 +136,32 @@ cudaError_t tables(pbe_rk4_tape* t, const double* N, cudaStream_t s)
     return e;
 }
 
-// k = RHS(Yin) with parameter set m, on the set's workspaces (bitwise the
-// result of the drop-in calls in gather mode).
-cudaError_t rhs(pbe_rk4_tape* t, int m, const double* Yin, cudaStream_t s)
+// k = RHS(Yin) with parameter set m, on the set's workspaces, and the stage update.
+// With both terms: aggregation prep with the breakage's, pair kernel, breakage gather
+// with the update.
+cudaError_t rhs(pbe_rk4_tape* t, int m, const double* Yin, const RkStage& st, cudaStream_t s)
 {
-    cudaError_t e = cudaMemsetAsync(t->k, 0, sizeof(double) * t->n, s);
-    if (e == cudaSuccess && t->kernel >= 0) {
+    cudaError_t e = cudaSuccess;
+    const bool agg = t->kernel >= 0, brk = t->selection >= 0;
+    BrkArgs b{};
+    if (brk) {
+        const pbe_brk_params_t& p = t->brk[m];
+        b = BrkArgs{Yin, t->x, t->t_q, t->bw_q, t->k, t->n, t->nq, t->selection, p.S0, p.v_ref,
+                    p.alpha, p.v_min};
+    }
+    bool prep_done = false;
+    if (agg) {
         const pbe_agg_params_t& p = t->agg[m];
         AggArgs a{Yin, t->x, t->k, t->n, t->kernel, p.beta0, p.beta_br, p.beta_sh};
-        e = agg_stage_launch(a, false, t->agg_ws[m], t->num_sms, s);
+        e = agg_stage_launch(a, t->agg_ws[m], t->num_sms, s, brk ? &b : nullptr, brk ? t->brk_ws[m] : nullptr,
+                             &prep_done);
+    } else {
+        e = cudaMemsetAsync(t->k, 0, sizeof(double) * t->n, s);
     }
-    if (e == cudaSuccess && t->selection >= 0) {
-        const pbe_brk_params_t& p = t->brk[m];
-        BrkArgs b{Yin, t->x, t->t_q, t->bw_q, t->k, t->n, t->nq, t->selection, p.S0, p.v_ref,
-                  p.alpha, p.v_min};
-        e = brk_stage_launch(b, t->brk_ws[m], s);
-    }
-    return e;
+    if (e != cudaSuccess) return e;
+    if (brk) return brk_stage_launch(b, t->brk_ws[m], s, prep_done, st);
+    launch_dep(rk_stage_kernel, dim3(blocks(t->n)), 256, 0, s, 1, t->k, t->n, st);
+    return cudaGetLastError();
 }
 
 // One RK4 step on N; Ys (nullable): stage states Y1..Y4 are written to Ys[q n].
@@ -165,12 +174,8 @@ cudaError_t step(pbe_rk4_tape* t, int m, double* N, double* Ys, cudaStream_t s)
     if (Ys) e = cudaMemcpyAsync(Ys, N, sizeof(double) * un, cudaMemcpyDeviceToDevice, s);
     for (int q = 0; q < 4 && e == cudaSuccess; ++q) {
         const double* in = (q == 0) ? N : (Ys ? Ys + q * un : t->Y);
-        e = rhs(t, m, in, s);
-        if (e != cudaSuccess) break;
         double* Yout = (q < 3) ? (Ys ? Ys + (q + 1) * un : t->Y) : t->Y;
-        launch_dep(rk_stage_kernel, dim3(blocks(t->n)), 256, 0, s, 1, N, t->k, t->acc, Yout, t->n, q, cs[q],
-                   dt6);
-        e = cudaGetLastError();
+        e = rhs(t, m, in, RkStage{N, t->acc, Yout, q, cs[q], dt6}, s);
     }
     return e;
 }
@@ -179,11 +184,13 @@ cudaError_t vjp(pbe_rk4_tape* t, int m, const double* Yq, double* g_agg, double*
                 cudaStream_t s)
 {
     cudaError_t e = cudaSuccess;
+    AggVjpArgs agg{};
     if (t->kernel >= 0) {
         const pbe_agg_params_t& p = t->agg[m];
         AggVjpArgs a{Yq, t->x, t->a, t->mu, g_agg + 3 * m, t->n, t->kernel, p.beta0, p.beta_br,
                      p.beta_sh};
-        e = agg_vjp_stage_launch(a, t->vjp_ws, t->num_sms, s);
+        agg = a;
+        e = agg_vjp_stage_launch(a, t->vjp_ws, t->num_sms, s, t->selection >= 0);
     }
     if (e == cudaSuccess && t->selection >= 0) {
         const pbe_brk_params_t& p = t->brk[m];
@@ -192,7 +199,7 @@ cudaError_t vjp(pbe_rk4_tape* t, int m, const double* Yq, double* g_agg, double*
         // the set's breakage tables (written by tables()): S per bin, fragment brackets
         BrkWs bw;
         brk_ws_layout(t->n, t->nq, static_cast<char*>(t->brk_ws[m]), &bw);
-        e = brk_vjp_launch(b, t->vjp_ws, s, bw.Ssel, bw.lo);
+        e = brk_vjp_launch(b, t->vjp_ws, s, bw.Ssel, bw.lo, t->kernel >= 0 ? &agg : nullptr);
     }
     return e;
 }
@@ -245,14 +252,17 @@ cudaError_t enqueue_backward(pbe_rk4_tape* t, const double* lamT, double* gN0, d
             e = cudaMemcpyAsync(lsum, lam, sizeof(double) * un, cudaMemcpyDeviceToDevice, s);
             for (int q = 3; q >= 0 && e == cudaSuccess; --q) {
                 const double w = (q == 0 || q == 3) ? c6 : 2.0 * c6;
-                launch_dep(adj_coeff_kernel, dim3(blocks(t->n)), 256, 0, s, 1, t->a, lam, t->mu, w,
-                           q < 3 ? cs[q] : 0.0, t->n, q == 3);
+                if (q == 3)
+                    launch_dep(adj_coeff_kernel, dim3(blocks(t->n)), 256, 0, s, 1, t->a, lam, t->mu, w, t->n);
+                else
+                    launch_dep(adj_next_kernel, dim3(blocks(t->n)), 256, 0, s, 1, lsum, t->a, lam, t->mu, w,
+                               cs[q], t->n);
                 e = cudaGetLastError();
                 if (e == cudaSuccess) e = vjp(t, m, Ys + q * un, g_agg, g_brk, s);
-                if (e == cudaSuccess) {
-                    launch_dep(adj_sum_kernel, dim3(blocks(t->n)), 256, 0, s, 1, lsum, t->mu, t->n);
-                    e = cudaGetLastError();
-                }
+            }
+            if (e == cudaSuccess) {
+                launch_dep(adj_sum_kernel, dim3(blocks(t->n)), 256, 0, s, 1, lsum, t->mu, t->n);
+                e = cudaGetLastError();
             }
             std::swap(lam, lsum);
         }

@@ -40,8 +40,8 @@
 // =============================================================================
 #include <cooperative_groups.h>
 
-#include "pbe_internal.cuh"
 #include "agg_lane.cuh"
+#include "tape_stage.cuh"
 
 namespace pbe_gb300 {
 namespace {
@@ -51,7 +51,7 @@ namespace {
 // so they keep the range of x_j / x_i on grids of any span; a shift between
 // exponents takes integer instructions only. Fixed order: reproducible.
 template <int K>
-__device__ __forceinline__ void prep_prefix(const double* m, double xm, int E, int i, int n,
+__device__ __forceinline__ void prep_prefix(const double* m, double xm, int E, int i, int n, int nb,
                                             const AggWs& ws, double* gsum)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -78,7 +78,7 @@ __device__ __forceinline__ void prep_prefix(const double* m, double xm, int E, i
         for (int q = 0; q < kMomN; ++q) { gsum[q] = P[q]; gsum[kMomN + q] = T[q]; }
     }
     asm volatile("bar.sync 1, %0;" :: "n"(kPrepThreads) : "memory");
-    const int nb = gridDim.x, b = blockIdx.x;
+    const int b = blockIdx.x;
     const int last = min(n - 1, b * kPrepThreads + kPrepThreads - 1);
 #pragma unroll
     for (int q = 0; q < kMomN; ++q) {
@@ -289,10 +289,18 @@ __device__ __forceinline__ int first_above(const double* __restrict__ x, int i, 
     return hi;
 }
 
+// What a stage call adds to its prep: rhs is zeroed, and the CTAs from nb on do the
+// breakage's prep of the stage (brk_stage_block).
+struct PrepStage {
+    double* rhs;
+    BrkArgs brk;
+    BrkWs bws;
+};
+
 template <int K, bool FULL>
 __global__ void __launch_bounds__(FULL ? kPrepFullThreads : kPrepStageThreads)
 agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int n, AggWs ws,
-                double b0, double bbr, double bsh)
+                double b0, double bbr, double bsh, int nb, PrepStage st)
 {
     const int dep = dep_wait();
     N += dep; x += dep; n += dep;
@@ -305,6 +313,13 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
     __shared__ GeoFit fit_s;
     __shared__ int d0_s[kPrepThreads / 32];
     __shared__ int last_s;
+    if constexpr (!FULL) {
+        if (static_cast<int>(blockIdx.x) >= nb) {
+            brk_stage_block(N, x, st.brk.t_q, st.brk.bw_q, n, st.brk.n_quad, st.bws,
+                            static_cast<int>(blockIdx.x) - nb, gsum);
+            return;
+        }
+    }
     const int tid = threadIdx.x, wp = tid >> 5, lane = tid & 31;
     const int i = blockIdx.x * kPrepThreads + (tid & (kPrepThreads - 1));
     const double xi = x[min(i, n - 1)];
@@ -326,6 +341,7 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
                 iai = ws.ia[i];
             }
             ws.h[i] = hi;
+            if (!FULL) st.rhs[i] = 0.0;
             m[0] = iai * Ni; m[1] = Ni; m[2] = ai * Ni; m[3] = (ai * ai) * Ni; m[4] = hi;
             xm = mantissa_of(xi);
             E = exponent_of(xi);
@@ -349,7 +365,7 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
         }
         const unsigned neg = __ballot_sync(0xffffffffu, !(Ni >= 0.0));   // negative, or NaN
         if (lane == 0) neg_s[wp] = neg != 0u;
-        prep_prefix<K>(m, xm, E, i, n, ws, gsum);
+        prep_prefix<K>(m, xm, E, i, n, nb, ws, gsum);
     } else if (wp >= (FULL ? 4 : 2)) {
         // window tables; FULL: the cube roots of the first two warps
         if constexpr (FULL) asm volatile("bar.sync 2, %0;" :: "n"(kPrepFullThreads) : "memory");
@@ -435,7 +451,7 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
         }
         ws.mom_part[blockIdx.x * 8 + 7] = (neg_s[0] | neg_s[1]) ? 1.0 : 0.0;
         __threadfence();                       // partials visible before the ticket
-        last_s = (atomicAdd(ws.counter + 2, 1) == static_cast<int>(gridDim.x) - 1);
+        last_s = (atomicAdd(ws.counter + 2, 1) == nb - 1);
     }
     __syncthreads();
     if (!last_s) return;
@@ -444,7 +460,6 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
     // block totals (prefix offsets, and the moments as its last sums); FULL, warp
     // 2: the largest deviation, warp 3: the smallest D0 candidate.
     __threadfence();
-    const int nb = gridDim.x;
     if (wp < 2) {
         prep_offsets<K>(x, n, nb, ws, wp, lane);
         if (wp == 1) {
@@ -814,7 +829,8 @@ agg_small_kernel(const double* __restrict__ N, const double* __restrict__ x, dou
         }
     }
     const double in = __shfl_up_sync(0xffffffffu, up, 1);
-    if (lane >= 1 && s < n) rhs[s] = rhs[s] + (((own + in) + clip) - death);
+    if (lane >= 1 && s < n)
+        rhs[s] = (KIND == kAggStage ? 0.0 : rhs[s]) + (((own + in) + clip) - death);   // a stage call writes rhs
 }
 
 // One cluster of the device can hold 16 CTAs of this kernel (a size beyond the
@@ -874,7 +890,8 @@ int agg_clip_tasks(int n)
 // the FULL prep only, kAggStage = the light prep + pair kernel on a
 // workspace whose tables an earlier kAggTables call wrote.
 template <int K, bool SC>
-cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_t s, int kind)
+cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_t s, int kind,
+                     const PrepStage* st, bool* brk_done)
 {
     const int n = a.n;
     if (!SC && n <= kSmallMaxN) {
@@ -897,13 +914,16 @@ cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_
     cudaError_t e = cudaSuccess;
     if (kind == kAggStage) {
         // counter[2] and [5] were left at 0 by the previous call on this workspace
-        launch_dep(agg_prep_kernel<K, false>, dim3(nb), kPrepStageThreads, 0, s, 1, a.N, a.x, n, ws,
-                   a.beta0, a.beta_br, a.beta_sh);
+        // (a stage's rhs is zeroed and its breakage prep done by further CTAs of the same launch)
+        const int bb = st->brk.n_quad > 0 ? brk_prep_blocks(n, st->brk.n_quad) : 0;
+        launch_dep(agg_prep_kernel<K, false>, dim3(nb + bb), kPrepStageThreads, 0, s, 1, a.N, a.x, n, ws, a.beta0,
+                   a.beta_br, a.beta_sh, nb, *st);
+        *brk_done = bb > 0;
     } else {
         e = cudaMemsetAsync(ws.counter, 0, 8 * sizeof(int), s);   // prep's block tickets
         if (e != cudaSuccess) return e;
         launch_dep(agg_prep_kernel<K, true>, dim3(nb), kPrepFullThreads, 0, s, 1, a.N, a.x, n, ws, a.beta0,
-                   a.beta_br, a.beta_sh);
+                   a.beta_br, a.beta_sh, nb, PrepStage{});
         if (kind == kAggTables) {
             e = cudaGetLastError();
             // this call's exact slots are no one's: the next prep starts its own list
@@ -919,15 +939,16 @@ cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_
 }
 
 template <bool SC>
-cudaError_t dispatch(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_t s, int kind)
+cudaError_t dispatch(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_t s, int kind,
+                     const PrepStage* st = nullptr, bool* brk_done = nullptr)
 {
     switch (a.kernel) {
-    case 0: return launch_k<0, SC>(a, ws, num_sms, s, kind);
-    case 1: return launch_k<1, SC>(a, ws, num_sms, s, kind);
-    case 2: return launch_k<2, SC>(a, ws, num_sms, s, kind);
-    case 3: return launch_k<3, SC>(a, ws, num_sms, s, kind);
-    case 4: return launch_k<4, SC>(a, ws, num_sms, s, kind);
-    case 5: return launch_k<5, SC>(a, ws, num_sms, s, kind);
+    case 0: return launch_k<0, SC>(a, ws, num_sms, s, kind, st, brk_done);
+    case 1: return launch_k<1, SC>(a, ws, num_sms, s, kind, st, brk_done);
+    case 2: return launch_k<2, SC>(a, ws, num_sms, s, kind, st, brk_done);
+    case 3: return launch_k<3, SC>(a, ws, num_sms, s, kind, st, brk_done);
+    case 4: return launch_k<4, SC>(a, ws, num_sms, s, kind, st, brk_done);
+    case 5: return launch_k<5, SC>(a, ws, num_sms, s, kind, st, brk_done);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -952,13 +973,19 @@ cudaError_t agg_tables_launch(const AggArgs& a, void* ws_base, int num_sms, cuda
     return dispatch<false>(a, ws, num_sms, s, kAggTables);
 }
 
-cudaError_t agg_stage_launch(const AggArgs& a, bool scatter, void* ws_base, int num_sms,
-                             cudaStream_t s)
+cudaError_t agg_stage_launch(const AggArgs& a, void* ws_base, int num_sms, cudaStream_t s,
+                             const BrkArgs* brk, void* brk_ws, bool* brk_done)
 {
     AggWs ws;
     agg_ws_layout(a.n, static_cast<char*>(ws_base), &ws);
-    return scatter ? dispatch<true>(a, ws, num_sms, s, kAggStage)
-                   : dispatch<false>(a, ws, num_sms, s, kAggStage);
+    PrepStage st{};
+    st.rhs = a.rhs;
+    if (brk) {
+        st.brk = *brk;
+        brk_ws_layout(a.n, brk->n_quad, static_cast<char*>(brk_ws), &st.bws);
+    }
+    *brk_done = false;
+    return dispatch<false>(a, ws, num_sms, s, kAggStage, &st, brk_done);
 }
 
 } // namespace pbe_gb300

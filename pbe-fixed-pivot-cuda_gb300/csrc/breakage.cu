@@ -21,31 +21,19 @@
 #include <cstdlib>
 #include <cstring>
 
-#include "pbe_internal.cuh"
+#include "tape_stage.cuh"
 
 namespace pbe_gb300 {
 namespace {
 
-// Shares of one fragment: (to lo, to lo+1). Clipped fragments put everything
-// into the first share.
-__device__ __forceinline__ void frag_shares(const double* __restrict__ x, int n, int lo, double v,
-                                            double contrib, double& clo, double& chi)
-{
-    if (lo < 0 || lo >= n - 1) { clo = contrib; chi = 0.0; return; }
-    const double xl = __ldg(x + lo), xh = __ldg(x + lo + 1);
-    const double q = contrib / (xh - xl);
-    clo = q * (xh - v);
-    chi = q * (v - xl);
-}
-
 // prep modes: kBrkFull computes everything per call; kBrkTables only the
 // grid-only tables (fragment brackets lo, run starts, S per bin) into the
 // workspace; kBrkStage the N-dependent shares from those tables, with the
-// arithmetic of kBrkFull (bitwise the same shares and sums).
+// arithmetic of kBrkFull (brk_stage_block).
 enum { kBrkFull = 0, kBrkTables = 1, kBrkStage = 2 };
 
 template <int F, int MODE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kBrkPrepBlock)
 brk_prep_kernel(const double* __restrict__ N, const double* __restrict__ x,
                 const double* __restrict__ t_q, const double* __restrict__ bw_q, int n, int nq,
                 BrkWs ws, double S0, double v_ref, double alpha, double v_min)
@@ -53,42 +41,20 @@ brk_prep_kernel(const double* __restrict__ N, const double* __restrict__ x,
     const int dep = dep_wait();
     N += dep; x += dep; t_q += dep; bw_q += dep; n += dep;
     __shared__ double sh[8];
-    const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const bool live = idx < static_cast<long long>(n) * nq;   // every lane takes part in the shuffle
-    const int lane = threadIdx.x & 31;
-    int q = 0, j = 0, lo = -2;
-    double clipped = 0.0;
-    double tq = 0.0;
-    if (live) {
-        q = static_cast<int>(idx / n);
-        j = static_cast<int>(idx - static_cast<long long>(q) * n);
-        const double xj = x[j];
-        tq = t_q[q];
-        const double v = xj * tq;
-        double S;
-        if constexpr (MODE == kBrkStage) {
-            S = ws.Ssel[j];
-            lo = ws.lo[idx];
-        } else {
-            S = selection<F>(xj, S0, v_ref, alpha, v_min);
-            lo = frag_bracket(x, n, v);
-        }
-        if constexpr (MODE == kBrkTables) {
-            ws.lo[idx] = lo;
-            if (q == 0) ws.Ssel[j] = S;
-        } else {
-            const double Nj = N[j];
-            const bool active = (S != 0.0) && (Nj > kBreakageNMin);
-            const double contrib = active ? S * Nj * bw_q[q] : 0.0;
-            double clo, chi;
-            frag_shares(x, n, lo, v, contrib, clo, chi);
-            ws.clo[idx] = clo;
-            ws.chi[idx] = chi;
-            if (lo < 0) clipped = clo;           // all of it goes to bin 0
-            if (q == 0) ws.SN[j] = active ? S * Nj : 0.0;
-        }
-    }
     if constexpr (MODE != kBrkStage) {
+        const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+        const bool live = idx < static_cast<long long>(n) * nq;   // every lane takes part in the shuffle
+        const int lane = threadIdx.x & 31;
+        int q = 0, j = 0, lo = -2;
+        double tq = 0.0;
+        if (live) {
+            q = static_cast<int>(idx / n);
+            j = static_cast<int>(idx - static_cast<long long>(q) * n);
+            tq = t_q[q];
+            lo = frag_bracket(x, n, x[j] * tq);
+            ws.lo[idx] = lo;
+            if (q == 0) ws.Ssel[j] = selection<F>(x[j], S0, v_ref, alpha, v_min);
+        }
         // bracket of the previous parent's fragment (same q): the lane below has it
         const int lo_left = __shfl_up_sync(0xffffffffu, lo, 1);
         if (live) {
@@ -101,16 +67,7 @@ brk_prep_kernel(const double* __restrict__ N, const double* __restrict__ x,
                 for (int m = max(lo + 1, -1); m <= n; ++m) fq[m + 1] = n;
         }
     }
-    if constexpr (MODE != kBrkTables) {
-        // this block's fragments clipped below x[0], summed in a fixed order (most
-        // blocks have none: one barrier tells)
-        if (__syncthreads_or(clipped != 0.0)) {
-            const double cs = block_sum(clipped, sh);
-            if (threadIdx.x == 0) ws.clipsum[blockIdx.x] = cs;
-        } else if (threadIdx.x == 0) {
-            ws.clipsum[blockIdx.x] = 0.0;
-        }
-    }
+    if constexpr (MODE == kBrkStage) brk_stage_block(N, x, t_q, bw_q, n, nq, ws, blockIdx.x, sh);
 }
 
 // Output bins in groups of 32/nqp per warp, nqp = n_quad rounded up to a power
@@ -120,7 +77,7 @@ brk_prep_kernel(const double* __restrict__ N, const double* __restrict__ x,
 // fragment clipped below x[0] (thousands on fine grids), pre-summed per prep
 // block.
 __global__ void __launch_bounds__(256)
-brk_gather_kernel(double* __restrict__ rhs, int n, int nq, BrkWs ws)
+brk_gather_kernel(double* __restrict__ rhs, int n, int nq, BrkWs ws, RkStage rk)
 {
     const int dep = dep_wait();
     rhs += dep; n += dep;
@@ -135,7 +92,7 @@ brk_gather_kernel(double* __restrict__ rhs, int n, int nq, BrkWs ws)
     // prep blocks' sums in a fixed order
     double clipped = 0.0;
     if (blockIdx.x == 0) {
-        const int nbp = static_cast<int>((static_cast<long long>(n) * nq + 255) / 256);
+        const int nbp = brk_prep_blocks(n, nq);
         double part = 0.0;
         for (int b = threadIdx.x; b < nbp; b += blockDim.x) part += ws.clipsum[b];
         clipped = block_sum(part, sh);
@@ -160,7 +117,9 @@ brk_gather_kernel(double* __restrict__ rhs, int n, int nq, BrkWs ws)
     for (int o = nqp >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (i < n && (lane % nqp) == 0) {
         if (i == 0) acc += clipped;
-        rhs[i] = (rhs[i] - ws.SN[i]) + acc;
+        const double k = (rhs[i] - ws.SN[i]) + acc;
+        rhs[i] = k;
+        if (rk.N) rk_update(rk, i, k);         // a stage's k is complete: on to the next state
     }
 }
 
@@ -609,10 +568,10 @@ brk_scatter_kernel(const double* __restrict__ N, const double* __restrict__ x,
 }
 
 template <int F>
-cudaError_t launch_f(const BrkArgs& a, bool scatter, void* ws_base, cudaStream_t s, int kind)
+cudaError_t launch_f(const BrkArgs& a, bool scatter, void* ws_base, cudaStream_t s, int kind,
+                     bool prep_done = false, const RkStage& rk = RkStage{})
 {
-    const long long m = static_cast<long long>(a.n) * a.n_quad;
-    const int grid = static_cast<int>((m + 255) / 256);
+    const int grid = brk_prep_blocks(a.n, a.n_quad);
     if (scatter) {
         launch_dep(brk_scatter_kernel<F>, dim3(grid), 256, 0, s, 1, a.N, a.x, a.t_q, a.bw_q, a.rhs, a.n,
                    a.n_quad, a.S0, a.v_ref, a.alpha, a.v_min);
@@ -633,17 +592,17 @@ cudaError_t launch_f(const BrkArgs& a, bool scatter, void* ws_base, cudaStream_t
                        a.n, a.n_quad, ws, a.S0, a.v_ref, a.alpha, a.v_min);
             return cudaGetLastError();
         }
-        if (kind == kBrkStage)
-            launch_dep(brk_prep_kernel<F, kBrkStage>, dim3(grid), 256, 0, s, 1, a.N, a.x, a.t_q, a.bw_q,
+        if (kind == kBrkFull)
+            launch_dep(brk_prep_kernel<F, kBrkTables>, dim3(grid), kBrkPrepBlock, 0, s, 1, a.N, a.x, a.t_q, a.bw_q,
                        a.n, a.n_quad, ws, a.S0, a.v_ref, a.alpha, a.v_min);
-        else
-            launch_dep(brk_prep_kernel<F, kBrkFull>, dim3(grid), 256, 0, s, 1, a.N, a.x, a.t_q, a.bw_q, a.n,
-                       a.n_quad, ws, a.S0, a.v_ref, a.alpha, a.v_min);
+        if (!prep_done)
+            launch_dep(brk_prep_kernel<F, kBrkStage>, dim3(grid), kBrkPrepBlock, 0, s, 1, a.N, a.x, a.t_q, a.bw_q,
+                       a.n, a.n_quad, ws, a.S0, a.v_ref, a.alpha, a.v_min);
         int nqp = 1;
         while (nqp < a.n_quad && nqp < 32) nqp <<= 1;
         const int per_block = 8 * (32 / nqp);               // bins per 256-thread block
         launch_dep(brk_gather_kernel, dim3((a.n + per_block - 1) / per_block), 256, 0, s, 1, a.rhs, a.n,
-                   a.n_quad, ws);
+                   a.n_quad, ws, rk);
     }
     return cudaGetLastError();
 }
@@ -651,13 +610,14 @@ cudaError_t launch_f(const BrkArgs& a, bool scatter, void* ws_base, cudaStream_t
 } // namespace
 
 namespace {
-cudaError_t brk_dispatch(const BrkArgs& a, bool scatter, void* ws_base, cudaStream_t s, int kind)
+cudaError_t brk_dispatch(const BrkArgs& a, bool scatter, void* ws_base, cudaStream_t s, int kind,
+                         bool prep_done = false, const RkStage& rk = RkStage{})
 {
     switch (a.selection) {
-    case 0: return launch_f<0>(a, scatter, ws_base, s, kind);
-    case 1: return launch_f<1>(a, scatter, ws_base, s, kind);
-    case 2: return launch_f<2>(a, scatter, ws_base, s, kind);
-    case 3: return launch_f<3>(a, scatter, ws_base, s, kind);
+    case 0: return launch_f<0>(a, scatter, ws_base, s, kind, prep_done, rk);
+    case 1: return launch_f<1>(a, scatter, ws_base, s, kind, prep_done, rk);
+    case 2: return launch_f<2>(a, scatter, ws_base, s, kind, prep_done, rk);
+    case 3: return launch_f<3>(a, scatter, ws_base, s, kind, prep_done, rk);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -678,9 +638,9 @@ cudaError_t brk_tables_launch(const BrkArgs& a, void* ws_base, cudaStream_t s)
     return brk_dispatch(a, false, ws_base, s, kBrkTables);
 }
 
-cudaError_t brk_stage_launch(const BrkArgs& a, void* ws_base, cudaStream_t s)
+cudaError_t brk_stage_launch(const BrkArgs& a, void* ws_base, cudaStream_t s, bool prep_done, const RkStage& rk)
 {
-    return brk_dispatch(a, false, ws_base, s, kBrkStage);
+    return brk_dispatch(a, false, ws_base, s, kBrkStage, prep_done, rk);
 }
 
 } // namespace pbe_gb300

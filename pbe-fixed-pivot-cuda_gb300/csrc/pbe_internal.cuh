@@ -612,7 +612,8 @@ struct VjpWs {
     double* mloc;      // [4 kMomN n]
     double* mtot;      // [4 kMomN nb_prep]
     double* moff;      // [4 kMomN nb_prep]
-    double* gpart;     // [max(ntile, n / 8) * 4] per-task / per-block parameter partials
+    double* gpart;     // [ntile * 4] per-task parameter partials of the aggregation
+    double* bpart;     // [n / 8 * 4] per-block ones of the breakage
     double* vpart;     // [ntile * kVjpMaxChunks * 2 kTileW] row sums per (tile, partner chunk)
     double* lup;       // [lane tasks * 64] lane-task sums of the rows as smaller members
     double* llo;       // [lane tasks * (C + 32)] lane-task sums of the rows as larger members
@@ -641,7 +642,8 @@ inline size_t vjp_ws_layout(int n, char* base, VjpWs* ws)
     w.mloc     = reinterpret_cast<double*>(take(4 * kMomN * dn));
     w.mtot     = reinterpret_cast<double*>(take(sizeof(double) * 4 * kMomN * nbp));
     w.moff     = reinterpret_cast<double*>(take(sizeof(double) * 4 * kMomN * nbp));
-    w.gpart    = reinterpret_cast<double*>(take(sizeof(double) * 4 * static_cast<size_t>(ntile > nbb ? ntile : nbb)));
+    w.gpart    = reinterpret_cast<double*>(take(sizeof(double) * 4 * static_cast<size_t>(ntile)));
+    w.bpart    = reinterpret_cast<double*>(take(sizeof(double) * 4 * static_cast<size_t>(nbb)));
     w.vpart    = reinterpret_cast<double*>(take(sizeof(double) * 2 * kTileW * kVjpMaxChunks *
                                                 static_cast<size_t>(ntile)));
     const int C = vjp_lane_chunk(n);
@@ -666,15 +668,18 @@ cudaError_t agg_vjp_launch(const AggVjpArgs& a, void* ws_base, int num_sms, cuda
 // For callers that keep a VJP workspace per set of pivots (the RK4 tape):
 // agg_vjp_tables_launch writes the grid-only tables (cube roots, lag tables,
 // bracket offsets, geometric flag); agg_vjp_stage_launch then runs the VJP for
-// any N and lambda on that workspace, with the result of agg_vjp_launch.
+// any N and lambda on that workspace, with the result of agg_vjp_launch; `defer` leaves
+// the parameter sums to the brk_vjp_launch that follows.
 cudaError_t agg_vjp_tables_launch(const AggVjpArgs& a, void* ws_base, int num_sms, cudaStream_t s);
-cudaError_t agg_vjp_stage_launch(const AggVjpArgs& a, void* ws_base, int num_sms, cudaStream_t s);
+cudaError_t agg_vjp_stage_launch(const AggVjpArgs& a, void* ws_base, int num_sms, cudaStream_t s, bool defer);
 // Ssel / lo_tab (nullable): the selection function per bin and the fragment
 // brackets [q n + j] of a breakage table workspace (brk_tables_launch) for the
 // same pivots, quadrature and parameters; the kernel then skips their
-// computation (same values).
+// computation (same values). after (nullable): the deferred aggregation VJP on the
+// same workspace, whose parameter sums are finished with this call's.
 cudaError_t brk_vjp_launch(const BrkVjpArgs& a, void* ws_base, cudaStream_t s,
-                           const double* Ssel = nullptr, const int* lo_tab = nullptr);
+                           const double* Ssel = nullptr, const int* lo_tab = nullptr,
+                           const AggVjpArgs* after = nullptr);
 
 // ---- profiling hook ----------------------------------------------------------
 // When both are non-null the aggregation launcher records g_prof_start right
@@ -692,6 +697,8 @@ struct BrkArgs {
     const double* N; const double* x; const double* t_q; const double* bw_q; double* rhs;
     int n; int n_quad; int selection; double S0, v_ref, alpha, v_min;
 };
+// One stage of an RK4 step (N null: none): rk_update of tape_stage.cuh.
+struct RkStage { double* N; double* acc; double* Y; int q; double c, dt6; };
 
 // true when `mode` (PBE_MODE_*) resolves to the scatter variant. Defined in api.cu.
 bool mode_is_scatter(int mode);
@@ -703,10 +710,12 @@ cudaError_t agg_launch(const AggArgs& a, bool scatter, void* ws_base, int num_sm
 // tape: agg_tables_launch writes the grid-only tables (cube roots, 1/dx, lag
 // tables, geometric flag, D0) into it; agg_stage_launch then evaluates the
 // RHS for any N on that workspace, recomputing only what depends on N, and
-// gives bitwise the result of agg_launch.
+// gives bitwise the result of agg_launch on a zeroed rhs: a stage call writes rhs,
+// whatever it held. With brk (brk_ws: a breakage workspace with its tables) it may do
+// the breakage's prep of the stage too, beside its own; *brk_done tells.
 cudaError_t agg_tables_launch(const AggArgs& a, void* ws_base, int num_sms, cudaStream_t s);
-cudaError_t agg_stage_launch(const AggArgs& a, bool scatter, void* ws_base, int num_sms,
-                             cudaStream_t s);
+cudaError_t agg_stage_launch(const AggArgs& a, void* ws_base, int num_sms, cudaStream_t s,
+                             const BrkArgs* brk, void* brk_ws, bool* brk_done);
 // Breakage: scatter needs no scratch (ws_base may be null).
 cudaError_t brk_launch(const BrkArgs& a, bool scatter, void* ws_base, cudaStream_t s);
 // Whether brk_launch uses scratch for these arguments.
@@ -714,10 +723,10 @@ bool brk_needs_scratch(const BrkArgs& a, bool scatter);
 // Gather mode on a kept workspace (the RK4 tape): brk_tables_launch writes the
 // grid-only tables (fragment brackets and run starts, the selection function
 // per bin) for the pivots, quadrature table and selection parameters;
-// brk_stage_launch then evaluates the RHS for any N on that workspace with
-// bitwise the result of brk_launch in gather mode.
+// brk_stage_launch then evaluates the RHS for any N on that workspace (its shares
+// already there if prep_done) and takes every bin's finished k into `rk`.
 cudaError_t brk_tables_launch(const BrkArgs& a, void* ws_base, cudaStream_t s);
-cudaError_t brk_stage_launch(const BrkArgs& a, void* ws_base, cudaStream_t s);
+cudaError_t brk_stage_launch(const BrkArgs& a, void* ws_base, cudaStream_t s, bool prep_done, const RkStage& rk);
 
 // Launches a kernel that begins with dep_wait: it may start before its predecessor in
 // the stream ends (its launch and its first instructions overlap the predecessor's

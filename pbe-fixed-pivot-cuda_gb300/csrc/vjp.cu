@@ -418,21 +418,22 @@ vjp_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
     }
 }
 
-// gp[0..nslots) += fixed-order sums of the per-tile partials
-// One block: parameter slot q (< nslots <= 4) summed by warp q over the
-// tasks' partials in a fixed order. nlane > 0: on a geometric grid the lane
-// rows kernel wrote nlane partials instead of ntile.
-__global__ void __launch_bounds__(128) vjp_gfin_kernel(int ntile, VjpWs ws, double* gp, int nslots,
-                                                       int nlane)
+// Parameter sums, one block: slots 0..2 of the aggregation's gp (warps 0..2; none if
+// null) from its tasks' partials -- ntile of them, or nlane > 0 on a geometric grid, where
+// the lane rows kernel wrote them -- and slots 0..3 of the breakage's bgp (warps 4..7;
+// none if null) from nb blocks', each by a warp in a fixed order.
+__global__ void __launch_bounds__(256) vjp_gfin_kernel(int ntile, int nlane, VjpWs ws, double* gp, int nb, double* bgp)
 {
     dep_wait();
-    const int q = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (q >= nslots) return;
-    if (nlane > 0 && ws.mom[10] != 0.0) ntile = nlane;
+    const int w = threadIdx.x >> 5, q = w & 3, l = threadIdx.x & 31;
+    double* out = w < 4 ? gp : bgp;
+    if (!out || w == 3) return;
+    const double* part = w < 4 ? ws.gpart : ws.bpart;
+    const int cnt = w >= 4 ? nb : (nlane > 0 && ws.mom[10] != 0.0) ? nlane : ntile;
     double s = 0.0;
-    for (int b = l; b < ntile; b += 32) s += ws.gpart[b * 4 + q];
+    for (int b = l; b < cnt; b += 32) s += part[b * 4 + q];
     s = warp_sum(s);
-    if (l == 0) gp[q] += s;
+    if (l == 0) out[q] += s;
 }
 
 // -------------------------------------------------------------------------
@@ -952,8 +953,15 @@ int vjp_lane_mode()
     return mode;
 }
 
+// Whether the lane-block kernels run (they leave grids that are not geometric to the tiles).
+bool vjp_lane_on(int n)
+{
+    const int C = vjp_lane_chunk(n);
+    return vjp_lane_mode() && vjp_lane_tasks(n, C) > 0 && vjp_lane_chunks(n, C) <= kVLaneMaxChunks;
+}
+
 template <int K>
-cudaError_t agg_vjp_k(const AggVjpArgs& a, const VjpWs& ws, int num_sms, cudaStream_t s, int kind)
+cudaError_t agg_vjp_k(const AggVjpArgs& a, const VjpWs& ws, int num_sms, cudaStream_t s, int kind, bool defer)
 {
     const int n = a.n;
     const int nb = (n + kPrepThreads - 1) / kPrepThreads;
@@ -967,7 +975,7 @@ cudaError_t agg_vjp_k(const AggVjpArgs& a, const VjpWs& ws, int num_sms, cudaStr
     if (e != cudaSuccess) return e;
     const int C = vjp_lane_chunk(n);
     const long long ltasks = vjp_lane_tasks(n, C);
-    const int lane_on = (vjp_lane_mode() && ltasks > 0 && vjp_lane_chunks(n, C) <= kVLaneMaxChunks) ? 1 : 0;
+    const int lane_on = vjp_lane_on(n) ? 1 : 0;
     if (kind == kVjpTables) {
         launch_dep(vjp_prep_kernel<kVjpTables>, dim3(nb), kPrepThreads, 0, s, 1, a.N, a.x, a.lam, n, ws);
         launch_dep(vjp_fin_kernel<kVjpTables>, dim3(1), 256, 0, s, 1, a.x, n, ws);
@@ -994,37 +1002,41 @@ cudaError_t agg_vjp_k(const AggVjpArgs& a, const VjpWs& ws, int num_sms, cudaStr
     if (lane_on)
         launch_dep(vjp_lane_rows_kernel<K>, dim3(nrb), kVRowsWarps * 32, 0, s, 1, a.N, a.x, a.lam, a.gN, ws,
                    n, C, a.beta0, a.beta_br, a.beta_sh);
-    launch_dep(vjp_gfin_kernel, dim3(1), 128, 0, s, 1, ntile, ws, a.gp, 3, lane_on ? nrb : 0);
+    if (!defer)
+        launch_dep(vjp_gfin_kernel, dim3(1), 256, 0, s, 1, ntile, lane_on ? nrb : 0, ws, a.gp, 0,
+                   static_cast<double*>(nullptr));
     return cudaGetLastError();
 }
 
 template <int F>
 cudaError_t brk_vjp_f(const BrkVjpArgs& a, const VjpWs& ws, cudaStream_t s, const double* Ssel,
-                      const int* lo_tab)
+                      const int* lo_tab, const AggVjpArgs* after)
 {
     int nqp = 1;
     while (nqp < a.n_quad && nqp < 32) nqp <<= 1;
     const int nb = static_cast<int>((static_cast<long long>(a.n) * nqp + 255) / 256);
-    launch_dep(brk_vjp_kernel<F>, dim3(nb), 256, 0, s, 1, a.N, a.x, a.t_q, a.bw_q, a.lam, a.gN, ws.gpart,
+    launch_dep(brk_vjp_kernel<F>, dim3(nb), 256, 0, s, 1, a.N, a.x, a.t_q, a.bw_q, a.lam, a.gN, ws.bpart,
                a.n, a.n_quad, nqp, a.S0, a.v_ref, a.alpha, a.v_min, Ssel, lo_tab);
-    launch_dep(vjp_gfin_kernel, dim3(1), 128, 0, s, 1, nb, ws, a.gp, 4, 0);
+    const int ntile = (a.n + VW - 1) / VW, nlane = vjp_lane_on(a.n) ? (a.n + kLaneBins - 1) / kLaneBins : 0;
+    launch_dep(vjp_gfin_kernel, dim3(1), 256, 0, s, 1, ntile, nlane, ws, after ? after->gp : nullptr, nb, a.gp);
     return cudaGetLastError();
 }
 
 } // namespace
 
 namespace {
-cudaError_t agg_vjp_dispatch(const AggVjpArgs& a, void* ws_base, int num_sms, cudaStream_t s, int kind)
+cudaError_t agg_vjp_dispatch(const AggVjpArgs& a, void* ws_base, int num_sms, cudaStream_t s, int kind,
+                             bool defer = false)
 {
     VjpWs ws;
     vjp_ws_layout(a.n, static_cast<char*>(ws_base), &ws);
     switch (a.kernel) {
-    case 0: return agg_vjp_k<0>(a, ws, num_sms, s, kind);
-    case 1: return agg_vjp_k<1>(a, ws, num_sms, s, kind);
-    case 2: return agg_vjp_k<2>(a, ws, num_sms, s, kind);
-    case 3: return agg_vjp_k<3>(a, ws, num_sms, s, kind);
-    case 4: return agg_vjp_k<4>(a, ws, num_sms, s, kind);
-    case 5: return agg_vjp_k<5>(a, ws, num_sms, s, kind);
+    case 0: return agg_vjp_k<0>(a, ws, num_sms, s, kind, defer);
+    case 1: return agg_vjp_k<1>(a, ws, num_sms, s, kind, defer);
+    case 2: return agg_vjp_k<2>(a, ws, num_sms, s, kind, defer);
+    case 3: return agg_vjp_k<3>(a, ws, num_sms, s, kind, defer);
+    case 4: return agg_vjp_k<4>(a, ws, num_sms, s, kind, defer);
+    case 5: return agg_vjp_k<5>(a, ws, num_sms, s, kind, defer);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -1038,21 +1050,21 @@ cudaError_t agg_vjp_tables_launch(const AggVjpArgs& a, void* ws_base, int num_sm
 {
     return agg_vjp_dispatch(a, ws_base, num_sms, s, kVjpTables);
 }
-cudaError_t agg_vjp_stage_launch(const AggVjpArgs& a, void* ws_base, int num_sms, cudaStream_t s)
+cudaError_t agg_vjp_stage_launch(const AggVjpArgs& a, void* ws_base, int num_sms, cudaStream_t s, bool defer)
 {
-    return agg_vjp_dispatch(a, ws_base, num_sms, s, kVjpStage);
+    return agg_vjp_dispatch(a, ws_base, num_sms, s, kVjpStage, defer);
 }
 
 cudaError_t brk_vjp_launch(const BrkVjpArgs& a, void* ws_base, cudaStream_t s, const double* Ssel,
-                           const int* lo_tab)
+                           const int* lo_tab, const AggVjpArgs* after)
 {
     VjpWs ws;
     vjp_ws_layout(a.n, static_cast<char*>(ws_base), &ws);
     switch (a.selection) {
-    case 0: return brk_vjp_f<0>(a, ws, s, Ssel, lo_tab);
-    case 1: return brk_vjp_f<1>(a, ws, s, Ssel, lo_tab);
-    case 2: return brk_vjp_f<2>(a, ws, s, Ssel, lo_tab);
-    case 3: return brk_vjp_f<3>(a, ws, s, Ssel, lo_tab);
+    case 0: return brk_vjp_f<0>(a, ws, s, Ssel, lo_tab, after);
+    case 1: return brk_vjp_f<1>(a, ws, s, Ssel, lo_tab, after);
+    case 2: return brk_vjp_f<2>(a, ws, s, Ssel, lo_tab, after);
+    case 3: return brk_vjp_f<3>(a, ws, s, Ssel, lo_tab, after);
     default: return cudaErrorInvalidValue;
     }
 }
