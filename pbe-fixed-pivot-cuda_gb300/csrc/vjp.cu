@@ -57,17 +57,24 @@ constexpr int VW = kVW;                 // rows per task
 // tables, bracket offsets, deviation) for callers that keep the workspace for
 // one set of pivots (the RK4 tape); kVjpStage the N- and lambda-dependent
 // part (x N, D, moments) on such a workspace, with kVjpFull's arithmetic.
+// Four pairs of warps share the 64 bins of a block, since the kernel is a chain of
+// dependent FP64 instructions: each pair does one of the four scans and its share of
+// the block's 25 moment sums, and before that (not kVjpStage) a part of the tables --
+// pair 0 the cube roots, pair 1 the brackets, pair 2 the bins' logarithms, pair 3 the
+// geometric fit and the cube root of x_0. (One pair for everything: n = 16384 31 us,
+// 23 with four; a stage at n = 3840 19.4 and 10.6.)
 // -------------------------------------------------------------------------
 enum { kVjpFull = 0, kVjpTables = 1, kVjpStage = 2 };
 
 // Running sums of v over the prep block's bins, from the first up (SUF = false)
 // or from the last down (true); SCALED: each bin's value is relative to 2^E
 // (prefix: the sum at bin i stands at 2^E_i, a term of a lower bin is scaled
-// down; suffix: at 2^-E_i, a term of a higher bin is scaled down).
+// down; suffix: at 2^-E_i, a term of a higher bin is scaled down). By one of the block's
+// pairs of warps, which meet at barrier 1 + pair; sv, se: the pair's.
 template <bool SUF, bool SCALED>
-__device__ __forceinline__ void block_scan(double* v, int E, double* sv, int* se)
+__device__ __forceinline__ void block_scan(double* v, int E, int pair, double* sv, int* se)
 {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & 1;
     static_assert(kPrepThreads == 64, "two warps");
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -80,13 +87,12 @@ __device__ __forceinline__ void block_scan(double* v, int E, double* sv, int* se
             if (SUF ? lane + o < 32 : lane >= o) v[q] += SCALED ? scale_down(u, sh) : u;
         }
     }
-    __syncthreads();
     if (SUF ? (w == 1 && lane == 0) : (w == 0 && lane == 31)) {
         *se = E;
 #pragma unroll
         for (int q = 0; q < kMomN; ++q) sv[q] = v[q];
     }
-    __syncthreads();
+    asm volatile("bar.sync %0, %1;" :: "r"(1 + pair), "n"(kPrepThreads) : "memory");
     if (SUF ? w == 0 : w == 1) {
         const int sh = SUF ? E - *se : *se - E;
 #pragma unroll
@@ -94,116 +100,136 @@ __device__ __forceinline__ void block_scan(double* v, int E, double* sv, int* se
     }
 }
 
+constexpr int kVPrepThreads = 4 * kPrepThreads;
+
 template <int MODE>
-__global__ void __launch_bounds__(kPrepThreads)
+__global__ void __launch_bounds__(kVPrepThreads)
 vjp_prep_kernel(const double* __restrict__ N, const double* __restrict__ x,
                 const double* __restrict__ lam, int n, VjpWs ws)
 {
     const int dep = dep_wait();
     N += dep; x += dep; lam += dep; n += dep;
     __shared__ double sh[kPrepThreads / 32][kVjpMom];
-    __shared__ double sv[kMomN];
-    __shared__ int se;
+    __shared__ double sv[4][kMomN];
+    __shared__ int se[4];
+    __shared__ double a_s[kPrepThreads], ia_s[kPrepThreads];
     __shared__ double ax0_s;
     __shared__ GeoFit fit_s;
-    const int i = blockIdx.x * kPrepThreads + threadIdx.x;
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int pair = threadIdx.x / kPrepThreads, t = threadIdx.x % kPrepThreads;
+    const int i = blockIdx.x * kPrepThreads + t;
+    const int lane = threadIdx.x & 31, wp = t >> 5;
     const int nb = gridDim.x, b = blockIdx.x;
-    if constexpr (MODE != kVjpStage) {
-        if (threadIdx.x == 0) {
-            ax0_s = cbrt(x[0]);
-            fit_s = geo_fit(x[0], x[n - 1], n);
-        }
-        __syncthreads();
-    }
-    double dev = 0.0;
-    int d0 = n;
     const double xi = x[min(i, n - 1)];          // bins beyond the last add zeros
-    double w[kMomN] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    double Ni = 0.0, li = 0.0, Di = 0.0, dl = 0.0;
-    if (i < n) {
-        double ai, iai;
-        if constexpr (MODE == kVjpStage) {
-            ai = ws.a[i];
-            iai = ws.ia[i];
-        } else {
+    int Ei = 0;
+    double fi = 0.0, ai = 0.0, iai = 0.0;
+    if constexpr (MODE != kVjpStage) {
+        if (pair == 0) {
             ai = cbrt(xi);
             iai = 1.0 / ai;
-            ws.a[i] = ai;
-            ws.ia[i] = iai;
-            const double x0 = x[0];
+            a_s[t] = ai;
+            ia_s[t] = iai;
+            if (i < n) { ws.a[i] = ai; ws.ia[i] = iai; }
+        } else if (pair == 1) {
+            int d0 = n;
+            if (i < n) {
+                const double v = x[0] + xi;
+                const int L = (dbits(v) >= dbits(x[n - 1])) ? kLagClipAll : bracket_from(x, n, v, i);
+                ws.Ld[i] = L;
+                if (L == i && i > 0) d0 = i;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) d0 = min(d0, __shfl_xor_sync(0xffffffffu, d0, o));
+            if (lane == 0) sh[wp][11] = static_cast<double>(d0);
+        } else if (pair == 2) {
+            Ei = ilogb(xi);
+            fi = log2(scalbn(xi, -Ei));
+        } else if (wp == 0) {
+            const double xe = x[lane == 1 ? n - 1 : 0];
+            const int Ee = ilogb(xe);
+            const double fe = log2(scalbn(xe, -Ee));
+            const double f1 = __shfl_sync(0xffffffffu, fe, 1);
+            const int E1 = __shfl_sync(0xffffffffu, Ee, 1);
+            if (lane == 0) fit_s = geo_fit_from(Ee, fe, E1, f1, n);
+        } else {
+            const double c0 = cbrt(x[0]);
+            if (lane == 0) ax0_s = c0;
+        }
+        __syncthreads();
+        ai = a_s[t];
+        iai = ia_s[t];
+        if (pair == 1 && i < n) {
             const double rho = ai / ax0_s;
             ws.Bf[i] = rho + 1.0 / rho + 2.0;
-            const double s = 1.0 + rho;
-            ws.Sf[i] = (s * s) * s;
-            ws.Sl[i] = (s * s) * s * (x0 / xi);
-            const double v = x0 + xi;
-            const int L = (dbits(v) >= dbits(x[n - 1])) ? kLagClipAll : bracket_from(x, n, v, i);
-            ws.Ld[i] = L;
-            if (L == i && i > 0) d0 = i;
-            if (n >= 2) {
-                dev = geo_dev(fit_s, xi, i);
-                if (!(dev == dev)) dev = 1.0;
-            }
+            const double u = 1.0 + rho;
+            ws.Sf[i] = (u * u) * u;
+            ws.Sl[i] = (u * u) * u * (x[0] / xi);
+        } else if (pair == 2) {
+            double dev = (i < n && n >= 2) ? geo_dev_from(fit_s, Ei, fi, i) : 0.0;
+            if (!(dev == dev)) dev = 1.0;        // NaN -> not geometric
+            dev = warp_max(dev);
+            if (lane == 0) sh[wp][10] = dev;
         }
-        if constexpr (MODE != kVjpTables) {
-            Ni = N[i];
-            li = lam[i];
-            if (i < n - 1) {
-                dl = lam[i + 1] - li;
-                Di = dl / (x[i + 1] - xi);
-            }
-            ws.h[i] = xi * Ni;
-            ws.D[i] = Di;
-            w[0] = iai; w[1] = 1.0; w[2] = ai; w[3] = ai * ai; w[4] = xi;
-        }
+    } else {
+        if (i < n) { ai = ws.a[i]; iai = ws.ia[i]; }
     }
     if constexpr (MODE != kVjpTables) {
-        const int E = exponent_of(xi);
-        const double xm = mantissa_of(xi);
-        // the block's share of the moments
-        const double u = (i < n - 1) ? 1.1102230246251565e-16 * (x[i + 1] / (x[i + 1] - xi)) : 0.0;
-        const double c[5] = {Ni, li * Ni, fabs(Ni), fabs(li * Ni), u * fabs(dl * Ni)};
-#pragma unroll
-        for (int g = 0; g < 5; ++g)
-#pragma unroll
-            for (int q = 0; q < kMomN; ++q) {
-                const double t = warp_sum(w[q] * c[g]);
-                if (lane == 0) sh[wp][(g < 2 ? 5 * g : 2 + 5 * g) + q] = t;
+        double w[kMomN] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        double Ni = 0.0, li = 0.0, Di = 0.0, dl = 0.0, u = 0.0;
+        if (i < n) {
+            Ni = N[i];
+            li = lam[i];
+            if (pair >= 2 && i < n - 1) {
+                const double xu = x[i + 1], dx = xu - xi;
+                dl = lam[i + 1] - li;
+                if (pair == 3) Di = dl / dx; else u = 1.1102230246251565e-16 * (xu / dx);
             }
-        // the sums over the bins
-        double v[kMomN];
-        auto store = [&](int k, int edge) {
+            if (pair == 0) ws.h[i] = xi * Ni;
+            if (pair == 3) ws.D[i] = Di;
+            w[0] = iai; w[1] = 1.0; w[2] = ai; w[3] = ai * ai; w[4] = xi;
+        }
+        // the block's share of the moments: slots 0.. (N), 5.. (lambda N), 12.. (|N|),
+        // 17.. (|lambda N|), 22.. (u |N| |lambda step|)
+        auto moments = [&](int slot, double c) {
 #pragma unroll
             for (int q = 0; q < kMomN; ++q) {
-                if (i < n) ws.mloc[static_cast<size_t>(k * kMomN + q) * n + i] = v[q];
-                if (i == edge) ws.mtot[(k * kMomN + q) * nb + b] = v[q];
+                const double m = warp_sum(w[q] * c);
+                if (lane == 0) sh[wp][slot + q] = m;
             }
         };
+        const int E = exponent_of(xi);
+        // the sums over the bins: group k = the pair
+        double v[kMomN];
+        auto fill = [&](double c) {
+#pragma unroll
+            for (int q = 0; q < kMomN; ++q) v[q] = w[q] * c;
+        };
+        if (pair == 0) {
+            moments(0, Ni);
+            fill(Ni);
+            block_scan<false, false>(v, E, pair, sv[pair], &se[pair]);
+        } else if (pair == 1) {
+            moments(5, li * Ni);
+            moments(17, fabs(li * Ni));
+            const double xm = mantissa_of(xi);
+#pragma unroll
+            for (int q = 0; q < kMomN; ++q) v[q] = (w[q] * Ni) * xm;
+            block_scan<false, true>(v, E, pair, sv[pair], &se[pair]);
+        } else if (pair == 2) {
+            moments(22, u * fabs(dl * Ni));
+            fill(li * Ni);
+            block_scan<true, false>(v, E, pair, sv[pair], &se[pair]);
+        } else {
+            moments(12, fabs(Ni));
+            fill(Ni * scalbn(Di, E));
+            block_scan<true, true>(v, E, pair, sv[pair], &se[pair]);
+        }
         const int first = b * kPrepThreads, last = min(n - 1, first + kPrepThreads - 1);
+        const int edge = pair >= 2 ? first : last;
 #pragma unroll
-        for (int q = 0; q < kMomN; ++q) v[q] = w[q] * Ni;
-        block_scan<false, false>(v, E, sv, &se);
-        store(0, last);
-#pragma unroll
-        for (int q = 0; q < kMomN; ++q) v[q] = (w[q] * Ni) * xm;
-        block_scan<false, true>(v, E, sv, &se);
-        store(1, last);
-#pragma unroll
-        for (int q = 0; q < kMomN; ++q) v[q] = w[q] * c[1];
-        block_scan<true, false>(v, E, sv, &se);
-        store(2, first);
-        const double ND = Ni * scalbn(Di, E);
-#pragma unroll
-        for (int q = 0; q < kMomN; ++q) v[q] = w[q] * ND;
-        block_scan<true, true>(v, E, sv, &se);
-        store(3, first);
-    }
-    if constexpr (MODE != kVjpStage) {
-        dev = warp_max(dev);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) d0 = min(d0, __shfl_xor_sync(0xffffffffu, d0, o));
-        if (lane == 0) { sh[wp][10] = dev; sh[wp][11] = static_cast<double>(d0); }
+        for (int q = 0; q < kMomN; ++q) {
+            if (i < n) ws.mloc[static_cast<size_t>(pair * kMomN + q) * n + i] = v[q];
+            if (i == edge) ws.mtot[(pair * kMomN + q) * nb + b] = v[q];
+        }
     }
     __syncthreads();
     if (threadIdx.x < kVjpMom) {
@@ -218,11 +244,13 @@ vjp_prep_kernel(const double* __restrict__ N, const double* __restrict__ x,
 // One block: the reductions over the prep blocks' partials, spread over the
 // warps: warps 0..3 scan the block totals of the four groups of sums into
 // offsets (each lane a run of consecutive blocks, a warp scan over the runs);
-// warps 4..7 the moments (kVjpFull, kVjpStage), the geometric flag and D0
+// warps 4..15 the moments (kVjpFull, kVjpStage), the geometric flag and D0
 // (kVjpFull, kVjpTables), lanes striding over the blocks, fixed butterflies.
 // Resets the task counters (kVjpFull, kVjpStage).
+constexpr int kVFinThreads = 512;
+
 template <int MODE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kVFinThreads)
 vjp_fin_kernel(const double* __restrict__ x, int n, VjpWs ws)
 {
     const int dep = dep_wait();
@@ -306,7 +334,7 @@ vjp_fin_kernel(const double* __restrict__ x, int n, VjpWs ws)
         }
         return;
     }
-    for (int r = wq - 4; r < 27; r += 4) {
+    for (int r = wq - 4; r < 27; r += kVFinThreads / 32 - 4) {
         double t = 0.0;
         if (r == 10 || r == 11) {
             if (MODE == kVjpStage) continue;
@@ -372,37 +400,32 @@ vjp_main_kernel(const double* __restrict__ N, const double* __restrict__ x,
     }
 }
 
-// Rows: one warp per row tile. Sums the tile's chunks in order, adds each
-// row's dL/dN_m and stores the tile's parameter partials (fixed order).
+// The rows of one row tile by a warp: sums the tile's chunks in order, adds each
+// row's dL/dN_m and stores the tile's parameter partials (fixed order). fin: kVRows
+// doubles of shared memory.
 template <int K>
-__global__ void __launch_bounds__(256)
-vjp_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
-                const double* __restrict__ lam, double* __restrict__ gN, VjpWs ws, int n,
-                int ntile, int nch, double b0, double bbr, double bsh, int lane_on)
+__device__ __forceinline__ void tile_rows(const double* __restrict__ N, const double* __restrict__ x,
+                                          const double* __restrict__ lam, double* __restrict__ gN,
+                                          const VjpWs& ws, int n, int tile, int nch, bool geo, double b0,
+                                          double bbr, double bsh, double* fin)
 {
-    const int dep = dep_wait();
-    N += dep; x += dep; lam += dep; gN += dep; n += dep;
-    __shared__ double fin[8][kVRows];
-    if (lane_on && ws.mom[10] != 0.0) return;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tile = blockIdx.x * 8 + w;
-    if (tile >= ntile) return;                    // whole warp
+    const int lane = threadIdx.x & 31;
     for (int r = lane; r < kVRows; r += 32) {
         double s = 0.0;
         for (int c = 0; c < nch; ++c) s += ws.vpart[(static_cast<size_t>(tile) * nch + c) * kVRows + r];
-        fin[w][r] = s;
+        fin[r] = s;
     }
     __syncwarp();
     VjpCellView v;
     v.x = x; v.N = N; v.h = ws.h; v.lam = lam; v.D = ws.D; v.a = ws.a; v.ia = ws.ia;
     v.Bf = ws.Bf; v.Sf = ws.Sf; v.Sl = ws.Sl; v.Ld = ws.Ld; v.lag0_scale = 1.0;
     v.n = n;
-    v.geo = ws.mom[10] != 0.0;
+    v.geo = geo;
     const int I = tile * VW;
     double gB = 0.0, gS = 0.0;
     if (lane < VW && I + lane < n) {
         double g;
-        vjp_tile_row<K>(v, I + lane, lane, fin[w], ws.mom, ws.mom + 5, b0, bbr, bsh, g, gB, gS);
+        vjp_tile_row<K>(v, I + lane, lane, fin, ws.mom, ws.mom + 5, b0, bbr, bsh, g, gB, gS);
         gN[I + lane] += g;
     }
     double s0 = 0.0, s1 = 0.0;
@@ -416,6 +439,20 @@ vjp_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
         ws.gpart[tile * 4 + 1] = (K == 3 || K == 5) ? s0 : 0.0;
         ws.gpart[tile * 4 + 2] = (K == 4 || K == 5) ? s1 : 0.0;
     }
+}
+
+template <int K>
+__global__ void __launch_bounds__(256)
+vjp_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
+                const double* __restrict__ lam, double* __restrict__ gN, VjpWs ws, int n,
+                int ntile, int nch, double b0, double bbr, double bsh)
+{
+    const int dep = dep_wait();
+    N += dep; x += dep; lam += dep; gN += dep; n += dep;
+    __shared__ double fin[8][kVRows];
+    const int w = threadIdx.x >> 5, tile = blockIdx.x * 8 + w;
+    if (tile < ntile)                             // whole warps
+        tile_rows<K>(N, x, lam, gN, ws, n, tile, nch, ws.mom[10] != 0.0, b0, bbr, bsh, fin[w]);
 }
 
 // Parameter sums, one block: slots 0..2 of the aggregation's gp (warps 0..2; none if
@@ -653,17 +690,22 @@ template <int K>
 __global__ void __launch_bounds__(kVRowsWarps * 32)
 vjp_lane_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
                      const double* __restrict__ lam, double* __restrict__ gN, VjpWs ws, int n,
-                     int C, double b0, double bbr, double bsh)
+                     int C, int ntile, int nch, double b0, double bbr, double bsh)
 {
     const int dep = dep_wait();
     N += dep; x += dep; lam += dep; gN += dep; n += dep;
+    __shared__ double fin[kVRowsWarps][kVRows];
     __shared__ double lw[kVRowsWarps][kLaneBins];
     __shared__ int base[kVLaneMaxChunks + 1];
     __shared__ double xs3[3][kLaneBins];           // exact rows: larger-member sum, smaller-member sums
     __shared__ double red[kVRowsWarps];
     __shared__ unsigned exact_s;
-    if (ws.mom[10] == 0.0) return;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (ws.mom[10] == 0.0) {                       // not geometric: the row tiles' sums
+        for (int tile = blockIdx.x * kVRowsWarps + w; tile < ntile; tile += gridDim.x * kVRowsWarps)
+            tile_rows<K>(N, x, lam, gN, ws, n, tile, nch, false, b0, bbr, bsh, fin[w]);
+        return;
+    }
     const int b = gridDim.x - 1 - blockIdx.x;      // top row blocks (the most lower blocks) first
     const int m = kLaneBins * b + lane;
     const int Dm = static_cast<int>(ws.mom[11]);   // lags below Dm were summed pair by pair
@@ -977,16 +1019,16 @@ cudaError_t agg_vjp_k(const AggVjpArgs& a, const VjpWs& ws, int num_sms, cudaStr
     const long long ltasks = vjp_lane_tasks(n, C);
     const int lane_on = vjp_lane_on(n) ? 1 : 0;
     if (kind == kVjpTables) {
-        launch_dep(vjp_prep_kernel<kVjpTables>, dim3(nb), kPrepThreads, 0, s, 1, a.N, a.x, a.lam, n, ws);
-        launch_dep(vjp_fin_kernel<kVjpTables>, dim3(1), 256, 0, s, 1, a.x, n, ws);
+        launch_dep(vjp_prep_kernel<kVjpTables>, dim3(nb), kVPrepThreads, 0, s, 1, a.N, a.x, a.lam, n, ws);
+        launch_dep(vjp_fin_kernel<kVjpTables>, dim3(1), kVFinThreads, 0, s, 1, a.x, n, ws);
         return cudaGetLastError();
     }
     if (kind == kVjpStage) {
-        launch_dep(vjp_prep_kernel<kVjpStage>, dim3(nb), kPrepThreads, 0, s, 1, a.N, a.x, a.lam, n, ws);
-        launch_dep(vjp_fin_kernel<kVjpStage>, dim3(1), 256, 0, s, 1, a.x, n, ws);
+        launch_dep(vjp_prep_kernel<kVjpStage>, dim3(nb), kVPrepThreads, 0, s, 1, a.N, a.x, a.lam, n, ws);
+        launch_dep(vjp_fin_kernel<kVjpStage>, dim3(1), kVFinThreads, 0, s, 1, a.x, n, ws);
     } else {
-        launch_dep(vjp_prep_kernel<kVjpFull>, dim3(nb), kPrepThreads, 0, s, 1, a.N, a.x, a.lam, n, ws);
-        launch_dep(vjp_fin_kernel<kVjpFull>, dim3(1), 256, 0, s, 1, a.x, n, ws);
+        launch_dep(vjp_prep_kernel<kVjpFull>, dim3(nb), kVPrepThreads, 0, s, 1, a.N, a.x, a.lam, n, ws);
+        launch_dep(vjp_fin_kernel<kVjpFull>, dim3(1), kVFinThreads, 0, s, 1, a.x, n, ws);
     }
     const int nrb = (n + kLaneBins - 1) / kLaneBins;
     if (lane_on) {
@@ -997,11 +1039,12 @@ cudaError_t agg_vjp_k(const AggVjpArgs& a, const VjpWs& ws, int num_sms, cudaStr
     }
     launch_dep(vjp_main_kernel<K>, dim3(grid), kMainThreads, smem, s, 1, a.N, a.x, a.lam, ws, n, ntile, nch,
                lane_on);
-    launch_dep(vjp_rows_kernel<K>, dim3((ntile + 7) / 8), 256, 0, s, 1, a.N, a.x, a.lam, a.gN, ws, n, ntile,
-               nch, a.beta0, a.beta_br, a.beta_sh, lane_on);
     if (lane_on)
         launch_dep(vjp_lane_rows_kernel<K>, dim3(nrb), kVRowsWarps * 32, 0, s, 1, a.N, a.x, a.lam, a.gN, ws,
-                   n, C, a.beta0, a.beta_br, a.beta_sh);
+                   n, C, ntile, nch, a.beta0, a.beta_br, a.beta_sh);
+    else
+        launch_dep(vjp_rows_kernel<K>, dim3((ntile + 7) / 8), 256, 0, s, 1, a.N, a.x, a.lam, a.gN, ws, n, ntile,
+                   nch, a.beta0, a.beta_br, a.beta_sh);
     if (!defer)
         launch_dep(vjp_gfin_kernel, dim3(1), 256, 0, s, 1, ntile, lane_on ? nrb : 0, ws, a.gp, 0,
                    static_cast<double*>(nullptr));
