@@ -255,9 +255,13 @@ __device__ __forceinline__ unsigned slot_warp(const SlotGrid& g, const SlotPass*
     } else {
         slot_pairs_any<K, NP>(g, p, s, slot, w, nw, R, TH);
     }
+    // (mom_exact_slot; not where x_{s+1} is within kMomGuard 2^53 = 2252 of x_0: bin s + 1
+    // gets at least x_0 / dx_s of every one of these pairs' rates, and u is within
+    // kMomGuard of that. 4096 cells of 48 sections: 503 us, 465 with this)
     bool ex = false;
-    if (slot && slot_cut(g, s) > 0) {
-        const double xu = __ldg(g.x + s + 1), idx = g.inv_dx[s];
+    const double xu = slot ? __ldg(g.x + s + 1) : 0.0;
+    if (slot && slot_cut(g, s) > 0 && xu > (kMomGuard * 9007199254740992.0) * __ldg(g.x)) {
+        const double idx = g.inv_dx[s];
 #pragma unroll
         for (int q = 0; q < NP; ++q) ex = ex || mom_exact_slot(p[q].Nk[s], p[q].Nk[s + 1], xu, idx);
     }
