@@ -61,6 +61,7 @@ struct pbe_batch_plan {
     int4* d_tasks = nullptr;
     std::vector<int> grid_direct;      // direct lags of a slot (D0), or n on a grid that is not geometric
     std::vector<char> grid_geo;        // grids verified geometric
+    int max_lags = 1;                  // most direct lags of a slot over the cells
     std::vector<double> t_q, bw_q;
     double* d_tq = nullptr;
     double* d_bw = nullptr;
@@ -523,11 +524,10 @@ cudaError_t create(pbe_batch_plan* p, int n_grids, const int* grid_n, const doub
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e == cudaSuccess) e = prep_shape(p, s);
     if (e != cudaSuccess) return e;
-    int max_lags = 1;
     for (int c = 0; c < n_cells; ++c)
-        max_lags = std::max(max_lags, std::min(cell_n[c], p->grid_direct[cell_grid[c]]));
+        p->max_lags = std::max(p->max_lags, std::min(cell_n[c], p->grid_direct[cell_grid[c]]));
     for (int cls = 0; cls < kClasses; ++cls)
-        p->group_size[cls] = rule_group_size(ntask, max_lags, p->num_sms);
+        p->group_size[cls] = rule_group_size(ntask, p->max_lags, p->num_sms);
     if (flags & (PBE_BATCH_TUNE | PBE_BATCH_RETUNE)) {
         e = autotune(p, (flags & PBE_BATCH_RETUNE) != 0, s);
         if (e != cudaSuccess) return e;
@@ -590,6 +590,8 @@ cudaError_t enqueue_rk4(pbe_batch_plan* p, double* N, const pbe_batch_cell_param
     cudaError_t e0 = sel_cache(p, prm, s);
     if (e0 != cudaSuccess) return e0;
     const BatchDev& d = p->d;
+    if (p->max_n <= kCellMaxN && p->max_lags <= kCellMaxLags)
+        return batch_cells_rk4(d, N, prm, dt, n_steps, p->max_n, s);
     const double h = 0.5 * dt, dt6 = dt / 6.0;
     cudaError_t e = cudaSuccess;
     for (int step = 0; step < n_steps && e == cudaSuccess; ++step) {

@@ -183,6 +183,16 @@ struct GmresDev {
 };
 
 // Launchers (batch_kernels.cu). All are asynchronous on `s`.
+// RK4 steps of small cells (every one of at most max_n <= kCellMaxN sections), a CTA
+// per cell.
+constexpr int kCellWarps = 4;
+constexpr int kCellMaxN = kCellWarps * kSlotBins;
+// (direct lags: one warp takes a block's. 64 cells of 96 sections with 28 lags 121 us a
+// step, 156 by the two kernels a stage; of 124 sections with 72 lags 215 and 162)
+constexpr int kCellMaxLags = 48;
+constexpr int kCellSteps = 64;
+cudaError_t batch_cells_rk4(const BatchDev& d, double* N, const pbe_batch_cell_params_t* params, double dt,
+                            int n_steps, int max_n, cudaStream_t s);
 cudaError_t batch_grid_tables(const BatchDev& d, const double* t_q, const double* bw_q,
                               int max_grid_n, cudaStream_t s);
 // Prep of a stage: state update per `stage`, stage arrays, moments, counter reset.

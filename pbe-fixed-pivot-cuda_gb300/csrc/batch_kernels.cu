@@ -275,8 +275,9 @@ __device__ void cell_breakage(const BatchDev& d, const BatchGridDev& gd, const d
 // The same term for the bins I .. I+SW-1 of a cell (those below n), by a
 // task's group into out[0 .. SW) (kBrkTasks): the same lanes per bin, loops and
 // butterfly, so the sums are bitwise those of cell_breakage.
+template <class Group>
 __device__ void tile_breakage(const BatchDev& d, const BatchGridDev& gd, const double* SN, int n,
-                              int I, double* out, const TileGroup& G)
+                              int I, double* out, const Group& G)
 {
     const int nqp = brk_lanes(d.nq);
     const int per_warp = 32 / nqp;
@@ -325,18 +326,15 @@ __device__ __forceinline__ void slot_passes(const BatchDev& d, const double* Y, 
 // visible) each CTA's part of the cell's clipped pairs (mom[10 + rank]) and of
 // its breakage term.
 // ---------------------------------------------------------------------------
+struct PrepShared {
+    double sh[8];
+    PrefixShared psm;
+};
+
 template <int K>
-__global__ void __launch_bounds__(256)
-batch_prep_kernel(BatchDev d, double* N, const pbe_batch_cell_params_t* __restrict__ params,
-                  int stage, double c, double dt6, StageCombine sc)
+__device__ void prep_cell(const BatchDev& d, double* N, const pbe_batch_cell_params_t* params, int cell,
+                          int stage, double c, double dt6, const StageCombine& sc, PrepShared& sm)
 {
-    const int dep = dep_wait();
-    params += dep;
-    __shared__ double sh[8];
-    __shared__ PrefixShared psm;
-    const cg::cluster_group cl = cg::this_cluster();
-    const int cell = blockIdx.x / cl.num_blocks();
-    if (d.skip && d.skip[cell]) return;             // whole cluster
     const BatchCellDev cd = d.cells[cell];
     const BatchGridDev gd = d.grids[cd.grid];
     const pbe_batch_cell_params_t P = params[cell];
@@ -381,18 +379,31 @@ batch_prep_kernel(BatchDev d, double* N, const pbe_batch_cell_params_t* __restri
     const double* Yk = (stage == kStageRhs || stage == kStageNext) ? Nc : Yc;
     double* mom = d.mom + static_cast<size_t>(cell) * kMomStride;
     if (agg) {
-        cell_prefix<K>(x, d.ga + gd.off, d.gia + gd.off, Yk, part, n, psm, d.pre + off, d.total, mom);
+        cell_prefix<K>(x, d.ga + gd.off, d.gia + gd.off, Yk, part, n, sm.psm, d.pre + off, d.total, mom);
     }
-    cl.sync();                             // the cell's stage arrays are complete; all shared reads done
+    cell_sync(part);                       // the cell's stage arrays are complete; all shared reads done
     if (agg) {
         const SlotGrid g = slot_grid(d, gd, n, P);
         SlotPass sp[1];
         slot_passes<1>(d, Yk - off, off, sp);
         const double clip = block_sum(slot_clip<K, 1>(g, sp, part.rank * blockDim.x + threadIdx.x,
-                                                      part.ranks * blockDim.x), sh);
+                                                      part.ranks * blockDim.x), sm.sh);
         if (threadIdx.x == 0) mom[10 + part.rank] = clip;
     }
     if (d.nq > 0 && !(d.brk & kBrkTasks)) cell_breakage(d, gd, d.SN + off, d.Bk + off, n, part.r0, part.r1);
+}
+
+template <int K>
+__global__ void __launch_bounds__(256)
+batch_prep_kernel(BatchDev d, double* N, const pbe_batch_cell_params_t* __restrict__ params,
+                  int stage, double c, double dt6, StageCombine sc)
+{
+    const int dep = dep_wait();
+    params += dep;
+    __shared__ PrepShared sm;
+    const int cell = blockIdx.x / cg::this_cluster().num_blocks();
+    if (d.skip && d.skip[cell]) return;             // whole cluster
+    prep_cell<K>(d, N, params, cell, stage, c, dt6, sc, sm);
 }
 
 // ---------------------------------------------------------------------------
@@ -462,6 +473,14 @@ batch_jvp_prep_kernel(BatchDev d, const double* __restrict__ v,
     if (d.nq > 0 && !(d.brk & kBrkTasks)) cell_breakage(d, gd, d.SN + off, d.Bk + off, n, part.r0, part.r1);
 }
 
+// A warp as a group of its own: no named barrier (a kernel whose barrier numbers are not
+// constants takes all 16 of a CTA, and an SM then holds four CTAs).
+struct WarpGroup {
+    int g, lane;
+    static constexpr int T = 32;
+    __device__ __forceinline__ void sync() const { __syncwarp(); }
+};
+
 // Shared memory of a CTA of the pair kernel (per group g < kMaxGroups).
 struct SlotShared {
     double red[kMaxGroups][2][32];        // per-warp R, TH of every slot
@@ -474,10 +493,11 @@ struct SlotShared {
 // slot, Brownian + shear: 4 per direct pair, 22 for the prefix part, 12 for the
 // death term and the bin.
 // ---------------------------------------------------------------------------
-template <int K, int NP>
+// Group: TileGroup, or WarpGroup for one warp.
+template <int K, int NP, class Group>
 __device__ void batch_task(const BatchDev& d, const double* __restrict__ Yg,
                            const pbe_batch_cell_params_t* __restrict__ params, double* out,
-                           bool accumulate, int4 tk, SlotShared& sm, const TileGroup& G)
+                           bool accumulate, int4 tk, SlotShared& sm, const Group& G)
 {
     const int c = tk.x, I = tk.y;
     if (d.skip && d.skip[c]) return;                // the whole group
@@ -578,6 +598,41 @@ batch_main_kernel(BatchDev d, const double* __restrict__ Y,
     batch_task<K, NP>(d, Y, params, out, accumulate != 0, tasks[bu.x + g], sm, G);
 }
 
+// ---------------------------------------------------------------------------
+// RK4 of small cells: a CTA per cell, a warp per slot block, up to kCellSteps steps
+// in one launch (cells do not see each other). With a prep and a pair kernel a stage,
+// 4096 cells of 48 sections took 462 us a step, most of it the arrays' way through
+// L2 and the latency of two short kernels at a few warps an SM; 411 us here (256 cells
+// of 48: 121 and 84).
+// ---------------------------------------------------------------------------
+template <int K>
+__global__ void __launch_bounds__(32 * kCellWarps, 7)
+batch_cells_rk4_kernel(BatchDev d, double* N, const pbe_batch_cell_params_t* __restrict__ params,
+                       double dt, int n_steps)
+{
+    const int dep = dep_wait();
+    params += dep;
+    __shared__ PrepShared psm;
+    __shared__ SlotShared sm;
+    const int cell = blockIdx.x, n = d.cells[cell].n, w = threadIdx.x >> 5;
+    const WarpGroup G{w, static_cast<int>(threadIdx.x & 31)};
+    const double h = 0.5 * dt, dt6 = dt / 6.0;
+    for (int step = 0; step < n_steps; ++step) {
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+            const int stage = q > 1 ? kStageThree : q == 1 ? kStageTwo : step == 0 ? kStageRhs : kStageNext;
+            prep_cell<K>(d, N, params, cell, stage, q == 3 ? dt : h, dt6, StageCombine{}, psm);
+            __syncthreads();
+            for (int I = SW * w; I < n; I += SW * static_cast<int>(blockDim.x >> 5)) {
+                batch_task<K, 1>(d, q == 0 ? N : d.Y, params, d.k, false, make_int4(cell, I, 0, 0), sm, G);
+                __syncwarp();
+            }
+            __syncthreads();
+        }
+    }
+    prep_cell<K>(d, N, params, cell, kStageFinish, 0.0, dt6, StageCombine{}, psm);
+}
+
 template <int K>
 cudaError_t main_k(const BatchDev& d, const double* Y, const pbe_batch_cell_params_t* params,
                    double* out, bool accumulate, const int4* bundles, const int4* tasks,
@@ -594,6 +649,31 @@ cudaError_t main_k(const BatchDev& d, const double* Y, const pbe_batch_cell_para
 }
 
 } // namespace
+
+cudaError_t batch_cells_rk4(const BatchDev& d, double* N, const pbe_batch_cell_params_t* params, double dt,
+                            int n_steps, int max_n, cudaStream_t s)
+{
+    auto run = [&](auto kern) {
+        // a warp per slot block, as far as the SMs hold all cells' CTAs at once (28 warps of
+        // 72 registers each); the prep's scan costs per warp
+        int warps = (max_n + SW - 1) / SW;
+        while (warps > 1 && static_cast<long long>(warps) * d.n_cells > 28LL * d.num_sms) --warps;
+        cudaError_t e = cudaSuccess;
+        for (int st = 0; st < n_steps && e == cudaSuccess; st += kCellSteps)   // launches of milliseconds
+            e = launch_dep(kern, dim3(d.n_cells), 32 * warps, 0, s, 1, d, N, params, dt,
+                           n_steps - st < kCellSteps ? n_steps - st : kCellSteps);
+        return e;
+    };
+    switch (d.kernel < 0 ? 0 : d.kernel) {
+    case 0: return run(batch_cells_rk4_kernel<0>);
+    case 1: return run(batch_cells_rk4_kernel<1>);
+    case 2: return run(batch_cells_rk4_kernel<2>);
+    case 3: return run(batch_cells_rk4_kernel<3>);
+    case 4: return run(batch_cells_rk4_kernel<4>);
+    case 5: return run(batch_cells_rk4_kernel<5>);
+    default: return cudaErrorInvalidValue;
+    }
+}
 
 cudaError_t batch_grid_tables(const BatchDev& d, const double* t_q, const double* bw_q,
                               int max_grid_n, cudaStream_t s)

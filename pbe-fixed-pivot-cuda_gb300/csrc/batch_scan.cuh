@@ -35,6 +35,12 @@ __device__ __forceinline__ CellPart cell_part(int n)
     return p;
 }
 
+// Barrier over the CTAs of the cell.
+__device__ __forceinline__ void cell_sync(const CellPart& part)
+{
+    if (part.ranks > 1) cg::this_cluster().sync(); else __syncthreads();
+}
+
 // Running sums over the cell's bins, from the first up (SUF = false) or from the
 // last down (true), into pre: with m_q = {1/a, 1, a, a^2, x}_q and (y, z) = val(i)
 //   pre[q stride + i]       = sum m_q y
@@ -128,7 +134,7 @@ __device__ void cell_scan(const double* __restrict__ x, const double* __restrict
         sm.ct[lane] = acc;
         if (lane == 0) sm.ce = ea;
     }
-    cl.sync();                                        // every CTA's totals are there
+    cell_sync(part);                                  // every CTA's totals are there
     if (w == 0 && lane < 2 * kMomN) {
         // the CTAs before this one, then the warps before each warp
         double base = 0.0;
