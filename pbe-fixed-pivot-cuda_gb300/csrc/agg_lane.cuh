@@ -35,7 +35,7 @@
 // Lags below D0 on fine grids (win_grid; gather mode; N without negative entries):
 // the runs from lag Dm on are long enough to separate too. In run e, lags [d1, d2),
 // slot s has k = s - e and the window j in [k - d2 + 1, k - d1], so
-//   R += sum_q c_q(x_k) N_k M_q,  TH += sum_q c_q N_k M_{q+3} + (x_k - x_s) R_run,
+//   R += N_k sum_q c_q(x_k) M_q,  TH += N_k (sum_q c_q M_{q+3} + (x_k - x_s) sum_q c_q M_q),
 // M_m = sum over the window of x_j^(m/3) N_j, from two table values (and whole
 // blocks of 64 between them): windows of any length and place without a
 // subtraction, so sums of one sign keep their relative precision. At 512 sections
@@ -192,10 +192,11 @@ __device__ __forceinline__ void lane_base(const LaneView& v, const AggWs& ws, in
         double P[kMomN], T[kMomN];
         prefix_moments<K>(ws, v.g.x, n, cut - 1, P, T);
         const double r = Ns * death_factor<K>(xv, as, ias, P, v.g.b0, v.g.bbr, v.g.bsh);
-        const double th = Ns * death_factor<K>(xv, as, ias, T, v.g.b0, v.g.bbr, v.g.bsh);
         if (s <= n - 2) {
+            // (shifted before N_s comes in: 1e-302 times a shift would leave the normal range)
+            const double f = death_factor<K>(xv, as, ias, T, v.g.b0, v.g.bbr, v.g.bsh);
             R = r;
-            TH = scale_down(th, exponent_of(__ldg(v.g.x + cut - 1)) - exponent_of(xv));
+            TH = Ns * scale_down(f, exponent_of(__ldg(v.g.x + cut - 1)) - exponent_of(xv));
         } else {
             D = -r;                                    // clipped: all of it stays in bin n - 1
         }
@@ -203,15 +204,17 @@ __device__ __forceinline__ void lane_base(const LaneView& v, const AggWs& ws, in
     D += Ns * death_factor<K>(xv, as, ias, v.M, v.g.b0, v.g.bbr, v.g.bsh);
 }
 
-// The runs eh .. el of slot s by windows: Rw += rates, Tw += rates (v - x_s), not
-// scaled. Every lane of the warp takes part.
+// The runs eh .. el of slot s by windows: Rw += rates, Tw += rates (v - x_s) 2^St_s.
+// Every lane of the warp takes part.
 template <int K>
 __device__ __forceinline__ void lane_windows(const LaneView& v, const AggWs& ws, int s, bool slot, int eh,
                                              int el, double& Rw, double& Tw)
 {
     const int n = v.g.n;
     const size_t ns = static_cast<size_t>(n);
-    const double xs = slot ? __ldg(v.g.x + s) : 0.0;
+    const double xs = slot ? __ldg(v.g.x + s) : 1.0;
+    const int E = win_exponent(v.g.x), E20 = E * (1 << 20);
+    const int dE = E - exponent_of(xs);              // from the tables' unit to the slot's, at most 0
     for (int e = eh; e >= el; --e) {
         const int d1 = __ldg(ws.rend + e + 1), d2 = __ldg(ws.rend + e);
         const int k = s - e, b = k - d1;
@@ -242,16 +245,20 @@ __device__ __forceinline__ void lane_windows(const LaneView& v, const AggWs& ws,
 #pragma unroll
             for (int m = 0; m < kWinMom; ++m)
                 if (need_window<K>(m)) M[m] += __ldg(ws.wtab + (4 * kWinMom + m) * ns + q * 64 + 63);
-        double r = 0.0;
+        double r = 0.0, t = 0.0;
 #pragma unroll
         for (int q = 0; q < kMomN; ++q) {
             if (!need_moment<K>(q)) continue;
             const double c = __ldg(ws.wc + q * ns + k);
             r = fma(c, M[q], r);
-            Tw = fma(c, M[q + 3], Tw);
+            t = fma(c, M[q + 3], t);
         }
-        Rw += r;
-        Tw = fma(__ldg(v.g.x + k) - xs, r, Tw);
+        // N_k comes last, and t is at the slot's exponent by then: with N_k = 1e-300 in c,
+        // or times x, the terms of a population's foot would underflow
+        t = fma(scale_pow2(__ldg(v.g.x + k) - xs, -E20), r, t);
+        const double Nk = __ldg(v.p.Nk + k);
+        Rw = fma(Nk, r, Rw);
+        Tw = fma(Nk, scale_down(t, dE), Tw);
     }
 }
 
@@ -296,7 +303,6 @@ __device__ void lane_finish(const LaneView& v, const AggWs& ws, const LaneArgs& 
     double sd = 0.0, own = 0.0, up = 0.0;              // the slot's own part of bin s, its w-part of bin s + 1
     if (w == 0 && finish && slot) {
         const int St = -exponent_of(__ldg(v.g.x + s));
-        u.Tw = scalbn(u.Tw, St);
         sd = scalbn(v.g.inv_dx[s], -St);
         own = fma(-(u.TH + u.Tw), sd, u.R + u.Rw);
         up = (u.TH + u.Tw) * sd;
@@ -310,7 +316,8 @@ __device__ void lane_finish(const LaneView& v, const AggWs& ws, const LaneArgs& 
             const double on = __shfl_down_sync(0xffffffffu, own, 1);
             if (finish && slot && u.Rw != 0.0) {
                 const double xu = __ldg(v.g.x + s + 1);
-                const double err = (1.1102230246251565e-16 * (xu * v.g.inv_dx[s])) * u.Rw;
+                const double err = (xu * v.g.inv_dx[s]) * u.Rw;     // 2^53 times the error
+                constexpr double kGuard = kMomGuard * 9007199254740992.0;
                 double dup = fmax(dn, 0.0);
                 if (lane == 31)
                     dup = __ldg(v.p.Nk + s + 1) * death_factor<K>(xu, v.g.a[s + 1], v.g.ia[s + 1],
@@ -318,7 +325,7 @@ __device__ void lane_finish(const LaneView& v, const AggWs& ws, const LaneArgs& 
                 const double here = fmax(own, 0.0) + (lane > 0 ? below : 0.0) + u.D;
                 const double next = up + (lane < 31 ? fmax(on, 0.0) : 0.0) + dup;
                 // (slot I - 1 matters to bin I alone here)
-                ex = !((lane == 0 || err <= kMomGuard * here) && err <= kMomGuard * next);
+                ex = !((lane == 0 || err <= kGuard * here) && err <= kGuard * next);
             }
             const unsigned m = __ballot_sync(0xffffffffu, ex);
             if (lane == 0) sm.mask = m;

@@ -34,15 +34,24 @@ __device__ __forceinline__ bool mom_exact_slot(double Ns, double Nup, double xup
 constexpr double kVjpGuard = 5e-13;
 
 // Window sums (agg_lane.cuh) pay on grids of about 64 sections an octave and more:
-// neighbour ratio at most kWinRatio = 2^(1/64). The tables hold x^2 N unscaled, so
-// the pivots stay within 2^-300 .. 2^300. Lags up to x_d = kWinStart x_0 are summed
+// neighbour ratio at most kWinRatio = 2^(1/64). Lags up to x_d = kWinStart x_0 are summed
 // pair by pair: from there on a run has at least 6 lags (1 + x_d / x_0, within
-// one), a window more than 4 bins, and costs 21 FP64 instructions against 4 a pair.
+// one), a window more than 4 bins, and costs 22 FP64 instructions against 4 a pair.
+// The tables hold moments up to x^2 N in units of 2^E of x_0, E = win_exponent (a multiple
+// of 3, so that cube roots scale exactly): N down to 1e-300 stays normal in them, where
+// x^2 N itself would underflow, and up to 1e187 finite within kWinOctaves.
 constexpr double kWinRatio = 1.0109;
 constexpr double kWinStart = 6.0;
+constexpr int kWinOctaves = 200;
 __device__ __forceinline__ bool win_grid(const double* __restrict__ x, int n)
 {
-    return n >= 2 && x[1] <= kWinRatio * x[0] && exponent_of(x[0]) > -300 && exponent_of(x[n - 1]) < 300;
+    return n >= 2 && x[1] <= kWinRatio * x[0] && exponent_of(x[n - 1]) - exponent_of(x[0]) <= kWinOctaves &&
+           exponent_of(x[0]) > -900;
+}
+__device__ __forceinline__ int win_exponent(const double* __restrict__ x)
+{
+    const int E = exponent_of(x[0]);
+    return 3 * ((E >= 0 ? E : E - 2) / 3);
 }
 // Moments m_{-1..6} (index m + 1) that kernel type K's windows need.
 template <int K>

@@ -98,19 +98,24 @@ __device__ __forceinline__ void prep_prefix(const double* m, double xm, int E, i
     }
 }
 
-// Window tables of one prep block (AggWs::wtab) and the coefficients of its bins as
-// larger members (AggWs::wc). p and s run through the prefix and suffix sums within
+// Window tables of one prep block (AggWs::wtab) and, FULL, the coefficients of its bins
+// as larger members (AggWs::wc). p and s run through the prefix and suffix sums within
 // aligned groups of 1, 2, 4 .. bins: joining two groups, the right half's prefixes
 // gain the left half's total and the left half's suffixes the right half's, one
 // add a lane, step and moment (p of the left half's last lane and s of the right
 // half's first are those totals).
-template <int K>
-__device__ __forceinline__ void prep_windows(const double* m, double xi, double Ni, double hi,
-                                             int i, int n, const AggWs& ws, double (*wtot)[kWinMom],
+template <int K, bool FULL>
+__device__ __forceinline__ void prep_windows(const double* __restrict__ x, double xi, double Ni, double ai,
+                                             double iai, int i, int n, const AggWs& ws, double (*wtot)[kWinMom],
                                              double b0, double bbr, double bsh)
 {
     const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & 1;   // two whole warps
     const size_t ns = static_cast<size_t>(n);
+    const int E = win_exponent(x), E20 = E * (1 << 20);
+    xi = scale_pow2(xi, -E20);
+    ai = scale_pow2(ai, -E20 / 3);
+    iai = scale_pow2(iai, E20 / 3);
+    const double m[kMomN] = {iai * Ni, Ni, ai * Ni, (ai * ai) * Ni, xi * Ni};
     double p[kWinMom], s[kWinMom];
 #pragma unroll
     for (int q = 0; q < kWinMom; ++q) {
@@ -139,17 +144,20 @@ __device__ __forceinline__ void prep_windows(const double* m, double xi, double 
         ws.wtab[(4 * kWinMom + q) * ns + i] = w ? p[q] + wtot[0][q] : p[q];
         ws.wtab[(5 * kWinMom + q) * ns + i] = w ? s[q] : s[q] + wtot[1][q];
     }
-    // beta(x_j, x_k) = sum_q c_q(x_k) m_q(x_j), m_q = {1/a, 1, a, a^2, x}
+    if constexpr (!FULL) return;
+    // beta(x_j, x_k) = sum_q c_q(x_k) m_q(x_j), m_q = {1/a, 1, a, a^2, x}, all in the tables'
+    // unit: Sum and Shear are of the first degree in x, Product of the second
     double c[kMomN] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    if constexpr (K == 0) c[1] = b0 * Ni;
-    if constexpr (K == 1) { c[1] = b0 * hi; c[4] = b0 * Ni; }
-    if constexpr (K == 2) c[4] = b0 * hi;
-    if constexpr (K == 3 || K == 5) { c[0] = bbr * m[2]; c[1] = 2.0 * bbr * Ni; c[2] = bbr * m[0]; }
+    if constexpr (K == 0) c[1] = b0;
+    if constexpr (K == 1) { b0 = scalbn(b0, E); c[1] = b0 * xi; c[4] = b0; }
+    if constexpr (K == 2) c[4] = scalbn(b0, 2 * E) * xi;
+    if constexpr (K == 3 || K == 5) { c[0] = bbr * ai; c[1] = 2.0 * bbr; c[2] = bbr * iai; }
     if constexpr (K == 4 || K == 5) {
-        c[1] = fma(bsh, hi, c[1]);
-        c[2] = fma(3.0 * bsh, m[3], c[2]);
-        c[3] = (3.0 * bsh) * m[2];
-        c[4] = bsh * Ni;
+        bsh = scalbn(bsh, E);
+        c[1] = fma(bsh, xi, c[1]);
+        c[2] = fma(3.0 * bsh, ai * ai, c[2]);
+        c[3] = (3.0 * bsh) * ai;
+        c[4] = bsh;
     }
 #pragma unroll
     for (int q = 0; q < kMomN; ++q)
@@ -253,7 +261,7 @@ __device__ __forceinline__ void prep_offsets(const double* __restrict__ x, int n
 // log2: some 40 clocks each): the parts of a block run theirs side by side.
 //
 // FULL = false (stage calls of a caller that keeps the workspace, e.g. the RK4
-// tape): every grid-only entry -- a, ia, inv_dx, Bd, Sd, Ld, J0, the window runs, the
+// tape): every grid-only entry -- a, ia, inv_dx, Bd, Sd, Ld, J0, wc, the window runs, the
 // geometric flag mom[5..6] and D0 in counter[1] -- is left as an earlier FULL
 // call on the same pivots and coefficients wrote it; only the N-dependent
 // values (h, moments, window tables) and the tickets are rewritten, with the
@@ -376,9 +384,7 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
                 ai = FULL ? a_s[tid & (kPrepThreads - 1)] : ws.a[i];
                 iai = FULL ? ia_s[tid & (kPrepThreads - 1)] : ws.ia[i];
             }
-            const double hi = xi * Ni;
-            const double m[5] = {iai * Ni, Ni, ai * Ni, (ai * ai) * Ni, hi};
-            prep_windows<K>(m, xi, Ni, hi, i, n, ws, wtot, b0, bbr, bsh);
+            prep_windows<K, FULL>(x, xi, Ni, ai, iai, i, n, ws, wtot, b0, bbr, bsh);
         }
     } else if constexpr (FULL) {
         // the fit's end points on lanes 0 and 1 of the third warp, the cube root of
@@ -814,7 +820,7 @@ agg_small_kernel(const double* __restrict__ N, const double* __restrict__ x, dou
             const double rr = Ns * death_factor<K>(xs, as, ias, P, b0, bbr, bsh);
             if (slot) {
                 R += rr;
-                TH += scale_down(Ns * death_factor<K>(xs, as, ias, T, b0, bbr, bsh), Ej + St);
+                TH += Ns * scale_down(death_factor<K>(xs, as, ias, T, b0, bbr, bsh), Ej + St);
             } else {
                 clip = rr;                             // bin n - 1: clipped
             }

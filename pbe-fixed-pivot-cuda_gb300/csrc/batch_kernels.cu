@@ -20,6 +20,8 @@
 //    writes its bins once: no atomics, and a fixed summation order for a fixed
 //    schedule. The slot below the first bin is summed by two tasks (1 in 32), so
 //    nothing is handed over between tasks.
+// RK4 of plans of small cells: batch_cells_rk4_kernel, a CTA per cell that runs the
+// bodies of both for all stages of its steps.
 // =============================================================================
 #include "batch_internal.cuh"
 #include "agg_slot.cuh"
@@ -546,9 +548,9 @@ __device__ void batch_task(const BatchDev& d, const double* __restrict__ Yg,
                 }
                 const double r = b * death_factor<K>(xv, as, ias, M, g.b0, g.bbr, g.bsh);
                 if (slot) {
-                    const double t = b * death_factor<K>(xv, as, ias, M1, g.b0, g.bbr, g.bsh);
+                    const double t = death_factor<K>(xv, as, ias, M1, g.b0, g.bbr, g.bsh);
                     R += r;
-                    TH += scale_down(t, exponent_of(__ldg(g.x + cut - 1)) + St);
+                    TH += b * scale_down(t, exponent_of(__ldg(g.x + cut - 1)) + St);
                 } else {
                     clip += r;                      // bin n - 1: clipped
                 }

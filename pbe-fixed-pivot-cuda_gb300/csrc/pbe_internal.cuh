@@ -313,7 +313,7 @@ struct AggWs {
     // its aligned block of 2^(v+3) bins (suffix in the left half, prefix in the
     // right half), v = 4 / 5 the prefix / suffix sum within i's block of 64 bins
     double* wtab;      // [6 * 8 n]
-    double* wc;        // [kMomN n] N_i times beta's coefficient of m_q(x_j) at x_k = x_i
+    double* wc;        // [kMomN n] beta's coefficient of m_q(x_j) at x_k = x_i (grid-only), in wtab's unit
     int*    rend;      // [n + 1] end (exclusive) of the run of lags with bracket offset e
     int*    xlist;     // [n] slots whose lags from D0 on keep the exact pair sum, counter[5] of them
     double* xsum;      // [2 n] their R, TH

@@ -106,3 +106,23 @@ def test_window_sums_match_oracle(kernel, b0, bbr, bsh, n, q):
             code, got = gpu_agg(N, x, p, mode)
             assert code == 0
             assert_close(got, ref, scale, "k=%d n=%d q=%g %s mode %d" % (kernel, n, q, what, mode))
+
+
+@pytest.mark.parametrize("kernel,b0,bbr,bsh", AGG_KERNELS, ids=[str(k[0]) for k in AGG_KERNELS])
+def test_window_sums_keep_a_populations_foot(kernel, b0, bbr, bsh):
+    """A population that falls to 1e-305 on a fine grid: bins that receive down to 1e-303
+    keep the relative bound of the others (1e-12 of their sum of |terms|, no floor): the
+    breakage guard N > 2.2e-308 and its adjoint see such values grow from nothing."""
+    n = 1500
+    x = pg.grids.geometric_pow2(n, 1e-21, 128.0)
+    p = agg_params(n, kernel, b0, bbr, bsh, x)
+    for c, width in ((300, 24.0), (500, 16.0)):
+        N = 1e12 * np.exp(-0.5 * ((np.arange(n) - c) / width) ** 2)
+        N[N < 1e-305] = 0.0
+        ref, scale, _ = oracle_agg(N, x, p)
+        code, got = gpu_agg(N, x, p, pg.MODE_GATHER)
+        assert code == 0
+        foot = (scale > 1e-303) & (scale < 1e-200)
+        assert foot.sum() > 10
+        err = np.abs(got - ref)[foot] / scale[foot]
+        assert err.max() <= 1e-12, (kernel, c, err.max())
