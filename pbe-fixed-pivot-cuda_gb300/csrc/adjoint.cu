@@ -30,6 +30,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <new>
+#include <utility>
 #include <vector>
 
 #include "tape_stage.cuh"
@@ -339,14 +340,20 @@ cudaError_t backward(pbe_rk4_tape* t, const double* lamT, double* gN0, double* g
     return e;
 }
 
-template <class T>
-cudaError_t tape_alloc(pbe_rk4_tape* t, T** out, size_t bytes)
+// Device memory of `want` (addresses to fill, sizes) as slices of one allocation.
+cudaError_t tape_alloc(pbe_rk4_tape* t, const std::vector<std::pair<void**, size_t>>& want)
 {
+    size_t total = 0;
+    for (const auto& w : want) total += w.second;
     void* q = nullptr;
-    cudaError_t e = cudaMalloc(&q, std::max<size_t>(bytes, 256));
+    cudaError_t e = cudaMalloc(&q, total);
     if (e != cudaSuccess) return e;
     t->allocs.push_back(q);
-    *out = static_cast<T*>(q);
+    char* p = static_cast<char*>(q);
+    for (const auto& w : want) {
+        *w.first = p;
+        p += w.second;
+    }
     return cudaSuccess;
 }
 
@@ -411,26 +418,23 @@ int pbe_rk4_tape_create(pbe_rk4_tape_t* tape, int n_steps, double dt, int checkp
     const size_t dn = sizeof(double) * static_cast<size_t>(n);
     const int nck = std::max(1, (n_steps + checkpoint_every - 1) / checkpoint_every);
     const int seg = std::min(checkpoint_every, std::max(n_steps, 1));
-    if (e == cudaSuccess) e = tape_alloc(t, &t->ckpt, dn * nck);
-    if (e == cudaSuccess) e = tape_alloc(t, &t->segY, dn * 4 * seg);
+    // one allocation for all (a cudaMalloc of a few MB takes about 100 us)
+    std::vector<std::pair<void**, size_t>> want;
+    auto take = [&](auto** p, size_t bytes) { want.emplace_back(reinterpret_cast<void**>(p), align256(bytes)); };
+    take(&t->ckpt, dn * nck);
+    take(&t->segY, dn * 4 * seg);
     for (double** p : {&t->k, &t->acc, &t->Y, &t->Ncur, &t->lam, &t->lsum, &t->a, &t->mu,
                        &t->Nio, &t->lam_in, &t->gN_out})
-        if (e == cudaSuccess) e = tape_alloc(t, p, dn);
-    if (e == cudaSuccess) e = tape_alloc(t, &t->g_int, sizeof(double) * 7 * n_sets);
+        take(p, dn);
+    take(&t->g_int, sizeof(double) * 7 * n_sets);
+    if (t->kernel >= 0) t->agg_ws.resize(static_cast<size_t>(n_sets));
+    if (t->selection >= 0) t->brk_ws.resize(static_cast<size_t>(n_sets));
+    for (void*& w : t->agg_ws) take(&w, agg_ws_layout(n, nullptr, nullptr));
+    for (void*& w : t->brk_ws) take(&w, brk_ws_layout(n, t->nq, nullptr, nullptr));
+    take(&t->vjp_ws, vjp_ws_layout(n, nullptr, nullptr));
+    if (e == cudaSuccess) e = tape_alloc(t, want);
     if (const char* g = std::getenv("PBE_GB300_TAPE_GRAPH")) t->use_graphs = std::strcmp(g, "0") != 0;
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&t->cap, cudaStreamNonBlocking);
-    for (int m = 0; m < n_sets && e == cudaSuccess; ++m) {
-        void* w = nullptr;
-        if (t->kernel >= 0) {
-            e = tape_alloc(t, &w, agg_ws_layout(n, nullptr, nullptr));
-            t->agg_ws.push_back(w);
-        }
-        if (e == cudaSuccess && t->selection >= 0) {
-            e = tape_alloc(t, &w, brk_ws_layout(n, t->nq, nullptr, nullptr));
-            t->brk_ws.push_back(w);
-        }
-    }
-    if (e == cudaSuccess) e = tape_alloc(t, &t->vjp_ws, vjp_ws_layout(n, nullptr, nullptr));
     if (e != cudaSuccess) { destroy(t); return e; }
     *tape = t;
     return cudaSuccess;
