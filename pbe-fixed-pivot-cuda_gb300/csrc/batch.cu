@@ -1,6 +1,6 @@
 // =============================================================================
 // batch.cu -- host side of the batched-cell path: plans, the task scheduler,
-// the tile-group autotuner, RK4 as one CUDA graph, the per-cell launch loop,
+// the group-size autotuner, RK4 as one CUDA graph, the per-cell launch loop,
 // and the pbe_batch_* C ABI (include/pbe_gb300.h).
 //
 // Schedule. Every cell is cut into pair tasks of kSlotBins bins; a task costs
@@ -18,7 +18,7 @@
 //
 // Autotuner. With PBE_BATCH_TUNE, each class present in the plan times the
 // pair kernel on its own tasks for T = 32, 64, 128, 256 (synthetic
-// state; the work of a tile does not depend on the values) and keeps the
+// state; the work of a task hardly depends on the values) and keeps the
 // fastest. Results are cached per process and device (key: SM count, kernel
 // type, breakage on/off, class) and, when PBE_GB300_TUNE_CACHE names a file,
 // in that file (one "sms kernel brk class T" line per entry).
