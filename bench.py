@@ -16,12 +16,12 @@ integrator asks for once per stage).
   e2e   : the same step through the C ABI from pinned HOST buffers: H2D copy of
           N, the RHS, D2H copy of rhs, all inside the timed events.
 
-  roofline: the pair kernel (agg_main_kernel) timed alone with CUDA events;
+  roofline: the pair kernel (agg_lane_kernel) timed alone with CUDA events;
           bound = the FP64 pipe, in FP64 instructions per second against the
           DFMA-chain probe's rate (one pipe slot per instruction). The
           reference-formula flop rate (22 flops per pair) is reported beside
-          it as reference_equivalent_*: it exceeds the peak because the
-          kernel executes about 4.5 FP64 instructions per pair.
+          it as reference_equivalent_*: it exceeds the peak because most
+          pairs are summed through prefix and window sums, not one by one.
   cpu_baseline: the oracle port on this host, all threads and one thread.
 
 --impl reference times the reference's path on the machine's host cores. The
@@ -65,105 +65,72 @@ PAIRS = N_BINS * (N_BINS + 1) // 2
 FRAGMENTS = N_BINS * N_QUAD
 FLOPS_PER_PAIR = 22      # algorithmic FP64 flops per pair interaction
 FLOPS_PER_FRAGMENT = 8   # per breakage fragment
-# FP64 instructions of the Brownian+shear pair kernel per pair evaluation:
-# lags with lo > k: rate (DMUL, DFMA, DMUL) + R += rate (DADD) + TH (DFMA) = 5;
-# lags with lo = k: q (DMUL, DFMA) + R (DADD) + TH (DFMA) = 4. The weight
-# numerator runs on the integer pipe. fp64_instr_per_launch() counts the
-# evaluations of both kinds the kernel performs on a given grid (each pair
-# once: tiles hand the w-part of their top slot to the tile above), plus 4 per
-# clipped pair (the clip tasks). On this workload the count is within 3 % of
-# ncu's FP64 instruction counters (dadd + dfma + dmul) for one launch.
-FP64_PHASE1, FP64_PHASE2 = 5, 4
+# FP64 instructions of the Brownian + shear pair kernels. A lane holds one output
+# slot, 32 lanes 31 bins (the slot below a block's first bin is summed twice). Per pair
+# evaluated 4 (q = B N_j + S x_j N_j: DMUL + DFMA; its sum: DADD; its weighted sum:
+# DFMA; the weight numerator runs on the integer pipe); per window of a run of lags 22
+# (8 table sums, 10 moment products, 4 to combine); per slot 34 (prefix part 22, death
+# term and bin 12); per clipped pair 4; per slot and run of direct lags with one bracket
+# offset 2 (its sums folded in). Lags from D0 on (pairs that land on their larger member)
+# cost nothing per pair; on fine grids the lags from Dm to D0 go by windows.
+LAG_CLIP = 0x3fffffff
+FP64_PAIR, FP64_WINDOW, FP64_SLOT, HALO = 4, 22, 34, 32.0 / 31.0
+WIN_RATIO, WIN_START = 1.0109, 6.0     # agg_moments.cuh
 
 
-def fp64_instr_per_launch(x) -> int:
-    n = len(x)
-    v = x[0] + x
-    L = np.searchsorted(x, v, side="right") - 1          # bracket of x_0 + x_d
-    L = np.where(v >= x[-1], 1 << 30, L)
-    # clipped pairs (summed by the clip tasks): rate (3) + accumulation (1)
-    d_all = np.arange(n)
-    jlo = np.where(L >= (1 << 30), 0, np.maximum(0, n - 1 - L))
-    clipped = int(np.maximum(0, (n - 1 - d_all) - jlo + 1).sum())
-    e0 = np.flatnonzero(L == np.arange(n))
-    D0 = int(e0[0]) if len(e0) else n
-    # pair (j, j + d) lands on slot j + L[d] <= n - 2
-    cnt = np.where(L <= n - 2, np.maximum(0, n - 1 - L), 0)
-    return (FP64_PHASE1 * int(cnt[d_all < D0].sum()) + FP64_PHASE2 * int(cnt[d_all >= D0].sum())
-            + 4 * clipped)
-# Lane-block pair kernel (agg_lane_kernel, geometric grids): one slot per lane,
-# blocks of 32 bins, lag chunks of max(256, n/16 rounded up to 64) lags split
-# evenly over 8 warps. Per non-clipped pair 4 FP64 instructions for
-# Brownian + shear (q = B N_j + S x_j N_j: DMUL + DFMA; its sum: DADD; its
-# weighted sum: DFMA); every run of lags with one bracket offset, in every
-# warp's share, costs 2 DFMA per lane when it is folded in; 4 per clipped pair.
-LANE_BINS, LANE_WARPS, LANE_MIN_CHUNK, LAG_CLIP = 32, 8, 256, 0x3fffffff
-
-
-def vjp_lane_fp64_instr(x) -> int:
-    """FP64 instructions of the lane-block aggregation VJP (Brownian + shear)
-    on a geometric grid: 7 per pair j < k (P, P Bf, P Sf, two sums of row j,
-    two FMAs into the sum of row k), 6 when the pair is clipped at x[n-1]
-    (P = lambda_{n-1}, no FMA)."""
+def lag_table(x):
+    """Brackets L of x_0 + x_d (LAG_CLIP at or above x[n-1]) and D0, the first lag >= 1
+    whose pairs land on their larger member."""
     n = len(x)
     v = x[0] + x
     L = np.searchsorted(x, v, side="right") - 1
-    L = np.where(v >= x[-1], LAG_CLIP, L)[1:]
-    d = np.arange(1, n)
+    L = np.where(v >= x[-1], LAG_CLIP, L)
+    e0 = np.flatnonzero((L == np.arange(n)) & (np.arange(n) > 0))
+    return L, int(e0[0]) if len(e0) else n
+
+
+def vjp_lane_fp64_instr(x, lags=None) -> int:
+    """FP64 instructions of the lane-block aggregation VJP (Brownian + shear)
+    on a geometric grid, lags 1 .. lags - 1 (all if None): 7 per pair j < k (P,
+    P Bf, P Sf, two sums of row j, two FMAs into the sum of row k), 6 when the
+    pair is clipped at x[n-1] (P = lambda_{n-1}, no FMA)."""
+    n = len(x)
+    L = lag_table(x)[0][1:lags]
+    d = np.arange(1, n)[:len(L)]
     nj = n - d                                            # rows j = 0 .. n-1-d
     jclip = np.where(L >= LAG_CLIP, 0, np.maximum(0, n - 1 - L))
     clipped = int(np.maximum(0, nj - jclip).sum())
     return 7 * int(nj.sum()) - clipped
 
 
-def lane_fp64_instr_per_launch(x) -> int:
+def slot_fp64_instr(x, windows: bool) -> int:
+    """FP64 instructions of the slot-per-lane pair kernels for one instance (model
+    above); windows: runs of lags by window sums where the grid allows them."""
     n = len(x)
-    v = x[0] + x
-    L = np.searchsorted(x, v, side="right") - 1          # bracket of x_0 + x_d
-    L = np.where(v >= x[-1], LAG_CLIP, L)
-    d_all = np.arange(n)
+    L, D0 = lag_table(x)
+    d = np.arange(n)
     jlo = np.where(L >= LAG_CLIP, 0, np.maximum(0, n - 1 - L))
-    clipped = int(np.maximum(0, (n - 1 - d_all) - jlo + 1).sum())
-    pairs = int(np.where(L <= n - 2, np.maximum(0, n - 1 - L), 0).sum())
-    e = L - d_all
-    chg = np.concatenate([[0], np.cumsum(e[1:] != e[:-1])])   # run starts at d >= 1
-    C = max(LANE_MIN_CHUNK, ((n + 15) // 16 + 63) // 64 * 64)
-    nblk = (n + LANE_BINS - 1) // LANE_BINS
-    ts, cs = [], []
-    c = 0
-    while True:
-        if c == 0:
-            cnt = nblk
-        elif c * C > n - 2:
-            cnt = 0
-        else:
-            cnt = min(nblk, (n - 1 - c * C) // LANE_BINS + 1)
-        if cnt == 0:
-            break
-        ts.append(np.arange(cnt))
-        cs.append(np.full(cnt, c))
-        c += 1
-    t = np.concatenate(ts)
-    c = np.concatenate(cs)
-    smax = np.minimum(n - LANE_BINS * t - 1, n - 2)
-    dA = c * C
-    dB = np.minimum(dA + C, smax + 1)
-    Lc = np.where(L >= LAG_CLIP, np.iinfo(np.int64).max, L)
-    dB = np.clip(np.searchsorted(Lc, smax, side="right"), dA, np.maximum(dA, dB))
-    per = (dB - dA + LANE_WARPS - 1) // LANE_WARPS
-    runs = 0
-    for w in range(LANE_WARPS):
-        d0 = dA + w * per
-        d1 = np.minimum(dB, d0 + per)
-        ok = d1 > d0
-        runs += int((1 + chg[np.maximum(d1 - 1, 0)] - chg[np.minimum(d0, n - 1)])[ok].sum())
-    return 4 * pairs + 2 * 32 * runs + 4 * clipped
+    clipped = int(np.maximum(0, (n - 1 - d) - jlo + 1)[d < D0].sum())
+    cnt = np.where(L <= n - 2, np.maximum(0, n - 1 - L), 0)     # slots of lag d, each one pair
+    Dm, win = min(D0, n), 0
+    if windows and n >= 2 and x[1] <= WIN_RATIO * x[0]:
+        e = np.where(L < LAG_CLIP, L - d, -1)
+        start = int(np.searchsorted(x, WIN_START * x[0]))
+        eh = int(e[start]) - 1 if start < n and e[start] >= 0 else 0
+        el = max(1, int(e[e >= 0].min()))
+        if eh >= el:
+            Dm = int(np.flatnonzero(e == eh)[0])
+            firsts = [int(np.flatnonzero(e == q)[0]) for q in range(el, eh + 1) if (e == q).any()]
+            win = sum(int(cnt[f]) for f in firsts)
+    ed = (L - d)[:Dm][L[:Dm] < LAG_CLIP]
+    runs = int(cnt[:len(ed)][np.concatenate([[True], ed[1:] != ed[:-1]])].sum()) if len(ed) else 0
+    return int(HALO * (2 * runs + FP64_PAIR * int(cnt[d < Dm].sum()) + FP64_WINDOW * win + FP64_SLOT * n) + 4 * clipped)
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum of one agg_main_kernel launch on
+# dram__bytes_read.sum + dram__bytes_write.sum of one pair-kernel launch on
 # this workload, read from an ncu capture of that launch (L2 flushed before it,
 # as in the timed loop); not measured by this script.
-MAIN_KERNEL_DRAM_BYTES = 1343488
+MAIN_KERNEL_DRAM_BYTES = 8250112
 # algorithmic bytes of one aggregation RHS: N and x read, rhs read and written
 ALGO_BYTES_PER_LAUNCH = 24 * N_BINS
 L2_FLUSH_BYTES = 512 << 20
@@ -322,13 +289,6 @@ def cpu_baseline(x, N, t_q, bw_q, ap, bp, seconds=3.0, serial_evals=3):
                      "semantics on x86_64 and aarch64, no -march=native)"}
 
 
-def fp64_instr_tiles(x, n_cell=None) -> int:
-    """FP64 instructions of the tile kernel for a cell with the first n_cell
-    pivots of x (same counting as fp64_instr_per_launch)."""
-    x = x[:n_cell] if n_cell else x
-    return fp64_instr_per_launch(x)
-
-
 def batched_section(dev, stream):
     """Batched cells: 4096 cells with n in {64..3840}, q in {4,8,16,32}
     (pbe_gb300.grids.config_batched_cells, seed 2026), Brownian+shear with a
@@ -395,13 +355,13 @@ def batched_section(dev, stream):
         agree = float((Y1 - Z).abs().max() / dN.abs().max())
     gs, nb = plan.schedule()
     plan.close()
-    # FP64 instructions of one batched RHS (tile evaluations, per cell)
+    # FP64 instructions of the pair kernel in one batched RHS, per cell
     instr = 0
     memo = {}
     for g, n in zip(cfg["cell_grid"], cfg["cell_n"]):
         key = (int(g), int(n))
         if key not in memo:
-            memo[key] = fp64_instr_tiles(cfg["grids"][g], int(n))
+            memo[key] = slot_fp64_instr(cfg["grids"][g][:int(n)], False)
         instr += memo[key]
     peak = fp64_peak_tflops(stream)
     cell_steps = n_cells * steps / (graph_ms / 1e3)
@@ -431,7 +391,8 @@ def batched_section(dev, stream):
                      "unit": "T FP64 instr/s",
                      "frac": round(instr / (rhs_ms / 1e3) / (peak * 1e12 / 2.0), 4) if peak else None,
                      "fp64_instr_per_rhs": instr,
-                     "fp64_instr_source": "instruction model of the tile kernel on the cells' grids",
+                     "fp64_instr_source": "instruction model of the pair kernel on the cells' grids "
+                                         "(the prep kernel's are not counted, its time is)",
                      "reference_equivalent_tflops": round(achieved, 4),
                      "reference_equivalent_unit": "22 FP64 flops per pair + 8 per fragment per s"},
         "schedule": {"group_size_by_log2n": gs, "bundles": nb, "tuned": True,
@@ -944,10 +905,10 @@ def main():
         rhs.zero_()
         pg.check(pg.aggregation_rhs(n_dev, dx, rhs, ap, stream=stream, mode=mode), "aggregation")
         pg.check(pg.breakage_rhs(n_dev, dx, dt, db, rhs, bp, stream=stream, mode=mode), "breakage")
-    # our kernels per step: aggregation prep + pair kernel; breakage prep +
-    # gather (gather mode) or one scatter kernel. (The aggregation call also
-    # enqueues one 32-byte cudaMemsetAsync of its counters, not counted.)
-    launches_per_step = 2 + (2 if mode == pg.MODE_GATHER else 1)
+    # our kernels per step: aggregation prep + pair kernel; breakage gather or scatter
+    # (threshold selection: no pre-pass). (The aggregation call also enqueues one
+    # 32-byte cudaMemsetAsync of its counters, not counted.)
+    launches_per_step = 2 + 1
 
     clocks = ClockSampler(local)
     with torch.cuda.stream(stream):
@@ -1055,7 +1016,7 @@ def main():
 
     peak = fp64_peak_tflops(stream)
     mk = statistics.mean(main_ms) * 1e-3 if main_ms else None
-    instr = lane_fp64_instr_per_launch(x)
+    instr = slot_fp64_instr(x, mode == pg.MODE_GATHER)
     # FP64 pipe: every FP64 instruction (DFMA, DMUL, DADD) takes one issue slot
     # of the pipe per thread; the DFMA-chain probe runs it at peak/2 slots per
     # second (2 flops per DFMA).
@@ -1064,7 +1025,7 @@ def main():
     ref_equiv = FLOPS_PER_PAIR * PAIRS / mk / 1e12 if mk else None
     roofline = {
         "bound": "fp64",
-        "kernel": "agg_lane_kernel<5> (+ agg_main_kernel<5>, which returns at once on this grid)",
+        "kernel": "agg_lane_kernel<5>",
         "achieved": round(achieved, 4) if achieved else None,
         "peak": round(slots_peak, 4) if slots_peak else None,
         "unit": "T FP64 instr/s",
@@ -1075,7 +1036,7 @@ def main():
         "algo_bytes": ALGO_BYTES_PER_LAUNCH,
         "kernel_ms": round(mk * 1e3, 5) if mk else None,
         "fp64_instr_per_launch": instr,
-        "fp64_instr_source": "instruction model of the lane-block kernel on this grid",
+        "fp64_instr_source": "instruction model of the pair kernel on this grid",
         "peak_source": "DFMA-chain probe timed in this run (libpbe_probe.so), of measured; "
                        "MEASURED_PEAKS.json has no FP64 entry",
         "reference_equivalent_tflops": round(ref_equiv, 4) if ref_equiv else None,
@@ -1115,7 +1076,7 @@ def main():
                                   "ms_per_step": round(other_ms, 5),
                                   "what": "the same step in the other accumulation mode, "
                                           "device-resident, L2 flushed"}
-        vjp_instr = vjp_lane_fp64_instr(x)
+        vjp_instr = vjp_lane_fp64_instr(x, lag_table(x)[1])
         vjp_ach = vjp_instr / (vjp_ms * 1e-3) / 1e12
         vjp_frac = round(vjp_ach / slots_peak, 4) if slots_peak else None
         sections["vjp"] = {"ms_per_eval": round(vjp_ms, 5),
@@ -1127,7 +1088,7 @@ def main():
                                         "frac": vjp_frac,
                                         "fp64_instr_per_eval": vjp_instr,
                                         "time": "the whole aggregation + breakage VJP step "
-                                                "(the pair kernel is ~93 % of it)"},
+                                                "(the pair kernel is ~87 % of it)"},
                            "what": "aggregation + breakage VJP (dL/dN and parameter gradients) "
                                    "of the same n=16384 step, device-resident, L2 flushed"}
     if n_gpus == 1 and not args.no_extras:

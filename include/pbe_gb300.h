@@ -55,7 +55,7 @@ enum {
 /* Birth accumulation mode.
  *   GATHER  : every output bin is reduced by one owner in a fixed order, no
  *             atomics; results are bitwise identical run to run.
- *   SCATTER : work tiles flush partial sums with FP64 atomicAdd; the order of
+ *   SCATTER : work tasks flush partial sums with FP64 atomicAdd; the order of
  *             the flushes (and hence the last bits) can vary run to run.
  *   DEFAULT : GATHER unless the environment variable PBE_GB300_MODE is
  *             "scatter" (read once per process). */
@@ -128,7 +128,7 @@ int pbe_breakage_rhs_ex(const double* N, const double* x, const double* t_q,
  * codes that forbid allocation once time stepping starts, plug-in interfaces
  * with no way to pass a workspace -- this runs the same kernels as
  * pbe_aggregation_rhs_ex with its scratch in a fixed device array compiled
- * into the library (about 8.5 MiB, held by every GPU that loads the library).
+ * into the library (about 28.7 MiB, held by every GPU that loads the library).
  *   Limit: params->n <= 32768; larger n returns cudaErrorInvalidValue.
  *   The first call on a device looks up that array's address; make it before
  *   any stream capture starts.
@@ -198,7 +198,7 @@ typedef struct pbe_batch_cell_params {
 
 /* flags of pbe_batch_create */
 enum {
-    PBE_BATCH_TUNE   = 1,  /* pick the tile group size per section-count class by timing
+    PBE_BATCH_TUNE   = 1,  /* pick the task group size per section-count class by timing
                               candidates on the device (results cached per process, and
                               in the file named by PBE_GB300_TUNE_CACHE when set)        */
     PBE_BATCH_RETUNE = 2,  /* like TUNE, ignoring cached results                          */
@@ -362,7 +362,7 @@ int pbe_batch_set_krylov_restarts(pbe_batch_t plan, int restarts);
 int pbe_batch_from_soa(pbe_batch_t plan, const double* soa, long long ld, double* N, void* stream);
 int pbe_batch_to_soa(pbe_batch_t plan, const double* N, double* soa, long long ld, void* stream);
 
-/* Schedule in use: group_size[c] (16 entries) = threads per tile task for
+/* Schedule in use: group_size[c] (16 entries) = threads per pair task for
  * cells with floor(log2(n)) == c (0 where no cell falls), *n_bundles = the
  * number of bundles in the persistent launch. Either pointer may be NULL. */
 int pbe_batch_schedule(pbe_batch_t plan, int* group_size, int* n_bundles);

@@ -1,5 +1,5 @@
 """Batched cells: many independent PBE instances with uneven section counts,
-evaluated by one persistent launch per RHS and integrated with RK4 steps
+evaluated by two launches per RHS and integrated with RK4 steps
 captured in one CUDA graph (C ABI pbe_batch_*, include/pbe_gb300.h).
 
 The reference has no batched interface: its callers loop over cells and call
@@ -59,7 +59,7 @@ class BatchPlan:
     """A plan over `cell_n` cells; cell c uses the first cell_n[c] pivots of
     grids[cell_grid[c]]. kernel: AGG_* or -1 (no aggregation); selection:
     SEL_* or -1 (no breakage) with the daughter table (t_q, bw_q).
-    tune / retune: time the tile group sizes per size class (cached);
+    tune / retune: time the task group sizes per size class (cached);
     breakage_gather: "prep" or "tasks" forces where the breakage term is
     gathered (bitwise the same result; by default the plan picks by its
     cell count)."""
