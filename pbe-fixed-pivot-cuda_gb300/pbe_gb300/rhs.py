@@ -20,19 +20,29 @@ Array = Union["torch.Tensor", int, None]  # noqa: F821
 
 
 _torch = None          # the module, once a call has needed it (an import statement a call costs 0.3 us)
+_raw_stream = None     # handle of a device's current stream
 
 
 def _load_torch():
-    global _torch
+    global _torch, _raw_stream
     import torch
 
+    # the handle without a Stream object (2.9 us a call on the host), where this torch has it
+    _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if _raw_stream is None:
+        def _raw_stream(device):
+            return torch.cuda.current_stream(device).cuda_stream
     _torch = torch
     return torch
 
 
 def _ptr(a: Array, name: str) -> Optional[int]:
     # a call has up to seven of these and a small one is bound by the host (64 sections,
-    # aggregation + breakage: 32 us of host time a pass): the common case first
+    # aggregation + breakage: 32 us of host time a pass). Addresses need no torch.
+    if a is None:
+        return None
+    if isinstance(a, int):
+        return a or None
     torch = _torch or _load_torch()
     if isinstance(a, torch.Tensor):
         if a.dtype is not torch.float64:
@@ -42,18 +52,13 @@ def _ptr(a: Array, name: str) -> Optional[int]:
         if not a.is_contiguous():
             raise TypeError("%s must be contiguous" % name)
         return a.data_ptr()
-    if a is None:
-        return None
-    if isinstance(a, int):
-        return a or None
     raise TypeError("%s must be a torch tensor or a device address" % name)
 
 
 def _stream(stream) -> Optional[int]:
     if stream is None:
-        # the current stream's handle without a Stream object (2.9 us a call on the host)
         torch = _torch or _load_torch()
-        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()) or None
+        return _raw_stream(torch.cuda.current_device()) or None
     if isinstance(stream, int):
         return stream or None
     return stream.cuda_stream or None
