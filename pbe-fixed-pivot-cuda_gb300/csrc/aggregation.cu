@@ -41,6 +41,7 @@
 #include <cooperative_groups.h>
 
 #include "agg_lane.cuh"
+#include "device_answer.h"
 #include "tape_stage.cuh"
 
 namespace pbe_gb300 {
@@ -839,17 +840,20 @@ agg_small_kernel(const double* __restrict__ N, const double* __restrict__ x, dou
         rhs[s] = (KIND == kAggStage ? 0.0 : rhs[s]) + (((own + in) + clip) - death);   // a stage call writes rhs
 }
 
-// One cluster of the device can hold 16 CTAs of this kernel (a size beyond the
-// portable 8, asked for once per kernel).
+// One cluster of the current device can hold 16 CTAs of this kernel (a size beyond the
+// portable 8, asked for once per kernel and device).
 template <int K, int KIND>
 bool small_cluster_ok(int ranks)
 {
     if (ranks <= 8) return true;
-    static const bool ok = []() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    static DeviceAnswer answer;
+    return answer.get(dev, []() {
         auto kern = agg_small_kernel<K, KIND>;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
             cudaGetLastError();
-            return false;
+            return 0;
         }
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(kSmallMaxCtas);
@@ -864,11 +868,10 @@ bool small_cluster_ok(int ranks)
         int num = 0;
         if (cudaOccupancyMaxActiveClusters(&num, kern, &cfg) != cudaSuccess) {
             cudaGetLastError();
-            return false;
+            return 0;
         }
-        return num > 0;
-    }();
-    return ok;
+        return num > 0 ? 1 : -1;
+    });
 }
 
 template <int K, int KIND>
