@@ -485,8 +485,8 @@ agg_prep_kernel(const double* __restrict__ N, const double* __restrict__ x, int 
             const bool geo = n >= 2 && m5 <= kGeoTol && x[1] <= 64.0 * x[0];
             ws.mom[5] = geo ? 1.0 : 0.0;
             ws.mom[6] = m5;
-            const int eh = __ldcg(ws.counter + 8);
-            ws.counter[10] = eh >= max(1, __ldcg(ws.counter + 9)) ? __ldcg(ws.rend + eh + 1) : 0;
+            const int entry = window_first_entry(__ldcg(ws.counter + 8), __ldcg(ws.counter + 9), n);
+            ws.counter[10] = entry >= 0 ? __ldcg(ws.rend + entry) : 0;
         }
     } else if (FULL && wp == 3) {
         int dmin = n;
@@ -929,7 +929,8 @@ cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_
                    a.beta_br, a.beta_sh, nb, *st);
         *brk_done = bb > 0;
     } else {
-        e = cudaMemsetAsync(ws.counter, 0, 8 * sizeof(int), s);   // prep's block tickets
+        // the prep's block tickets; and what pivots that are no numbers leave unwritten
+        e = cudaMemsetAsync(ws.counter, 0, kAggCounters * sizeof(int), s);
         if (e != cudaSuccess) return e;
         launch_dep(agg_prep_kernel<K, true>, dim3(nb), kPrepFullThreads, 0, s, 1, a.N, a.x, n, ws, a.beta0,
                    a.beta_br, a.beta_sh, nb, PrepStage{});

@@ -293,7 +293,7 @@ struct AggWs {
     double* clip_part; // [kMaxClipTasks] sums of clipped pair rates, one per clip task
     int*    J0;        // [n]  first j with fl(x_j + x_i) >= x_{i+1} (at most i)
     int*    cticket;   // [nblk] tasks of the block done
-    int*    counter;   // [16] [0] task counter, [1] first lag with Ld[d] == d,
+    int*    counter;   // [kAggCounters] [0] task counter, [1] first lag with Ld[d] == d,
                        //      [2] prep blocks done, [3] bin n-1 contributors done,
                        //      [5] entries of xlist,
                        //      [6] CTAs of the pair kernel done, [8] the first (largest)
@@ -319,8 +319,18 @@ struct AggWs {
     double* xsum;      // [2 n] their R, TH
 };
 constexpr int kMomN = 5;               // moments per prefix (the death term's)
+constexpr int kAggCounters = 16;       // entries of AggWs::counter, all cleared before a FULL prep
 constexpr int kWinMom = 8;             // moments of a window: kMomN of N and, x_j / x_j^(-1/3) on, of x N
 constexpr int kWinTabs = 6 * kWinMom;  // window table values per bin
+
+// Entry of AggWs::rend that holds the first lag of the runs summed by windows, given the
+// largest offset eh of those runs and the last run's el (counter[8], counter[9]); -1 when
+// there are none. Pivots that are not increasing numbers (a NaN) leave the two without
+// a meaning, so they are checked against the table.
+__host__ __device__ constexpr int window_first_entry(int eh, int el, int n)
+{
+    return eh >= (el > 1 ? el : 1) && eh < n ? eh + 1 : -1;
+}
 
 __host__ __device__ constexpr int agg_prep_blocks(int n) { return (n + kPrepThreads - 1) / kPrepThreads; }
 
@@ -441,7 +451,7 @@ constexpr size_t agg_ws_bytes(int n)
          + align256(sizeof(double) * 8)
          + align256(sizeof(double) * kMaxClipTasks)
          + align256(sizeof(int) * static_cast<size_t>(slot_blocks(n)))
-         + align256(sizeof(int) * 16)
+         + align256(sizeof(int) * kAggCounters)
          + align256(sizeof(double) * lane_partial_doubles(n))
          + align256(sizeof(double) * 2 * kMomN * static_cast<size_t>(n))
          + 2 * align256(sizeof(double) * 2 * kMomN * static_cast<size_t>(agg_prep_blocks(n)))
@@ -471,7 +481,7 @@ inline size_t agg_ws_layout(int n, char* base, AggWs* ws)
     w.clip_part = reinterpret_cast<double*>(take(sizeof(double) * kMaxClipTasks));
     w.J0        = reinterpret_cast<int*>(take(sizeof(int) * static_cast<size_t>(n)));
     w.cticket   = reinterpret_cast<int*>(take(sizeof(int) * static_cast<size_t>(slot_blocks(n))));
-    w.counter   = reinterpret_cast<int*>(take(sizeof(int) * 16));
+    w.counter   = reinterpret_cast<int*>(take(sizeof(int) * kAggCounters));
     w.lpart     = reinterpret_cast<double*>(take(sizeof(double) * lane_partial_doubles(n)));
     w.mloc      = reinterpret_cast<double*>(take(sizeof(double) * 2 * kMomN * static_cast<size_t>(n)));
     const size_t nbm = sizeof(double) * 2 * kMomN * static_cast<size_t>(agg_prep_blocks(n));
