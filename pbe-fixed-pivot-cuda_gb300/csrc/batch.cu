@@ -19,9 +19,11 @@
 // Autotuner. With PBE_BATCH_TUNE, each class present in the plan times the
 // pair kernel on its own tasks for T = 32, 64, 128, 256 (synthetic
 // state; the work of a task hardly depends on the values) and keeps the
-// fastest. Results are cached per process and device (key: SM count, kernel
-// type, breakage on/off, class) and, when PBE_GB300_TUNE_CACHE names a file,
-// in that file (one "sms kernel brk class T" line per entry).
+// fastest. What is fastest depends on what the rule for the default looks at, so the
+// results are cached per process by SM count, kernel type, breakage on/off, class, and
+// the class's tasks, direct lags (both in powers of two) and kinds of grids; when
+// PBE_GB300_TUNE_CACHE names a file, in that file too (a "slot" line per entry: lines
+// of any other form, as earlier schedulers wrote them, are passed over).
 //
 // RK4. A step is four (prep, main) launch pairs; the prep of a stage applies
 // the previous stage's update in place (batch_internal.cuh, BatchStage).
@@ -35,13 +37,13 @@
 // with an optional tolerance and restarts (batch_implicit.cu).
 // =============================================================================
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
-#include <tuple>
 #include <vector>
 
 #include "batch_internal.cuh"
@@ -139,12 +141,28 @@ int rule_group_size(long long tasks, int max_lags, int num_sms)
 }
 
 // ---- tune cache ----------------------------------------------------------------
-using TuneKey = std::tuple<int, int, int, int>;   // sms, kernel, brk, class
+// sms, kernel, brk, class, log2 tasks, log2 direct lags, kinds of grids (1 geometric, 2 other)
+using TuneKey = std::array<int, 7>;
 std::mutex g_tune_mu;
 std::map<TuneKey, int> g_tune;
 bool g_tune_file_read = false;
 
 const char* tune_file() { return std::getenv("PBE_GB300_TUNE_CACHE"); }
+
+TuneKey tune_key(const pbe_batch_plan& p, int cls)
+{
+    long long tasks = 0;
+    int lags = 1, grids = 0;
+    for (int c = 0; c < p.n_cells; ++c) {
+        if (n_class(p.cell_n[c]) != cls) continue;
+        const int g = p.cell_grid[c];
+        tasks += (p.cell_n[c] + SW - 1) / SW;
+        lags = std::max(lags, std::min(p.cell_n[c], p.grid_direct[g]));
+        grids |= p.grid_geo[g] ? 1 : 2;
+    }
+    auto log2i = [](long long v) { int e = 0; while (v >>= 1) ++e; return e; };
+    return TuneKey{p.num_sms, p.kernel, p.nq > 0 ? 1 : 0, cls, log2i(tasks), log2i(lags), grids};
+}
 
 void tune_cache_load_locked()
 {
@@ -154,9 +172,14 @@ void tune_cache_load_locked()
     if (!path || !*path) return;
     FILE* f = std::fopen(path, "r");
     if (!f) return;
-    int a, b, c, e, t;
-    while (std::fscanf(f, "%d %d %d %d %d", &a, &b, &c, &e, &t) == 5)
-        if (t == 32 || t == 64 || t == 128 || t == 256) g_tune[TuneKey(a, b, c, e)] = t;
+    char line[160];
+    while (std::fgets(line, sizeof line, f)) {
+        TuneKey k;
+        int t = 0;
+        if (std::sscanf(line, "slot %d %d %d %d %d %d %d %d", &k[0], &k[1], &k[2], &k[3], &k[4], &k[5], &k[6],
+                        &t) == 8 && (t == 32 || t == 64 || t == 128 || t == 256))
+            g_tune[k] = t;
+    }
     std::fclose(f);
 }
 
@@ -167,8 +190,7 @@ void tune_cache_store_locked(const TuneKey& k, int t)
     if (!path || !*path) return;
     FILE* f = std::fopen(path, "a");
     if (!f) return;
-    std::fprintf(f, "%d %d %d %d %d\n", std::get<0>(k), std::get<1>(k), std::get<2>(k),
-                 std::get<3>(k), t);
+    std::fprintf(f, "slot %d %d %d %d %d %d %d %d\n", k[0], k[1], k[2], k[3], k[4], k[5], k[6], t);
     std::fclose(f);
 }
 
@@ -344,7 +366,7 @@ cudaError_t autotune(pbe_batch_plan* p, bool retune, cudaStream_t s)
     }
     for (int cls = 0; cls < kClasses && e == cudaSuccess; ++cls) {
         if (!present[cls]) continue;
-        const TuneKey key(p->num_sms, p->kernel, p->nq > 0 ? 1 : 0, cls);
+        const TuneKey key = tune_key(*p, cls);
         auto it = g_tune.find(key);
         if (!retune && it != g_tune.end()) { p->group_size[cls] = it->second; continue; }
         int T = p->group_size[cls];
