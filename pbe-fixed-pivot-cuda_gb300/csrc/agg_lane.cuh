@@ -32,7 +32,8 @@
 // bin, where a tiny w's rounding would show) the slot keeps its exact pair sum,
 // a task of its own (exact_slot_task).
 //
-// Lags below D0 on fine grids (win_grid; gather mode; N without negative entries):
+// Lags below D0 on fine grids (win_grid; gather mode; N without negative entries, and
+// coefficients of one sign):
 // the runs from lag Dm on are long enough to separate too. In run e, lags [d1, d2),
 // slot s has k = s - e and the window j in [k - d2 + 1, k - d1], so
 //   R += N_k sum_q c_q(x_k) M_q,  TH += N_k (sum_q c_q M_{q+3} + (x_k - x_s) sum_q c_q M_q),
@@ -316,14 +317,15 @@ __device__ void lane_finish(const LaneView& v, const AggWs& ws, const LaneArgs& 
             const double on = __shfl_down_sync(0xffffffffu, own, 1);
             if (finish && slot && u.Rw != 0.0) {
                 const double xu = __ldg(v.g.x + s + 1);
-                const double err = (xu * v.g.inv_dx[s]) * u.Rw;     // 2^53 times the error
+                const double sg = rate_sign<K>(v.g.b0, v.g.bbr, v.g.bsh);
+                const double err = (xu * v.g.inv_dx[s]) * (sg * u.Rw);   // 2^53 times the error
                 constexpr double kGuard = kMomGuard * 9007199254740992.0;
-                double dup = fmax(dn, 0.0);
+                double dup = fmax(sg * dn, 0.0);
                 if (lane == 31)
-                    dup = __ldg(v.p.Nk + s + 1) * death_factor<K>(xu, v.g.a[s + 1], v.g.ia[s + 1],
-                                                                  v.M, v.g.b0, v.g.bbr, v.g.bsh);
-                const double here = fmax(own, 0.0) + (lane > 0 ? below : 0.0) + u.D;
-                const double next = up + (lane < 31 ? fmax(on, 0.0) : 0.0) + dup;
+                    dup = sg * (__ldg(v.p.Nk + s + 1) * death_factor<K>(xu, v.g.a[s + 1], v.g.ia[s + 1],
+                                                                        v.M, v.g.b0, v.g.bbr, v.g.bsh));
+                const double here = fmax(sg * own, 0.0) + sg * ((lane > 0 ? below : 0.0) + u.D);
+                const double next = sg * up + (lane < 31 ? fmax(sg * on, 0.0) : 0.0) + dup;
                 // (slot I - 1 matters to bin I alone here)
                 ex = !((lane == 0 || err <= kGuard * here) && err <= kGuard * next);
             }

@@ -53,6 +53,18 @@ __device__ __forceinline__ int win_exponent(const double* __restrict__ x)
     const int E = exponent_of(x[0]);
     return 3 * ((E >= 0 ? E : E - 2) / 3);
 }
+// Sign that all pair rates of a population without negative entries share: the windows'
+// rule compares sums of such rates, so it takes them times this. 0: none (Brownian and
+// shear coefficients of opposite signs), no windows.
+template <int K>
+__device__ __forceinline__ double rate_sign(double b0, double bbr, double bsh)
+{
+    if constexpr (K <= 2) return b0 < 0.0 ? -1.0 : 1.0;
+    else if constexpr (K == 3) return bbr < 0.0 ? -1.0 : 1.0;
+    else if constexpr (K == 4) return bsh < 0.0 ? -1.0 : 1.0;
+    else if ((bbr < 0.0 && bsh > 0.0) || (bbr > 0.0 && bsh < 0.0)) return 0.0;
+    else return bbr < 0.0 || bsh < 0.0 ? -1.0 : 1.0;
+}
 // Moments m_{-1..6} (index m + 1) that kernel type K's windows need.
 template <int K>
 __device__ __forceinline__ constexpr bool need_window(int m)
