@@ -317,15 +317,15 @@ __device__ void lane_finish(const LaneView& v, const AggWs& ws, const LaneArgs& 
             const double on = __shfl_down_sync(0xffffffffu, own, 1);
             if (finish && slot && u.Rw != 0.0) {
                 const double xu = __ldg(v.g.x + s + 1);
-                const double sg = rate_sign<K>(v.g.b0, v.g.bbr, v.g.bsh);
-                const double err = (xu * v.g.inv_dx[s]) * (sg * u.Rw);   // 2^53 times the error
+                const int fl = rates_flip<K>(v.g.b0, v.g.bbr, v.g.bsh);
+                const double err = (xu * v.g.inv_dx[s]) * flip_sign(u.Rw, fl);   // 2^53 times the error
                 constexpr double kGuard = kMomGuard * 9007199254740992.0;
-                double dup = fmax(sg * dn, 0.0);
+                double dup = fmax(flip_sign(dn, fl), 0.0);
                 if (lane == 31)
-                    dup = sg * (__ldg(v.p.Nk + s + 1) * death_factor<K>(xu, v.g.a[s + 1], v.g.ia[s + 1],
-                                                                        v.M, v.g.b0, v.g.bbr, v.g.bsh));
-                const double here = fmax(sg * own, 0.0) + sg * ((lane > 0 ? below : 0.0) + u.D);
-                const double next = sg * up + (lane < 31 ? fmax(sg * on, 0.0) : 0.0) + dup;
+                    dup = flip_sign(__ldg(v.p.Nk + s + 1) * death_factor<K>(xu, v.g.a[s + 1], v.g.ia[s + 1],
+                                                                            v.M, v.g.b0, v.g.bbr, v.g.bsh), fl);
+                const double here = fmax(flip_sign(own, fl), 0.0) + flip_sign((lane > 0 ? below : 0.0) + u.D, fl);
+                const double next = flip_sign(up, fl) + (lane < 31 ? fmax(flip_sign(on, fl), 0.0) : 0.0) + dup;
                 // (slot I - 1 matters to bin I alone here)
                 ex = !((lane == 0 || err <= kGuard * here) && err <= kGuard * next);
             }

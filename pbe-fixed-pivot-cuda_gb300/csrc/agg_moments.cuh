@@ -53,17 +53,23 @@ __device__ __forceinline__ int win_exponent(const double* __restrict__ x)
     const int E = exponent_of(x[0]);
     return 3 * ((E >= 0 ? E : E - 2) / 3);
 }
-// Sign that all pair rates of a population without negative entries share: the windows'
-// rule compares sums of such rates, so it takes them times this. 0: none (Brownian and
-// shear coefficients of opposite signs), no windows.
+// All pair rates of a population without negative entries have one sign (Brownian and
+// shear coefficients of opposite signs: not so, no windows). The windows' rule compares
+// sums of such rates, taken positive: the sign bit to flip.
 template <int K>
-__device__ __forceinline__ double rate_sign(double b0, double bbr, double bsh)
+__device__ __forceinline__ bool rates_one_sign(double bbr, double bsh)
 {
-    if constexpr (K <= 2) return b0 < 0.0 ? -1.0 : 1.0;
-    else if constexpr (K == 3) return bbr < 0.0 ? -1.0 : 1.0;
-    else if constexpr (K == 4) return bsh < 0.0 ? -1.0 : 1.0;
-    else if ((bbr < 0.0 && bsh > 0.0) || (bbr > 0.0 && bsh < 0.0)) return 0.0;
-    else return bbr < 0.0 || bsh < 0.0 ? -1.0 : 1.0;
+    return K != 5 || !((bbr < 0.0 && bsh > 0.0) || (bbr > 0.0 && bsh < 0.0));
+}
+template <int K>
+__device__ __forceinline__ int rates_flip(double b0, double bbr, double bsh)
+{
+    const bool neg = K <= 2 ? b0 < 0.0 : ((K != 4 && bbr < 0.0) || (K != 3 && bsh < 0.0));
+    return neg ? static_cast<int>(0x80000000u) : 0;
+}
+__device__ __forceinline__ double flip_sign(double v, int flip)
+{
+    return __hiloint2double(__double2hiint(v) ^ flip, __double2loint(v));
 }
 // Moments m_{-1..6} (index m + 1) that kernel type K's windows need.
 template <int K>

@@ -551,7 +551,7 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
     const int nblk = slot_blocks(n);
     // direct pairs of a slot: its lags below D0; on other grids at most its rows
     int Dm = min(v.g.D0, n), eh = 0, el = 1;
-    if (!SCATTER && v.g.geo && ws.mom[7] == 0.0 && rate_sign<K>(b0, bbr, bsh) != 0.0 && win_grid(x, n)) {
+    if (!SCATTER && v.g.geo && ws.mom[7] == 0.0 && rates_one_sign<K>(bbr, bsh) && win_grid(x, n)) {
         eh = ws.counter[8];
         el = max(1, ws.counter[9]);
         if (eh >= el) Dm = ws.counter[10];
