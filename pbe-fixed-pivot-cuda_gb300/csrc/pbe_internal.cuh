@@ -627,7 +627,7 @@ struct VjpWs {
     double* vpart;     // [ntile * kVjpMaxChunks * 2 kTileW] row sums per (tile, partner chunk)
     double* lup;       // [lane tasks * 64] lane-task sums of the rows as smaller members
     double* llo;       // [lane tasks * (C + 32)] lane-task sums of the rows as larger members
-    int*    counter;   // [8]: 0 tile tasks, 1 lane tasks
+    int*    counter;   // [8]: 0 tile tasks, 1 lane tasks, 2 lags summed pair by pair (vjp_direct_lags)
 };
 
 inline size_t vjp_ws_layout(int n, char* base, VjpWs* ws)

@@ -244,17 +244,59 @@ vjp_prep_kernel(const double* __restrict__ N, const double* __restrict__ x,
 // One block: the reductions over the prep blocks' partials, spread over the
 // warps: warps 0..3 scan the block totals of the four groups of sums into
 // offsets (each lane a run of consecutive blocks, a warp scan over the runs);
-// warps 4..15 the moments (kVjpFull, kVjpStage), the geometric flag and D0
+// warps 4..14 the moments (kVjpFull, kVjpStage), the geometric flag and D0
 // (kVjpFull, kVjpTables), lanes striding over the blocks, fixed butterflies.
-// Resets the task counters (kVjpFull, kVjpStage).
+// Resets the task counters (kVjpFull, kVjpStage). Then warp 15 tries 32 rows spread over
+// the grid for the rule of the exact rows (vjp_row_exact) and decides for the lags of
+// all (vjp_direct_lags into counter[2]): rows of one kind lie together, so a row among them
+// that keeps its exact sum stands for many.
 constexpr int kVFinThreads = 512;
+
+// Row m of a geometric grid takes its lags from D0 on pair by pair (vjp_lane_rows_kernel
+// derives the rule).
+struct RowOfRule {
+    double x, a, ia, l, ul;      // the row's pivot, its powers 1/3 and -1/3, |lambda_m|, u_m |lambda_{m+1}|
+    __device__ __forceinline__ RowOfRule(const double* __restrict__ xp, const double* __restrict__ lam,
+                                         const VjpWs& ws, int n, int m)
+        : x(xp[m]), a(ws.a[m]), ia(ws.ia[m]), l(fabs(lam[m])), ul(0.0)
+    {
+        if (m < n - 1) {
+            const double xu = xp[m + 1];
+            ul = 1.1102230246251565e-16 * (xu / (xu - x)) * fabs(lam[m + 1]);
+        }
+    }
+};
+// mom: slots 12.. of VjpWs::mom.
+template <int K>
+__device__ __forceinline__ bool vjp_row_exact(const RowOfRule& r, const double* mom, double b0, double bbr,
+                                              double bsh)
+{
+    const double c0 = fabs(b0), c1 = fabs(bbr), c2 = fabs(bsh);
+    const double A = death_factor<K>(r.x, r.a, r.ia, mom, c0, c1, c2);
+    const double AL = death_factor<K>(r.x, r.a, r.ia, mom + 5, c0, c1, c2);
+    const double err = fma(r.ul, A, death_factor<K>(r.x, r.a, r.ia, mom + 10, c0, c1, c2));
+    return err > kVjpGuard * fma(r.l, A, AL);
+}
+
+// Lags summed pair by pair: those below D0; all of them where `rows` of the 32 rows tried
+// are exact and exact rows would take longer. An exact row takes its block 8 to 12 n
+// clocks, one after the other (taken as 16 a row tried, at most the block's 32); all lags
+// instead of those below D0 take the chip 0.01 (n - D0)^2 clocks. (lambda 1 above the
+// largest particles and 0 below, where nearly every row is exact: by exact rows 64
+// sections took 387 us, 960 443 and 16384 2.67 ms.)
+__device__ __forceinline__ int vjp_direct_lags(int n, int D0, int rows)
+{
+    const double d = static_cast<double>(n - D0);
+    return 1200.0 * min(32, 16 * rows) * n > d * d ? n : min(n, D0);
+}
 
 template <int MODE>
 __global__ void __launch_bounds__(kVFinThreads)
-vjp_fin_kernel(const double* __restrict__ x, int n, VjpWs ws)
+vjp_fin_kernel(const double* __restrict__ x, const double* __restrict__ lam, int n, VjpWs ws, int kernel,
+               double b0, double bbr, double bsh)
 {
     const int dep = dep_wait();
-    x += dep; n += dep;
+    x += dep; lam += dep; n += dep;
     const int nb = (n + kPrepThreads - 1) / kPrepThreads;
     const int wq = threadIdx.x >> 5, lq = threadIdx.x & 31;
     if (wq < 4) {
@@ -334,7 +376,35 @@ vjp_fin_kernel(const double* __restrict__ x, int n, VjpWs ws)
         }
         return;
     }
-    for (int r = wq - 4; r < 27; r += kVFinThreads / 32 - 4) {
+    __shared__ double mom_s[27];
+    if (wq == kVFinThreads / 32 - 1) {
+        if (MODE == kVjpTables) return;
+        const int m = static_cast<int>((2LL * lq + 1) * n / 64);
+        const RowOfRule row(x, lam, ws, n, m);
+        asm volatile("bar.sync 1, %0;" :: "n"(kVFinThreads - 128) : "memory");   // warps 4..15
+        const int D0 = static_cast<int>(MODE == kVjpFull ? mom_s[11] : ws.mom[11]);
+        const bool geo = (MODE == kVjpFull ? mom_s[10] : ws.mom[10]) != 0.0;
+        const double* M = mom_s + 12;
+        bool ex = false;
+        if (geo && (m >= D0 || m + D0 < n)) {
+            switch (kernel) {
+            case 0: ex = vjp_row_exact<0>(row, M, b0, bbr, bsh); break;
+            case 1: ex = vjp_row_exact<1>(row, M, b0, bbr, bsh); break;
+            case 2: ex = vjp_row_exact<2>(row, M, b0, bbr, bsh); break;
+            case 3: ex = vjp_row_exact<3>(row, M, b0, bbr, bsh); break;
+            case 4: ex = vjp_row_exact<4>(row, M, b0, bbr, bsh); break;
+            default: ex = vjp_row_exact<5>(row, M, b0, bbr, bsh); break;
+            }
+        }
+        const unsigned rows = __ballot_sync(0xffffffffu, ex);
+        if (lq == 0) {
+            ws.counter[0] = 0;
+            ws.counter[1] = 0;
+            ws.counter[2] = vjp_direct_lags(n, D0, __popc(rows));
+        }
+        return;
+    }
+    for (int r = wq - 4; r < 27; r += kVFinThreads / 32 - 5) {
         double t = 0.0;
         if (r == 10 || r == 11) {
             if (MODE == kVjpStage) continue;
@@ -353,12 +423,10 @@ vjp_fin_kernel(const double* __restrict__ x, int n, VjpWs ws)
             for (int b = lq; b < nb; b += 32) t += ws.mom_part[b * kVjpMom + r];
             t = warp_sum(t);
         }
-        if (lq == 0) ws.mom[r] = t;
+        if (lq == 0) { ws.mom[r] = t; mom_s[r] = t; }
     }
-    if (threadIdx.x == 128 && MODE != kVjpTables) {
-        ws.counter[0] = 0;
-        ws.counter[1] = 0;
-    }
+    if (MODE != kVjpTables)
+        asm volatile("bar.sync 1, %0;" :: "n"(kVFinThreads - 128) : "memory");
 }
 
 // Pair sums: task = (row tile, partner chunk); the whole CTA is one group.
@@ -486,7 +554,8 @@ __global__ void __launch_bounds__(256) vjp_gfin_kernel(int ntile, int nlane, Vjp
 // instructions per pair (P; P Bf, P Sf; two sums of the smaller member; two
 // FMAs into W) against 8 for the two visits of the tile path.
 // Only the lags below D0: from there on every pair lands on its larger member's
-// own slot, lo = k, and the sums separate (vjp_lane_rows_kernel).
+// own slot, lo = k, and the sums separate (vjp_lane_rows_kernel; vjp_direct_lags
+// tells when all lags are summed here after all).
 // Tasks (row block, lag chunk) run chunk by chunk; all but the lowest-lag rows'
 // have equal length. Determinism: the windows of the CTA's warps are added in
 // warp order; the rows kernel adds the tasks' sums in a fixed order.
@@ -521,7 +590,7 @@ vjp_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
     const double lamlast = lam[n - 1];
     const int ew = (C + kLaneWarps - 1) / kLaneWarps + 32;
     double* eb = esm + w * ew;
-    const int Dm = static_cast<int>(ws.mom[11]);
+    const int Dm = ws.counter[2];
 
     for (;;) {
         if (tid == 0) s_task = atomicAdd(ws.counter + 1, 1);
@@ -680,7 +749,7 @@ __device__ __forceinline__ void bin_sums(const VjpWs& ws, const double* __restri
 // u_k = 2^-53 x_{k+1}/dx_k. Bounded over all partners with the moments of
 // |N|, |lambda N| and u |N| |lambda step|, it may move a row by at most
 // kVjpGuard of the row's sum of |terms|; rows where it could (a lambda that is
-// nonzero on few bins) take their lags from D0 on pair by pair.
+// nonzero on few bins) take their lags from D0 on pair by pair (vjp_row_exact).
 #ifndef PBE_VROWS_WARPS
 #define PBE_VROWS_WARPS 16
 #endif
@@ -708,7 +777,7 @@ vjp_lane_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
     }
     const int b = gridDim.x - 1 - blockIdx.x;      // top row blocks (the most lower blocks) first
     const int m = kLaneBins * b + lane;
-    const int Dm = static_cast<int>(ws.mom[11]);   // lags below Dm were summed pair by pair
+    const int Dm = ws.counter[2];                  // lags below Dm were summed pair by pair
     int nchunks = 0;                               // chunks that hold such lags
     while (nchunks < kVLaneMaxChunks && 1 + nchunks * C < Dm && vjp_lane_chunk_blocks(n, nchunks, C) > 0) ++nchunks;
     if (threadIdx.x == 0) {
@@ -718,21 +787,11 @@ vjp_lane_rows_kernel(const double* __restrict__ N, const double* __restrict__ x,
             sacc += vjp_lane_chunk_blocks(n, c, C);
         }
     }
-    // rows that take the lags from D0 on pair by pair
+    // rows that take the other lags so too
     if (w == 0) {
         bool ex = false;
-        if (m < n && (m >= Dm || m + Dm < n)) {
-            const double xm = x[m], am = ws.a[m], iam = ws.ia[m];
-            const double c0 = fabs(b0), c1 = fabs(bbr), c2 = fabs(bsh);
-            const double A = death_factor<K>(xm, am, iam, ws.mom + 12, c0, c1, c2);
-            const double AL = death_factor<K>(xm, am, iam, ws.mom + 17, c0, c1, c2);
-            double err = death_factor<K>(xm, am, iam, ws.mom + 22, c0, c1, c2);
-            if (m < n - 1) {
-                const double xu = x[m + 1];
-                err = fma(1.1102230246251565e-16 * (xu / (xu - xm)) * fabs(lam[m + 1]), A, err);
-            }
-            ex = err > kVjpGuard * fma(fabs(lam[m]), A, AL);
-        }
+        if (m < n && (m >= Dm || m + Dm < n))
+            ex = vjp_row_exact<K>(RowOfRule(x, lam, ws, n, m), ws.mom + 12, b0, bbr, bsh);
         const unsigned em = __ballot_sync(0xffffffffu, ex);
         if (lane == 0) exact_s = em;
     }
@@ -1020,15 +1079,18 @@ cudaError_t agg_vjp_k(const AggVjpArgs& a, const VjpWs& ws, int num_sms, cudaStr
     const int lane_on = vjp_lane_on(n) ? 1 : 0;
     if (kind == kVjpTables) {
         launch_dep(vjp_prep_kernel<kVjpTables>, dim3(nb), kVPrepThreads, 0, s, 1, a.N, a.x, a.lam, n, ws);
-        launch_dep(vjp_fin_kernel<kVjpTables>, dim3(1), kVFinThreads, 0, s, 1, a.x, n, ws);
+        launch_dep(vjp_fin_kernel<kVjpTables>, dim3(1), kVFinThreads, 0, s, 1, a.x, a.lam, n, ws, a.kernel, a.beta0,
+                   a.beta_br, a.beta_sh);
         return cudaGetLastError();
     }
     if (kind == kVjpStage) {
         launch_dep(vjp_prep_kernel<kVjpStage>, dim3(nb), kVPrepThreads, 0, s, 1, a.N, a.x, a.lam, n, ws);
-        launch_dep(vjp_fin_kernel<kVjpStage>, dim3(1), kVFinThreads, 0, s, 1, a.x, n, ws);
+        launch_dep(vjp_fin_kernel<kVjpStage>, dim3(1), kVFinThreads, 0, s, 1, a.x, a.lam, n, ws, a.kernel, a.beta0,
+                   a.beta_br, a.beta_sh);
     } else {
         launch_dep(vjp_prep_kernel<kVjpFull>, dim3(nb), kVPrepThreads, 0, s, 1, a.N, a.x, a.lam, n, ws);
-        launch_dep(vjp_fin_kernel<kVjpFull>, dim3(1), kVFinThreads, 0, s, 1, a.x, n, ws);
+        launch_dep(vjp_fin_kernel<kVjpFull>, dim3(1), kVFinThreads, 0, s, 1, a.x, a.lam, n, ws, a.kernel, a.beta0,
+                   a.beta_br, a.beta_sh);
     }
     const int nrb = (n + kLaneBins - 1) / kLaneBins;
     if (lane_on) {
