@@ -441,7 +441,7 @@ __device__ void lane_task(const LaneView& v, const AggWs& ws, const LaneArgs& la
         slot_pairs_geo<K, 1>(v.g, &v.p, s, slot, smax, dw0, min(dB, dw0 + per),
                              ew_operand_c(xs, -exponent_of(xs)), r, th);
     } else {
-        slot_pairs_any<K, 1>(v.g, &v.p, s, slot, c * kLaneWarps + w, la.parts * kLaneWarps, r, th);
+        slot_pairs_any<K, 1>(v.g, &v.p, s, slot, s + 1, c * kLaneWarps + w, la.parts * kLaneWarps, r, th);
     }
     sm.red[w][0][lane] = R + r;
     sm.red[w][1][lane] = TH + th;

@@ -40,27 +40,6 @@ __device__ __forceinline__ double q_slot(double B, double S, double Nj, double h
     else return fma(S, hj, B * Nj);
 }
 
-// Pair rate on any grid from per-bin values (a = x^(1/3), ia = 1/a, h = x N):
-// beta of src/aggregation_kernels.cuh:56-89 with the divisions replaced by
-// products with the reciprocal cube roots.
-template <int K>
-__device__ __forceinline__ double rate_gen(bool diag, double b0, double bbr, double bsh,
-                                           double Nj, double hj, double aj, double iaj,
-                                           double Nk, double hk, double ak, double iak)
-{
-    double r;
-    if constexpr (K == 0) r = (b0 * Nj) * Nk;
-    else if constexpr (K == 1) r = b0 * fma(hj, Nk, Nj * hk);
-    else if constexpr (K == 2) r = (b0 * hj) * hk;
-    else {
-        double beta = 0.0;
-        if constexpr (K == 3 || K == 5) beta = bbr * (fma(aj, iak, ak * iaj) + 2.0);
-        if constexpr (K == 4 || K == 5) { const double s = aj + ak; beta = fma(bsh * s, s * s, beta); }
-        r = (beta * Nj) * Nk;
-    }
-    return diag ? 0.5 * r : r;
-}
-
 // sum_k beta(x_i, x_k) N_k from the moments
 // M[0] = sum N/a, M[1] = sum N, M[2] = sum a N, M[3] = sum a^2 N, M[4] = sum x N.
 template <int K>

@@ -131,29 +131,88 @@ __device__ __forceinline__ void slot_pairs_geo(const SlotGrid& g, const SlotPass
     }
 }
 
-// beta(x_j, x_k) a_j b_k from per-bin values, every pass.
+// beta(x_j, x_k) of one row j as a polynomial in a_k, 1/a_k (no minus signs in it):
+//   Brownian  beta_br (a_j/a_k + a_k/a_j + 2),
+//   shear     beta_sh (a_j + a_k)^3 = beta_sh (x_j + 3 a_j^2 a_k + 3 a_j a_k^2 + a_k^3).
+// Five FP64 instructions a row and up to four a pair, where a pair alone takes eight.
+template <int K>
+struct RowBeta {
+    double c0, c1, c2, c3, ci;
+    __device__ __forceinline__ RowBeta(const SlotGrid& g, int j)
+    {
+        c0 = c1 = c2 = c3 = ci = 0.0;
+        if constexpr (K >= 3) {
+            const double aj = g.a[j];
+            if constexpr (K == 3 || K == 5) { c0 = 2.0 * g.bbr; c1 = g.bbr * g.ia[j]; ci = g.bbr * aj; }
+            if constexpr (K == 4 || K == 5) {
+                c3 = g.bsh;
+                c2 = (3.0 * g.bsh) * aj;
+                c1 = fma(c2, aj, c1);
+                c0 = fma(g.bsh, __ldg(g.x + j), c0);
+            }
+        }
+    }
+    __device__ __forceinline__ double operator()(double ak, double iak) const
+    {
+        if constexpr (K == 3) return fma(ci, iak, fma(c1, ak, c0));
+        const double shear = fma(ak, fma(ak, fma(ak, c3, c2), c1), c0);
+        if constexpr (K == 4) return shear;
+        return fma(ci, iak, shear);
+    }
+};
+
+// beta(x_j, x_k) a_j b_k from per-bin values, every pass (row: the row's RowBeta).
 template <int K, int NP>
-__device__ __forceinline__ double slot_rate_any(const SlotGrid& g, const SlotPass* p, int j, int k)
+__device__ __forceinline__ double slot_rate_any(const SlotGrid& g, const SlotPass* p, const RowBeta<K>& row, int j,
+                                                int k)
 {
-    const double aj = K >= 3 ? g.a[j] : 0.0, iaj = K >= 3 ? g.ia[j] : 0.0;
-    const double ak = K >= 3 ? g.a[k] : 0.0, iak = K >= 3 ? g.ia[k] : 0.0;
+    double beta = 0.0;
+    if constexpr (K >= 3) beta = row(g.a[k], g.ia[k]);
     double r = 0.0;
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
-        const double v = rate_gen<K>(j == k, g.b0, g.bbr, g.bsh, p[q].Aj[j],
-                                     NeedH<K>::k ? p[q].AHj[j] : 0.0, aj, iaj,
-                                     p[q].Nk[k], NeedH<K>::k ? p[q].Hk[k] : 0.0, ak, iak);
+        double v;
+        if constexpr (K == 0) v = (g.b0 * p[q].Aj[j]) * p[q].Nk[k];
+        else if constexpr (K == 1) v = g.b0 * fma(p[q].AHj[j], p[q].Nk[k], p[q].Aj[j] * p[q].Hk[k]);
+        else if constexpr (K == 2) v = (g.b0 * p[q].AHj[j]) * p[q].Hk[k];
+        else v = (beta * p[q].Aj[j]) * p[q].Nk[k];
         r = q == 0 ? v : r + v;
     }
-    return r;
+    return j == k ? 0.5 * r : r;
+}
+
+// First j <= s + 1 with 2 x_j >= x_{s+1}, sought from `guess`: from there on a row has
+// no larger member with which it stays below x_{s+1}. On a linear grid that is half of
+// the rows.
+__device__ __forceinline__ int slot_rows_end(const double* __restrict__ x, int s, int guess)
+{
+    const long long top = dbits(__ldg(x + s + 1));
+    auto end = [&](int j) { return dbits(2.0 * __ldg(x + j)) >= top; };
+    int lo, hi, step = 1;                              // lo: not yet (or -1); hi: 2 x_hi >= x_{s+1}
+    const int g = min(max(guess, 0), s);
+    if (end(g)) {
+        hi = g;
+        while (hi - step > 0 && end(hi - step)) { hi -= step; step <<= 1; }
+        lo = hi - step > 0 ? hi - step : -1;
+    } else {
+        lo = g;
+        while (lo + step <= s && !end(lo + step)) { lo += step; step <<= 1; }
+        hi = min(s + 1, lo + step);
+    }
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (end(mid)) hi = mid; else lo = mid;
+    }
+    return hi;
 }
 
 // Share w of nw of slot s's rows on any grid, but for the pairs of the prefix
 // sums: for each row j the larger members k with x_s <= fl(x_j + x_k) < x_{s+1}
-// lie in one run below the previous row's, so a lane walks down k as j grows.
+// lie in one run below the previous row's, so a lane walks down k as j grows. Rows
+// from jt on have none (slot_rows_end, or s + 1).
 template <int K, int NP>
 __device__ __forceinline__ void slot_pairs_any(const SlotGrid& g, const SlotPass* p, int s, bool slot,
-                                               int w, int nw, double& R, double& TH)
+                                               int jt, int w, int nw, double& R, double& TH)
 {
     if (!slot) return;
     const double* __restrict__ x = g.x;
@@ -162,8 +221,8 @@ __device__ __forceinline__ void slot_pairs_any(const SlotGrid& g, const SlotPass
     const int St20 = -exponent_of(xs) * (1 << 20);
     const int Js = slot_cut(g, s);
     const int j0 = s > 0 ? min(Js, slot_cut(g, s - 1)) : Js;
-    const int per = (s + 1 - j0 + nw - 1) / nw;
-    const int ja = j0 + w * per, jb = min(s + 1, ja + per);
+    const int per = (max(0, jt - j0) + nw - 1) / nw;
+    const int ja = j0 + w * per, jb = min(jt, ja + per);
     if (ja >= jb) return;
     // last k <= s with fl(x_ja + x_k) < x_{s+1} (below ja: the rows are done)
     const double xa = __ldg(x + ja);
@@ -176,11 +235,12 @@ __device__ __forceinline__ void slot_pairs_any(const SlotGrid& g, const SlotPass
         const double xj = __ldg(x + j);
         while (k >= j && dbits(xj + __ldg(x + k)) >= hi) --k;
         if (k < j) break;
+        const RowBeta<K> row(g, j);
         for (int q = k; q >= j; --q) {
             const double v = xj + __ldg(x + q);
             if (dbits(v) < lo) break;
             if (q == s && j < Js) continue;            // in the prefix sums
-            const double r = slot_rate_any<K, NP>(g, p, j, q);
+            const double r = slot_rate_any<K, NP>(g, p, row, j, q);
             R += r;
             TH = fma(r, scale_pow2(v - xs, St20), TH);
         }
@@ -200,6 +260,8 @@ __device__ __forceinline__ void slot_exact_part(const SlotGrid& g, const SlotPas
     const int cut = slot_cut(g, s);
     r = 0.0;
     t = 0.0;
+    constexpr int kU = NP == 1 ? 2 : 1;                // (two of the two-pass sums spill)
+#pragma unroll kU
     for (int j = tid; j < cut; j += nt) {
         double rate, th;
         if (g.geo) {
@@ -212,7 +274,7 @@ __device__ __forceinline__ void slot_exact_part(const SlotGrid& g, const SlotPas
                                     NeedH<K>::k ? p[q].Hk[s] : 0.0);
             th = sum_minus_scaled_pre(pa, __ldg(g.x + j), pc);
         } else {
-            rate = slot_rate_any<K, NP>(g, p, j, s);
+            rate = slot_rate_any<K, NP>(g, p, RowBeta<K>(g, j), j, s);
             th = scale_pow2((__ldg(g.x + j) + xs) - xs, St * (1 << 20));
         }
         r += rate;
@@ -231,30 +293,15 @@ __device__ __forceinline__ void slot_exact(const SlotGrid& g, const SlotPass* p,
     TH = warp_sum(t);
 }
 
-// Warp w of nw's part of the 32 slots s = I - 1 + lane (I the first bin): the
-// direct pairs, and its turns of the slots that keep their exact pair sums
-// (spread over the warps). Returns the mask of those slots; the prefix part of
-// the others is left to the caller.
+// Warp w of nw's turns of those among the 32 slots s = I - 1 + lane (I the first bin) that
+// keep their exact pair sums (spread over the warps), added to R, TH. Returns the mask of
+// those slots; the prefix part of the others is left to the caller.
 template <int K, int NP>
-__device__ __forceinline__ unsigned slot_warp(const SlotGrid& g, const SlotPass* p, int I, int w, int nw,
-                                              double& R, double& TH)
+__device__ __forceinline__ unsigned slot_exact_turns(const SlotGrid& g, const SlotPass* p, int I, int w, int nw,
+                                                     double& R, double& TH)
 {
     const int l = threadIdx.x & 31, s = I - 1 + l, n = g.n;
     const bool slot = s >= 0 && s <= n - 2;
-    R = 0.0;
-    TH = 0.0;
-    if (g.geo) {
-        // equal contiguous shares of the lags below D0 (each warp sees its runs in order)
-        const int smax = min(I - 1 + 31, n - 2);
-        const double xs = slot ? __ldg(g.x + s) : 1.0;
-        const int lags = min(min(n, g.D0), smax + 1);
-        const int per = (lags + nw - 1) / nw;
-        const int d0 = w * per;
-        slot_pairs_geo<K, NP>(g, p, s, slot, smax, d0, min(lags, d0 + per),
-                              ew_operand_c(xs, -exponent_of(xs)), R, TH);
-    } else {
-        slot_pairs_any<K, NP>(g, p, s, slot, w, nw, R, TH);
-    }
     // (mom_exact_slot; not where x_{s+1} is within kMomGuard 2^53 = 2252 of x_0: bin s + 1
     // gets at least x_0 / dx_s of every one of these pairs' rates, and u is within
     // kMomGuard of that. 4096 cells of 48 sections: 503 us, 465 with this)
@@ -279,12 +326,46 @@ __device__ __forceinline__ unsigned slot_warp(const SlotGrid& g, const SlotPass*
     return exact;
 }
 
+// Warp w of nw's direct lags of the 32 slots s = I - 1 + lane on a geometric grid:
+// equal contiguous shares of the lags below D0 (each warp sees its runs in order).
+template <int K, int NP>
+__device__ __forceinline__ void slot_lags(const SlotGrid& g, const SlotPass* p, int I, int w, int nw,
+                                          double& R, double& TH)
+{
+    const int s = I - 1 + (threadIdx.x & 31), n = g.n;
+    const bool slot = s >= 0 && s <= n - 2;
+    const int smax = min(I - 1 + 31, n - 2);
+    const double xs = slot ? __ldg(g.x + s) : 1.0;
+    const int lags = min(min(n, g.D0), smax + 1);
+    const int per = (lags + nw - 1) / nw;
+    const int d0 = w * per;
+    slot_pairs_geo<K, NP>(g, p, s, slot, smax, d0, min(lags, d0 + per), ew_operand_c(xs, -exponent_of(xs)), R, TH);
+}
+
 // Clipped pairs (x_j + x_k >= x[n-1], all deposited on bin n-1,
 // src/aggregation_kernels.cuh:191-192) but for those of the prefix sums of slot
 // n - 1, share of thread tid of nt: a warp per lag with its lanes over j on a
-// geometric grid, a thread per row otherwise.
+// geometric grid, lanes over a row's larger members otherwise. Neighbouring warps have shares of about
+// equal length and far ones have not, so CTAs that share a cell take warps in turn
+// (slot_clip_tid).
+__device__ __forceinline__ int slot_clip_tid(int rank, int ranks)
+{
+    return ((static_cast<int>(threadIdx.x >> 5) * ranks + rank) << 5) + static_cast<int>(threadIdx.x & 31);
+}
+
+// A row's larger members over as many lanes as a cell's CTAs have threads for: a pair is a
+// chain of some ten dependent FP64 instructions, and n / 2 of them in a row took 31 us at
+// 155 linear sections.
+__device__ __forceinline__ int slot_clip_lanes(int n, int nt)
+{
+    int G = 1;
+    while (G < 32 && 2 * G * n <= nt) G <<= 1;
+    return G;
+}
+
+// G: lanes a row (a power of two).
 template <int K, int NP>
-__device__ double slot_clip(const SlotGrid& g, const SlotPass* p, int tid, int nt)
+__device__ double slot_clip(const SlotGrid& g, const SlotPass* p, int tid, int nt, int G)
 {
     const int n = g.n;
     double acc = 0.0;
@@ -303,7 +384,7 @@ __device__ double slot_clip(const SlotGrid& g, const SlotPass* p, int tid, int n
         }
     } else {
         const long long top = dbits(__ldg(g.x + n - 1));
-        for (int j = tid; j < n; j += nt) {
+        for (int j = tid / G; j < n; j += nt / G) {
             const double xj = __ldg(g.x + j);
             int lo = j, hi = n - 1;                    // x_j + x[n-1] >= x[n-1] always holds
             while (lo < hi) {
@@ -311,8 +392,11 @@ __device__ double slot_clip(const SlotGrid& g, const SlotPass* p, int tid, int n
                 if (dbits(xj + __ldg(g.x + mid)) >= top) hi = mid; else lo = mid + 1;
             }
             // k = n - 1 is in the prefix sums, but for the diagonal pair
-            for (int k = lo; k < n - 1 || (k == n - 1 && j == n - 1); ++k)
-                acc += slot_rate_any<K, NP>(g, p, j, k);
+            const int sub = tid & (G - 1);
+            const RowBeta<K> row(g, j);
+#pragma unroll 2
+            for (int k = lo + sub; k < n - 1; k += G) acc += slot_rate_any<K, NP>(g, p, row, j, k);
+            if (j == n - 1 && sub == 0) acc += slot_rate_any<K, NP>(g, p, row, j, j);
         }
     }
     return acc;

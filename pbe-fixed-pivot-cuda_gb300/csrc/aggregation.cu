@@ -567,7 +567,8 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
         if (task < nclip) {
             // a part of the clipped pairs (but for the prefix part of slot n - 1),
             // summed over the CTA in a fixed order
-            double sc = warp_sum(slot_clip<K, 1>(v.g, &v.p, task * kMainThreads + tid, nclip * kMainThreads));
+            // (a thread a row: 2049 irregular sections 125 us, 132 with two)
+            double sc = warp_sum(slot_clip<K, 1>(v.g, &v.p, task * kMainThreads + tid, nclip * kMainThreads, 1));
             if ((tid & 31) == 0) sm.sum[tid >> 5] = sc;
             __syncthreads();
             if (tid == 0) {
@@ -615,6 +616,7 @@ enum { kAggFull = 0, kAggTables = 1, kAggStage = 2 };
 constexpr int kSmallBins = 31;
 constexpr int kSmallMaxCtas = 16;
 constexpr int kSmallMaxN = kSmallBins * kSmallMaxCtas;
+constexpr int kSmallClipRows = 32;     // most rows of clipped pairs that the last CTA sums alone
 
 template <int K, int KIND>
 __global__ void __launch_bounds__(kMainThreads)
@@ -638,6 +640,8 @@ agg_small_kernel(const double* __restrict__ N, const double* __restrict__ x, dou
     __shared__ int geo_all;
     __shared__ double red[kLaneWarps][2][32];
     __shared__ double csum[kLaneWarps];
+    __shared__ double cpart[kSmallMaxCtas];            // last CTA: the CTAs' parts of the clipped pairs
+    __shared__ int jt_s[32];                           // end of every slot's rows (slot_pairs_any)
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int r = static_cast<int>(cl.block_rank()), ranks = static_cast<int>(cl.num_blocks());
     const int I = kSmallBins * r;
@@ -690,6 +694,24 @@ agg_small_kernel(const double* __restrict__ N, const double* __restrict__ x, dou
             }
             if (lane == 31) te_s = E;
         }
+    }
+    if (w == 4) {
+        // end of every slot's rows (slot_pairs_any), sought from where a geometric grid through
+        // the end points would have half of x_{s+1}; kept in xlist, which this kernel has no
+        // use for
+        const int s = I - 1 + lane;
+        int jt = 0;
+        if (s >= 0 && s <= n - 2) {
+            if constexpr (KIND == kAggStage) {
+                jt = ws.xlist[s];
+            } else {
+                const float lx0 = log2_approx(__ldg(x)), span = log2_approx(__ldg(x + n - 1)) - lx0;
+                const float gf = (log2_approx(__ldg(x + s + 1)) - 1.0f - lx0) * (static_cast<float>(n - 1) / span);
+                jt = slot_rows_end(x, s, static_cast<int>(fminf(fmaxf(gf, 0.0f), static_cast<float>(s))));
+                if (KIND == kAggTables) ws.xlist[s] = jt;
+            }
+        }
+        jt_s[lane] = jt;
     }
     if constexpr (KIND != kAggStage) {
         if (w == 1) {
@@ -786,22 +808,39 @@ agg_small_kernel(const double* __restrict__ N, const double* __restrict__ x, dou
     const SlotGrid g{x, ws.a, ws.ia, ws.inv_dx, ws.Bd, ws.Sd, ws.Ld, ws.J0, n, D0_all, geo_all != 0,
                      b0, bbr, bsh};
     const SlotPass p{N, ws.h, N, ws.h, N, ws.h};
-    double R, TH;
-    const unsigned exact = slot_warp<K, 1>(g, &p, I, w, kLaneWarps, R, TH);
+    const int s = I - 1 + lane;                        // this lane's slot and bin
+    const bool slot = s >= 0 && s <= n - 2;
+    double R = 0.0, TH = 0.0;
+    if (g.geo) slot_lags<K, 1>(g, &p, I, w, kLaneWarps, R, TH);
+    else slot_pairs_any<K, 1>(g, &p, s, slot, jt_s[lane], w, kLaneWarps, R, TH);
+    const unsigned exact = slot_exact_turns<K, 1>(g, &p, I, w, kLaneWarps, R, TH);
     red[w][0][lane] = R;
     red[w][1][lane] = TH;
-    if (last == n - 1) {
-        const double c = warp_sum(slot_clip<K, 1>(g, &p, tid, kMainThreads));
+    // the clipped pairs: of few rows (D0 of a geometric grid, those from J0(n - 2) on of
+    // another) by the last CTA, else (fine or linear grids: up to half of all pairs) a
+    // share per CTA (all of them in the last one: 480 sections at 128 an octave 99 us, 248
+    // linear ones 140)
+    const bool alone = ranks == 1 || (g.geo ? g.D0 : n - ws.J0[n - 2]) <= kSmallClipRows;
+    if (!alone || r == ranks - 1) {
+        const int nt = (alone ? 1 : ranks) * kMainThreads;
+        const double c = warp_sum(slot_clip<K, 1>(g, &p, alone ? tid : slot_clip_tid(r, ranks), nt,
+                                                  slot_clip_lanes(n, nt)));
         if (lane == 0) csum[w] = c;
     }
     __syncthreads();
+    if (!alone) {
+        if (tid == 0) {
+            double sum = 0.0;
+            for (int q = 0; q < kLaneWarps; ++q) sum += csum[q];
+            *cl.map_shared_rank(&cpart[r], static_cast<unsigned>(ranks - 1)) = sum;
+        }
+        cl.sync();                                     // the parts are there; nobody left before
+    }
     if (w != 0) return;
     R = 0.0;
     TH = 0.0;
 #pragma unroll
     for (int q = 0; q < kLaneWarps; ++q) { R += red[q][0][lane]; TH += red[q][1][lane]; }
-    const int s = I - 1 + lane;                        // this lane's slot and bin
-    const bool slot = s >= 0 && s <= n - 2;
     double death = 0.0, clip = 0.0, own = 0.0, up = 0.0;
     if (s >= 0 && s < n) {
         const double xs = x[s], as = g.a[s], ias = g.ia[s], Ns = N[s];
@@ -831,8 +870,8 @@ agg_small_kernel(const double* __restrict__ N, const double* __restrict__ x, dou
             own = fma(-TH, sd, R);
             up = TH * sd;
         } else {
-#pragma unroll
-            for (int q = 0; q < kLaneWarps; ++q) clip += csum[q];
+            if (alone) for (int q = 0; q < kLaneWarps; ++q) clip += csum[q];
+            else for (int q = 0; q < ranks; ++q) clip += cpart[q];
         }
     }
     const double in = __shfl_up_sync(0xffffffffu, up, 1);

@@ -54,6 +54,7 @@ struct BatchDev {
     // per grid bin (packed by BatchGridDev::off)
     double* gx; double* ga; double* gia; double* ginv_dx; double* gBd; double* gSd; int* gLd;
     int* gJ0;       // first j with fl(x_j + x_i) >= x_{i+1} (at most i)
+    int* gJt;       // first j with 2 x_j >= x_{i+1}: end of slot i's rows (slot_pairs_any)
     double* gSl;    // shear factor of lag d seen from the larger member: (1 + rho)^3 x_0 / x_d
     // breakage fragment tables: bfirst[foff + q (n+2) + m + 1] = first j with
     // lo(q, j) >= m; bwlo / bwhi[woff + q n + j] = bw_q times the shares of the

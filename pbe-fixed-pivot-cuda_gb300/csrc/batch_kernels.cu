@@ -83,6 +83,7 @@ batch_grid_kernel(BatchDev d)
             }
         }
         d.gJ0[gd->off + i] = jl;
+        d.gJt[gd->off + i] = i < n - 1 ? slot_rows_end(x, i, i) : 0;
         if (n >= 2) {
             double e = geo_dev(fit, xi, i);
             if (!(e == e)) e = 1.0;
@@ -388,8 +389,9 @@ __device__ void prep_cell(const BatchDev& d, double* N, const pbe_batch_cell_par
         const SlotGrid g = slot_grid(d, gd, n, P);
         SlotPass sp[1];
         slot_passes<1>(d, Yk - off, off, sp);
-        const double clip = block_sum(slot_clip<K, 1>(g, sp, part.rank * blockDim.x + threadIdx.x,
-                                                      part.ranks * blockDim.x), sm.sh);
+        const int nt = part.ranks * static_cast<int>(blockDim.x);
+        const double clip = block_sum(slot_clip<K, 1>(g, sp, slot_clip_tid(part.rank, part.ranks), nt,
+                                                      slot_clip_lanes(n, nt)), sm.sh);
         if (threadIdx.x == 0) mom[10 + part.rank] = clip;
     }
     if (d.nq > 0 && !(d.brk & kBrkTasks)) cell_breakage(d, gd, d.SN + off, d.Bk + off, n, part.r0, part.r1);
@@ -468,8 +470,9 @@ batch_jvp_prep_kernel(BatchDev d, const double* __restrict__ v,
         const SlotGrid g = slot_grid(d, gd, n, P);
         SlotPass sp[2];
         slot_passes<2>(d, v, off, sp);
-        const double clip = block_sum(slot_clip<K, 2>(g, sp, part.rank * blockDim.x + threadIdx.x,
-                                                      part.ranks * blockDim.x), sh);
+        const int nt = part.ranks * static_cast<int>(blockDim.x);
+        const double clip = block_sum(slot_clip<K, 2>(g, sp, slot_clip_tid(part.rank, part.ranks), nt,
+                                                      slot_clip_lanes(n, nt)), sh);
         if (threadIdx.x == 0) mom[10 + part.rank] = clip;
     }
     if (d.nq > 0 && !(d.brk & kBrkTasks)) cell_breakage(d, gd, d.SN + off, d.Bk + off, n, part.r0, part.r1);
@@ -516,7 +519,12 @@ __device__ void batch_task(const BatchDev& d, const double* __restrict__ Yg,
     const bool slot = s >= 0 && s <= n - 2;
     const int St = slot ? -exponent_of(__ldg(g.x + s)) : 0;
     double R = 0.0, TH = 0.0;
-    const unsigned exact = agg ? slot_warp<K, NP>(g, p, I, w, nw, R, TH) : 0u;
+    unsigned exact = 0u;
+    if (agg) {
+        if (g.geo) slot_lags<K, NP>(g, p, I, w, nw, R, TH);
+        else slot_pairs_any<K, NP>(g, p, s, slot, slot ? __ldg(d.gJt + gd.off + s) : 0, w, nw, R, TH);
+        exact = slot_exact_turns<K, NP>(g, p, I, w, nw, R, TH);
+    }
     const bool brk = d.nq > 0;
     const bool brk_tasks = (d.brk & kBrkTasks) != 0;
     if (brk && brk_tasks) tile_breakage(d, gd, d.SN + off, n, I, sm.extra[G.g], G);
