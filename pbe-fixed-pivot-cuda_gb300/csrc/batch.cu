@@ -133,9 +133,15 @@ int n_class(int n)
 // Up to 8 CTAs of 256 threads per SM, more than fit at once, so that the last tasks of a
 // launch are short (48 cells of 256..2048 bins, forward and VJP: 25.96 ms with 2, 22.21
 // with 4, 21.79 with 8; 256 cells of up to 3840 the same with all three).
+// Tasks that leave an SM below 512 threads are chains of latencies whatever their lags
+// (a lag's pair, a slot that keeps its exact sum, a row of another grid): their warps
+// then come without that limit (an RHS of 128 cells of 100 sections 44 us with a warp a
+// task, 34 with 4; one cell of 200 with every other section empty 62 and 38; 16 cells of
+// 31 linear sections 67 and 40).
 int rule_group_size(long long tasks, int max_lags, int num_sms)
 {
     int T = 32;
+    while (T < kMainThreads && tasks * 2 * T <= 512LL * num_sms) T <<= 1;
     while (T < kMainThreads && tasks * T < 8LL * kMainThreads * num_sms && max_lags * 32 >= 16 * 2 * T) T <<= 1;
     return T;
 }
@@ -239,12 +245,18 @@ void build_schedule(const pbe_batch_plan& p, const int* gs, const bool* want,
     struct B { long long cost; int cls; int first; int cnt; };
     std::vector<B> bl;
     std::vector<std::vector<HostTask>> sorted(kClasses);
+    // tasks side by side in a CTA share its SM's FP64 pipe: while there are SMs without
+    // one, each gets a CTA of its own (16 cells of 31 linear bins: 82 us for an RHS with 8
+    // tasks a CTA)
+    size_t all = 0;
+    for (const auto& v : per) all += v.size();
+    const size_t spread = std::max<size_t>(1, all / static_cast<size_t>(std::max(1, p.num_sms)));
     for (int cls = 0; cls < kClasses; ++cls) {
         auto& v = per[cls];
         if (v.empty()) continue;
         std::stable_sort(v.begin(), v.end(),
                          [](const HostTask& a, const HostTask& b) { return a.cost > b.cost; });
-        const int per_b = kMainThreads / gs[cls];
+        const size_t per_b = std::min<size_t>(kMainThreads / gs[cls], spread);
         for (size_t i = 0; i < v.size(); i += per_b) {
             const int cnt = static_cast<int>(std::min<size_t>(per_b, v.size() - i));
             long long cost = 0;
@@ -380,7 +392,7 @@ cudaError_t autotune(pbe_batch_plan* p, bool retune, cudaStream_t s)
     return e;
 }
 
-// Direct lags of every grid (from its tables) and the launch shape of the prep
+// Direct lags of every grid (from its tables) and the launch shapes of the prep
 // kernels: a thread per two bins of an average cell, up to 256; where the cells
 // are too few for the SMs, clusters of up to 8 CTAs share a cell (a prep of one
 // CTA per cell costs about 30 FP64 operations a bin on one SM: 60 us at n = 3840).
@@ -400,9 +412,22 @@ cudaError_t prep_shape(pbe_batch_plan* p, cudaStream_t s)
     }
     const long long avg = p->total / p->n_cells;
     int ranks = 1;
-    while (ranks < 8 && 2LL * ranks * p->n_cells <= 4LL * p->num_sms && p->max_n >= 256 * ranks) ranks <<= 1;
+    while (ranks < 8 && ((2LL * ranks * p->n_cells <= 4LL * p->num_sms && p->max_n >= 256 * ranks) ||
+                         (ranks < 4 && 2LL * ranks * p->n_cells <= p->num_sms && p->max_n >= 128 * ranks)))
+        ranks <<= 1;
+    // (a thread per bin where every cell has SMs to itself: an RHS of one cell of 64
+    // sections 50 us with two bins a thread, 40 with one)
+    const bool few = static_cast<long long>(ranks) * p->n_cells <= p->num_sms;
     int threads = 32;
-    while (threads < 256 && (ranks > 1 || 2LL * threads < avg)) threads <<= 1;
+    while (threads < 256 && (ranks > 1 || (few ? threads : 2LL * threads) < avg)) threads <<= 1;
+    // the VJP's prep: its two scans pay per warp (48 cells of 256..2048 bins, 8 CTAs each:
+    // 83 us with 256 threads, 62 with 64), so three bins a thread, and one where every
+    // cell has SMs to itself (one cell of 200: 92 us a VJP with 32 threads, 66 with 128,
+    // 72 with 256)
+    const long long bins = (avg + ranks - 1) / ranks;
+    int vthreads = 32;
+    while (vthreads < 128 && (few ? 1LL : 3LL) * vthreads < bins) vthreads <<= 1;
+    d.vjp_prep_threads = vthreads;
     d.prep_ranks = ranks;
     d.prep_threads = threads;
     return cudaSuccess;

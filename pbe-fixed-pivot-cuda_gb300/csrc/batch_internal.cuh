@@ -48,8 +48,8 @@ struct BatchDev {
     // Bk); plans of few cells take it, so that one large cell's prep does not
     // hold up the launch, while many cells balance the prep CTAs anyway.
     int brk;
-    // launch shape of the prep kernels: CTAs per cell (a cluster) and threads per CTA
-    int prep_ranks, prep_threads;
+    // launch shapes of the prep kernels: CTAs per cell (a cluster) and threads per CTA (the VJP's)
+    int prep_ranks, prep_threads, vjp_prep_threads;
     long long total;   // packed length of the per-bin arrays
     // per grid bin (packed by BatchGridDev::off)
     double* gx; double* ga; double* gia; double* ginv_dx; double* gBd; double* gSd; int* gLd;

@@ -532,10 +532,7 @@ cudaError_t vjp_k(const BatchDev& d, const BatchVjpDev& vd, const double* N, con
                   double* gN, double* gparams, const pbe_batch_cell_params_t* params,
                   cudaStream_t s)
 {
-    // its two scans pay per thread: fewer threads than the forward's prep (48 cells of
-    // 256..2048 bins, 8 CTAs each: 83 us with 256 threads, 62 with 64)
-    const int vthreads = d.prep_threads > 128 ? d.prep_threads / 4 : 32;
-    cudaError_t e = launch_prep(d, batch_vjp_prep_kernel<K>, vthreads, s, d, vd, N, lam, gN, params);
+    cudaError_t e = launch_prep(d, batch_vjp_prep_kernel<K>, d.vjp_prep_threads, s, d, vd, N, lam, gN, params);
     if (e != cudaSuccess) return e;
     if (d.kernel >= 0) {
         if (vd.n_rbundles > 0)
