@@ -63,6 +63,7 @@ struct pbe_batch_plan {
     int4* d_tasks = nullptr;
     std::vector<int> grid_direct;      // direct lags of a slot (D0), or n on a grid that is not geometric
     std::vector<char> grid_geo;        // grids verified geometric
+    bool vjp_rows = false;             // the VJP of cells on them goes by blocks of rows (vjp_setup)
     int max_lags = 1;                  // most direct lags of a slot over the cells
     std::vector<double> t_q, bw_q;
     double* d_tq = nullptr;
@@ -218,8 +219,8 @@ long long pair_task_cost(int direct, int I) { return std::min(direct, I + SW) + 
 // Bundles for the cells of the classes selected by `want` (all when null),
 // each class with its group size gs[class]; sorted by work, largest first.
 // kTasksPair: the pair kernel's tasks of every cell; kTasksRows: the VJP's blocks
-// of 32 rows of the cells on geometric grids; kTasksTiles: its row tiles of the
-// other cells (their work does not depend on the first row). slot_off: first task
+// of 32 rows of the cells on geometric grids, if the plan takes rows (vjp_setup);
+// kTasksTiles: its row tiles of the other cells (their work does not depend on the first row). slot_off: first task
 // slot of each cell (VJP).
 enum TaskKind { kTasksPair, kTasksRows, kTasksTiles };
 void build_schedule(const pbe_batch_plan& p, const int* gs, const bool* want,
@@ -232,13 +233,13 @@ void build_schedule(const pbe_batch_plan& p, const int* gs, const bool* want,
         const int cls = n_class(n);
         if (want && !want[cls]) continue;
         const int direct = p.grid_direct[p.cell_grid[c]];
-        const bool geo = p.grid_geo[p.cell_grid[c]] != 0;
+        const bool rows = p.vjp_rows && p.grid_geo[p.cell_grid[c]] != 0;
         if (kind == kTasksPair) {
             for (int I = 0; I < n; I += SW) per[cls].push_back({c, I, 0, pair_task_cost(direct, I)});
-        } else if (kind == kTasksRows && geo) {
+        } else if (kind == kTasksRows && rows) {
             for (int I = 0; I < n; I += 32)
                 per[cls].push_back({c, I, slot_off[c] + I / 32, std::min(direct, std::max(n - I, I + 32)) + 8LL});
-        } else if (kind == kTasksTiles && !geo) {
+        } else if (kind == kTasksTiles && !rows) {
             for (int I = 0; I < n; I += W) per[cls].push_back({c, I, slot_off[c] + I / W, vjp_task_cost(n, gs[cls])});
         }
     }
@@ -752,12 +753,34 @@ cudaError_t vjp_setup(pbe_batch_plan* p, cudaStream_t s)
     if (p->vjp_ready) return cudaSuccess;
     BatchVjpDev& vd = p->vd;
     const size_t C = static_cast<size_t>(p->total);
+    // Cells on geometric grids: blocks of 32 rows that meet the lags below D0 twice, or,
+    // as on other grids, tiles of 12 rows that meet all partners once. Rows do less work,
+    // but at worst (rows that keep their exact sums) as much, in fewer tasks, which a plan
+    // of few cells cannot spread. So by the worst case, with pair visits as work: on an SM
+    // alone a task takes 3.2 ns a visit of its rows, a full chip 2.1 (rows) or 3.0 (tiles,
+    // and the worth of 2500 visits a tile for its sums) ns times visits over SMs; the
+    // rows' prep is some 3 us longer. Measured, rows, rows at worst and tiles: 1 cell of
+    // 960 sections at 32 an octave 91, 139 and 65 us; 4 of 300 at 4 an octave 57, 82, 52;
+    // 16 of 480 at 32 94, 113 and 120; 64 of 200 at 32 76, 85 and 107.
+    double row_max = 0.0, row_sum = 0.0, tile_max = 0.0, tile_sum = 0.0;
+    for (int c = 0; c < p->n_cells; ++c) {
+        const int n = p->cell_n[c], g = p->cell_grid[c];
+        if (!p->grid_geo[g]) continue;
+        const double r = 32.0 * n, t = 12.0 * n + 2500.0;
+        row_max = std::max(row_max, r);
+        tile_max = std::max(tile_max, t);
+        row_sum += r * ((n + 31) / 32);
+        tile_sum += t * ((n + W - 1) / W);
+    }
+    p->vjp_rows = std::max(3.2 * row_max, 2.1 * row_sum / p->num_sms) + 3000.0 <
+                  std::max(3.2 * tile_max, 3.0 * tile_sum / p->num_sms);
+    vd.rows = p->vjp_rows ? 1 : 0;
     std::vector<int> slot_off(static_cast<size_t>(p->n_cells) + 1, 0);
     long long tiles = 0, rows = 0;
     int max_lags = 1;
     for (int c = 0; c < p->n_cells; ++c) {
         const int n = p->cell_n[c], g = p->cell_grid[c];
-        const bool by_rows = p->grid_geo[g] != 0;
+        const bool by_rows = p->vjp_rows && p->grid_geo[g] != 0;
         const int cnt = by_rows ? (n + 31) / 32 : (n + W - 1) / W;
         slot_off[c + 1] = slot_off[c] + cnt;
         (by_rows ? rows : tiles) += cnt;

@@ -105,18 +105,19 @@ struct BatchVjpDev {
     double* D;             // lambda slopes per cell bin
     // [n_cells * kVjpMomStride] moments of N (0..4) and of lambda N (5..9); by each
     // CTA r of the cell's prep cluster, at 16 + 18 r: its parts of the moments of
-    // |N|, |lambda N| and u |N| |lambda step| (5 each, VjpWs::mom) and of the
-    // breakage parameter gradients (3)
+    // |N|, |lambda N| and u |N| |lambda step| (5 each, VjpWs::mom; CTA 0's become the
+    // cell's) and of the breakage parameter gradients (3)
     double* mom;
     double* pre;           // [2 * 2 kMomN * total] sums over the bins: VjpWs::mloc's four groups
     double* tpart;         // [2 * slots]: parameter partials per task
     const int* tile_off;   // [n_cells + 1]: first task slot of each cell
-    // row tiles of the cells on grids that are not geometric: bundles {first task,
+    int rows;              // the cells on geometric grids go by blocks of rows (else by tiles)
+    // row tiles of the other cells: bundles {first task,
     // tasks, group size, 0}, tasks {cell, first row, slot, 0}
     const int4* bundles;
     const int4* tasks;
     int n_bundles;
-    // blocks of 32 rows of the cells on geometric grids
+    // blocks of 32 rows
     const int4* rbundles;
     const int4* rtasks;
     int n_rbundles;

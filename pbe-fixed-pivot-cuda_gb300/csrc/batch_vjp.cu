@@ -108,7 +108,7 @@ batch_vjp_prep_kernel(BatchDev d, BatchVjpDev vd, const double* __restrict__ N,
         // by rows: the moments of |N|, |lambda N| and u |N| |lambda step|, parts of this
         // CTA (the sums over the bins give those of N and lambda N); by tiles: the
         // moments of N and lambda N
-        const bool rows = gd.geo != 0;
+        const bool rows = gd.geo != 0 && vd.rows != 0;
         double m[3][kMomN];
 #pragma unroll
         for (int g = 0; g < 3; ++g)
@@ -153,13 +153,13 @@ batch_vjp_prep_kernel(BatchDev d, BatchVjpDev vd, const double* __restrict__ N,
             mine[threadIdx.x] = s;
         }
         cl.sync();                         // D and the parts of the whole cell
-        if (!rows) {
-            if (part.rank == 0 && threadIdx.x < 2 * kMomN) {
-                double s = 0.0;
-                for (int r = 0; r < part.ranks; ++r) s += mom[16 + 18 * r + threadIdx.x];
-                mom[threadIdx.x] = s;
-            }
-        } else {
+        // the CTAs' parts together: by tiles in slots 0.., by rows in CTA 0's own
+        if (part.rank == 0 && threadIdx.x < (rows ? 3 : 2) * kMomN) {
+            double s = 0.0;
+            for (int r = 0; r < part.ranks; ++r) s += mom[16 + 18 * r + threadIdx.x];
+            mom[(rows ? 16 : 0) + threadIdx.x] = s;
+        }
+        if (rows) {
             double* pre = vd.pre + off;
             const double* D = vd.D + off;
             cell_scan<K, false>(x, a, ia,
@@ -256,10 +256,12 @@ __device__ __forceinline__ void row_exact(const VjpCellView& v, int m, int Dm, d
         if constexpr (K == 3 || K == 5) s0 = fma(P * Nk, __ldg(v.Bf + d), s0);
         if constexpr (K == 4 || K == 5) s1 = fma(P * Nk, S, s1);
     };
+#pragma unroll 4
     for (int j = lane; j <= m - Dm; j += 32) {
         const double P = m < n - 1 ? fma(sum_minus_scaled_pre(ma, __ldg(v.x + j), mc), Dk, lm) : lamlast;
         add(j, m - j, P, K >= 4 ? __ldg(v.Sl + m - j) : 0.0);
     }
+#pragma unroll 4
     for (int k = m + Dm + lane; k < n; k += 32) {
         const double xk = __ldg(v.x + k);
         double P = __ldg(v.lam + k);
@@ -324,10 +326,9 @@ batch_vjp_row_kernel(BatchDev d, BatchVjpDev vd, const double* __restrict__ N,
     bool ex = false;
     if (valid && (m >= Dm || m + Dm < n)) {
         const double c0 = fabs(P.beta0), c1 = fabs(P.beta_br), c2 = fabs(P.beta_sh);
-        double S[3] = {0.0, 0.0, 0.0};
-        for (int r = 0; r < d.prep_ranks; ++r)
+        double S[3];
 #pragma unroll
-            for (int q = 0; q < 3; ++q) S[q] += death_factor<K>(xm, am, iam, mom + 16 + 18 * r + 5 * q, c0, c1, c2);
+        for (int q = 0; q < 3; ++q) S[q] = death_factor<K>(xm, am, iam, mom + 16 + 5 * q, c0, c1, c2);
         double err = S[2];
         if (m < n - 1)
             err = fma(1.1102230246251565e-16 * (__ldg(v.x + m + 1) * __ldg(d.ginv_dx + gd.off + m)) *

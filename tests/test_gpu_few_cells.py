@@ -88,3 +88,27 @@ def test_cells_keep_a_populations_foot(kernel, b0, bbr, bsh, cells):
         assert foot.sum() >= 3
         err = np.abs(got - ref)[:, foot] / scale[foot]
         assert err.max() <= 1e-12, (kernel, n, err.max())
+
+
+def test_one_cells_vjp_keeps_up_with_an_irregular_one():
+    """One cell of 960 sections at 128 an octave: by blocks of rows 1.6 times a cell on an
+    irregular grid (row tiles), 0.8 by tiles."""
+    import torch
+
+    us = []
+    for x in (pg.grids.geometric_pow2(960, 1e-21, 128.0), make_grid("generic", 960, np.random.default_rng(960))):
+        N = t(1e12 * np.exp(-0.5 * ((np.arange(960) - 320) / 80.0) ** 2))
+        lam = t(np.random.default_rng(3).standard_normal(960))
+        with pg.BatchPlan([x], [960], [0], 5) as plan:
+            prm = t(pg.batch.cell_params(1, beta_br=6.73e-18, beta_sh=66.67))
+            gN, gp = torch.zeros_like(N), torch.zeros(1, 8, dtype=torch.float64, device=dev())
+            ts = []
+            for r in range(30):
+                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                e0.record()
+                pg.check(plan.rhs_vjp(N, lam, gN, gp, prm))
+                e1.record()
+                e1.synchronize()
+                ts.append(e0.elapsed_time(e1))
+        us.append(float(np.median(ts[5:])))
+    assert us[0] <= 1.2 * us[1], us
