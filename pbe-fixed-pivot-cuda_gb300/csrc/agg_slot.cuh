@@ -231,18 +231,20 @@ __device__ __forceinline__ void slot_pairs_any(const SlotGrid& g, const SlotPass
         const int mid = (kb + k + 1) >> 1;
         if (dbits(xa + __ldg(x + mid)) < hi) kb = mid; else k = mid - 1;
     }
-    for (int j = ja; j < jb; ++j) {
+    for (int j = ja; j < jb && k >= j; ++j) {
         const double xj = __ldg(x + j);
-        while (k >= j && dbits(xj + __ldg(x + k)) >= hi) --k;
+        double v = xj + __ldg(x + k);
+        while (dbits(v) >= hi && --k >= j) v = xj + __ldg(x + k);
         if (k < j) break;
         const RowBeta<K> row(g, j);
-        for (int q = k; q >= j; --q) {
-            const double v = xj + __ldg(x + q);
-            if (dbits(v) < lo) break;
-            if (q == s && j < Js) continue;            // in the prefix sums
-            const double r = slot_rate_any<K, NP>(g, p, row, j, q);
-            R += r;
-            TH = fma(r, scale_pow2(v - xs, St20), TH);
+        for (int q = k; dbits(v) >= lo;) {
+            if (q != s || j >= Js) {                   // (else in the prefix sums)
+                const double r = slot_rate_any<K, NP>(g, p, row, j, q);
+                R += r;
+                TH = fma(r, scale_pow2(v - xs, St20), TH);
+            }
+            if (--q < j) break;
+            v = xj + __ldg(x + q);
         }
     }
 }
