@@ -39,8 +39,8 @@
 //   R += N_k sum_q c_q(x_k) M_q,  TH += N_k (sum_q c_q M_{q+3} + (x_k - x_s) sum_q c_q M_q),
 // M_m = sum over the window of x_j^(m/3) N_j, from two table values (and whole
 // blocks of 64 between them): windows of any length and place without a
-// subtraction, so sums of one sign keep their relative precision. At 512 sections
-// an octave 1189 lags stay pairs and 135 runs cover the other 3690. The rounding of
+// subtraction, so sums of one sign keep their relative precision. At n = 16384 and 512
+// sections an octave 1330 lags stay pairs and 112 runs cover the other 3549. The rounding of
 // fl(x_j + x_k), left out as above, moves bins s and s + 1 by at most u R_win; the
 // finishing warp compares that with what these bins are known to receive and lose
 // (kMomGuard), and slots beyond it sum those lags pair by pair.
@@ -73,9 +73,9 @@ namespace pbe_gb300 {
 constexpr int kLaneWarps = kMainThreads / 32;       // warps sharing a task's lags
 // Shares of a block's pairs (`lags`: pairs of a slot). Long shares: enough tasks
 // to give every CTA four, so that the last ones end together. A task costs a few
-// microseconds beside its pairs (fetch, staging, sums, ticket), so where that would
-// leave a share less than 192 pairs a slot, as many shares as fit the CTAs in one
-// round (n = 3840, 456 CTAs: 8 shares in two rounds 57 us, 3 shares in one 42). At
+// microseconds beside its pairs (fetch, sums, ticket), so where that would leave a share
+// less than 192 pairs a slot, as many shares as fit the CTAs in one round (608 CTAs, the
+// whole call: n = 3840 8 shares in two rounds 70 us, 4 in one 65; n = 8191 98 and 88). At
 // least 32 pairs a share (4 per warp).
 __host__ __device__ constexpr int lane_parts(int lags, int nblk, int ctas)
 {

@@ -552,7 +552,7 @@ cudaError_t create(pbe_batch_plan* p, int n_grids, const int* grid_n, const doub
     if (e != cudaSuccess) return e;
     d.cells = dcells;
     // zero the stage arrays once: entries a kernel type never writes stay
-    // finite for the loads that the tile body issues unconditionally
+    // (entries that no call has written yet read as zero)
     for (double* a : {d.Y, d.Nj, d.Hj, d.Hk, d.SN, d.Bk, d.k, d.kacc})
         if (e == cudaSuccess) e = cudaMemsetAsync(a, 0, C * sizeof(double), s);
     if (e == cudaSuccess)

@@ -26,10 +26,10 @@
 namespace pbe_gb300 {
 namespace {
 
-// prep modes: kBrkFull computes everything per call; kBrkTables only the
-// grid-only tables (fragment brackets lo, run starts, S per bin) into the
-// workspace; kBrkStage the N-dependent shares from those tables, with the
-// arithmetic of kBrkFull (brk_stage_block).
+// What a call does: kBrkFull everything (one pass, or by PBE_GB300_BRK_PATH=prep the
+// tables, the shares and the gather in turn); kBrkTables only the grid-only tables
+// (fragment brackets lo, run starts, S per bin) into the workspace; kBrkStage the
+// N-dependent shares from those tables (brk_stage_block) and the gather.
 enum { kBrkFull = 0, kBrkTables = 1, kBrkStage = 2 };
 
 template <int F, int MODE>

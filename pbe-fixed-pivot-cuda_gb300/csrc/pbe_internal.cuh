@@ -336,11 +336,11 @@ __host__ __device__ constexpr int agg_prep_blocks(int n) { return (n + kPrepThre
 
 constexpr size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
-// Lane-block pair tasks (agg_lane.cuh): blocks of kLaneBins output bins
-// aligned to the top of the grid, cut into lag chunks of lane_chunk_len(n)
-// lags (at least n / 16 by default, so at most 17 chunks per block). Task (block t,
-// chunk c) has the index sum_{c' < c} lane_chunk_blocks(c') + t; its chunk
-// partial (R, TH of 32 slots) is stored under that index.
+// Blocks of kLaneBins bins cut into lag chunks of lane_chunk_len(n) lags. The VJP's lane
+// kernel uses the blocks and its own chunks (vjp_lane_chunk). The forward's chunks, and the
+// orders by length (lane_last_rank, vjp_lane_last_rank), belong to no kernel any more: the
+// forward cuts by shares (lane_parts) and the VJP runs chunk by chunk. The host test of
+// those tables still compiles them.
 constexpr int kLaneBins = 32;
 #ifndef PBE_LANE_MIN_CHUNK
 #define PBE_LANE_MIN_CHUNK 256
@@ -354,8 +354,7 @@ __host__ __device__ constexpr int lane_block_smax(int n, int t)
     return (n - kLaneBins * t - 1) < n - 2 ? (n - kLaneBins * t - 1) : n - 2;
 }
 // Lag chunk length: at least n / PBE_LANE_CHUNK_DIV (16), a multiple of 64, at
-// least kLaneMinChunk. At n = 3840 the chunk lengths 128 to 512 measured
-// within 2 % of each other; at n = 16384, 576 to 1408 within 1 %.
+// least kLaneMinChunk.
 #ifndef PBE_LANE_CHUNK_DIV
 #define PBE_LANE_CHUNK_DIV 16
 #endif
@@ -383,11 +382,9 @@ __host__ __device__ constexpr long long lane_tasks(int n, int C)
     for (int c = 0; lane_chunk_blocks(n, c, C) > 0; ++c) s += lane_chunk_blocks(n, c, C);
     return s;
 }
-// Launch order of the lane tasks (largest first, so the last wave is filled
-// with the shortest tasks): first every chunk that is not its block's last
-// (all C lags long), chunk by chunk; then each block's last chunk, longest
-// first (ties: lower block first). Entry k of the order is lane_task_at(k).
-// Full chunks: chunk c of the blocks that also have chunk c + 1.
+// An order of those tasks, largest first: every chunk that is not its block's last (all C
+// lags long), chunk by chunk; then each block's last chunk, longest first (ties: lower
+// block first). Full chunks: chunk c of the blocks that also have chunk c + 1.
 __host__ __device__ constexpr int lane_full_tasks(int n, int C)
 {
     int s = 0;
@@ -568,9 +565,8 @@ __host__ __device__ constexpr long long vjp_lane_tasks(int n, int C)
     for (int c = 0; vjp_lane_chunk_blocks(n, c, C) > 0; ++c) s += vjp_lane_chunk_blocks(n, c, C);
     return s;
 }
-// Launch order (largest first, as the forward's lane tasks): every chunk that is
-// not its row block's last, chunk by chunk, then each block's last chunk,
-// longest first (ties: lower block first).
+// The same order of the VJP's tasks (the kernel runs them chunk by chunk instead, so that
+// it need not know the last one below D0 beforehand).
 __host__ __device__ constexpr int vjp_lane_full_tasks(int n, int C)
 {
     int s = 0;

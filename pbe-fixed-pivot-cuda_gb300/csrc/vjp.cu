@@ -732,9 +732,9 @@ __device__ __forceinline__ void bin_sums(const VjpWs& ws, const double* __restri
 }
 
 // Rows of the lane path: one CTA per row block b (rows 32 b + lane). Warp g
-// adds the larger-member sums of the row blocks b' = g, g + 32, ... <= b (the
+// adds the larger-member sums of the row blocks b' = g, g + 16, ... <= b (the
 // chunk holding lag d = m - 32 b' and, for the first 32 lags of a chunk, the
-// tail of the chunk before); warp 0 adds the 32 in order, the block's own
+// tail of the chunk before); warp 0 adds the 16 warps' in order, the block's own
 // smaller-member sums chunk by chunk, the diagonal pair, the lags from D0 on,
 // the death moments, and stores dL/dN_m and the block's parameter partials.
 //
