@@ -250,8 +250,8 @@ __device__ __forceinline__ void slot_pairs_any(const SlotGrid& g, const SlotPass
 }
 
 // Thread tid of nt's share of the prefix part of slot s, pair by pair: for the
-// slots of mom_exact_slot.
-template <int K, int NP>
+// slots of mom_exact_slot. U: pairs in flight.
+template <int K, int NP, int U = 1>
 __device__ __forceinline__ void slot_exact_part(const SlotGrid& g, const SlotPass* p, int s, int tid,
                                                 int nt, double& r, double& t)
 {
@@ -262,8 +262,7 @@ __device__ __forceinline__ void slot_exact_part(const SlotGrid& g, const SlotPas
     const int cut = slot_cut(g, s);
     r = 0.0;
     t = 0.0;
-    constexpr int kU = NP == 1 ? 2 : 1;                // (two of the two-pass sums spill)
-#pragma unroll kU
+#pragma unroll U
     for (int j = tid; j < cut; j += nt) {
         double rate, th;
         if (g.geo) {
@@ -285,12 +284,12 @@ __device__ __forceinline__ void slot_exact_part(const SlotGrid& g, const SlotPas
 }
 
 // The same by one warp, summed by a fixed butterfly. Valid in every lane.
-template <int K, int NP>
+template <int K, int NP, int U>
 __device__ __forceinline__ void slot_exact(const SlotGrid& g, const SlotPass* p, int s, double& R,
                                            double& TH)
 {
     double r, t;
-    slot_exact_part<K, NP>(g, p, s, threadIdx.x & 31, 32, r, t);
+    slot_exact_part<K, NP, U>(g, p, s, threadIdx.x & 31, 32, r, t);
     R = warp_sum(r);
     TH = warp_sum(t);
 }
@@ -298,7 +297,7 @@ __device__ __forceinline__ void slot_exact(const SlotGrid& g, const SlotPass* p,
 // Warp w of nw's turns of those among the 32 slots s = I - 1 + lane (I the first bin) that
 // keep their exact pair sums (spread over the warps), added to R, TH. Returns the mask of
 // those slots; the prefix part of the others is left to the caller.
-template <int K, int NP>
+template <int K, int NP, int U = 1>
 __device__ __forceinline__ unsigned slot_exact_turns(const SlotGrid& g, const SlotPass* p, int I, int w, int nw,
                                                      double& R, double& TH)
 {
@@ -320,7 +319,7 @@ __device__ __forceinline__ unsigned slot_exact_turns(const SlotGrid& g, const Sl
         const int le = __ffs(m) - 1;
         if (turn == w) {
             double r, t;
-            slot_exact<K, NP>(g, p, I - 1 + le, r, t);
+            slot_exact<K, NP, U>(g, p, I - 1 + le, r, t);
             if (l == le) { R += r; TH += t; }
         }
         turn = turn + 1 == nw ? 0 : turn + 1;

@@ -641,7 +641,6 @@ agg_small_kernel(const double* __restrict__ N, const double* __restrict__ x, dou
     __shared__ double red[kLaneWarps][2][32];
     __shared__ double csum[kLaneWarps];
     __shared__ double cpart[kSmallMaxCtas];            // last CTA: the CTAs' parts of the clipped pairs
-    __shared__ int jt_s[32];                           // end of every slot's rows (slot_pairs_any)
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int r = static_cast<int>(cl.block_rank()), ranks = static_cast<int>(cl.num_blocks());
     const int I = kSmallBins * r;
@@ -694,24 +693,6 @@ agg_small_kernel(const double* __restrict__ N, const double* __restrict__ x, dou
             }
             if (lane == 31) te_s = E;
         }
-    }
-    if (w == 4) {
-        // end of every slot's rows (slot_pairs_any), sought from where a geometric grid through
-        // the end points would have half of x_{s+1}; kept in xlist, which this kernel has no
-        // use for
-        const int s = I - 1 + lane;
-        int jt = 0;
-        if (s >= 0 && s <= n - 2) {
-            if constexpr (KIND == kAggStage) {
-                jt = ws.xlist[s];
-            } else {
-                const float lx0 = log2_approx(__ldg(x)), span = log2_approx(__ldg(x + n - 1)) - lx0;
-                const float gf = (log2_approx(__ldg(x + s + 1)) - 1.0f - lx0) * (static_cast<float>(n - 1) / span);
-                jt = slot_rows_end(x, s, static_cast<int>(fminf(fmaxf(gf, 0.0f), static_cast<float>(s))));
-                if (KIND == kAggTables) ws.xlist[s] = jt;
-            }
-        }
-        jt_s[lane] = jt;
     }
     if constexpr (KIND != kAggStage) {
         if (w == 1) {
@@ -811,8 +792,18 @@ agg_small_kernel(const double* __restrict__ N, const double* __restrict__ x, dou
     const int s = I - 1 + lane;                        // this lane's slot and bin
     const bool slot = s >= 0 && s <= n - 2;
     double R = 0.0, TH = 0.0;
-    if (g.geo) slot_lags<K, 1>(g, &p, I, w, kLaneWarps, R, TH);
-    else slot_pairs_any<K, 1>(g, &p, s, slot, jt_s[lane], w, kLaneWarps, R, TH);
+    if (g.geo) {
+        slot_lags<K, 1>(g, &p, I, w, kLaneWarps, R, TH);
+    } else {
+        // the rows' end sought from where a geometric grid through the end points would have it
+        int jt = 0;
+        if (slot) {
+            const float lx0 = log2_approx(__ldg(x)), span = log2_approx(__ldg(x + n - 1)) - lx0;
+            const float gf = (log2_approx(__ldg(x + s + 1)) - 1.0f - lx0) * (static_cast<float>(n - 1) / span);
+            jt = slot_rows_end(x, s, static_cast<int>(fminf(fmaxf(gf, 0.0f), static_cast<float>(s))));
+        }
+        slot_pairs_any<K, 1>(g, &p, s, slot, jt, w, kLaneWarps, R, TH);
+    }
     const unsigned exact = slot_exact_turns<K, 1>(g, &p, I, w, kLaneWarps, R, TH);
     red[w][0][lane] = R;
     red[w][1][lane] = TH;

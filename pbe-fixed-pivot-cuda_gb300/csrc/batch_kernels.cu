@@ -23,6 +23,8 @@
 // RK4 of plans of small cells: batch_cells_rk4_kernel, a CTA per cell that runs the
 // bodies of both for all stages of its steps.
 // =============================================================================
+#include <type_traits>
+
 #include "batch_internal.cuh"
 #include "agg_slot.cuh"
 #include "batch_scan.cuh"
@@ -523,7 +525,10 @@ __device__ void batch_task(const BatchDev& d, const double* __restrict__ Yg,
     if (agg) {
         if (g.geo) slot_lags<K, NP>(g, p, I, w, nw, R, TH);
         else slot_pairs_any<K, NP>(g, p, s, slot, slot ? __ldg(d.gJt + gd.off + s) : 0, w, nw, R, TH);
-        exact = slot_exact_turns<K, NP>(g, p, I, w, nw, R, TH);
+        // (two pairs of an exact slot in flight: an RHS of one cell of 3840 with every other
+        // section empty 210 us, 180 so; not with two passes or 72 registers, where they spill)
+        constexpr int kU = NP == 1 && !std::is_same<Group, WarpGroup>::value ? 2 : 1;
+        exact = slot_exact_turns<K, NP, kU>(g, p, I, w, nw, R, TH);
     }
     const bool brk = d.nq > 0;
     const bool brk_tasks = (d.brk & kBrkTasks) != 0;
