@@ -914,7 +914,7 @@ cudaError_t launch_small(const AggArgs& a, const AggWs& ws, cudaStream_t s, int 
                                      s, static_cast<unsigned>(ranks), a.N, a.x, a.rhs, ws, a.n, a.beta0,
                                      a.beta_br, a.beta_sh);
     if (prof) cudaEventRecord(g_prof_stop, s);
-    return e != cudaSuccess ? e : cudaGetLastError();
+    return launch_result(e);
 }
 
 // Tasks that sum the clipped pairs (about n + 1.2 q^2 pairs on a grid with q bins

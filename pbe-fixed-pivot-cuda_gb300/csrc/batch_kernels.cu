@@ -677,7 +677,7 @@ cudaError_t batch_cells_rk4(const BatchDev& d, double* N, const pbe_batch_cell_p
         for (int st = 0; st < n_steps && e == cudaSuccess; st += kCellSteps)   // launches of milliseconds
             e = launch_dep(kern, dim3(d.n_cells), 32 * warps, 0, s, 1, d, N, params, dt,
                            n_steps - st < kCellSteps ? n_steps - st : kCellSteps);
-        return e;
+        return launch_result(e);
     };
     switch (d.kernel < 0 ? 0 : d.kernel) {
     case 0: return run(batch_cells_rk4_kernel<0>);

@@ -200,8 +200,8 @@ template <class... P, class... A>
 cudaError_t launch_prep(const BatchDev& d, void (*kern)(P...), int threads, cudaStream_t s, A... args)
 {
     const unsigned ranks = static_cast<unsigned>(d.prep_ranks);
-    return launch_dep(kern, dim3(static_cast<unsigned>(d.n_cells) * ranks), static_cast<unsigned>(threads), 0, s,
-                      ranks, args...);
+    return launch_result(launch_dep(kern, dim3(static_cast<unsigned>(d.n_cells) * ranks),
+                                    static_cast<unsigned>(threads), 0, s, ranks, args...));
 }
 
 } // namespace pbe_gb300

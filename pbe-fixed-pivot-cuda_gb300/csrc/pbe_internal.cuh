@@ -758,4 +758,12 @@ inline cudaError_t launch_dep(void (*kern)(P...), dim3 grid, unsigned threads, s
     return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
+// For callers that return a launch's result: a failed launch also stays pending in the
+// runtime, where the next call would find it and take it for its own.
+inline cudaError_t launch_result(cudaError_t e)
+{
+    const cudaError_t pending = cudaGetLastError();
+    return e != cudaSuccess ? e : pending;
+}
+
 } // namespace pbe_gb300
