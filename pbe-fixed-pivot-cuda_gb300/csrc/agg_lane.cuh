@@ -103,6 +103,7 @@ struct LaneArgs {
     int parts;           // tasks per block
     int Dm;              // lags summed pair by pair (geometric grids)
     int eh, el;          // runs eh .. el (descending) summed by windows; eh < el: none
+    int flip;            // rates_flip
 };
 
 // The call as its tasks see it: the grid with the lag tables, the one pass
@@ -317,7 +318,7 @@ __device__ void lane_finish(const LaneView& v, const AggWs& ws, const LaneArgs& 
             const double on = __shfl_down_sync(0xffffffffu, own, 1);
             if (finish && slot && u.Rw != 0.0) {
                 const double xu = __ldg(v.g.x + s + 1);
-                const int fl = rates_flip<K>(v.g.b0, v.g.bbr, v.g.bsh);
+                const int fl = la.flip;
                 const double err = (xu * v.g.inv_dx[s]) * flip_sign(u.Rw, fl);   // 2^53 times the error
                 constexpr double kGuard = kMomGuard * 9007199254740992.0;
                 double dup = fmax(flip_sign(dn, fl), 0.0);

@@ -534,7 +534,7 @@ template <int K, bool SCATTER>
 __global__ void __launch_bounds__(kMainThreads, kLaneCtas)
 agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
                 double* __restrict__ rhs, AggWs ws, int n, int nclip, double b0, double bbr,
-                double bsh)
+                double bsh, int flip)
 {
     const int dep = dep_wait();
     N += dep; x += dep; rhs += dep; n += dep;
@@ -551,7 +551,7 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
     const int nblk = slot_blocks(n);
     // direct pairs of a slot: its lags below D0; on other grids at most its rows
     int Dm = min(v.g.D0, n), eh = 0, el = 1;
-    if (!SCATTER && v.g.geo && ws.mom[7] == 0.0 && rates_one_sign<K>(bbr, bsh) && win_grid(x, n)) {
+    if (!SCATTER && v.g.geo && ws.mom[7] == 0.0 && flip != kRatesMixed && win_grid(x, n)) {
         eh = ws.counter[8];
         el = max(1, ws.counter[9]);
         if (eh >= el) Dm = ws.counter[10];
@@ -560,7 +560,7 @@ agg_lane_kernel(const double* __restrict__ N, const double* __restrict__ x,
     const int parts = lane_parts(v.g.geo ? Dm + 5 * max(0, eh - el + 1) : n, nblk, gridDim.x);
     const int nexact = ws.counter[5];
     const int ntasks = nclip + nexact + nblk * parts;
-    const LaneArgs la{ws.lpart, ws.cticket, parts, Dm, eh, el};
+    const LaneArgs la{ws.lpart, ws.cticket, parts, Dm, eh, el, flip};
     for (int next = blockIdx.x;;) {                      // the first task by the CTA's own index
         int task = next;
         if (task >= ntasks) break;
@@ -973,7 +973,7 @@ cudaError_t launch_k(const AggArgs& a, const AggWs& ws, int num_sms, cudaStream_
     const bool prof = g_prof_start && g_prof_stop;
     if (prof) cudaEventRecord(g_prof_start, s);
     launch_dep(kern, dim3(grid), kMainThreads, 0, s, 1, a.N, a.x, a.rhs, ws, n, nclip, a.beta0, a.beta_br,
-               a.beta_sh);
+               a.beta_sh, rates_flip(a.kernel, a.beta0, a.beta_br, a.beta_sh));
     if (prof) cudaEventRecord(g_prof_stop, s);
     return cudaGetLastError();
 }
